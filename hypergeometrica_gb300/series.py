@@ -21,7 +21,7 @@ device-resident multiply service; R is one batched signed sum
 P, Q, B and R of every node stay in device memory, one arena per height,
 until the parent has combined them.  For a series given by polynomials the
 tree stops at nodes of at most 2^NODE_HEIGHT terms, each computed whole by
-one device thread (hg_series_nodes_device); a range's partial is the same
+one warp (hg_series_nodes_device); a range's partial is the same
 integers however the range is split.  Because the tree is the reference's,
 every partial it holds, not just the root, equals the reference's.
 """
@@ -197,8 +197,11 @@ def trim_sizes(vecs) -> np.ndarray:
 SMALL_MAX_LIMBS = 64  # HG_SMALL_MAX_LIMBS
 # Tree nodes of height <= NODE_HEIGHT (at most 2^NODE_HEIGHT terms) whose
 # parent is higher are computed whole on the device (hg_series_nodes_device)
-# instead of level by level.
-NODE_HEIGHT = 6
+# instead of level by level.  A level more costs its products' and sums' host
+# round trips, a node height more about doubles the node kernel: 89,034
+# Chudnovsky terms take 17.7, 15.6, 13.4 and 12.5 ms at heights 5 to 8,
+# 1,424,505 take 108, 88, 73 and 68, 2,000 take 5.4, 4.3, 3.7 and 4.4.
+NODE_HEIGHT = 7
 
 
 def _multiply_records(rec: np.ndarray, service) -> None:

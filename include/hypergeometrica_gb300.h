@@ -323,7 +323,7 @@ int hg_series_leaves_device(const hg_poly *polys, uint64_t lower, uint64_t count
 
 /* binary-split (src/binary-splitting.lisp:112-133) of whole nodes: the
  * partial P, Q, B, R over terms [ranges[2 i], ranges[2 i + 1]) for each of
- * the n nodes, one device thread per node folding its terms left to right
+ * the n nodes, one warp per node folding its terms left to right
  * (a range's partial is the same integers however the range is split).
  * Value j of node i goes to limbs[(j n + i) width ..] (magnitude) and
  * sign_size[(j n + i) 2] = sign (+1 for zero), [.. + 1] = length without

@@ -283,3 +283,37 @@ def test_small_schoolbook_batch(hg):
     for k, ((o, nout), v) in enumerate(zip(outs, want)):
         got = o.cpu().numpy().view(np.uint64)[:nout]
         assert _as_int(got) == v, k
+
+
+# Series that take the node kernel to its edges: values of one to four limbs
+# (their products q b and p b inside and past 256 bits), zero terms and
+# partials, sums that cancel.
+NODE_SERIES = {
+    "alternating": (((3, -2), None), ((1,), None), ((-1,), None), ((1,), None)),
+    "zero in p and a": (((-9, 1), None), ((2, 1), None), ((-20, 1), None), ((5, 3), 1)),
+    "four limbs": (((1,), None), ((1, 0, 0, 0, 7), None), ((-(1 << 62), 0, 0, 0, 0, 0, 0, -9), None),
+                   ((1, 1 << 61, 0, 0, 0, 0, 0, 11), 1)),
+    "all ones": ((((1 << 63) - 1,), None), (((1 << 63) - 1,), None), ((-(1 << 63) + 1,), None), (((1 << 63) - 1,), None)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(NODE_SERIES))
+def test_device_nodes_edges(hg, name):
+    """Nodes of 1 .. 130 terms (eight are evaluated at once, a warp takes 32
+    limbs at once): the node kernel's partials equal the recursion's."""
+    from hypergeometrica_gb300 import series as S
+
+    ser = S._poly_series(*NODE_SERIES[name])
+    base = 1 << 20 if name == "four limbs" else 0
+    lo = np.array([0, 0, 0, 3, 2, 0, 17, 0, 1], dtype=np.int64) + base
+    hi = np.array([1, 8, 9, 19, 34, 64, 82, 128, 131], dtype=np.int64) + base
+    upper = int(hi.max())
+    assert S._device_leaves_fit(ser, upper)
+    limbs, ss, width = S._device_nodes(ser, lo, hi, upper)
+    host = limbs.cpu().numpy().view(np.uint64).reshape(4, lo.size, width)
+    for i in range(lo.size):
+        want = O.binary_split((ser.a, ser.b, ser.p, ser.q), int(lo[i]), int(hi[i]))
+        for j, v in enumerate(want):
+            size = (abs(v).bit_length() + 63) // 64
+            assert tuple(ss[j, i]) == (-1 if v < 0 else 1, size), (i, j)
+            assert _as_int(host[j, i, :size]) == abs(v), (i, j)
