@@ -414,15 +414,80 @@ std::vector<PassPlan> plan_passes(int L) {
   return v;
 }
 
-PassArgs base_args(int L, int nops) {
+// ---- truncated transforms -------------------------------------------------
+//
+// A product of n limbs needs n points.  Where n is at most 7/8 of the power
+// of two above it, the transform keeps 5, 6 or 7 eighths of the 2^L points
+// (hg_ntt_strided.cu): the passes inside the outer one, the middle and the
+// workspace shrink by that factor.  The outer pass cuts by its top row bits,
+// so it needs 16, 128 or 256 rows (64 for 6/8).
+uint64_t kept_points(int L, int kh) { return kh == 8 ? uint64_t(1) << L : (uint64_t(1) << (L - 3)) * kh; }
+
+struct TransformPlan {
+  int L = 0;
+  int kh = 8;  // eighths kept
+  std::vector<PassPlan> passes;
+  uint64_t points() const { return kept_points(L, kh); }
+};
+
+// Passes of a 2^L-point transform that keeps kh eighths: the outer pass has
+// 16 rows where the other bits still fit the same number of passes (the
+// smaller the outer pass, the more of the work is cut), else the plan of the
+// whole transform, else 128 rows (2^17 and 2^18 points).
+std::vector<PassPlan> plan_kept(int L, int kh) {
+  std::vector<PassPlan> v = plan_passes(L);
+  if (kh == 8) return v;
+  const int rem = L - v.back().logT;
+  const int k = static_cast<int>(v.size()) - 1;
+  std::vector<int> parts;
+  if (k >= 2 && rem - 4 >= 4 * (k - 1) && rem - 4 <= 8 * (k - 1)) {
+    parts.push_back(4);
+    for (int i = 0; i < k - 1; ++i) parts.push_back((rem - 4) / (k - 1) + (i < (rem - 4) % (k - 1) ? 1 : 0));
+  } else if (!truncation_ok(v[0].logR, kh)) {
+    parts.push_back(7);
+  } else {
+    return v;
+  }
+  v.clear();
+  int logS = L;
+  for (int part : parts) {
+    logS -= part;
+    v.push_back({part, logS, kTileBits});
+  }
+  v.push_back({logS, 0, logS});
+  return v;
+}
+
+// Eighths of 2^L points that a product of `size` limbs keeps (2^(L-1) < size
+// <= 2^L): transforms of one contiguous pass (L <= 12) are whole, and so is
+// every one with chunking off (hg_set_chunking).
+std::atomic<int> g_chunking{1};  // hg_set_chunking
+int plan_eighths(int L, uint64_t size, bool whole = false) {
+  if (whole || L <= kTileBits || !g_chunking.load()) return 8;
+  const uint64_t eighth = uint64_t(1) << (L - 3);
+  const uint64_t kh = (size + eighth - 1) / eighth;
+  return kh < 5 ? 5 : static_cast<int>(kh);
+}
+
+TransformPlan plan_transform(int L, uint64_t size, bool whole = false) {
+  TransformPlan t;
+  t.L = L;
+  t.kh = plan_eighths(L, size, whole);
+  t.passes = plan_kept(L, t.kh);
+  return t;
+}
+
+// Arguments of the passes over arrays of `points` residues (2^L unless truncated).
+PassArgs base_args(int L, int nops, uint64_t points = 0) {
   PassArgs a{};
   a.nops = nops;
   a.logN = L;
+  a.points = points ? points : uint64_t(1) << L;
   a.prime_lo = 0;
   a.nprimes = kPrimes;
-  a.prime_stride = uint64_t(1) << L;
+  a.prime_stride = a.points;
   a.nprod = 1;
-  a.ws_stride = static_cast<uint64_t>(kPrimes) << L;
+  a.ws_stride = static_cast<uint64_t>(kPrimes) * a.points;
   for (int i = 0; i < kPrimes; ++i) {
     a.pc[i] = g_ctx.pc[i];
     a.tb[i] = g_ctx.tb[i];
@@ -431,11 +496,31 @@ PassArgs base_args(int L, int nops) {
   return a;
 }
 
+// Shape `a` for the strided pass pp.  The outer pass runs over every column
+// and keeps points / S of its rows; the passes inside run on points / M blocks.
+void set_strided(PassArgs &a, const PassPlan &pp) {
+  const bool outer = pp.logR + pp.logS == a.logN;
+  a.logR = pp.logR;
+  a.logS = pp.logS;
+  a.logT = pp.logT;
+  a.krows = outer ? static_cast<int>(a.points >> pp.logS) : 1 << pp.logR;
+  a.tiles = (outer ? uint64_t(1) << a.logN : a.points) >> pp.logT;
+}
+
+// Shape `a` for the contiguous pass pp.
+void set_contig(PassArgs &a, const PassPlan &pp) {
+  a.logR = pp.logT;
+  a.logS = 0;
+  a.logT = pp.logT;
+  a.krows = 1 << pp.logT;
+  a.tiles = a.points >> pp.logT;
+}
+
 // Algorithmic bytes of a launch over nops operands: every residue written
 // once, every input read once (limbs when a pass reduces them itself).
 double pass_bytes(const PassArgs &a, int readers, int writers) {
   const double words =
-      static_cast<double>(a.nprimes) * static_cast<double>(uint64_t(1) << a.logN) * static_cast<double>(a.nprod);
+      static_cast<double>(a.nprimes) * static_cast<double>(a.points) * static_cast<double>(a.nprod);
   double bytes = 8.0 * words * writers;
   for (int op = 0; op < readers; ++op)
     bytes += a.limbs[op] ? 8.0 * static_cast<double>(a.nlimbs[op]) : 8.0 * words;
@@ -506,10 +591,7 @@ cudaError_t run_strided_range(PassArgs a, const std::vector<PassPlan> &plan, boo
   const int np = static_cast<int>(plan.size()) - 1;
   for (int s = s0; s < s1 && s < np; ++s) {
     const PassPlan &pp = plan[inverse ? np - 1 - s : s];
-    a.logR = pp.logR;
-    a.logS = pp.logS;
-    a.logT = pp.logT;
-    a.tiles = (uint64_t(1) << a.logN) >> pp.logT;
+    set_strided(a, pp);
     const bool last_inverse = inverse && s == np - 1;
     a.ptw = pass_twiddles(pp.logR + pp.logS, pp.logR, inverse, st, last_inverse ? scale_last : nullptr);
     if (last_inverse && scaled) *scaled = scale_last && a.ptw;
@@ -533,10 +615,7 @@ cudaError_t run_strided(const PassArgs &a, const std::vector<PassPlan> &plan, bo
 
 // The contiguous pass (the plan's last entry) in the given mode.
 cudaError_t run_contig(PassArgs a, const PassPlan &pp, int mode, cudaStream_t st) {
-  a.logR = pp.logR;
-  a.logS = 0;
-  a.logT = pp.logT;
-  a.tiles = (uint64_t(1) << a.logN) >> pp.logT;
+  set_contig(a, pp);
   const int readers = mode == kContigMul ? 2 : 1;
   const int cls = mode == kContigFwd ? HG_KC_NTT_FORWARD : (mode == kContigInv ? HG_KC_NTT_INVERSE : HG_KC_MIDDLE);
   ProfScope ps(cls, st, pass_bytes(a, readers, 1));
@@ -643,13 +722,11 @@ constexpr double kChunkGain = 0.95;
 // C = (2^L - ns) rounded down to a multiple of 8 (>= 2^(L-1) because
 // 2^L >= 2 pow2(ns) >= 16), so that at most two chunk products meet at any
 // position of the result.
-std::atomic<int> g_chunking{1};  // hg_set_chunking
-
 bool plan_chunks(uint64_t nl, uint64_t ns, ChunkPlan &cp) {
   if (ns == 0 || nl < ns || !g_chunking.load()) return false;
   const int Lf = ilog2_ceil(nl + ns);
   const auto cost = [](double transforms, int L) { return transforms * std::ldexp(L + kPassCost, L); };
-  double best = kChunkGain * cost(3.0, Lf);
+  double best = kChunkGain * cost(3.0, Lf) / 8 * plan_eighths(Lf, nl + ns);
   bool found = false;
   const int Lmin = std::max(4, ilog2_ceil(ns) + 1);
   for (int L = Lmin; L < Lf && L <= Lmin + 4; ++L) {
@@ -807,7 +884,8 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
   const int L = ilog2_ceil(size);
   int rc = check_len(L);
   if (rc) return rc;
-  const uint64_t N = uint64_t(1) << L;
+  const TransformPlan tp = plan_transform(L, size);
+  const uint64_t N = tp.points();
   const size_t words = static_cast<size_t>(kPrimes) * N;
   HG_CUDA(ws_acquire(st), "workspace ordering");
   if (c.lane->A.bytes < words * 8 || (!square && c.lane->B.bytes < words * 8)) {
@@ -817,8 +895,8 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
   }
   // Strided forward passes, the fused middle (last forward pass of both
   // operands + pointwise product + first inverse pass), strided inverse passes.
-  const std::vector<PassPlan> plan = plan_passes(L);
-  PassArgs a = base_args(L, square ? 1 : 2);
+  const std::vector<PassPlan> &plan = tp.passes;
+  PassArgs a = base_args(L, square ? 1 : 2, N);
   a.data[0] = c.lane->A.u64();
   a.data[1] = c.lane->B.u64();
   a.limbs[0] = x;
@@ -833,12 +911,12 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
               "operand upload");
   }
   if (host && plan.size() > 1) {
-    // The first strided pass covers one block of N = R S residues; its tile t
-    // reads columns [t C, (t + 1) C) (C = 4096 / R) of every row.
+    // The first strided pass covers one block of 2^L = R S residues; its tile
+    // t reads columns [t C, (t + 1) C) (C = 4096 / R) of every row.
     const PassPlan &p0 = plan[0];
     const uint64_t S = uint64_t(1) << p0.logS;
     const uint64_t C = uint64_t(1) << (kTileBits - p0.logR);
-    const uint64_t ntiles = N >> kTileBits;
+    const uint64_t ntiles = (uint64_t(1) << L) >> kTileBits;
     const int K = static_cast<int>(std::min<uint64_t>(kUploadSlices, ntiles));
     const int nops = square ? 1 : 2;
     const uint64_t *ptw = pass_twiddles(p0.logR + p0.logS, p0.logR, false, st);
@@ -860,9 +938,7 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
         f.data[0] = op ? c.lane->B.u64() : c.lane->A.u64();
         f.limbs[0] = op ? y : x;
         f.nlimbs[0] = op ? ny : nx;
-        f.logR = p0.logR;
-        f.logS = p0.logS;
-        f.logT = p0.logT;
+        set_strided(f, p0);
         f.tile_lo = t0;
         f.tiles = t1 - t0;
         f.ptw = ptw;
@@ -886,7 +962,7 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
     if (plan.size() > 1) m.limbs[0] = m.limbs[1] = nullptr;
     HG_CUDA(run_contig(m, plan.back(), square ? kContigSqr : kContigMul, st), "middle pass");
   }
-  PassArgs inv = base_args(L, 1);
+  PassArgs inv = base_args(L, 1, N);
   inv.data[0] = c.lane->A.u64();
   uint64_t sc[kPrimes];
   bool scaled = false;
@@ -899,7 +975,7 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
   uint64_t tiles = 0;
   {
     ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(nproc), 2);  // local scan + fix
-    HG_CUDA(launch_crt_carry(c.lane->A.u64(), L, crt_const(L, scaled), out, nout, ss, st, &tiles),
+    HG_CUDA(launch_crt_carry(c.lane->A.u64(), N, crt_const(L, scaled), out, nout, ss, st, &tiles),
             "reconstruction");
   }
   HG_CUDA(ws_release(st), "workspace ordering");
@@ -969,25 +1045,16 @@ int noalloc_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, ui
   a.nlimbs[1] = square ? 0 : ny;
   if (L > kTileBits) {
     PassArgs f = a;
-    f.logR = 4;
-    f.logS = logC;
-    f.logT = kTileBits;
-    f.tiles = N >> kTileBits;
+    set_strided(f, {4, logC, kTileBits});
     HG_CUDA(launch_ntt_strided(f, false, st), "forward transform");
     a.limbs[0] = a.limbs[1] = nullptr;
   }
-  a.logR = logC;
-  a.logS = 0;
-  a.logT = logC;
-  a.tiles = N >> logC;
+  set_contig(a, {logC, 0, logC});
   HG_CUDA(launch_ntt_contig(a, square ? kContigSqr : kContigMul, st), "middle pass");
   if (L > kTileBits) {
     PassArgs inv = base_args(L, 1);
     inv.data[0] = scratch;
-    inv.logR = 4;
-    inv.logS = logC;
-    inv.logT = kTileBits;
-    inv.tiles = N >> kTileBits;
+    set_strided(inv, {4, logC, kTileBits});
     HG_CUDA(launch_ntt_strided(inv, true, st), "inverse transform");
   }
   if (nout > N) HG_CUDA(cudaMemsetAsync(out + N, 0, (nout - N) * sizeof(uint64_t), st), "zero tail");
@@ -1004,7 +1071,7 @@ int noalloc_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, ui
   ss.epoch = 1;
   ss.err = err_word();
   uint64_t used = 0;
-  HG_CUDA(launch_crt_carry(scratch, L, crt_const(L), out, nout, ss, st, &used), "reconstruction");
+  HG_CUDA(launch_crt_carry(scratch, N, crt_const(L), out, nout, ss, st, &used), "reconstruction");
   return HG_OK;
 }
 
@@ -1299,9 +1366,10 @@ int spectrum(uint64_t *a, size_t n, int mod_num, bool inverse, cudaStream_t st) 
 // Products of one transform length (and kind) run by one launch per pass.
 // Candidate pass splits of a 2^L transform: the default plan and, for
 // L >= 12, every contiguous block size T with the remaining L - T bits in
-// as few strided passes of 4..8 bits as possible.
-std::vector<std::vector<PassPlan>> plan_candidates(int L) {
-  std::vector<std::vector<PassPlan>> out{plan_passes(L)};
+// as few strided passes of 4..8 bits as possible (where the outer one can
+// keep kh eighths of its rows).
+std::vector<std::vector<PassPlan>> plan_candidates(int L, int kh) {
+  std::vector<std::vector<PassPlan>> out{plan_kept(L, kh)};
   if (L < kTileBits) return out;
   for (int T = 4; T <= kTileBits; ++T) {
     const int rem = L - T;
@@ -1318,6 +1386,7 @@ std::vector<std::vector<PassPlan>> plan_candidates(int L) {
     // A strided pass over R rows needs columns of at least 2^(12 - logR)
     // words so that its 4096-word tile spans whole rows.
     if (logS + v.back().logR < kTileBits) continue;
+    if (!truncation_ok(v[0].logR, kh)) continue;
     v.push_back({logS, 0, logS});
     bool same = v.size() == out[0].size();
     for (size_t i = 0; same && i < v.size(); ++i)
@@ -1327,9 +1396,9 @@ std::vector<std::vector<PassPlan>> plan_candidates(int L) {
   return out;
 }
 
-// Schedules chosen by timing, keyed by (L, square, products in the group).
+// Schedules chosen by timing, keyed by (L, eighths kept, square, products in the group).
 std::mutex g_tune_mu;
-std::map<std::tuple<int, bool, uint64_t>, std::vector<PassPlan>> g_tuned;
+std::map<std::tuple<int, int, bool, uint64_t>, std::vector<PassPlan>> g_tuned;
 
 }  // namespace
 }  // namespace hg
@@ -1353,12 +1422,12 @@ namespace {
 int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::vector<PassPlan> &plan,
               cudaStream_t st) {
   const int nops = g.square ? 1 : 2;
-  const uint64_t N = uint64_t(1) << g.L;
+  const uint64_t N = kept_points(g.L, g.kh);
   const uint64_t slab = static_cast<uint64_t>(kPrimes) * N;
   const ProductDesc *d = bb.desc + g.first;
   uint64_t *ws = bb.ws;
   if (g.tails) HG_CUDA(launch_zero_tails(d, g.nprod, N, st), "zero tails");
-  PassArgs a = base_args(g.L, nops);
+  PassArgs a = base_args(g.L, nops, N);
   a.err = bb.err;
   a.batch = d;
   a.read_limbs = 1;
@@ -1370,7 +1439,7 @@ int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::ve
   PassArgs m = a;
   if (plan.size() > 1) m.read_limbs = 0;
   HG_CUDA(run_contig(m, plan.back(), g.square ? kContigSqr : kContigMul, st), "middle pass");
-  PassArgs inv = base_args(g.L, 1);
+  PassArgs inv = base_args(g.L, 1, N);
   inv.err = bb.err;
   inv.batch = d;
   inv.nprod = g.nprod;
@@ -1387,7 +1456,7 @@ int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::ve
   ss.err = bb.err;
   {
     ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(N) * static_cast<double>(g.nprod), 2);  // tiles + fix
-    HG_CUDA(launch_crt_carry_batch(ws, slab, g.L, crt_const(g.L, scaled), d, g.nprod, ss, st), "reconstruction");
+    HG_CUDA(launch_crt_carry_batch(ws, slab, N, crt_const(g.L, scaled), d, g.nprod, ss, st), "reconstruction");
   }
   return HG_OK;
 }
@@ -1405,14 +1474,44 @@ BatchBufs batch_bufs(hg_batch *b) {
 // one, with the same arguments.
 constexpr uint64_t kPersistWorkspaceCap = uint64_t(16) << 30;  // bytes
 
+// The persistent schedule's groups: whole transforms, all products of one
+// length and kind together (they are contiguous in the descriptors).  Its
+// phases run the per-thread-load bodies, whose outer inverse pass is not
+// truncated.
+std::vector<BatchGroup> persist_groups(const BatchPlan &bp) {
+  std::vector<BatchGroup> v;
+  uint64_t tuned = 0;  // products of the part whose tuned plan the group takes
+  std::lock_guard<std::mutex> lk(g_tune_mu);
+  for (const BatchGroup &g : bp.groups) {
+    if (v.empty() || v.back().L != g.L || v.back().square != g.square) {
+      v.push_back(g);
+      v.back().kh = 8;
+      v.back().tails = false;
+      v.back().nprod = 0;
+      v.back().plan = plan_passes(g.L);
+      tuned = 0;
+    }
+    v.back().nprod += g.nprod;
+    const auto it = g_tuned.find(std::make_tuple(g.L, g.kh, g.square, g.nprod));
+    if (it != g_tuned.end() && g.nprod > tuned) {
+      v.back().plan = it->second;
+      tuned = g.nprod;
+    }
+  }
+  for (BatchGroup &g : v)
+    for (uint64_t k = g.first; k < g.first + g.nprod; ++k)
+      if (bp.desc[k].nout > (uint64_t(1) << g.L)) g.tails = true;
+  return v;
+}
+
 struct PersistLayout {
   std::vector<uint64_t> ws_off, flag_off;  // per group, words
   uint64_t ws_words = 0, flag_words = 0;
 };
 
-PersistLayout persist_layout(const BatchPlan &bp) {
+PersistLayout persist_layout(const std::vector<BatchGroup> &groups) {
   PersistLayout l;
-  for (const BatchGroup &g : bp.groups) {
+  for (const BatchGroup &g : groups) {
     const uint64_t N = uint64_t(1) << g.L;
     l.ws_off.push_back(l.ws_words);
     l.flag_off.push_back(l.flag_words);
@@ -1450,10 +1549,7 @@ std::vector<PersistPhase> group_phases(const BatchGroup &g, const BatchBufs &bb,
   a.data[1] = ws + g.nprod * slab;
   for (int s = 0; s < np; ++s) {
     PassArgs f = a;
-    f.logR = plan[s].logR;
-    f.logS = plan[s].logS;
-    f.logT = plan[s].logT;
-    f.tiles = N >> plan[s].logT;
+    set_strided(f, plan[s]);
     f.ptw = pass_twiddles(f.logR + f.logS, f.logR, false, st);
     PersistPhase p = phase(kPhaseStrided, f.logR, f.tiles * g.nprod * static_cast<uint64_t>(nops) * kPrimes);
     p.a = f;
@@ -1463,10 +1559,7 @@ std::vector<PersistPhase> group_phases(const BatchGroup &g, const BatchBufs &bb,
   {
     PassArgs m = a;
     const int T = plan.back().logT;
-    m.logR = T;
-    m.logS = 0;
-    m.logT = T;
-    m.tiles = N >> T;
+    set_contig(m, plan.back());
     const int mode = g.square ? kContigSqr : kContigMul;
     if (T < 4) {
       PersistPhase p = phase(kPhaseTiny, mode, (g.nprod * kPrimes + 255) / 256);
@@ -1493,10 +1586,7 @@ std::vector<PersistPhase> group_phases(const BatchGroup &g, const BatchBufs &bb,
   for (int s = 0; s < np; ++s) {
     const PassPlan &pp = plan[np - 1 - s];
     PassArgs f = inv;
-    f.logR = pp.logR;
-    f.logS = pp.logS;
-    f.logT = pp.logT;
-    f.tiles = N >> pp.logT;
+    set_strided(f, pp);
     const bool last = s == np - 1;  // the last inverse pass: its table prescaled
     f.ptw = pass_twiddles(f.logR + f.logS, f.logR, true, st, last && can_scale ? sc : nullptr);
     if (last) scaled = can_scale && f.ptw;
@@ -1533,7 +1623,8 @@ int persist_build(hg_batch *b) {
   b->items = 0;
   const BatchPlan &bp = b->bp;
   if (bp.groups.empty() || !persist_grid()) return HG_OK;
-  const PersistLayout l = persist_layout(bp);
+  const std::vector<BatchGroup> groups = persist_groups(bp);
+  const PersistLayout l = persist_layout(groups);
   if (l.ws_words * 8 > kPersistWorkspaceCap) return HG_OK;
   if (b->ws.bytes < l.ws_words * 8) HG_CUDA(b->ws.ensure(l.ws_words * 8), "batch workspace");
   if (b->flags.bytes < l.flag_words * 8) HG_CUDA(b->flags.ensure(l.flag_words * 8), "batch scan flags");
@@ -1541,8 +1632,8 @@ int persist_build(hg_batch *b) {
   const BatchBufs bb = batch_bufs(b);
   std::vector<std::vector<PersistPhase>> per;
   std::vector<PersistPhase> indep;  // zeroing: waits for nothing
-  for (size_t gi = 0; gi < bp.groups.size(); ++gi) {
-    const BatchGroup &g = bp.groups[gi];
+  for (size_t gi = 0; gi < groups.size(); ++gi) {
+    const BatchGroup &g = groups[gi];
     per.push_back(group_phases(g, bb, bb.ws + l.ws_off[gi], bb.flags + l.flag_off[gi], g_ctx.lane->stream));
     if (g.tails) {
       PersistPhase z{};
@@ -1625,7 +1716,7 @@ int batch_autotune(hg_batch *b) {
   const BatchBufs bb = batch_bufs(b);
   for (size_t gi = 0; gi < b->bp.groups.size() && rc == HG_OK; ++gi) {
     BatchGroup &g = b->bp.groups[gi];
-    const auto key = std::make_tuple(g.L, g.square, g.nprod);
+    const auto key = std::make_tuple(g.L, g.kh, g.square, g.nprod);
     {
       std::lock_guard<std::mutex> lk(g_tune_mu);
       auto it = g_tuned.find(key);
@@ -1634,7 +1725,7 @@ int batch_autotune(hg_batch *b) {
         continue;
       }
     }
-    const auto cands = plan_candidates(g.L);
+    const auto cands = plan_candidates(g.L, g.kh);
     float best = 1e30f;
     for (const auto &plan : cands) {
       float ms = 0;
@@ -1737,7 +1828,7 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
   } else {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     for (BatchGroup &g : b->bp.groups) {
-      auto it = g_tuned.find(std::make_tuple(g.L, g.square, g.nprod));
+      auto it = g_tuned.find(std::make_tuple(g.L, g.kh, g.square, g.nprod));
       if (it != g_tuned.end()) g.plan = it->second;
     }
   }
@@ -1769,11 +1860,17 @@ uint64_t product_workspace_bytes(uint64_t nx, uint64_t ny, bool square) {
   return static_cast<uint64_t>(square ? 1 : 2) * kPrimes * N * 8;
 }
 
+// Points a batch's cut must save per prime and operand to be a group of its
+// own: about 40 us of a full GPU's work, what a group's chain of launches
+// takes at least.
+constexpr uint64_t kCutPoints = uint64_t(1) << 19;
+
 int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchPlan &bp) {
   bp = BatchPlan();
   struct Item {
     int L;
     bool square;
+    int kh;
     size_t i;
   };
   std::vector<Item> live;
@@ -1786,28 +1883,49 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
       zeros.push_back(i);
       continue;
     }
-    live.push_back({ilog2_ceil(p.nx + p.ny), square, i});
+    const int L = ilog2_ceil(p.nx + p.ny);
+    live.push_back({L, square, plan_eighths(L, p.nx + p.ny), i});
   }
   std::stable_sort(live.begin(), live.end(), [](const Item &a, const Item &c) {
-    return a.L != c.L ? a.L < c.L : a.square < c.square;
+    return a.L != c.L ? a.L < c.L : a.square != c.square ? a.square < c.square : a.kh < c.kh;
   });
-  bp.desc.reserve(n);
+  // Every group is a chain of launches that depend on each other, so a cut
+  // that few products would use is not worth a group of its own: they join
+  // the next larger cut of their length unless it would process at least
+  // kCutPoints points more.
   for (size_t s = 0; s < live.size();) {
     size_t e = s;
     while (e < live.size() && live[e].L == live[s].L && live[e].square == live[s].square) ++e;
+    for (size_t c = s; c < e;) {
+      size_t d = c;
+      while (d < e && live[d].kh == live[c].kh) ++d;
+      if (d < e && (static_cast<uint64_t>(d - c) * (live[d].kh - live[c].kh) << live[c].L) / 8 < kCutPoints)
+        for (size_t k = c; k < d; ++k) live[k].kh = live[d].kh;
+      else
+        c = d;
+    }
+    s = e;
+  }
+  bp.desc.reserve(n);
+  for (size_t s = 0; s < live.size();) {
+    size_t e = s;
+    while (e < live.size() && live[e].L == live[s].L && live[e].square == live[s].square && live[e].kh == live[s].kh)
+      ++e;
     const int L = live[s].L;
     const bool square = live[s].square;
-    const uint64_t N = uint64_t(1) << L;
+    const uint64_t N = kept_points(L, live[s].kh);
     const uint64_t per = static_cast<uint64_t>(square ? 1 : 2) * kPrimes * N * 8;
-    if (per > ws_cap_bytes)
+    const uint64_t whole = (static_cast<uint64_t>(square ? 1 : 2) * kPrimes * 8) << L;
+    if (whole > ws_cap_bytes)
       return fail(HG_ERR_ARG, "a 2^%d-point product needs %llu workspace bytes, more than the %llu available", L,
-                  (unsigned long long)per, (unsigned long long)ws_cap_bytes);
+                  (unsigned long long)whole, (unsigned long long)ws_cap_bytes);
     const uint64_t chunk = std::max<uint64_t>(1, ws_cap_bytes / per);
     for (size_t c = s; c < e; c += chunk) {
       BatchGroup g;
       g.L = L;
       g.square = square;
-      g.plan = plan_passes(L);
+      g.kh = live[s].kh;
+      g.plan = plan_kept(L, g.kh);
       g.first = bp.desc.size();
       g.nprod = std::min<uint64_t>(chunk, e - c);
       g.flags_off = bp.flag_words;

@@ -270,9 +270,8 @@ __global__ void zero_tails_kernel(const ProductDesc *batch, uint64_t N) {
 
 uint64_t carry_tiles(uint64_t n) { return (n + kCarryTile - 1) / kCarryTile; }
 
-cudaError_t launch_crt_carry(const uint64_t *res, int logN, const CrtConst &cc, uint64_t *out, uint64_t nout,
+cudaError_t launch_crt_carry(const uint64_t *res, uint64_t n, const CrtConst &cc, uint64_t *out, uint64_t nout,
                              const ScanState &ss, cudaStream_t st, uint64_t *tiles_used) {
-  const uint64_t n = 1ull << logN;
   const uint64_t nproc = nout < n ? nout : n;
   const uint64_t tiles = carry_tiles(nproc);
   *tiles_used = tiles;
@@ -281,9 +280,8 @@ cudaError_t launch_crt_carry(const uint64_t *res, int logN, const CrtConst &cc, 
   return launch_carry(CrtProducer{res, n, cc}, out, nproc, tiles, ss, st);
 }
 
-cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, int logN, const CrtConst &cc,
+cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint64_t n, const CrtConst &cc,
                                    const ProductDesc *batch, uint64_t nprod, const ScanState &ss, cudaStream_t st) {
-  const uint64_t n = 1ull << logN;
   const uint64_t tpp = carry_tiles(n);
   const uint64_t tiles = tpp * nprod;
   if (tiles == 0) return cudaSuccess;

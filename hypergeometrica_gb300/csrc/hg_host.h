@@ -19,6 +19,7 @@ struct PassPlan {
 // Products of one transform length and kind, run as one launch per pass.
 struct BatchGroup {
   int L = 0;
+  int kh = 8;                      // eighths of the 2^L points that are kept (8: a whole transform)
   bool square = false;
   bool tails = false;              // some product has nout > N
   std::vector<PassPlan> plan;

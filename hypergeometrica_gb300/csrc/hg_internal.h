@@ -86,6 +86,10 @@ struct PassArgs {
   int logR;                    // log2 rows (transform points) of this pass
   int logS;                    // log2 stride; 0 = contiguous pass
   int logT;                    // log2 residues per tile
+  // Residues of each array: 2^logN, or fewer in a truncated transform
+  // (krows rows of the outer pass, see hg_ntt_strided.cu).
+  uint64_t points;
+  int krows;                   // strided passes: rows of a block that are kept (R unless truncated)
   int prime_lo, nprimes;
   uint64_t prime_stride;       // words between the arrays of consecutive primes
   uint64_t nprod;              // products in the launch
@@ -144,6 +148,12 @@ struct ScanState {
   int *err;                    // device error word
 };
 
+// Whether a truncated transform's outer pass of 2^logR rows can keep kh
+// eighths of them (8: all).
+__host__ __device__ __forceinline__ constexpr bool truncation_ok(int logR, int kh) {
+  return kh == 8 || (kh == 6 && logR == 6) || (kh >= 5 && kh <= 7 && (logR == 4 || logR >= 7));
+}
+
 // Kernel launchers.
 // Strided pass (hg_ntt_strided.cu): 4 <= logR <= 8, logT = 12.
 cudaError_t launch_ntt_strided(const PassArgs &a, bool inverse, cudaStream_t st);
@@ -153,11 +163,11 @@ cudaError_t launch_ntt_strided(const PassArgs &a, bool inverse, cudaStream_t st)
 // logR == logT <= 12.
 constexpr int kContigFwd = 0, kContigInv = 1, kContigMul = 2, kContigSqr = 3, kContigMulSpec = 4;
 cudaError_t launch_ntt_contig(const PassArgs &a, int mode, cudaStream_t st);
-cudaError_t launch_crt_carry(const uint64_t *res, int logN, const CrtConst &cc, uint64_t *out, uint64_t nout,
+cudaError_t launch_crt_carry(const uint64_t *res, uint64_t n, const CrtConst &cc, uint64_t *out, uint64_t nout,
                              const ScanState &ss, cudaStream_t st, uint64_t *tiles_used);
-// Reconstruction + carry for nprod products of transform length 2^logN whose
-// residues start ws_stride words apart at res.
-cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, int logN, const CrtConst &cc,
+// Reconstruction + carry for nprod products of n residues per prime that
+// start ws_stride words apart at res.
+cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint64_t n, const CrtConst &cc,
                                    const ProductDesc *batch, uint64_t nprod, const ScanState &ss, cudaStream_t st);
 // Reconstruction + carry of a product computed in chunks: chunk k's
 // residues ([3][2^logN], unscaled inverse) start k * ws_stride words past
@@ -173,7 +183,8 @@ cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, int
 // result = (sign, size).  top is one device word of scratch.
 cudaError_t launch_large_sum(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t *b, uint64_t nb, int64_t sb,
                              uint64_t *out, long long *top, int64_t *result, const ScanState &ss, cudaStream_t st);
-// Zero out[N, nout) of every product (out[0, nout) when N == 0).
+// Zero out[N, nout) of every product (out[0, nout) when N == 0), N the
+// residues per prime.
 cudaError_t launch_zero_tails(const ProductDesc *batch, uint64_t nprod, uint64_t N, cudaStream_t st);
 cudaError_t launch_schoolboy_carry(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64_t ny, uint64_t *out,
                                    uint64_t nout, const ScanState &ss, cudaStream_t st, uint64_t *tiles_used);

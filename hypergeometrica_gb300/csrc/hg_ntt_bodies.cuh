@@ -22,7 +22,9 @@ constexpr int kFwd = 0, kInv = 1, kMul = 2, kSqr = 3, kMulSpec = 4;
 // per-thread global loads and stores; tw holds 2^(LOGR-1) (twiddle,
 // companion) pairs and sm 4096 words of shared memory.  The pass that reads
 // and reduces limbs from batch descriptors or chunks runs here.
-template <int LOGR, bool INV>
+// CUT (forward only): the outer pass of a truncated transform, which keeps
+// P.krows rows.
+template <int LOGR, bool INV, bool CUT = false>
 __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid, ulonglong2 *tw, uint64_t *sm) {
   constexpr int T = kTileBits;
   constexpr int LOGTC = T - LOGR;  // log2 columns per tile
@@ -70,7 +72,10 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
       const uint64_t *t = P.ptw + (static_cast<uint64_t>(prime) << logM) +
                           (static_cast<uint64_t>(rhi) << (4 + logS)) + s;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = mont_mul(v[i], __ldg(t + (static_cast<uint64_t>(i) << logS)), p, c);
+      for (int i = 0; i < 16; ++i) {
+        if (CUT && LOGR == 4 && i >= 10 && i >= P.krows) break;  // rows a truncated transform drops
+        v[i] = mont_mul(v[i], __ldg(t + (static_cast<uint64_t>(i) << logS)), p, c);
+      }
       return;
     }
     uint32_t rrev = 0;
@@ -98,7 +103,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const uint64_t o = off + i * step;
-        v[i] = check_index(o, uint64_t(1) << P.logN) ? data[o] : 0;
+        v[i] = check_index(o, P.points) ? data[o] : 0;
         check_below(v[i], p);
       }
     }
@@ -110,14 +115,19 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
       xt = thread_base<A0>(tid);
       from_smem<A0>(v, sm, xt);
     }
+    // The thread's 16 rows, of which a truncated transform keeps the first
+    // `keep` (the rows of a 16-row group together; 10, 12 or 14 of 16 when R = 16).
+    const int keep = CUT ? P.krows - static_cast<int>((xt >> (ROWOFF + 4)) << 4) : 16;
+    if (CUT && LOGR > 4 && keep <= 0) return;
     stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true>(v, tw, xt, p, c);  // then the inter-pass twiddle
     inter_pass(v, xt, tb.hi_fwd, tb.lo_fwd);
     offsets(xt, A0, off, step);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
+      if (CUT && LOGR == 4 && i >= 10 && i >= keep) break;
       const uint64_t o = off + i * step;
       check_below(v[i], p);
-      if (check_index(o, uint64_t(1) << P.logN)) data[o] = v[i];
+      if (check_index(o, P.points)) data[o] = v[i];
     }
   } else {
     uint32_t xt = thread_base<A0>(tid);
@@ -126,7 +136,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const uint64_t o = off + i * step;
-      v[i] = check_index(o, uint64_t(1) << P.logN) ? data[o] : 0;
+      v[i] = check_index(o, P.points) ? data[o] : 0;
       check_below(v[i], 2 * p);
     }
     inter_pass(v, xt, tb.hi_inv, tb.lo_inv);
@@ -144,7 +154,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     for (int i = 0; i < 16; ++i) {
       const uint64_t o = off + i * step;
       check_below(v[i], 2 * p);
-      if (check_index(o, uint64_t(1) << P.logN)) data[o] = v[i];
+      if (check_index(o, P.points)) data[o] = v[i];
     }
   }
 }

@@ -170,6 +170,107 @@ __device__ __forceinline__ void from_smem(uint64_t (&v)[16], uint64_t *sm, uint3
   for (int i = 0; i < 16; ++i) v[i] = s[static_cast<uint32_t>(i) << A];
 }
 
+// The inverse of a truncated transform's top row bits, on registers.
+//
+// A truncated transform (van der Hoeven's truncated Fourier transform) keeps
+// the first krows of the outer pass's R rows of outputs: krows S points
+// determine a product of at most krows S coefficients.  Its inverse gets, per
+// column, the R-point transform's first outputs, and knows that the rows of
+// the result past krows are zero.  After the stages of the low row bits (run
+// on the known rows only, as in a whole transform), each thread holds 2^JN
+// values that differ in the top JN row bits (register bits J = JL .. 3):
+// the first K are the transform's, the others are known results (zero at
+// the top level).  run<J, JL, K, OFF, ZT> solves the n = 2^(J - JL + 1)
+// values at OFF for the first K results, scaled by n as the unscaled inverse
+// leaves them; results past K are already known.  With u and v the half-size
+// transforms' inputs (u_h = x_h + x_(h+n/2), v_h = (x_h - x_(h+n/2)) w^h):
+//   K > n/2: every u is an inverse of known outputs.  For h >= K - n/2 the
+//     upper result is known, so v_h = (u_h - 2 x_(h+n/2)) w^h is too and x_h
+//     = u_h - x_(h+n/2); the rest of v is the same problem at half the size,
+//     and its butterflies are the inverse's own.
+//   K <= n/2: u_h is known for h >= K, the rest of u is the same problem, and
+//     x_h = u_h - x_(h+n/2).
+// Every value is in [0, 2p) before and after.
+template <int LOGR, int A, int ROWOFF, bool TZERO>
+struct TruncatedInverse {
+  const ulonglong2 *twi, *twf;  // (w_R^-e, companion), (w_R^e, companion), e < R / 2
+  uint32_t xt;
+  uint64_t p;
+  uint32_t c;
+
+  // Entry of the stage on register bit J's row bit for register i.
+  template <int J>
+  __device__ __forceinline__ uint32_t entry(int i) const {
+    constexpr int b = J + A - ROWOFF;
+    constexpr uint32_t lowmask = (1u << b) - 1u;
+    constexpr int sh = LOGR - 1 - b;
+    const uint32_t te = TZERO ? 0u : ((xt >> ROWOFF) & lowmask) << sh;
+    return te + ((((static_cast<uint32_t>(i) << A) >> ROWOFF) & lowmask) << sh);
+  }
+
+  template <int J>
+  __device__ __forceinline__ void butterfly(uint64_t (&v)[16], int i) const {
+    const uint64_t u = fold_p(v[i], p), w = v[i | (1 << J)];
+    uint64_t t;
+    if (TZERO && entry<J>(i) == 0) {
+      t = fold_p(w, p);
+    } else {
+      const ulonglong2 tt = twi[entry<J>(i)];
+      t = shoup_mul(w, tt.x, tt.y, p, c);
+    }
+    v[i] = u + t;
+    v[i | (1 << J)] = u - t + p;
+  }
+
+  // 2 a - b mod p in (0, 2p)
+  __device__ __forceinline__ uint64_t twice_less(uint64_t a, uint64_t b) const {
+    return fold_p(2 * fold_p(a, p), p) - fold_p(b, p) + p;
+  }
+
+  template <int J, int JL, int K, int OFF, bool ZT>
+  __device__ __forceinline__ void run(uint64_t (&v)[16]) const {
+    if constexpr (J >= JL) {
+      constexpr int half = 1 << (J - JL), U = 1 << J;
+      if constexpr (K == 2 * half) {
+        run<J - 1, JL, half, OFF, false>(v);
+        run<J - 1, JL, half, OFF | U, false>(v);
+#pragma unroll
+        for (int q = 0; q < (half << JL); ++q) butterfly<J>(v, OFF | q);
+      } else if constexpr (K > half) {
+        constexpr int K1 = K - half;
+        run<J - 1, JL, half, OFF, false>(v);
+#pragma unroll
+        for (int q = (K1 << JL); q < (half << JL); ++q) {
+          const int i = OFF | q;
+          const uint64_t u = v[i], x = v[i | U];  // x: known (zero when ZT)
+          const uint64_t d = ZT ? u : fold_p(u, p) - fold_p(x, p) + p;
+          if (TZERO && entry<J>(i) == 0) {
+            v[i | U] = d;
+          } else {
+            const ulonglong2 t = twf[entry<J>(i)];
+            v[i | U] = shoup_mul(d, t.x, t.y, p, c);
+          }
+          v[i] = ZT ? 2 * fold_p(u, p) : twice_less(u, x);
+        }
+        run<J - 1, JL, K1, OFF | U, false>(v);
+#pragma unroll
+        for (int q = 0; q < (K1 << JL); ++q) butterfly<J>(v, OFF | q);
+      } else {
+        static_assert(!ZT, "a truncated transform keeps more than half its rows");
+#pragma unroll
+        for (int q = (K << JL); q < (half << JL); ++q) {  // u_h = (x_h + x_(h+n/2)) at half the scale
+          const int i = OFF | q;
+          const uint64_t s = add_mod(fold_p(v[i], p), fold_p(v[i | U], p), p);
+          v[i] = (s + ((s & 1) ? p : 0)) >> 1;
+        }
+        run<J - 1, JL, K, OFF, false>(v);
+#pragma unroll
+        for (int q = 0; q < (K << JL); ++q) v[OFF | q] = twice_less(v[OFF | q], v[OFF | q | U]);
+      }
+    }
+  }
+};
+
 // Multiply register i by beta * gamma^bitrev4(i) (Montgomery-form beta, gamma):
 // the twiddle w_M^(s * bitrev_R(r)) of the 16 rows r = rhi*16 + i of one
 // column, with beta = w_M^(s * bitrev(rhi)), gamma = w_M^(s * R/16).

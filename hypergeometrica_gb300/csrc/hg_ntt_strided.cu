@@ -25,6 +25,15 @@
 // their 16 residues with constant shared-memory offsets, and after the
 // stages one bulk copy writes the tile back.  No thread computes a global
 // address or issues a global load or store for the residues.
+//
+// Truncated transforms: a product of n coefficients needs n points, not the
+// power of two above.  The outer pass (M = N) may keep only its first krows
+// rows of outputs (krows S >= n): the passes inside then run on krows of the
+// R blocks, and the outer inverse pass solves each column's krows values
+// from krows outputs and the R - krows results known to be zero
+// (TruncatedInverse).  krows is 5/8, 6/8 or 7/8 of R, cut by the top three row
+// bits (by the top two for R = 64: 6/8 only), which sit in one thread's
+// registers in the round that ends the pass.
 #include <algorithm>
 #include <cudaTypedefs.h>
 #include <mutex>
@@ -41,12 +50,14 @@ using namespace bodies;
 // Four CTAs of 256 threads per SM (64 registers, a few spilled words): on
 // the 2^25-point passes faster than three (80 registers), two (128) or five
 // (48).
-template <int LOGR, bool INV>
+template <int LOGR, bool INV, bool CUT = false>
 __global__ void __launch_bounds__(kTileThreads, 4) ntt_strided_kernel(const PassArgs P) {
   __shared__ ulonglong2 tw[1 << (LOGR - 1)];
   __shared__ uint64_t sm[LOGR > 4 ? (1 << kTileBits) : 1];
-  strided_ldg_body<LOGR, INV>(P, blockIdx.x, tw, sm);
+  strided_ldg_body<LOGR, INV, CUT>(P, blockIdx.x, tw, sm);
 }
+
+constexpr int kCut = 0;  // KH of a truncated transform's outer forward pass
 
 // Tensor maps of one TMA-staged pass: the box each CTA loads (residues, or
 // the limbs of a first forward pass) and stores, per operand, and the box of
@@ -80,7 +91,13 @@ struct TmaLimbs {
 // complete one with plain loads before reducing every limb modulo p.  When
 // the upper half of the block lies past the limbs (P.ztop bit op), the first
 // stage skips its zero inputs.
-template <int LOGR, bool INV, bool TABLE, bool LIMBS>
+//
+// KH < 8: the outer pass of a truncated transform.  Inverse: KH/8 of the rows
+// are known.  Forward (KH = kCut, whatever the number): the kept rows are
+// P.krows, and threads whose 16 rows are all dropped stop after the exchange
+// (R > 16).  A whole transform's passes are instances of their own: taking the
+// rows from P.krows there made the 2^25-point product 2% slower.
+template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KH>
 __global__ void __launch_bounds__(kTileThreads, 4)
     ntt_strided_tma_kernel(const __grid_constant__ TmaMaps maps, const PassArgs P, const TmaLimbs L) {
   constexpr int T = kTileBits;
@@ -93,8 +110,15 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   constexpr uint32_t kTileBytes = (1u << T) * sizeof(uint64_t);
   static_assert(LOGR >= 4 && LOGR <= 8, "strided passes have 4..8 row bits");
   static_assert(!LIMBS || !INV, "only a forward pass reads limbs");
+  static_assert(KH == 8 || (!INV && KH == kCut && LIMBS) || (INV && KH >= 5 && (LOGR == 4 || LOGR >= 7 || (LOGR == 6 && KH == 6))),
+                "rows a truncated inverse can cut");
+  constexpr int KI = INV ? KH : 8;
+  constexpr int kRows = (1 << LOGR) * KI / 8;  // inverse: known rows
+  constexpr bool kCutFwd = !INV && KH < 8;
+  const int krows = kCutFwd ? P.krows : kRows;
   extern __shared__ __align__(128) uint64_t tile[];  // [1 << T] residues, then [1 << T] twiddles
   __shared__ ulonglong2 tw[1 << (LOGR - 1)];
+  __shared__ ulonglong2 twf[INV && KH < 8 ? 1 << (LOGR - 1) : 1];
   __shared__ __align__(8) uint64_t bar;
 
   const uint32_t tid = threadIdx.x;
@@ -120,7 +144,9 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   }
   __syncthreads();
   if (tid == 0) {
-    tma::mbar_arrive_expect_tx(&bar, TABLE ? 2 * kTileBytes : kTileBytes);
+    const uint32_t row_bytes = kTileBytes >> LOGR;
+    tma::mbar_arrive_expect_tx(&bar, (INV ? kRows * row_bytes : kTileBytes) +
+                                         (TABLE ? static_cast<uint32_t>(krows) * row_bytes : 0u));
     if constexpr (LIMBS)
       tma::load_2d(tile, &maps.in[op], &bar, s0, blk << LOGR);
     else
@@ -128,6 +154,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     if (TABLE) tma::load_3d(twt, &maps.tw, &bar, s0, 0, prime);
   }
   load_sub_twiddles(tw, INV ? tb.sub_inv : tb.sub_fwd, LOGR, tid, kTileThreads);
+  if constexpr (INV && KH < 8) load_sub_twiddles(twf, tb.sub_fwd, LOGR, tid, kTileThreads);
   const bool landed = tma::mbar_wait_bounded(&bar, 0);
   if (!__syncthreads_and(landed)) {  // also orders the sub-twiddle table
     if (tid == 0) latch_error(P.err, kDevCopyTimeout);
@@ -139,7 +166,10 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   auto inter_pass = [&](uint64_t (&v)[16], uint32_t xt, const uint64_t *hi, const uint64_t *lo) {
     if constexpr (TABLE) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = mont_mul(v[i], twt[xt | (static_cast<uint32_t>(i) << A0)], p, c);
+      for (int i = 0; i < 16; ++i) {
+        if (LOGR == 4 && KH < 8 && i >= 10 && i >= krows) break;  // rows that are not kept
+        v[i] = mont_mul(v[i], twt[xt | (static_cast<uint32_t>(i) << A0)], p, c);
+      }
     } else {
       const uint64_t s = static_cast<uint64_t>(s0) + (xt & ((1u << LOGTC) - 1u));
       const uint32_t rhi = (xt >> (ROWOFF + 4)) & ((1u << (LOGR - 4)) - 1u);
@@ -199,35 +229,75 @@ __global__ void __launch_bounds__(kTileThreads, 4)
       xt = thread_base<A0>(tid);
       from_smem<A0>(v, tile, xt);
     }
-    stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true>(v, tw, xt, p, c);
-    inter_pass(v, xt, tb.hi_fwd, tb.lo_fwd);
+    // A truncated transform drops the rows past krows: whole 16-row groups
+    // (the thread's, warp by warp), or the last rows of the one group (R = 16).
+    const bool kept = !kCutFwd || LOGR == 4 || static_cast<int>((xt >> (ROWOFF + 4)) << 4) < krows;
+    if (kept) {
+      stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true>(v, tw, xt, p, c);
+      inter_pass(v, xt, tb.hi_fwd, tb.lo_fwd);
+    }
     __syncthreads();
+    if (kept) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      check_below(v[i], p);  // after the Montgomery inter-pass twiddle
-      tile[xt | (static_cast<uint32_t>(i) << A0)] = v[i];
+      for (int i = 0; i < 16; ++i) {
+        if (!(kCutFwd && LOGR == 4 && i >= krows)) check_below(v[i], p);  // after the Montgomery inter-pass twiddle
+        tile[xt | (static_cast<uint32_t>(i) << A0)] = v[i];
+      }
     }
   } else {
+    // Registers of the rows [0, kRows) hold the known outputs, the others nothing.
+    constexpr int NK0 = LOGR == 4 ? kRows : 16;  // layout A0: registers of a thread with known rows
+    constexpr int NK1 = 2 * KI;                  // the pass's last layout: register i is row bits LOGR-4 .. LOGR-1
     xt = thread_base<A0>(tid);
+    const bool known = KI == 8 || LOGR == 4 || static_cast<int>((xt >> (ROWOFF + 4)) << 4) < kRows;
+    if (known) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      v[i] = tile[xt | (static_cast<uint32_t>(i) << A0)];
-      check_below(v[i], 2 * p);  // inverse residues live in [0, 2p)
+      for (int i = 0; i < 16; ++i) {
+        if (i >= NK0) {
+          v[i] = 0;
+          continue;
+        }
+        v[i] = tile[xt | (static_cast<uint32_t>(i) << A0)];
+        check_below(v[i], 2 * p);  // inverse residues live in [0, 2p)
+      }
+      inter_pass(v, xt, tb.hi_inv, tb.lo_inv);
+      if constexpr (KI == 8 || LOGR > 4) {
+        stages<4, 0, A0, ROWOFF, 0, LOGR, true, true, true>(v, tw, xt, p, c);
+      } else {  // the stage on row bit 0 of the known rows, then the top three bits
+#pragma unroll
+        for (int i = 0; i < kRows; i += 2) {
+          const uint64_t u = v[i], w = v[i + 1];
+          v[i] = u + w;
+          v[i + 1] = u - w + p;
+        }
+        TruncatedInverse<LOGR, A0, ROWOFF, true>{tw, twf, xt, p, c}.template run<3, 1, KI, 0, true>(v);
+      }
     }
-    inter_pass(v, xt, tb.hi_inv, tb.lo_inv);
-    stages<4, 0, A0, ROWOFF, 0, LOGR, true, true, true>(v, tw, xt, p, c);
     constexpr int AS = (G == 2) ? A1 : A0;
     if constexpr (G == 2) {
       __syncthreads();
-      to_smem<A0>(tile, v, xt);
+      if (known) to_smem<A0>(tile, v, xt);
       __syncthreads();
       xt = thread_base<A1>(tid);
-      from_smem<A1>(v, tile, xt);
-      stages<NB1, 4 - NB1, A1, ROWOFF, 4, LOGR, true, false>(v, tw, xt, p, c);
+#pragma unroll
+      for (int i = 0; i < NK1; ++i) v[i] = tile[xt | (static_cast<uint32_t>(i) << A1)];
+      if constexpr (KI == 8) {
+        stages<NB1, 4 - NB1, A1, ROWOFF, 4, LOGR, true, false>(v, tw, xt, p, c);
+      } else {
+        const TruncatedInverse<LOGR, A1, ROWOFF, false> top{tw, twf, xt, p, c};
+        if constexpr (LOGR == 8) {
+#pragma unroll
+          for (int i = 0; i < NK1; i += 2) top.template butterfly<0>(v, i);  // row bit 4 of the known rows
+        }
+        if constexpr (LOGR == 6)
+          top.template run<3, 2, KI / 2, 0, true>(v);
+        else
+          top.template run<3, 1, KI, 0, true>(v);
+      }
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
+    for (int i = 0; i < NK1; ++i) {
       check_below(v[i], 2 * p);
       tile[xt | (static_cast<uint32_t>(i) << AS)] = v[i];
     }
@@ -266,6 +336,8 @@ template <int LOGR>
 cudaError_t launch_r(const PassArgs &a, bool inverse, unsigned grid, cudaStream_t st) {
   if (inverse)
     ntt_strided_kernel<LOGR, true><<<grid, kTileThreads, 0, st>>>(a);
+  else if (a.krows < (1 << LOGR))
+    ntt_strided_kernel<LOGR, false, true><<<grid, kTileThreads, 0, st>>>(a);
   else
     ntt_strided_kernel<LOGR, false><<<grid, kTileThreads, 0, st>>>(a);
   return cudaGetLastError();
@@ -300,17 +372,18 @@ cudaError_t encode(CUtensorMap *m, const void *base, int rank, const cuuint64_t 
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// The residue arrays of one operand as a 5-D tensor: column s (S), row r (R),
-// block (N / M), prime (nprimes, prime_stride apart), product (nprod,
-// ws_stride apart); the box is one tile, C columns by R rows.
+// The residue arrays of one operand as a 5-D tensor: column s (S), row r (R,
+// or the kept rows of a truncated outer pass), block (points / M), prime
+// (nprimes, prime_stride apart), product (nprod, ws_stride apart); the box is
+// one tile, C columns by the rows.
 cudaError_t residue_map(CUtensorMap *m, const uint64_t *base, const PassArgs &a) {
-  const uint64_t S = uint64_t(1) << a.logS, R = uint64_t(1) << a.logR, M = R * S;
-  const uint64_t N = uint64_t(1) << a.logN;
-  const cuuint64_t dims[5] = {S, R, N / M, static_cast<cuuint64_t>(a.nprimes), a.nprod};
-  const uint64_t pstride = a.nprimes > 1 ? a.prime_stride : N;
-  const uint64_t wstride = a.nprod > 1 ? a.ws_stride : N * static_cast<uint64_t>(a.nprimes);
+  const uint64_t S = uint64_t(1) << a.logS, R = uint64_t(1) << a.logR, K = static_cast<uint64_t>(a.krows);
+  const uint64_t M = R * S;
+  const cuuint64_t dims[5] = {S, K, K < R ? 1 : a.points / M, static_cast<cuuint64_t>(a.nprimes), a.nprod};
+  const uint64_t pstride = a.nprimes > 1 ? a.prime_stride : a.points;
+  const uint64_t wstride = a.nprod > 1 ? a.ws_stride : a.points * static_cast<uint64_t>(a.nprimes);
   const cuuint64_t strides[4] = {S * 8, M * 8, pstride * 8, wstride * 8};
-  const cuuint32_t box[5] = {static_cast<cuuint32_t>((uint64_t(1) << kTileBits) / R), static_cast<cuuint32_t>(R), 1,
+  const cuuint32_t box[5] = {static_cast<cuuint32_t>((uint64_t(1) << kTileBits) / R), static_cast<cuuint32_t>(K), 1,
                              1, 1};
   return encode(m, base, 5, dims, strides, box);
 }
@@ -321,23 +394,24 @@ cudaError_t twiddle_map(CUtensorMap *m, const uint64_t *ptw, const PassArgs &a) 
   const uint64_t S = uint64_t(1) << a.logS, R = uint64_t(1) << a.logR;
   const cuuint64_t dims[3] = {S, R, static_cast<cuuint64_t>(kPrimes)};
   const cuuint64_t strides[2] = {S * 8, R * S * 8};
-  const cuuint32_t box[3] = {static_cast<cuuint32_t>((uint64_t(1) << kTileBits) / R), static_cast<cuuint32_t>(R), 1};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>((uint64_t(1) << kTileBits) / R),
+                             static_cast<cuuint32_t>(a.krows), 1};
   return encode(m, ptw, 3, dims, strides, box);
 }
 
-template <int LOGR, bool INV, bool TABLE, bool LIMBS>
+template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KH = 8>
 cudaError_t launch_tma_v(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l, unsigned grid, cudaStream_t st) {
   constexpr size_t bytes = (TABLE ? 2 : 1) * (size_t(1) << kTileBits) * sizeof(uint64_t);
   // Raise the dynamic shared-memory limit once per instantiation (not on
   // every launch, so that launches can be captured in a CUDA graph).
   static bool raised = false;
   if (bytes > 48 * 1024 && !raised) {
-    cudaError_t e = cudaFuncSetAttribute(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS>,
+    cudaError_t e = cudaFuncSetAttribute(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e != cudaSuccess) return e;
     raised = true;
   }
-  ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS><<<grid, kTileThreads, bytes, st>>>(m, a, l);
+  ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH><<<grid, kTileThreads, bytes, st>>>(m, a, l);
   return cudaGetLastError();
 }
 
@@ -345,9 +419,29 @@ template <int LOGR>
 cudaError_t launch_tma_r(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l, bool inverse, bool limbs,
                          unsigned grid, cudaStream_t st) {
   const bool table = a.ptw != nullptr;
+  if (inverse && a.krows < (1 << LOGR)) {
+    const int kh = 8 * a.krows >> LOGR;
+    if constexpr (LOGR != 5) {
+      if (kh == 6)
+        return table ? launch_tma_v<LOGR, true, true, false, 6>(m, a, l, grid, st)
+                     : launch_tma_v<LOGR, true, false, false, 6>(m, a, l, grid, st);
+    }
+    if constexpr (LOGR != 5 && LOGR != 6) {
+      if (kh == 5)
+        return table ? launch_tma_v<LOGR, true, true, false, 5>(m, a, l, grid, st)
+                     : launch_tma_v<LOGR, true, false, false, 5>(m, a, l, grid, st);
+      if (kh == 7)
+        return table ? launch_tma_v<LOGR, true, true, false, 7>(m, a, l, grid, st)
+                     : launch_tma_v<LOGR, true, false, false, 7>(m, a, l, grid, st);
+    }
+    return cudaErrorInvalidValue;
+  }
   if (inverse)
     return table ? launch_tma_v<LOGR, true, true, false>(m, a, l, grid, st)
                  : launch_tma_v<LOGR, true, false, false>(m, a, l, grid, st);
+  if (limbs && a.krows < (1 << LOGR))
+    return table ? launch_tma_v<LOGR, false, true, true, kCut>(m, a, l, grid, st)
+                 : launch_tma_v<LOGR, false, false, true, kCut>(m, a, l, grid, st);
   if (limbs)
     return table ? launch_tma_v<LOGR, false, true, true>(m, a, l, grid, st)
                  : launch_tma_v<LOGR, false, false, true>(m, a, l, grid, st);
@@ -416,6 +510,14 @@ cudaError_t launch_ntt_strided(const PassArgs &a, bool inverse, cudaStream_t st)
     return cudaErrorInvalidValue;
   const unsigned g = static_cast<unsigned>(grid);
   const bool limbs = reads_limbs(a);
+  const int R = 1 << a.logR;
+  if (a.krows < R) {  // truncated: the outer pass, its forward side from limbs, by rows the kernels can cut
+    if (a.logR + a.logS != a.logN || !truncation_ok(a.logR, 8 * a.krows >> a.logR) || (8 * a.krows) % R ||
+        a.points != static_cast<uint64_t>(a.krows) << a.logS || (inverse ? !tma_aligned(a) : !limbs))
+      return cudaErrorInvalidValue;
+  } else if (a.krows != R || (a.points >> (a.logR + a.logS)) == 0) {
+    return cudaErrorInvalidValue;
+  }
   if (tma_aligned(a) && (!limbs || tma_limbs_ok(a))) {
     TmaMaps m;
     TmaLimbs l{};

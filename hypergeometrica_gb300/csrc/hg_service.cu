@@ -35,7 +35,7 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 constexpr int kMaxSlots = 8;
-constexpr size_t kSlotTickets = 128;  // carry-scan tickets per slot (one per group)
+constexpr size_t kSlotTickets = 512;  // carry-scan tickets per slot (one per group)
 
 struct SvcRequest {
   ProductDesc d;

@@ -1,0 +1,117 @@
+"""Truncated transforms: a product whose size is at most 7/8 of the power of
+two above it keeps 5, 6 or 7 eighths of the points.  Every length class that
+has its own plan (13 .. 22 bits: one or two strided passes, outer passes of
+16, 64, 128 and 256 rows) at the edges of each cut, against the oracle where
+that is quick and against the whole transform (set_chunking(False)) limb for
+limb.
+"""
+
+import numpy as np
+import pytest
+
+from hypergeometrica_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(a):
+    import torch
+
+    return torch.from_numpy(a.view(np.int64).copy()).cuda()
+
+
+def _np(t):
+    return t.cpu().numpy().view(np.uint64)
+
+
+def _sizes(L):
+    """Product sizes around every cut of 2^L points, and odd ones between."""
+    n, e = 1 << L, 1 << (L - 3)
+    out = [n // 2 + 1]
+    for k in (5, 6, 7):
+        out += [k * e - 1, k * e, k * e + 1]
+    return out + [n - 1, n, n // 2 + e // 3, 6 * e + e // 5]
+
+
+@pytest.mark.parametrize("L", range(13, 23))
+def test_products_and_squares(hg, oracle, L):
+    import torch
+
+    from hypergeometrica_gb300 import device as D
+    from hypergeometrica_gb300._lib import set_chunking
+
+    for j, size in enumerate(_sizes(L)):
+        nx = size - size * (3 + j % 4) // 8
+        ny = size - nx
+        dist = ("uniform", "ones", "sparse")[j % 3]
+        x, y = W.limbs(100 * L + j, nx, dist), W.limbs(7000 + 100 * L + j, ny, "uniform" if dist == "sparse" else dist)
+        tx, ty = _dev(x), _dev(y)
+        pad = (0, 1, 5000)[j % 3]  # limbs of out past the product, written as zeros
+        got = torch.full((size + pad,), -1, dtype=torch.int64, device="cuda")
+        D.mul(tx, ty, got)
+        sq = torch.full((2 * (size // 2) + pad,), -1, dtype=torch.int64, device="cuda")
+        D.sqr(tx, sq, nx=min(nx, size // 2))
+        D.sync()
+        if L <= 15:
+            want = oracle.mpz_mul_ntt(x, y)[:size]
+            wsq = oracle.mpz_square(x[: size // 2])[: 2 * min(nx, size // 2)]
+        else:
+            assert set_chunking(False)
+            try:
+                w, ws = torch.empty_like(got), torch.empty_like(sq)
+                D.mul(tx, ty, w)
+                D.sqr(tx, ws, nx=min(nx, size // 2))
+                D.sync()
+            finally:
+                set_chunking(True)
+            want, wsq = _np(w)[:size], _np(ws)
+        assert np.array_equal(_np(got)[:size], want), (L, size)
+        assert not _np(got)[size:].any(), (L, size)
+        k = min(len(wsq), sq.numel())
+        assert np.array_equal(_np(sq)[:k], wsq[:k]) and not _np(sq)[k:].any(), (L, size)
+
+
+def test_host_products(hg, oracle):
+    """hg_mul from host memory: column slices of a truncated outer pass."""
+    for size in (5 << 10, (5 << 10) + 1, 6 << 11, 7 << 12, 21000, 23000):
+        nx = size * 5 // 8
+        x, y = W.limbs(size, nx), W.limbs(size + 1, size - nx)
+        assert hg.int_from_digits(hg.mpz_mul_ntt(hg.MPZ(1, x), hg.MPZ(-1, y)).storage) == \
+            hg.int_from_digits(oracle.mpz_mul_ntt(x, y))
+
+
+@pytest.mark.parametrize("autotune", [False, True])
+def test_batches(hg, autotune):
+    """Mixed lengths and cuts in one batch, on both schedules, with results
+    longer than the product; against products of whole transforms."""
+    import torch
+
+    from hypergeometrica_gb300 import device as D
+    from hypergeometrica_gb300._lib import set_chunking
+
+    sizes = sorted({s for L in (12, 13, 14, 15, 17, 18) for s in _sizes(L)})
+    items, want = [], []
+    assert set_chunking(False)
+    try:
+        for k, size in enumerate(sizes):
+            nx = size * (4 + k % 3) // 8
+            x = _dev(W.limbs(31 * k + 1, nx, ("uniform", "ones")[k % 2]))
+            y = None if k % 5 == 4 else _dev(W.limbs(31 * k + 2, size - nx))
+            n = 2 * nx if y is None else size
+            nout = n + (0, 3, 9000)[k % 3]
+            items.append((x, y, torch.full((nout,), -1, dtype=torch.int64, device="cuda")))
+            w = torch.empty(nout, dtype=torch.int64, device="cuda")
+            D.sqr(x, w) if y is None else D.mul(x, y, w)
+            want.append(w)
+        D.sync()
+    finally:
+        set_chunking(True)
+    for schedule in ("per_pass", "persistent", None):
+        b = D.Batch(items, autotune=autotune, schedule=schedule)
+        for _, _, out in items:
+            out.fill_(-1)
+        b.run()
+        D.sync()
+        for k, (it, w) in enumerate(zip(items, want)):
+            assert torch.equal(it[2], w), (schedule, sizes[k])
+        b.close()
