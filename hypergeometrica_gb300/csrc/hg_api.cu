@@ -129,8 +129,7 @@ constexpr int kUploadSlices = 4;
 struct Lane {
   cudaStream_t stream = nullptr;
   DevBuf A, B, X, Y, OUT, flags;
-  DevBuf misc;  // bytes [0, 8) carry-scan ticket, [8, 12) error word (lane 0's is the library's), [16, 24) large-sum top index
-  unsigned long long ticket_count = 0;
+  DevBuf misc;  // bytes [0, 4) carry-scan finished count, [8, 12) error word (lane 0's is the library's), [16, 24) large-sum top index
   uint32_t epoch = 0;
   cudaEvent_t ws_done = nullptr;
   cudaStream_t copy_stream = nullptr;  // host entry points: operand uploads
@@ -420,7 +419,14 @@ std::vector<PassPlan> plan_passes(int L) {
 // of two above it, the transform keeps 5, 6 or 7 eighths of the 2^L points
 // (hg_ntt_strided.cu): the passes inside the outer one, the middle and the
 // workspace shrink by that factor.  The outer pass cuts by its top row bits,
-// so it needs 16, 128 or 256 rows (64 for 6/8).
+// so it needs 16, 128 or 256 rows (64 for 6/8).  Products, us, beside the
+// whole transform of the same size (one product, warm):
+//   points   5/8            6/8            7/8            8/8
+//   2^18     59.8 (74.2)    61.8 (74.2)    72.8 (74.1)    74.4
+//   2^21     272 (363)      302 (365)      329 (367)      369
+//   2^25     3947 (5521)    4543 (5561)    5132 (5600)    5638
+// Below 2^17 points a product is bound by the latency of its launches and the
+// cut gives 1-6%; it is nowhere slower.
 uint64_t kept_points(int L, int kh) { return kh == 8 ? uint64_t(1) << L : (uint64_t(1) << (L - 3)) * kh; }
 
 struct TransformPlan {
@@ -430,12 +436,26 @@ struct TransformPlan {
   uint64_t points() const { return kept_points(L, kh); }
 };
 
+// Tiles of 4096 residues (three primes) up to which a launch leaves SMs idle:
+// plans for it spread the work instead of saving passes over memory.
+constexpr uint64_t kIdleTiles = 192;
+
 // Passes of a 2^L-point transform that keeps kh eighths: the outer pass has
 // 16 rows where the other bits still fit the same number of passes (the
 // smaller the outer pass, the more of the work is cut), else the plan of the
 // whole transform, else 128 rows (2^17 and 2^18 points).
-std::vector<PassPlan> plan_kept(int L, int kh) {
+//
+// nprod products at a time that leave SMs idle (kIdleTiles) take contiguous
+// blocks of 2^9 residues (2^10 from 2^17 points on): more CTAs, and more of
+// the stages where both operands run side by side.  A product of 2^16 points:
+// 43.1 us with 2^12-residue blocks, 37.0 with 2^9; of 2^17: 49.2 and 45.6; of
+// 2^18: 73.0 and 68.8 (one product, warm).
+std::vector<PassPlan> plan_kept(int L, int kh, uint64_t nprod = 1) {
   std::vector<PassPlan> v = plan_passes(L);
+  if (L > kTileBits && L <= 18 && (3 * nprod << L) >> kTileBits <= kIdleTiles) {
+    const int T = L < 17 ? 9 : 10;
+    if (truncation_ok(L - T, kh)) return {{L - T, T, kTileBits}, {T, 0, T}};
+  }
   if (kh == 8) return v;
   const int rem = L - v.back().logT;
   const int k = static_cast<int>(v.size()) - 1;
@@ -627,7 +647,7 @@ cudaError_t run_contig(PassArgs a, const PassPlan &pp, int mode, cudaStream_t st
 // reconstruction receives the coefficients mod p_j; false where the moduli
 // do not meet the prescaled reconstruction's bounds (p0 < 2 p1, p0 < 2 p2,
 // 3 p2 < 2^64).
-bool prescale_factors(int L, uint64_t (&s)[kPrimes]) {
+bool prescale_factors_of(int L, uint64_t (&s)[kPrimes]) {
   const uint64_t p0 = g_ctx.moduli[0], p1 = g_ctx.moduli[1], p2 = g_ctx.moduli[2];
   if (!(p0 < 2 * p1 && p0 < 2 * p2 && p2 < ~uint64_t(0) / 3)) return false;
   const uint64_t N = uint64_t(1) << L;
@@ -638,7 +658,7 @@ bool prescale_factors(int L, uint64_t (&s)[kPrimes]) {
   return true;
 }
 
-CrtConst crt_const(int L, bool prescaled = false) {
+CrtConst crt_const_of(int L, bool prescaled) {
   CrtConst k{};
   k.prescaled = prescaled ? 1u : 0u;
   const uint64_t p0 = g_ctx.moduli[0], p1 = g_ctx.moduli[1], p2 = g_ctx.moduli[2];
@@ -661,6 +681,31 @@ CrtConst crt_const(int L, bool prescaled = false) {
   return k;
 }
 
+// The two above depend on the length alone and take some ten modular powers
+// (15 us of host time per product): worked out once per length.
+struct LengthConst {
+  std::once_flag once;
+  CrtConst crt[2];  // unscaled, prescaled
+  uint64_t scale[kPrimes];
+  bool scalable;
+};
+const LengthConst &length_const(int L) {
+  static LengthConst table[kLogNmax + 1];  // the scheme's moduli never change
+  LengthConst &t = table[L];
+  std::call_once(t.once, [&] {
+    t.crt[0] = crt_const_of(L, false);
+    t.crt[1] = crt_const_of(L, true);
+    t.scalable = prescale_factors_of(L, t.scale);
+  });
+  return t;
+}
+const CrtConst &crt_const(int L, bool prescaled = false) { return length_const(L).crt[prescaled ? 1 : 0]; }
+bool prescale_factors(int L, uint64_t (&s)[kPrimes]) {
+  const LengthConst &t = length_const(L);
+  for (int j = 0; j < kPrimes; ++j) s[j] = t.scale[j];
+  return t.scalable;
+}
+
 // Serialise use of the shared workspace across streams.
 cudaError_t ws_acquire(cudaStream_t st) {
   if (g_ctx.lane->ws_pending) return cudaStreamWaitEvent(st, g_ctx.lane->ws_done, 0);
@@ -680,12 +725,10 @@ int scan_state(uint64_t tiles, ScanState *ss) {
     HG_CUDA(cudaMemset(c.lane->flags.p, 0, c.lane->flags.bytes), "flag init");
   }
   if (++c.lane->epoch == 0) c.lane->epoch = 1;
-  ss->ticket = static_cast<unsigned long long *>(c.lane->misc.p);
-  ss->ticket_base = c.lane->ticket_count;
+  ss->done = static_cast<unsigned *>(c.lane->misc.p);
   ss->flags = static_cast<unsigned long long *>(c.lane->flags.p);
   ss->epoch = c.lane->epoch;
   ss->err = err_word();
-  c.lane->ticket_count += tiles;
   return HG_OK;
 }
 
@@ -812,7 +855,7 @@ int chunk_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint
   if (rc) return rc;
   uint64_t tiles = 0;
   {
-    ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(size), 2);  // local scan + fix
+    ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(size), carry_short(size) ? 1 : 2);
     HG_CUDA(launch_crt_carry_chunks(c.lane->A.u64(), slab, L, cp.chunk, cp.nchunks, crt_const(L, scaled), out, size,
                                     ss, st, &tiles),
             "reconstruction");
@@ -974,7 +1017,7 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
   if (rc) return rc;
   uint64_t tiles = 0;
   {
-    ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(nproc), 2);  // local scan + fix
+    ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(nproc), carry_short(nproc) ? 1 : 2);
     HG_CUDA(launch_crt_carry(c.lane->A.u64(), N, crt_const(L, scaled), out, nout, ss, st, &tiles),
             "reconstruction");
   }
@@ -985,15 +1028,15 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
 // ---- products on a fixed scratch array (hg_mul_device_noalloc) ----------
 //
 // Scratch layout, in words: operand 0's residues [3][2^16], operand 1's
-// residues [3][2^16], the carry scan's ticket word, then one flag word per
-// carry tile (16 at 2^16).  Static device memory is zero when the module
+// residues [3][2^16], the carry scan's count word, then one flag word per
+// carry tile (64 at 2^16).  Static device memory is zero when the module
 // loads; the residue area needs no initial value (the first pass writes
-// every word it later reads), and the call clears the ticket and flag words
+// every word it later reads), and the call clears the count and flag words
 // on its stream before each reconstruction.
 constexpr int kNoAllocLogN = 16;
 constexpr uint64_t kNoAllocN = uint64_t(1) << kNoAllocLogN;
 constexpr uint64_t kNoAllocResWords = 2ull * kPrimes * kNoAllocN;
-constexpr uint64_t kNoAllocScanWords = 64;
+constexpr uint64_t kNoAllocScanWords = 128;
 constexpr int kNoAllocDevices = 64;
 static_assert(kNoAllocN == HG_NOALLOC_MAX_LIMBS, "public limit and scratch size disagree");
 
@@ -1065,8 +1108,7 @@ int noalloc_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, ui
   uint64_t *scan = scratch + kNoAllocResWords;
   HG_CUDA(cudaMemsetAsync(scan, 0, (tiles + 1) * sizeof(uint64_t), st), "scan state reset");
   ScanState ss;
-  ss.ticket = reinterpret_cast<unsigned long long *>(scan);
-  ss.ticket_base = 0;
+  ss.done = reinterpret_cast<unsigned *>(scan);
   ss.flags = reinterpret_cast<unsigned long long *>(scan + 1);
   ss.epoch = 1;
   ss.err = err_word();
@@ -1093,7 +1135,7 @@ int small_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint
   if (rc) return rc;
   uint64_t tiles = 0;
   {
-    ProfScope ps(HG_KC_SMALL, st, 8.0 * static_cast<double>(nx + (y ? ny : 0) + size), 2);
+    ProfScope ps(HG_KC_SMALL, st, 8.0 * static_cast<double>(nx + (y ? ny : 0) + size), carry_short(size) ? 1 : 2);
     if (y)
       HG_CUDA(launch_schoolboy_carry(x, nx, y, ny, out, size, ss, st, &tiles), "schoolboy product");
     else
@@ -1368,8 +1410,8 @@ int spectrum(uint64_t *a, size_t n, int mod_num, bool inverse, cudaStream_t st) 
 // L >= 12, every contiguous block size T with the remaining L - T bits in
 // as few strided passes of 4..8 bits as possible (where the outer one can
 // keep kh eighths of its rows).
-std::vector<std::vector<PassPlan>> plan_candidates(int L, int kh) {
-  std::vector<std::vector<PassPlan>> out{plan_kept(L, kh)};
+std::vector<std::vector<PassPlan>> plan_candidates(int L, int kh, uint64_t nprod) {
+  std::vector<std::vector<PassPlan>> out{plan_kept(L, kh, nprod)};
   if (L < kTileBits) return out;
   for (int T = 4; T <= kTileBits; ++T) {
     const int rem = L - T;
@@ -1449,13 +1491,13 @@ int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::ve
   bool scaled = false;
   HG_CUDA(run_strided(inv, plan, true, st, prescale_factors(g.L, sc) ? sc : nullptr, &scaled), "inverse transform");
   ScanState ss;
-  ss.ticket = bb.tickets + gi;
-  ss.ticket_base = 0;
+  ss.done = reinterpret_cast<unsigned *>(bb.tickets + gi);
   ss.flags = bb.flags + g.flags_off;
   ss.epoch = 1;
   ss.err = bb.err;
   {
-    ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(N) * static_cast<double>(g.nprod), 2);  // tiles + fix
+    ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(N) * static_cast<double>(g.nprod),
+                 carry_short(N, g.nprod) ? 1 : 2);
     HG_CUDA(launch_crt_carry_batch(ws, slab, N, crt_const(g.L, scaled), d, g.nprod, ss, st), "reconstruction");
   }
   return HG_OK;
@@ -1602,8 +1644,7 @@ std::vector<PersistPhase> group_phases(const BatchGroup &g, const BatchBufs &bb,
   c.batch = d;
   c.tpp = persist_carry_tiles(N);
   c.tiles = c.tpp * g.nprod;
-  c.ss.ticket = nullptr;
-  c.ss.ticket_base = 0;
+  c.ss.done = nullptr;
   c.ss.flags = flags;
   c.ss.epoch = 1;
   c.ss.err = bb.err;
@@ -1725,7 +1766,7 @@ int batch_autotune(hg_batch *b) {
         continue;
       }
     }
-    const auto cands = plan_candidates(g.L, g.kh);
+    const auto cands = plan_candidates(g.L, g.kh, g.nprod);
     float best = 1e30f;
     for (const auto &plan : cands) {
       float ms = 0;
@@ -1925,7 +1966,7 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
       g.L = L;
       g.square = square;
       g.kh = live[s].kh;
-      g.plan = plan_kept(L, g.kh);
+      g.plan = plan_kept(L, g.kh, g.nprod);
       g.first = bp.desc.size();
       g.nprod = std::min<uint64_t>(chunk, e - c);
       g.flags_off = bp.flag_words;
@@ -1933,7 +1974,7 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
         bp.desc.push_back(items[live[k].i]);
         if (bp.desc.back().nout > N) g.tails = true;
       }
-      bp.flag_words += carry_tiles(N) * g.nprod;
+      bp.flag_words += carry_tiles(N, g.nprod) * g.nprod;
       bp.ws_words = std::max<uint64_t>(bp.ws_words, per / 8 * g.nprod);
       bp.groups.push_back(std::move(g));
     }
@@ -1970,8 +2011,8 @@ int large_sum_device(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t 
   if (rc) return rc;
   long long *top = reinterpret_cast<long long *>(static_cast<char *>(g_ctx.lane->misc.p) + 16);
   {
-    // (top search,) local scan, fix, sign and size
-    ProfScope ps(HG_KC_OTHER, st, 24.0 * static_cast<double>(nproc), sa != sb ? 4 : 3);
+    // (top search,) scan (and fix), sign and size
+    ProfScope ps(HG_KC_OTHER, st, 24.0 * static_cast<double>(nproc), (sa != sb ? 3 : 2) + (carry_short(nproc) ? 0 : 1));
     HG_CUDA(launch_large_sum(a, na, sa, b, nb, sb, out, top, result, ss, st), "large sum");
   }
   HG_CUDA(ws_release(st), "workspace ordering");
@@ -2027,7 +2068,8 @@ int hg_batch_schedule(const hg_batch *batch, int *persistent, size_t *launches) 
   }
   size_t n = batch->bp.nzero ? 1 : 0;
   for (const hg::BatchGroup &g : batch->bp.groups)
-    n += (g.tails ? 1 : 0) + 2 * (g.plan.size() - 1) + 1 + 2;  // zero tails, passes, middle, carry + fix
+    n += (g.tails ? 1 : 0) + 2 * (g.plan.size() - 1) + 1  // zero tails, passes, middle, carry (+ fix)
+         + (hg::carry_short(hg::kept_points(g.L, g.kh), g.nprod) ? 1 : 2);
   *launches = n;
   return HG_OK;
 }
@@ -2096,7 +2138,6 @@ int hg_shutdown(void) {
         e = nullptr;
       }
     L.ws_pending = L.d2h_pending = false;
-    L.ticket_count = 0;
     L.epoch = 0;
   }
   c.lane = &c.lanes[0];

@@ -15,7 +15,7 @@
 namespace hg {
 namespace carry {
 
-constexpr int kCarryPer = 8;  // positions per thread
+constexpr int kCarryPer = 8;  // positions per thread (4 in short launches, hg_crt.cu)
 
 template <int TILE>
 __device__ __forceinline__ uint64_t carry_tiles_dev(uint64_t n) { return (n + TILE - 1) / TILE; }
@@ -60,25 +60,26 @@ struct CrtProducerT {
     return garner(r[i], r[n + i], r[2 * n + i]);
   }
 
-  // Eight consecutive positions from i0 (a multiple of 8): 16-byte loads.
-  __device__ __forceinline__ void eight(uint64_t off, uint64_t i0, uint64_t nproc, V3 (&v)[8]) const {
-    if (i0 + 8 <= nproc) {
-      uint64_t r[3][8];
+  // PER consecutive positions from i0 (a multiple of PER, 4 or 8): 16-byte loads.
+  template <int PER>
+  __device__ __forceinline__ void many(uint64_t off, uint64_t i0, uint64_t nproc, V3 (&v)[PER]) const {
+    if (i0 + PER <= nproc) {
+      uint64_t r[3][PER];
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(res + off + j * n + i0);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < PER / 2; ++q) {
           const ulonglong2 w = load2(src + q);
           r[j][2 * q] = w.x;
           r[j][2 * q + 1] = w.y;
         }
       }
 #pragma unroll
-      for (int k8 = 0; k8 < 8; ++k8) v[k8] = garner(r[0][k8], r[1][k8], r[2][k8]);
+      for (int k8 = 0; k8 < PER; ++k8) v[k8] = garner(r[0][k8], r[1][k8], r[2][k8]);
     } else {
 #pragma unroll
-      for (int k8 = 0; k8 < 8; ++k8) v[k8] = (i0 + k8 < nproc) ? at(off, i0 + k8) : V3{0, 0, 0};
+      for (int k8 = 0; k8 < PER; ++k8) v[k8] = (i0 + k8 < nproc) ? at(off, i0 + k8) : V3{0, 0, 0};
     }
   }
 
@@ -143,14 +144,14 @@ __device__ __forceinline__ unsigned long long flag_word(uint32_t epoch, uint32_t
 // stream, then adds the true carry-in.  No CTA waits on another, so the
 // tiles stream at the memory and integer-pipe rate.
 //
-// carry_body is one CTA of NT threads on tile gt (NT * 8 positions);
+// carry_body is one CTA of NT threads on tile gt (NT * PER positions);
 // s_prev holds NT * 9 words and s_warp NT / 32 pairs of shared memory.
-template <class Producer, int NT>
+template <class Producer, int NT, int PER = kCarryPer>
 __device__ __forceinline__ void carry_body(const Producer &prod, uint64_t *__restrict__ out, uint64_t nproc,
                                            const ScanState &ss, const ProductDesc *batch, uint64_t tpp,
                                            uint64_t ws_stride, uint64_t n, uint64_t gt, uint64_t (*s_prev)[9],
                                            GP *s_warp) {
-  constexpr int kCarryTile = NT * kCarryPer;
+  constexpr int kCarryTile = NT * PER;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   // Product k's residues are addressed through an explicit word offset.
   uint64_t tile = gt, off = 0;
@@ -161,13 +162,16 @@ __device__ __forceinline__ void carry_body(const Producer &prod, uint64_t *__res
     out = batch[k].out;
     nproc = batch[k].nout < n ? batch[k].nout : n;
   }
-  const uint64_t i0 = tile * kCarryTile + static_cast<uint64_t>(tid) * kCarryPer;
+  const uint64_t i0 = tile * kCarryTile + static_cast<uint64_t>(tid) * PER;
 
-  V3 v[kCarryPer];
-  prod.eight(off, i0, nproc, v);
-  s_prev[tid][0] = v[5].w0; s_prev[tid][1] = v[5].w1; s_prev[tid][2] = v[5].w2;
-  s_prev[tid][3] = v[6].w0; s_prev[tid][4] = v[6].w1; s_prev[tid][5] = v[6].w2;
-  s_prev[tid][6] = v[7].w0; s_prev[tid][7] = v[7].w1; s_prev[tid][8] = v[7].w2;
+  V3 v[PER];
+  prod.template many<PER>(off, i0, nproc, v);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    s_prev[tid][3 * k] = v[PER - 3 + k].w0;
+    s_prev[tid][3 * k + 1] = v[PER - 3 + k].w1;
+    s_prev[tid][3 * k + 2] = v[PER - 3 + k].w2;
+  }
   V3 pm3{0, 0, 0}, pm2{0, 0, 0}, pm1{0, 0, 0};
   if (tid == 0 && i0 >= 3) {
     pm3 = prod.at(off, i0 - 3);
@@ -193,10 +197,10 @@ __device__ __forceinline__ void carry_body(const Producer &prod, uint64_t *__res
   };
   uint64_t whp;
   (void)wsum(pm1.w0, pm2.w1, pm3.w2, whp);  // W_(i0-1)
-  uint64_t al[kCarryPer];
+  uint64_t al[PER];
   uint32_t gbits = 0, pbits = 0;
 #pragma unroll
-  for (int k = 0; k < kCarryPer; ++k) {
+  for (int k = 0; k < PER; ++k) {
     const V3 &c1 = (k >= 1) ? v[k - 1] : pm1;
     const V3 &c2 = (k >= 2) ? v[k - 2] : (k == 1 ? pm1 : pm2);
     uint64_t wh;
@@ -208,10 +212,10 @@ __device__ __forceinline__ void carry_body(const Producer &prod, uint64_t *__res
     pbits |= ((a == ~0ull) && !ah ? 1u : 0u) << k;
     whp = wh;
   }
-  // Thread aggregate over its 8 positions (position 0 least significant).
+  // Thread aggregate over its positions (position 0 least significant).
   GP t{0, 1};
 #pragma unroll
-  for (int k = 0; k < kCarryPer; ++k) t = gp_compose(t, GP{(gbits >> k) & 1u, (pbits >> k) & 1u});
+  for (int k = 0; k < PER; ++k) t = gp_compose(t, GP{(gbits >> k) & 1u, (pbits >> k) & 1u});
 
   // Inclusive warp scan, then across warps.
   GP inc = t;
@@ -244,15 +248,15 @@ __device__ __forceinline__ void carry_body(const Producer &prod, uint64_t *__res
   uint64_t *s_out = &s_prev[0][0];
   auto oswz = [](uint32_t w) { return w ^ ((w >> 3) & 7u); };
 #pragma unroll
-  for (int k = 0; k < kCarryPer; ++k) {
+  for (int k = 0; k < PER; ++k) {
     const uint64_t z = al[k] + cin;
     cin = ((gbits >> k) & 1u) | (((pbits >> k) & 1u) & cin);
-    s_out[oswz(static_cast<uint32_t>(tid * kCarryPer + k))] = z;
+    s_out[oswz(static_cast<uint32_t>(tid * PER + k))] = z;
   }
   __syncthreads();
   const uint64_t tbase = tile * kCarryTile;
 #pragma unroll
-  for (int k = 0; k < kCarryPer; ++k) {
+  for (int k = 0; k < PER; ++k) {
     const uint32_t w = static_cast<uint32_t>(tid + k * NT);
     if (tbase + w < nproc) out[tbase + w] = s_out[oswz(w)];
   }

@@ -28,6 +28,15 @@ using namespace carry;
 constexpr int kCarryThreads = 256;
 constexpr int kCarryMinBlocks = 4;
 constexpr int kCarryTile = kCarryThreads * kCarryPer;
+// Launches of at most kShortCarry limbs leave SMs idle and are bound by the
+// latency of one thread's positions and by the launches themselves: they run
+// tiles of 1024 limbs (four positions a thread), and the CTA that finishes
+// last applies the carries itself instead of a second launch (one thread per
+// tile reads the aggregates, so at most 256 tiles): a product of 2^13 points
+// 35.9 -> 31.8 us, of 2^16 points 47.2 -> 43.1.
+constexpr int kShortPer = 4;
+constexpr int kShortTile = kCarryThreads * kShortPer;
+constexpr uint64_t kShortCarry = static_cast<uint64_t>(kShortTile) * kCarryThreads;
 
 // The product of a long operand cut into chunks of `chunk` limbs with a
 // short one: chunk k's cyclic product (2^logN > chunk + short - 1 points, no
@@ -69,21 +78,22 @@ struct ChunkProducerT {
     return crt.garner(sum_res(r0, r1, 0), sum_res(r0, r1, 1), sum_res(r0, r1, 2));
   }
 
-  // Eight positions from i0 (a multiple of 8, as is chunk): one chunk pair.
-  __device__ __forceinline__ void eight(uint64_t, uint64_t i0, uint64_t nproc, V3 (&v)[8]) const {
-    if (i0 + 8 > nproc) {
+  // PER positions from i0 (a multiple of PER, as is chunk): one chunk pair.
+  template <int PER>
+  __device__ __forceinline__ void many(uint64_t, uint64_t i0, uint64_t nproc, V3 (&v)[PER]) const {
+    if (i0 + PER > nproc) {
 #pragma unroll
-      for (int k8 = 0; k8 < 8; ++k8) v[k8] = (i0 + k8 < nproc) ? at(0, i0 + k8) : V3{0, 0, 0};
+      for (int k8 = 0; k8 < PER; ++k8) v[k8] = (i0 + k8 < nproc) ? at(0, i0 + k8) : V3{0, 0, 0};
       return;
     }
     const uint64_t *r0, *r1;
     sources(i0, r0, r1);
-    uint64_t r[3][8];
+    uint64_t r[3][PER];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const uint64_t p = crt.k.pc[j].p;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < PER / 2; ++q) {
         ulonglong2 a = make_ulonglong2(0, 0), b = make_ulonglong2(0, 0);
         if (r0) a = __ldg(reinterpret_cast<const ulonglong2 *>(r0 + j * crt.n) + q);
         if (r1) b = __ldg(reinterpret_cast<const ulonglong2 *>(r1 + j * crt.n) + q);
@@ -92,7 +102,7 @@ struct ChunkProducerT {
       }
     }
 #pragma unroll
-    for (int k8 = 0; k8 < 8; ++k8) v[k8] = crt.garner(r[0][k8], r[1][k8], r[2][k8]);
+    for (int k8 = 0; k8 < PER; ++k8) v[k8] = crt.garner(r[0][k8], r[1][k8], r[2][k8]);
   }
 };
 
@@ -105,9 +115,10 @@ struct ConvProducer {
 
   __host__ __device__ __forceinline__ bool drop_top() const { return false; }
 
-  __device__ __forceinline__ void eight(uint64_t, uint64_t i0, uint64_t nproc, V3 (&v)[8]) const {
+  template <int PER>
+  __device__ __forceinline__ void many(uint64_t, uint64_t i0, uint64_t nproc, V3 (&v)[PER]) const {
 #pragma unroll
-    for (int k8 = 0; k8 < 8; ++k8) v[k8] = (i0 + k8 < nproc) ? at(0, i0 + k8) : V3{0, 0, 0};
+    for (int k8 = 0; k8 < PER; ++k8) v[k8] = (i0 + k8 < nproc) ? at(0, i0 + k8) : V3{0, 0, 0};
   }
 
   __device__ __forceinline__ V3 at(uint64_t, uint64_t i) const {
@@ -167,14 +178,13 @@ struct SumProducer {
     return V3{lo, c, 0};
   }
 
-  __device__ __forceinline__ void prefetch(uint64_t, uint64_t, uint64_t) const {}
-
   __device__ __forceinline__ V3 at(uint64_t, uint64_t i) const { return value(i, a_larger()); }
 
-  __device__ __forceinline__ void eight(uint64_t, uint64_t i0, uint64_t nproc, V3 (&v)[8]) const {
+  template <int PER>
+  __device__ __forceinline__ void many(uint64_t, uint64_t i0, uint64_t nproc, V3 (&v)[PER]) const {
     const bool ax = a_larger();
 #pragma unroll
-    for (int k8 = 0; k8 < 8; ++k8) v[k8] = (i0 + k8 < nproc) ? value(i0 + k8, ax) : V3{0, 0, 0};
+    for (int k8 = 0; k8 < PER; ++k8) v[k8] = (i0 + k8 < nproc) ? value(i0 + k8, ax) : V3{0, 0, 0};
   }
 };
 
@@ -218,22 +228,109 @@ __global__ void sum_finish_kernel(const uint64_t *out, uint64_t nproc, SumProduc
   }
 }
 
-// One tile per CTA, in ticket order.
+// One tile per CTA.
 template <class Producer>
 __global__ void __launch_bounds__(kCarryThreads, kCarryMinBlocks)
     carry_kernel(const Producer prod0, uint64_t *__restrict__ out, uint64_t nproc, ScanState ss,
                  const ProductDesc *batch, uint64_t tpp, uint64_t ws_stride, uint64_t n) {
   __shared__ uint64_t s_prev[kCarryThreads][9];
   __shared__ GP s_warp[kCarryThreads / 32];
-  __shared__ unsigned long long s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(ss.ticket, 1ull) - ss.ticket_base;
-  __syncthreads();
-  const uint64_t gt = s_tile;
-  if (gt >= gridDim.x) {  // ticket out of step with this launch: touch nothing
-    if (threadIdx.x == 0) atomicCAS(ss.err, kDevOk, kDevTicket);
-    return;
+  carry_body<Producer, kCarryThreads>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, blockIdx.x, s_prev, s_warp);
+}
+
+// The carries of a whole short launch, by the CTA that finished last: thread
+// t composes tile t's carry-in from the aggregates of its product's tiles
+// below (fix_body says why only the tile's leading limbs equal to 2^64 - 1
+// and the first limb after them change).  Most tiles are done by their
+// thread's first limb; the others go to whole warps.
+__device__ __forceinline__ void fix_all(uint64_t *out, uint64_t nproc, uint64_t tiles, const ScanState &ss,
+                                        bool drop_top, const ProductDesc *batch, uint64_t tpp, uint64_t n,
+                                        GP *s_warp, uint32_t *s_long) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const uint64_t gt = static_cast<uint64_t>(tid);
+  uint64_t t = gt;
+  if (batch && gt < tiles) {
+    const uint64_t k = gt / tpp;
+    t = gt - k * tpp;
+    out = batch[k].out;
+    nproc = batch[k].nout < n ? batch[k].nout : n;
   }
-  carry_body<Producer, kCarryThreads>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, gt, s_prev, s_warp);
+  const uint64_t ntiles = carry_tiles_dev<kShortTile>(nproc);
+  const bool live = gt < tiles && t < ntiles;
+  GP own{0, 0};
+  if (live) {
+    const unsigned long long w = __ldcg(ss.flags + gt);
+    if ((w >> 32) != ss.epoch || (w & 3u) != 1u) atomicCAS(ss.err, kDevOk, kDevTicket);
+    own = GP{static_cast<uint32_t>((w >> 2) & 1u), static_cast<uint32_t>((w >> 3) & 1u)};
+  }
+  // Inclusive scan; a product's first tile has carry-in 0, so what is below it does not matter.
+  GP inc = GP{own.g, t == 0 ? 0u : own.p};
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t og = __shfl_up_sync(0xffffffffu, inc.g, d);
+    const uint32_t op = __shfl_up_sync(0xffffffffu, inc.p, d);
+    if (lane >= d) inc = gp_compose(GP{og, op}, inc);
+  }
+  if (lane == 31) s_warp[wid] = inc;
+  s_long[tid] = 0;
+  __syncthreads();
+  GP below{0, 0};
+  for (int w = 0; w < wid; ++w) below = gp_compose(below, s_warp[w]);
+  const uint32_t og = __shfl_up_sync(0xffffffffu, inc.g, 1), op = __shfl_up_sync(0xffffffffu, inc.p, 1);
+  if (lane > 0) below = gp_compose(below, GP{og, op});
+  const uint32_t cin = live && t > 0 ? below.g : 0;
+  if (live && t == ntiles - 1 && !drop_top && (own.g | (own.p & cin))) atomicCAS(ss.err, kDevOk, kDevCarryOverflow);
+  if (cin) {
+    const uint64_t w = __ldcg(out + t * kShortTile);
+    if (w != ~0ull)
+      out[t * kShortTile] = w + 1;
+    else
+      s_long[tid] = 1;
+  }
+  __syncthreads();
+  for (uint64_t k = wid; k < tiles; k += kCarryThreads / 32) {
+    if (!s_long[k]) continue;
+    uint64_t tile = k, np = nproc;
+    uint64_t *o = out;
+    if (batch) {
+      const uint64_t pr = k / tpp;
+      tile = k - pr * tpp;
+      o = batch[pr].out;
+      np = batch[pr].nout < n ? batch[pr].nout : n;
+    }
+    const uint64_t end = (tile + 1) * kShortTile < np ? (tile + 1) * kShortTile : np;
+    for (uint64_t i = tile * kShortTile; i < end; i += 32) {
+      const uint64_t at = i + lane;
+      const uint64_t w = at < end ? __ldcg(o + at) : 0;
+      const unsigned stop = __ballot_sync(0xffffffffu, at < end && w != ~0ull);
+      const int f = stop ? __ffs(stop) - 1 : 32;
+      if (lane < f && at < end) o[at] = 0;
+      if (lane == f) o[at] = w + 1;
+      if (stop) break;
+    }
+  }
+}
+
+// A short launch: tiles, then the carries by the CTA that finishes last.
+// ss.done counts the launch's finished CTAs and wraps back to 0 with the last.
+template <class Producer>
+__global__ void __launch_bounds__(kCarryThreads, kCarryMinBlocks)
+    carry_short_kernel(const Producer prod0, uint64_t *out, uint64_t nproc, ScanState ss, const ProductDesc *batch,
+                       uint64_t tpp, uint64_t ws_stride, uint64_t n, bool drop_top) {
+  __shared__ uint64_t s_prev[kCarryThreads][9];
+  __shared__ GP s_warp[kCarryThreads / 32];
+  __shared__ unsigned s_done;
+  carry_body<Producer, kCarryThreads, kShortPer>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, blockIdx.x, s_prev,
+                                                 s_warp);
+  __threadfence();  // this thread's limbs (thread 0: also the aggregate) before the count
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_done = atomicInc(ss.done, gridDim.x - 1);
+    __threadfence();
+  }
+  __syncthreads();
+  if (s_done != gridDim.x - 1) return;
+  fix_all(out, nproc, gridDim.x, ss, drop_top, batch, tpp, n, s_warp, reinterpret_cast<uint32_t *>(&s_prev[0][0]));
 }
 
 __global__ void __launch_bounds__(kFixWarps * 32)
@@ -243,13 +340,19 @@ __global__ void __launch_bounds__(kFixWarps * 32)
                        static_cast<uint64_t>(blockIdx.x) * kFixWarps + (threadIdx.x >> 5));
 }
 
-// The two launches of a carry over `tiles` tiles (a batch: tpp per product).
+// A carry over `tiles` tiles (a batch: tpp per product): one launch where it
+// is short, else the tiles and the fix.
 template <class Producer>
-cudaError_t launch_carry(const Producer &prod, uint64_t *out, uint64_t nproc, uint64_t tiles, const ScanState &ss,
-                         cudaStream_t st, const ProductDesc *batch = nullptr, uint64_t tpp = 0,
+cudaError_t launch_carry(const Producer &prod, uint64_t *out, uint64_t nproc, uint64_t tiles, bool is_short,
+                         const ScanState &ss, cudaStream_t st, const ProductDesc *batch = nullptr, uint64_t tpp = 0,
                          uint64_t ws_stride = 0, uint64_t n = 0) {
   if (tiles == 0) return cudaSuccess;
-  if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
+  if (tiles > 0x7fffffffull || (is_short && tiles > kCarryThreads)) return cudaErrorInvalidValue;
+  if (is_short) {
+    carry_short_kernel<Producer><<<static_cast<unsigned>(tiles), kCarryThreads, 0, st>>>(
+        prod, out, nproc, ss, batch, tpp, ws_stride, n, prod.drop_top());
+    return cudaGetLastError();
+  }
   carry_kernel<Producer><<<static_cast<unsigned>(tiles), kCarryThreads, 0, st>>>(prod, out, nproc, ss, batch, tpp,
                                                                                 ws_stride, n);
   cudaError_t e = cudaGetLastError();
@@ -268,7 +371,12 @@ __global__ void zero_tails_kernel(const ProductDesc *batch, uint64_t N) {
 
 }  // namespace
 
-uint64_t carry_tiles(uint64_t n) { return (n + kCarryTile - 1) / kCarryTile; }
+bool carry_short(uint64_t n, uint64_t nprod) { return (n + kShortTile - 1) / kShortTile * nprod <= kCarryThreads; }
+
+uint64_t carry_tiles(uint64_t n, uint64_t nprod) {
+  const uint64_t tile = carry_short(n, nprod) ? kShortTile : kCarryTile;
+  return (n + tile - 1) / tile;
+}
 
 cudaError_t launch_crt_carry(const uint64_t *res, uint64_t n, const CrtConst &cc, uint64_t *out, uint64_t nout,
                              const ScanState &ss, cudaStream_t st, uint64_t *tiles_used) {
@@ -276,20 +384,22 @@ cudaError_t launch_crt_carry(const uint64_t *res, uint64_t n, const CrtConst &cc
   const uint64_t tiles = carry_tiles(nproc);
   *tiles_used = tiles;
   if (tiles == 0) return cudaSuccess;
-  if (cc.prescaled) return launch_carry(carry::CrtProducerT<false, true>{res, n, cc}, out, nproc, tiles, ss, st);
-  return launch_carry(CrtProducer{res, n, cc}, out, nproc, tiles, ss, st);
+  const bool sh = carry_short(nproc);
+  if (cc.prescaled) return launch_carry(carry::CrtProducerT<false, true>{res, n, cc}, out, nproc, tiles, sh, ss, st);
+  return launch_carry(CrtProducer{res, n, cc}, out, nproc, tiles, sh, ss, st);
 }
 
 cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint64_t n, const CrtConst &cc,
                                    const ProductDesc *batch, uint64_t nprod, const ScanState &ss, cudaStream_t st) {
-  const uint64_t tpp = carry_tiles(n);
+  const uint64_t tpp = carry_tiles(n, nprod);
   const uint64_t tiles = tpp * nprod;
+  const bool sh = carry_short(n, nprod);
   if (tiles == 0) return cudaSuccess;
   if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
   if (cc.prescaled)
-    return launch_carry(carry::CrtProducerT<false, true>{res, n, cc}, nullptr, 0, tiles, ss, st, batch, tpp, ws_stride,
-                        n);
-  return launch_carry(CrtProducer{res, n, cc}, nullptr, 0, tiles, ss, st, batch, tpp, ws_stride, n);
+    return launch_carry(carry::CrtProducerT<false, true>{res, n, cc}, nullptr, 0, tiles, sh, ss, st, batch, tpp,
+                        ws_stride, n);
+  return launch_carry(CrtProducer{res, n, cc}, nullptr, 0, tiles, sh, ss, st, batch, tpp, ws_stride, n);
 }
 
 cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, int logN, uint64_t chunk,
@@ -303,9 +413,9 @@ cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, int
   if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
   if (cc.prescaled)
     return launch_carry(ChunkProducerT<carry::CrtProducerT<false, true>>{{res, n, cc}, ws_stride, chunk, nchunks}, out,
-                        nproc, tiles, ss, st);
+                        nproc, tiles, carry_short(nproc), ss, st);
   return launch_carry(ChunkProducerT<CrtProducer>{CrtProducer{res, n, cc}, ws_stride, chunk, nchunks}, out, nproc,
-                      tiles, ss, st);
+                      tiles, carry_short(nproc), ss, st);
 }
 
 cudaError_t launch_large_sum(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t *b, uint64_t nb, int64_t sb,
@@ -323,7 +433,7 @@ cudaError_t launch_large_sum(const uint64_t *a, uint64_t na, int64_t sa, const u
     top_diff_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(a, na, b, nb, n, top);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  cudaError_t e = launch_carry(prod, out, nproc, tiles, ss, st);
+  cudaError_t e = launch_carry(prod, out, nproc, tiles, carry_short(nproc), ss, st);
   if (e != cudaSuccess) return e;
   sum_finish_kernel<<<1, 256, 0, st>>>(out, nproc, prod, sa, sb, result);
   return cudaGetLastError();
@@ -342,7 +452,7 @@ cudaError_t launch_schoolboy_carry(const uint64_t *x, uint64_t nx, const uint64_
   const uint64_t tiles = carry_tiles(nproc);
   *tiles_used = tiles;
   if (tiles == 0) return cudaSuccess;
-  return launch_carry(ConvProducer{x, nx, y, ny, 0}, out, nproc, tiles, ss, st);
+  return launch_carry(ConvProducer{x, nx, y, ny, 0}, out, nproc, tiles, carry_short(nproc), ss, st);
 }
 
 cudaError_t launch_digit_carry(const uint64_t *x, uint64_t nx, uint64_t d, uint64_t *out, uint64_t nout,
@@ -351,7 +461,7 @@ cudaError_t launch_digit_carry(const uint64_t *x, uint64_t nx, uint64_t d, uint6
   const uint64_t tiles = carry_tiles(nproc);
   *tiles_used = tiles;
   if (tiles == 0) return cudaSuccess;
-  return launch_carry(ConvProducer{x, nx, nullptr, 1, d}, out, nproc, tiles, ss, st);
+  return launch_carry(ConvProducer{x, nx, nullptr, 1, d}, out, nproc, tiles, carry_short(nproc), ss, st);
 }
 
 #if HG_CHECKED

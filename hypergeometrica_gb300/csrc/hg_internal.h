@@ -139,10 +139,9 @@ struct CrtConst {
   uint32_t pad;
 };
 
-// Carry launch state: tile tickets and the tiles' published aggregates.
+// Carry launch state: the finished-tile count and the tiles' published aggregates.
 struct ScanState {
-  unsigned long long *ticket;  // monotonically increasing tile ticket
-  unsigned long long ticket_base;
+  unsigned *done;              // 0 before and after every launch (launches sharing it are ordered)
   unsigned long long *flags;   // one word per tile
   uint32_t epoch;              // distinguishes launches sharing `flags`
   int *err;                    // device error word
@@ -197,8 +196,10 @@ cudaError_t launch_scale(uint64_t *a, uint64_t n, uint64_t mont_factor, PrimeCon
 cudaError_t launch_pass_twiddles(uint64_t *out, int logM, int logR, bool inverse, const NttTables *tb,
                                  const PrimeConst *pc, int nprimes, cudaStream_t st, const uint64_t *scale = nullptr);
 
-// Tiles a carry-scan launch over n positions uses.
-uint64_t carry_tiles(uint64_t n);
+// Tiles per product that a carry over nprod products of n positions uses, and
+// whether it is one launch (short) or two.
+uint64_t carry_tiles(uint64_t n, uint64_t nprod = 1);
+bool carry_short(uint64_t n, uint64_t nprod = 1);
 
 #if HG_CHECKED
 // The fault word of each translation unit with kernels (checked builds),

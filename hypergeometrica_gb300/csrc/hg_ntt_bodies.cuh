@@ -189,15 +189,26 @@ __device__ __forceinline__ void round_g(uint64_t (&v)[16], const ulonglong2 *tw,
 // before them (wait) keeps the writes from overtaking threads that still
 // read the buffer's last exchange, and is left out where no thread has read
 // the buffer since the last barrier the whole CTA passed.
-template <int T, int g, int h>
+//
+// BAR: the threads that take part (a whole number of warps), where the rest
+// of the CTA does not; 0 for the whole CTA.
+template <int BAR>
+__device__ __forceinline__ void block_barrier() {
+  if constexpr (BAR == 0)
+    __syncthreads();
+  else
+    asm volatile("bar.sync 1, %0;" ::"n"(BAR) : "memory");
+}
+
+template <int T, int g, int h, int BAR = 0>
 __device__ __forceinline__ void regroup(uint64_t (&v)[16], uint64_t *sm, uint32_t &xt, uint32_t tid,
                                         bool wait = true) {
   using Gr = Groups<T>;
   constexpr int Ag = Gr::template A<g>(), Ah = Gr::template A<h>();
   if constexpr (Ag == Ah) return;
-  if (wait) __syncthreads();
+  if (wait) block_barrier<BAR>();
   to_smem<Ag, true>(sm, v, xt);
-  __syncthreads();
+  block_barrier<BAR>();
   xt = thread_base<Ah>(tid);
   from_smem<Ah, true>(v, sm, xt);
 }
@@ -234,17 +245,17 @@ __device__ __forceinline__ void forward_rounds(uint64_t (&v)[16], Exchanges x, c
 
 // All inverse rounds, from group 0 up to the top group.  CANON_IN: the
 // residues come from the pointwise product, in [0, p).
-template <int T, bool CANON_IN = false>
+template <int T, bool CANON_IN = false, int BAR = 0>
 __device__ __forceinline__ void inverse_rounds(uint64_t (&v)[16], Exchanges x, const ulonglong2 *tw, uint32_t &xt,
                                                uint32_t tid, uint64_t p, uint32_t c) {
   constexpr int G = Groups<T>::G;
   round_g<T, 0, true, CANON_IN>(v, tw, xt, p, c);
   if constexpr (G >= 2) {
-    regroup<T, 0, 1>(v, x.sm1, xt, tid, x.wait1);
+    regroup<T, 0, 1, BAR>(v, x.sm1, xt, tid, x.wait1);
     round_g<T, 1, true>(v, tw, xt, p, c);
   }
   if constexpr (G == 3) {
-    regroup<T, 1, 2>(v, x.sm2, xt, tid, x.wait2);
+    regroup<T, 1, 2, BAR>(v, x.sm2, xt, tid, x.wait2);
     round_g<T, 2, true>(v, tw, xt, p, c);
   }
 }
