@@ -235,6 +235,7 @@ __global__ void __launch_bounds__(kCarryThreads, kCarryMinBlocks)
                  const ProductDesc *batch, uint64_t tpp, uint64_t ws_stride, uint64_t n) {
   __shared__ uint64_t s_prev[kCarryThreads][9];
   __shared__ GP s_warp[kCarryThreads / 32];
+  pdl_wait();
   carry_body<Producer, kCarryThreads>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, blockIdx.x, s_prev, s_warp);
 }
 
@@ -320,6 +321,7 @@ __global__ void __launch_bounds__(kCarryThreads, kCarryMinBlocks)
   __shared__ uint64_t s_prev[kCarryThreads][9];
   __shared__ GP s_warp[kCarryThreads / 32];
   __shared__ unsigned s_done;
+  pdl_wait();
   carry_body<Producer, kCarryThreads, kShortPer>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, blockIdx.x, s_prev,
                                                  s_warp);
   __threadfence();  // this thread's limbs (thread 0: also the aggregate) before the count
@@ -336,6 +338,7 @@ __global__ void __launch_bounds__(kCarryThreads, kCarryMinBlocks)
 __global__ void __launch_bounds__(kFixWarps * 32)
     carry_fix_kernel(uint64_t *out, uint64_t nproc, uint64_t tiles, ScanState ss, bool drop_top,
                      const ProductDesc *batch, uint64_t tpp, uint64_t n) {
+  pdl_wait();
   fix_body<kCarryTile>(out, nproc, tiles, ss, drop_top, batch, tpp, n,
                        static_cast<uint64_t>(blockIdx.x) * kFixWarps + (threadIdx.x >> 5));
 }
@@ -348,19 +351,16 @@ cudaError_t launch_carry(const Producer &prod, uint64_t *out, uint64_t nproc, ui
                          uint64_t ws_stride = 0, uint64_t n = 0) {
   if (tiles == 0) return cudaSuccess;
   if (tiles > 0x7fffffffull || (is_short && tiles > kCarryThreads)) return cudaErrorInvalidValue;
-  if (is_short) {
-    carry_short_kernel<Producer><<<static_cast<unsigned>(tiles), kCarryThreads, 0, st>>>(
-        prod, out, nproc, ss, batch, tpp, ws_stride, n, prod.drop_top());
-    return cudaGetLastError();
-  }
-  carry_kernel<Producer><<<static_cast<unsigned>(tiles), kCarryThreads, 0, st>>>(prod, out, nproc, ss, batch, tpp,
-                                                                                ws_stride, n);
-  cudaError_t e = cudaGetLastError();
+  const dim3 grid(static_cast<unsigned>(tiles));
+  if (is_short)
+    return launch_dep(carry_short_kernel<Producer>, grid, kCarryThreads, 0, st, prod, out, nproc, ss, batch, tpp,
+                      ws_stride, n, prod.drop_top());
+  cudaError_t e = launch_dep(carry_kernel<Producer>, grid, kCarryThreads, 0, st, prod, out, nproc, ss, batch, tpp,
+                             ws_stride, n);
   if (e != cudaSuccess) return e;
   const uint64_t blocks = (tiles + kFixWarps - 1) / kFixWarps;
-  carry_fix_kernel<<<static_cast<unsigned>(blocks), kFixWarps * 32, 0, st>>>(out, nproc, tiles, ss, prod.drop_top(),
-                                                                             batch, tpp, n);
-  return cudaGetLastError();
+  return launch_dep(carry_fix_kernel, dim3(static_cast<unsigned>(blocks)), kFixWarps * 32, 0, st, out, nproc, tiles,
+                    ss, prod.drop_top(), batch, tpp, n);
 }
 
 // out[N, nout) = 0 for product blockIdx.x.

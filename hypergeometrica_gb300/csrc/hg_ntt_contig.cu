@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(kTileThreads, contig_min_blocks(T)) ntt_contig
   extern __shared__ uint64_t smem[];
   const uint64_t bx = blockIdx.x;
   const int by = static_cast<int>(blockIdx.y);
+  pdl_wait();
 #include "hg_contig_body.inc"
 }
 
@@ -62,6 +63,7 @@ __global__ void __launch_bounds__(MODE == kMul ? 2 << (T - 4) : 1 << (T - 4)) nt
   const uint64_t poff = prod * P.ws_stride + static_cast<uint64_t>(prime - P.prime_lo) * P.prime_stride;
   const uint64_t base = tile << T;
   uint64_t *sm = smem + (op << T);
+  pdl_wait();
   uint64_t nl = 0;
   const uint64_t *limbs = MODE == kInv ? nullptr : pass_limbs(P, prod, op, nl);
   uint64_t v[16];
@@ -102,6 +104,7 @@ __global__ void __launch_bounds__(MODE == kMul ? 2 << (T - 4) : 1 << (T - 4)) nt
 }
 
 __global__ void ntt_tiny_kernel(const PassArgs P, int mode) {
+  pdl_wait();
   tiny_body(P, mode, blockIdx.x, static_cast<int>(blockIdx.y));
 }
 
@@ -131,8 +134,7 @@ cudaError_t launch_tm(const PassArgs &a, uint64_t nblk, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     raised = true;
   }
-  ntt_contig_kernel<T, MODE><<<grid, kTileThreads, bytes, st>>>(a);
-  return cudaGetLastError();
+  return launch_dep(ntt_contig_kernel<T, MODE>, grid, kTileThreads, bytes, st, a);
 }
 
 template <int T, int MODE>
@@ -145,9 +147,9 @@ cudaError_t launch_small(const PassArgs &a, uint64_t nblk, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     raised = true;
   }
-  ntt_contig_small_kernel<T, MODE><<<dim3(static_cast<unsigned>(nblk), static_cast<unsigned>(a.nprimes)),
-                                     (MODE == kMul ? 2 : 1) << (T - 4), bytes, st>>>(a);
-  return cudaGetLastError();
+  return launch_dep(ntt_contig_small_kernel<T, MODE>,
+                    dim3(static_cast<unsigned>(nblk), static_cast<unsigned>(a.nprimes)),
+                    (MODE == kMul ? 2 : 1) << (T - 4), bytes, st, a);
 }
 
 template <int MODE>
@@ -186,8 +188,8 @@ cudaError_t launch_ntt_contig(const PassArgs &a, int mode, cudaStream_t st) {
     return cudaErrorInvalidValue;
   if (a.logT < 4) {
     if (mode == kMulSpec || a.logT < 1 || a.logT != a.logN || a.tiles != 1 || a.nprod > 0x7fffffffull) return cudaErrorInvalidValue;
-    ntt_tiny_kernel<<<dim3(static_cast<unsigned>(a.nprod), static_cast<unsigned>(a.nprimes)), 1, 0, st>>>(a, mode);
-    return cudaGetLastError();
+    return launch_dep(ntt_tiny_kernel, dim3(static_cast<unsigned>(a.nprod), static_cast<unsigned>(a.nprimes)), 1, 0,
+                      st, a, mode);
   }
   switch (mode) {
     case kFwd: return launch_mode<kFwd>(a, nblk, st);

@@ -54,6 +54,7 @@ template <int LOGR, bool INV, bool CUT = false>
 __global__ void __launch_bounds__(kTileThreads, 4) ntt_strided_kernel(const PassArgs P) {
   __shared__ ulonglong2 tw[1 << (LOGR - 1)];
   __shared__ uint64_t sm[LOGR > 4 ? (1 << kTileBits) : 1];
+  pdl_wait();
   strided_ldg_body<LOGR, INV, CUT>(P, blockIdx.x, tw, sm);
 }
 
@@ -147,14 +148,16 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     const uint32_t row_bytes = kTileBytes >> LOGR;
     tma::mbar_arrive_expect_tx(&bar, (INV ? kRows * row_bytes : kTileBytes) +
                                          (TABLE ? static_cast<uint32_t>(krows) * row_bytes : 0u));
+    if (TABLE) tma::load_3d(twt, &maps.tw, &bar, s0, 0, prime);  // no kernel of the stream writes the tables
+    pdl_wait();
     if constexpr (LIMBS)
       tma::load_2d(tile, &maps.in[op], &bar, s0, blk << LOGR);
     else
       tma::load_5d(tile, &maps.in[op], &bar, s0, 0, blk, prime - P.prime_lo, static_cast<int>(prod));
-    if (TABLE) tma::load_3d(twt, &maps.tw, &bar, s0, 0, prime);
   }
   load_sub_twiddles(tw, INV ? tb.sub_inv : tb.sub_fwd, LOGR, tid, kTileThreads);
   if constexpr (INV && KH < 8) load_sub_twiddles(twf, tb.sub_fwd, LOGR, tid, kTileThreads);
+  if constexpr (LIMBS) pdl_wait();  // a partial row's limbs are read by every thread
   const bool landed = tma::mbar_wait_bounded(&bar, 0);
   if (!__syncthreads_and(landed)) {  // also orders the sub-twiddle table
     if (tid == 0) latch_error(P.err, kDevCopyTimeout);
@@ -335,12 +338,9 @@ __global__ void pass_twiddles_kernel(uint64_t *out, int logM, int logR, bool inv
 template <int LOGR>
 cudaError_t launch_r(const PassArgs &a, bool inverse, unsigned grid, cudaStream_t st) {
   if (inverse)
-    ntt_strided_kernel<LOGR, true><<<grid, kTileThreads, 0, st>>>(a);
-  else if (a.krows < (1 << LOGR))
-    ntt_strided_kernel<LOGR, false, true><<<grid, kTileThreads, 0, st>>>(a);
-  else
-    ntt_strided_kernel<LOGR, false><<<grid, kTileThreads, 0, st>>>(a);
-  return cudaGetLastError();
+    return launch_dep(ntt_strided_kernel<LOGR, true>, grid, kTileThreads, 0, st, a);
+  if (a.krows < (1 << LOGR)) return launch_dep(ntt_strided_kernel<LOGR, false, true>, grid, kTileThreads, 0, st, a);
+  return launch_dep(ntt_strided_kernel<LOGR, false>, grid, kTileThreads, 0, st, a);
 }
 
 // ---- tensor maps ----------------------------------------------------------
@@ -411,8 +411,7 @@ cudaError_t launch_tma_v(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l,
     if (e != cudaSuccess) return e;
     raised = true;
   }
-  ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH><<<grid, kTileThreads, bytes, st>>>(m, a, l);
-  return cudaGetLastError();
+  return launch_dep(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH>, grid, kTileThreads, bytes, st, m, a, l);
 }
 
 template <int LOGR>
