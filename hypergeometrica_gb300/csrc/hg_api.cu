@@ -129,7 +129,7 @@ constexpr int kUploadSlices = 4;
 struct Lane {
   cudaStream_t stream = nullptr;
   DevBuf A, B, X, Y, OUT, flags;
-  DevBuf misc;  // bytes [0, 4) carry-scan finished count, [8, 12) error word (lane 0's is the library's), [16, 24) large-sum top index
+  DevBuf misc;  // bytes [0, 4) carry-scan finished count, [8, 12) error word (lane 0's is the library's), [16, 40) a long sum's SumWords
   uint32_t epoch = 0;
   cudaEvent_t ws_done = nullptr;
   cudaStream_t copy_stream = nullptr;  // host entry points: operand uploads
@@ -365,6 +365,7 @@ int init_locked(const uint64_t *moduli, int k, const uint64_t *roots, int maxlg,
     HG_CUDA(cudaEventCreateWithFlags(&L.d2h_done, cudaEventDisableTiming), "event creation");
     HG_CUDA(L.misc.ensure(64), "scan state allocation");
     HG_CUDA(cudaMemset(L.misc.p, 0, 64), "scan state init");
+    HG_CUDA(cudaMemset(static_cast<char *>(L.misc.p) + 16, 0xff, 2 * sizeof(long long)), "scan state init");
   }
   c.lane = &c.lanes[0];
   c.ready = true;
@@ -605,14 +606,17 @@ void release_pass_twiddles() {
 // pass), forward in order or inverse in reverse order.  scale_last (inverse
 // only): the last inverse pass reads its table multiplied by these
 // Montgomery-form factors, and *scaled says whether it did (it forms its
-// twiddles unscaled when no table can be had).
+// twiddles unscaled when no table can be had).  out_scale (inverse, one
+// prime): the last inverse pass multiplies what it writes by this factor.
 cudaError_t run_strided_range(PassArgs a, const std::vector<PassPlan> &plan, bool inverse, int s0, int s1,
-                              cudaStream_t st, const uint64_t *scale_last = nullptr, bool *scaled = nullptr) {
+                              cudaStream_t st, const uint64_t *scale_last = nullptr, bool *scaled = nullptr,
+                              uint64_t out_scale = 0) {
   const int np = static_cast<int>(plan.size()) - 1;
   for (int s = s0; s < s1 && s < np; ++s) {
     const PassPlan &pp = plan[inverse ? np - 1 - s : s];
     set_strided(a, pp);
     const bool last_inverse = inverse && s == np - 1;
+    a.scale = last_inverse ? out_scale : 0;
     a.ptw = pass_twiddles(pp.logR + pp.logS, pp.logR, inverse, st, last_inverse ? scale_last : nullptr);
     if (last_inverse && scaled) *scaled = scale_last && a.ptw;
     cudaError_t e;
@@ -687,6 +691,7 @@ struct LengthConst {
   std::once_flag once;
   CrtConst crt[2];  // unscaled, prescaled
   uint64_t scale[kPrimes];
+  uint64_t ninv[kPrimes];  // 1/2^L mod p
   bool scalable;
 };
 const LengthConst &length_const(int L) {
@@ -696,6 +701,7 @@ const LengthConst &length_const(int L) {
     t.crt[0] = crt_const_of(L, false);
     t.crt[1] = crt_const_of(L, true);
     t.scalable = prescale_factors_of(L, t.scale);
+    for (int j = 0; j < kPrimes; ++j) t.ninv[j] = invmod_h((uint64_t(1) << L) % g_ctx.moduli[j], g_ctx.moduli[j]);
   });
   return t;
 }
@@ -1392,13 +1398,12 @@ int spectrum(uint64_t *a, size_t n, int mod_num, bool inverse, cudaStream_t st) 
     HG_CUDA(run_strided(pa, plan, false, st), "forward transform");
     HG_CUDA(run_contig(pa, plan.back(), kContigFwd, st), "forward transform");
   } else {
-    HG_CUDA(run_contig(pa, plan.back(), kContigInv, st), "inverse transform");
-    HG_CUDA(run_strided(pa, plan, true, st), "inverse transform");
-  }
-  if (inverse) {
     const uint64_t p = g_ctx.moduli[mod_num];
-    ProfScope ps(HG_KC_OTHER, st, 16.0 * static_cast<double>(n));
-    HG_CUDA(launch_scale(a, n, mont_h(invmod_h(n % p, p), p), g_ctx.pc[mod_num], st), "1/N scaling");
+    const uint64_t f = mont_h(length_const(L).ninv[mod_num], p);  // 1/N
+    const int np = static_cast<int>(plan.size()) - 1;
+    pa.scale = np ? 0 : f;
+    HG_CUDA(run_contig(pa, plan.back(), kContigInv, st), "inverse transform");
+    HG_CUDA(run_strided_range(pa, plan, true, 0, np, st, nullptr, nullptr, f), "inverse transform");
   }
   return HG_OK;
 }
@@ -2009,11 +2014,11 @@ int large_sum_device(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t 
   ScanState ss;
   rc = scan_state(carry_tiles(nproc), &ss);
   if (rc) return rc;
-  long long *top = reinterpret_cast<long long *>(static_cast<char *>(g_ctx.lane->misc.p) + 16);
+  SumWords *words = reinterpret_cast<SumWords *>(static_cast<char *>(g_ctx.lane->misc.p) + 16);
   {
     // (top search,) scan (and fix), sign and size
     ProfScope ps(HG_KC_OTHER, st, 24.0 * static_cast<double>(nproc), (sa != sb ? 3 : 2) + (carry_short(nproc) ? 0 : 1));
-    HG_CUDA(launch_large_sum(a, na, sa, b, nb, sb, out, top, result, ss, st), "large sum");
+    HG_CUDA(launch_large_sum(a, na, sa, b, nb, sb, out, words, result, ss, st), "large sum");
   }
   HG_CUDA(ws_release(st), "workspace ordering");
   return HG_OK;
@@ -2143,6 +2148,7 @@ int hg_shutdown(void) {
   c.lane = &c.lanes[0];
   c.tables.release();
   release_pass_twiddles();
+  lib_release_descs();
   c.ready = false;
   // The scratch array's device address belongs to the module as loaded in
   // the current context: after a context reset the module loads again, so

@@ -188,13 +188,9 @@ struct SumProducer {
   }
 };
 
-// *top = max index i < n with a_i != b_i (the caller set it to -1).
-__global__ void top_diff_kernel(const uint64_t *a, uint64_t na, const uint64_t *b, uint64_t nb, uint64_t n,
-                                long long *top) {
-  long long best = -1;
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
-    if ((i < na ? a[i] : 0) != (i < nb ? b[i] : 0)) best = static_cast<long long>(i);
+// The highest index (or -1) found by a grid: each warp's best goes to *top,
+// which was -1.
+__device__ __forceinline__ void grid_max(long long best, long long *top) {
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
     const long long o = __shfl_down_sync(0xffffffffu, best, d);
@@ -203,29 +199,43 @@ __global__ void top_diff_kernel(const uint64_t *a, uint64_t na, const uint64_t *
   if ((threadIdx.x & 31) == 0 && best >= 0) atomicMax(top, best);
 }
 
-// result = (sign, size) of out[0, nproc): the highest nonzero limb, scanned
-// from the top 2048 limbs at a time by one CTA.
+// *top = max index i < n with a_i != b_i.
+__global__ void top_diff_kernel(const uint64_t *a, uint64_t na, const uint64_t *b, uint64_t nb, uint64_t n,
+                                long long *top) {
+  pdl_wait();
+  long long best = -1;
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
+    if ((i < na ? a[i] : 0) != (i < nb ? b[i] : 0)) best = static_cast<long long>(i);
+  grid_max(best, top);
+}
+
+// result = (sign, size) of out[0, nproc): the highest nonzero limb, searched by
+// the whole grid (a difference may have many zero limbs at its top: one CTA
+// that searched them from the top took 24 us for 2^16-limb Newton residuals).
+// The CTA that finishes last writes the result and leaves the search words
+// and its own count as the next sum expects them.
 __global__ void sum_finish_kernel(const uint64_t *out, uint64_t nproc, SumProducer prod, int64_t sa, int64_t sb,
-                                  int64_t *result) {
-  __shared__ long long s_top;
-  if (threadIdx.x == 0) s_top = -1;
+                                  int64_t *result, SumWords *w) {
+  __shared__ unsigned s_done;
+  pdl_wait();
+  long long best = -1;
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < nproc; i += stride)
+    if (out[i]) best = static_cast<long long>(i);
+  grid_max(best, &w->top_out);
+  __threadfence();
   __syncthreads();
-  for (uint64_t hi = nproc; hi > 0;) {
-    const uint64_t lo = hi > 2048 ? hi - 2048 : 0;
-    for (uint64_t i = lo + threadIdx.x; i < hi; i += blockDim.x)
-      if (out[i]) atomicMax(&s_top, static_cast<long long>(i));
-    __syncthreads();
-    const bool found = s_top >= 0;  // read by all before any update for the next chunk
-    __syncthreads();
-    if (found) break;
-    hi = lo;
-  }
-  if (threadIdx.x == 0) {
-    const int64_t size = s_top + 1;
-    const int64_t sign = prod.a_larger() ? sa : sb;
-    result[0] = size ? sign : 1;
-    result[1] = size;
-  }
+  if (threadIdx.x == 0) s_done = atomicInc(&w->done, gridDim.x - 1);
+  __syncthreads();
+  if (s_done != gridDim.x - 1 || threadIdx.x != 0) return;
+  __threadfence();
+  const int64_t size = *static_cast<volatile long long *>(&w->top_out) + 1;
+  const int64_t sign = prod.a_larger() ? sa : sb;
+  result[0] = size ? sign : 1;
+  result[1] = size;
+  w->top_out = -1;
+  w->top_diff = -1;
 }
 
 // One tile per CTA.
@@ -363,6 +373,61 @@ cudaError_t launch_carry(const Producer &prod, uint64_t *out, uint64_t nproc, ui
                     ss, prod.drop_top(), batch, tpp, n);
 }
 
+// A schoolboy product of at most kSchoolMax limbs, whole, in one CTA: one
+// thread per position, the operands in shared memory.  The general kernel
+// above gives such a product a handful of threads with four positions each
+// and reads the operands from global memory: 64 x 48 limbs took 25 us (eight
+// positions a thread; four: the whole host call 57.5 us, with this kernel 46.9).
+constexpr uint32_t kSchoolMax = 1024;
+
+__global__ void __launch_bounds__(kSchoolMax)
+    school_kernel(const uint64_t *x, uint32_t nx, const uint64_t *y, uint32_t ny, uint64_t *out, uint32_t n, int *err) {
+  __shared__ uint64_t s_x[kSchoolMax], s_y[kSchoolMax];  // then words 1 and 2 of the columns
+  __shared__ GP s_warp[32];
+  __shared__ uint32_t s_h[32];
+  const uint32_t i = threadIdx.x, lane = i & 31, wid = i >> 5;
+  pdl_wait();
+  if (i < nx) s_x[i] = x[i];
+  if (i < ny) s_y[i] = y[i];
+  __syncthreads();
+  V3 v{0, 0, 0};
+  if (i < n) {
+    const uint32_t jlo = i >= nx ? i - nx + 1 : 0, jhi = i < ny ? i + 1 : ny;
+#pragma unroll 4
+    for (uint32_t j = jlo; j < jhi; ++j) {
+      const uint64_t a = s_x[i - j], b = s_y[j];
+      add128_to(v, a * b, __umul64hi(a, b));
+    }
+  }
+  __syncthreads();
+  s_x[i] = v.w1;
+  s_y[i] = v.w2;
+  __syncthreads();
+  // W_i = v0_i + v1_(i-1) + v2_(i-2) = wl + wh 2^64, A_i = wl_i + wh_(i-1), as in carry_body.
+  const uint64_t u1 = i >= 1 ? s_x[i - 1] : 0, u2 = i >= 2 ? s_y[i - 2] : 0;
+  uint64_t wl = v.w0 + u1;
+  uint32_t wh = wl < u1;
+  wl += u2;
+  wh += wl < u2;
+  if (lane == 31) s_h[wid] = wh;
+  uint32_t whp = __shfl_up_sync(0xffffffffu, wh, 1);
+  __syncthreads();
+  if (lane == 0) whp = wid ? s_h[wid - 1] : 0;
+  const uint64_t A = wl + whp;
+  const uint32_t G = __ballot_sync(0xffffffffu, A < whp), P = __ballot_sync(0xffffffffu, A == ~0ull);
+  if (lane == 0) {  // the warp's carry out: with carry-in 0, and whether it passes one on
+    const uint64_t c0 = (static_cast<uint64_t>(G) << 1) + P;
+    s_warp[wid] = GP{static_cast<uint32_t>(c0 >> 32), P == 0xffffffffu ? 1u : 0u};
+  }
+  __syncthreads();
+  GP below{0, 0};
+  for (uint32_t w = 0; w < wid; ++w) below = gp_compose(below, s_warp[w]);
+  const uint64_t sum = ((static_cast<uint64_t>(G) << 1) | below.g) + P;
+  const uint32_t c = static_cast<uint32_t>((sum ^ P) >> lane) & 1u;
+  if (i < n) out[i] = A + c;
+  if (i == n - 1 && ((A < whp) || (A == ~0ull && c))) latch_error(err, kDevCarryOverflow);
+}
+
 // out[N, nout) = 0 for product blockIdx.x.
 __global__ void zero_tails_kernel(const ProductDesc *batch, uint64_t N) {
   const ProductDesc d = batch[blockIdx.x];
@@ -419,24 +484,19 @@ cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, int
 }
 
 cudaError_t launch_large_sum(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t *b, uint64_t nb, int64_t sb,
-                             uint64_t *out, long long *top, int64_t *result, const ScanState &ss, cudaStream_t st) {
+                             uint64_t *out, SumWords *words, int64_t *result, const ScanState &ss, cudaStream_t st) {
   const uint64_t n = na > nb ? na : nb;
   const bool sub = sa != sb;
   const uint64_t nproc = sub ? n : n + 1;
   const uint64_t tiles = carry_tiles(nproc);
   if (tiles == 0 || tiles > 0x7fffffffull) return cudaErrorInvalidValue;
-  SumProducer prod{a, b, na, nb, n, sub ? top : nullptr};
-  if (sub) {
-    cudaError_t e = cudaMemsetAsync(top, 0xff, sizeof(long long), st);
-    if (e != cudaSuccess) return e;
-    const uint64_t blocks = (n + 255) / 256 < 152 * 8 ? (n + 255) / 256 : 152 * 8;
-    top_diff_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(a, na, b, nb, n, top);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
-  cudaError_t e = launch_carry(prod, out, nproc, tiles, carry_short(nproc), ss, st);
-  if (e != cudaSuccess) return e;
-  sum_finish_kernel<<<1, 256, 0, st>>>(out, nproc, prod, sa, sb, result);
-  return cudaGetLastError();
+  const SumProducer prod{a, b, na, nb, n, sub ? &words->top_diff : nullptr};
+  const auto grid = [](uint64_t m) { return dim3(static_cast<unsigned>(m < 152 * 4 * 1024 ? (m + 1023) / 1024 : 152 * 4)); };
+  cudaError_t e = cudaSuccess;
+  if (sub) e = launch_dep(top_diff_kernel, grid(n), 256, 0, st, a, na, b, nb, n, &words->top_diff);
+  if (e == cudaSuccess) e = launch_carry(prod, out, nproc, tiles, carry_short(nproc), ss, st);
+  if (e == cudaSuccess) e = launch_dep(sum_finish_kernel, grid(nproc), 256, 0, st, out, nproc, prod, sa, sb, result, words);
+  return e;
 }
 
 cudaError_t launch_zero_tails(const ProductDesc *batch, uint64_t nprod, uint64_t N, cudaStream_t st) {
@@ -452,6 +512,10 @@ cudaError_t launch_schoolboy_carry(const uint64_t *x, uint64_t nx, const uint64_
   const uint64_t tiles = carry_tiles(nproc);
   *tiles_used = tiles;
   if (tiles == 0) return cudaSuccess;
+  if (nproc == nx + ny && nproc <= kSchoolMax)
+    return launch_dep(school_kernel, dim3(1), static_cast<unsigned>((nproc + 31) & ~uint64_t(31)), 0, st, x,
+                      static_cast<uint32_t>(nx), y, static_cast<uint32_t>(ny), out, static_cast<uint32_t>(nproc),
+                      ss.err);
   return launch_carry(ConvProducer{x, nx, y, ny, 0}, out, nproc, tiles, carry_short(nproc), ss, st);
 }
 

@@ -64,6 +64,9 @@ int large_sum_device(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t 
 // products, run every group.  Takes no lock and allocates nothing.
 int enqueue_batch(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st);
 
+// Give back the descriptor memory that hg_sum.cu keeps (hg_shutdown).
+void lib_release_descs();
+
 // The library's state, for code outside hg_api.cu.
 std::recursive_mutex &lib_mutex();
 bool lib_ready();

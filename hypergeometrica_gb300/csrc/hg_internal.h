@@ -102,6 +102,10 @@ struct PassArgs {
   // (M, R, direction), Montgomery form, [prime][r][s] with M words per prime
   // (all primes of the scheme), or null to form them from tb.
   const uint64_t *ptw;
+  // Spectrum entry point: the transform's last inverse pass (strided or
+  // contiguous) multiplies every residue by this Montgomery-form factor, which
+  // leaves it in [0, p); 0 elsewhere (one prime per launch).
+  uint64_t scale;
   int *err;                    // device error word (a tile copy that did not land)
 };
 
@@ -210,11 +214,18 @@ cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint
 cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, int logN, uint64_t chunk,
                                     uint64_t nchunks, const CrtConst &cc, uint64_t *out, uint64_t nproc,
                                     const ScanState &ss, cudaStream_t st, uint64_t *tiles_used);
+// Search words of a long sum, in device memory: -1, -1 and 0 before and after
+// every sum (sums that share them are ordered).
+struct SumWords {
+  long long top_diff;  // highest limb where the operands differ
+  long long top_out;   // highest nonzero limb of the result
+  unsigned done;
+};
 // sa |a| + sb |b| into out[0, n + 1) (n = max(na, nb); out[0, n) when the
 // signs differ) over the whole GPU, with the carry scan of the products;
-// result = (sign, size).  top is one device word of scratch.
+// result = (sign, size).
 cudaError_t launch_large_sum(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t *b, uint64_t nb, int64_t sb,
-                             uint64_t *out, long long *top, int64_t *result, const ScanState &ss, cudaStream_t st);
+                             uint64_t *out, SumWords *words, int64_t *result, const ScanState &ss, cudaStream_t st);
 // Zero out[N, nout) of every product (out[0, nout) when N == 0), N the
 // residues per prime.
 cudaError_t launch_zero_tails(const ProductDesc *batch, uint64_t nprod, uint64_t N, cudaStream_t st);
@@ -222,8 +233,6 @@ cudaError_t launch_schoolboy_carry(const uint64_t *x, uint64_t nx, const uint64_
                                    uint64_t nout, const ScanState &ss, cudaStream_t st, uint64_t *tiles_used);
 cudaError_t launch_digit_carry(const uint64_t *x, uint64_t nx, uint64_t d, uint64_t *out, uint64_t nout,
                                const ScanState &ss, cudaStream_t st, uint64_t *tiles_used);
-cudaError_t launch_scale(uint64_t *a, uint64_t n, uint64_t mont_factor, PrimeConst pc, cudaStream_t st);
-
 // Fill out[j * M + r * S + s] = w_M^(+-s * bitrev_R(r)) (Montgomery form) for
 // the primes j = 0 .. nprimes - 1 of tb, M = 2^logM, R = 2^logR, S = M / R.
 cudaError_t launch_pass_twiddles(uint64_t *out, int logM, int logR, bool inverse, const NttTables *tb,

@@ -22,8 +22,8 @@ constexpr int kFwd = 0, kInv = 1, kMul = 2, kSqr = 3, kMulSpec = 4;
 // per-thread global loads and stores; tw holds 2^(LOGR-1) (twiddle,
 // companion) pairs and sm 4096 words of shared memory.  The pass that reads
 // and reduces limbs from batch descriptors or chunks runs here.
-// CUT (forward only): the outer pass of a truncated transform, which keeps
-// P.krows rows.
+// CUT: forward, the outer pass of a truncated transform, which keeps P.krows
+// rows; inverse, a transform's last pass that scales by P.scale.
 template <int LOGR, bool INV, bool CUT = false>
 __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid, ulonglong2 *tw, uint64_t *sm) {
   constexpr int T = kTileBits;
@@ -154,7 +154,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     for (int i = 0; i < 16; ++i) {
       const uint64_t o = off + i * step;
       check_below(v[i], 2 * p);
-      if (check_index(o, P.points)) data[o] = v[i];
+      if (check_index(o, P.points)) data[o] = CUT ? mont_mul(v[i], P.scale, p, c) : v[i];
     }
   }
 }
@@ -285,6 +285,12 @@ __device__ __forceinline__ void zero16(uint64_t (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = 0;
 }
 
+// v <- v f (Montgomery-form f), in [0, p).
+__device__ __forceinline__ void scale16(uint64_t (&v)[16], uint64_t f, uint64_t p, uint32_t c) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = mont_mul(v[i], f, p, c);
+}
+
 template <int A>
 __device__ __forceinline__ void store_block(const uint64_t (&v)[16], uint64_t *data, uint64_t base, uint32_t xt,
                                             uint64_t bound = ~0ull) {
@@ -353,7 +359,7 @@ __device__ __forceinline__ void tiny_body(const PassArgs &P, int mode, uint64_t 
       }
     }
   }
-  for (int i = 0; i < n; ++i) P.data[0][poff + i] = a[0][i];
+  for (int i = 0; i < n; ++i) P.data[0][poff + i] = P.scale ? mont_mul(a[0][i], P.scale, p, c) : a[0][i];
 }
 
 }  // namespace bodies

@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(MODE == kMul ? 2 << (T - 4) : 1 << (T - 4)) nt
     xt = thread_base<A0>(lt);
     load_block<A0>(v, P.data[0] + poff, nullptr, 0, base, xt, p, 2 * p);
     inverse_rounds<T>(v, through(sm), swz_table(tb, T, true), xt, lt, p, c);
+    if (P.scale) scale16(v, P.scale, p, c);
     store_block<ATOP>(v, P.data[0] + poff, base, xt, 2 * p);
     return;
   } else {
@@ -106,12 +107,6 @@ __global__ void __launch_bounds__(MODE == kMul ? 2 << (T - 4) : 1 << (T - 4)) nt
 __global__ void ntt_tiny_kernel(const PassArgs P, int mode) {
   pdl_wait();
   tiny_body(P, mode, blockIdx.x, static_cast<int>(blockIdx.y));
-}
-
-__global__ void scale_kernel(uint64_t *a, uint64_t n, uint64_t f, uint64_t p, uint32_t c) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-    a[i] = mont_mul(a[i], f, p, c);
 }
 
 // Two CTAs of 4096 residues per SM: up to there the small kernel's spread is
@@ -199,15 +194,6 @@ cudaError_t launch_ntt_contig(const PassArgs &a, int mode, cudaStream_t st) {
     case kMulSpec: return launch_mode<kMulSpec>(a, nblk, st);
     default: return cudaErrorInvalidValue;
   }
-}
-
-cudaError_t launch_scale(uint64_t *a, uint64_t n, uint64_t f, PrimeConst pc, cudaStream_t st) {
-  const int threads = 256;
-  uint64_t blocks = (n + threads - 1) / threads;
-  if (blocks > 152ull * 16) blocks = 152ull * 16;
-  if (blocks == 0) return cudaSuccess;
-  scale_kernel<<<static_cast<unsigned>(blocks), threads, 0, st>>>(a, n, f, pc.p, pc.c);
-  return cudaGetLastError();
 }
 
 }  // namespace hg

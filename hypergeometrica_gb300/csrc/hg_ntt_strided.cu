@@ -98,7 +98,11 @@ struct TmaLimbs {
 // P.krows, and threads whose 16 rows are all dropped stop after the exchange
 // (R > 16).  A whole transform's passes are instances of their own: taking the
 // rows from P.krows there made the 2^25-point product 2% slower.
-template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KH>
+//
+// SCALE (inverse only): the last pass of the spectrum entry point, which
+// multiplies every residue by P.scale as it leaves (a launch and a pass over
+// memory less: 2^20 points there and back 67.4 -> 61.0 us).
+template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KH, bool SCALE>
 __global__ void __launch_bounds__(kTileThreads, 4)
     ntt_strided_tma_kernel(const __grid_constant__ TmaMaps maps, const PassArgs P, const TmaLimbs L) {
   constexpr int T = kTileBits;
@@ -298,6 +302,10 @@ __global__ void __launch_bounds__(kTileThreads, 4)
           top.template run<3, 1, KI, 0, true>(v);
       }
     }
+    if constexpr (SCALE) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = mont_mul(v[i], P.scale, p, c);
+    }
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < NK1; ++i) {
@@ -337,6 +345,7 @@ __global__ void pass_twiddles_kernel(uint64_t *out, int logM, int logR, bool inv
 
 template <int LOGR>
 cudaError_t launch_r(const PassArgs &a, bool inverse, unsigned grid, cudaStream_t st) {
+  if (inverse && a.scale) return launch_dep(ntt_strided_kernel<LOGR, true, true>, grid, kTileThreads, 0, st, a);
   if (inverse)
     return launch_dep(ntt_strided_kernel<LOGR, true>, grid, kTileThreads, 0, st, a);
   if (a.krows < (1 << LOGR)) return launch_dep(ntt_strided_kernel<LOGR, false, true>, grid, kTileThreads, 0, st, a);
@@ -399,19 +408,20 @@ cudaError_t twiddle_map(CUtensorMap *m, const uint64_t *ptw, const PassArgs &a) 
   return encode(m, ptw, 3, dims, strides, box);
 }
 
-template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KH = 8>
+template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KH = 8, bool SCALE = false>
 cudaError_t launch_tma_v(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l, unsigned grid, cudaStream_t st) {
   constexpr size_t bytes = (TABLE ? 2 : 1) * (size_t(1) << kTileBits) * sizeof(uint64_t);
   // Raise the dynamic shared-memory limit once per instantiation (not on
   // every launch, so that launches can be captured in a CUDA graph).
   static bool raised = false;
   if (bytes > 48 * 1024 && !raised) {
-    cudaError_t e = cudaFuncSetAttribute(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH>,
+    cudaError_t e = cudaFuncSetAttribute(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH, SCALE>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e != cudaSuccess) return e;
     raised = true;
   }
-  return launch_dep(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH>, grid, kTileThreads, bytes, st, m, a, l);
+  return launch_dep(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH, SCALE>, grid, kTileThreads, bytes, st, m, a,
+                    l);
 }
 
 template <int LOGR>
@@ -435,6 +445,9 @@ cudaError_t launch_tma_r(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l,
     }
     return cudaErrorInvalidValue;
   }
+  if (inverse && a.scale)
+    return table ? launch_tma_v<LOGR, true, true, false, 8, true>(m, a, l, grid, st)
+                 : launch_tma_v<LOGR, true, false, false, 8, true>(m, a, l, grid, st);
   if (inverse)
     return table ? launch_tma_v<LOGR, true, true, false>(m, a, l, grid, st)
                  : launch_tma_v<LOGR, true, false, false>(m, a, l, grid, st);

@@ -36,8 +36,10 @@ struct SumDesc {
 };
 
 // Sums of at least this many limbs run over the whole GPU (large_sum_device)
-// instead of in one CTA.
+// instead of in one CTA, which takes about 2 us per 2048 limbs; a sum alone
+// in its call has the GPU to itself and goes there earlier.
 constexpr uint64_t kLargeSum = uint64_t(1) << 15;
+constexpr uint64_t kLargeSumAlone = uint64_t(1) << 13;
 
 struct VecDesc {
   const uint64_t *p;
@@ -233,6 +235,31 @@ __global__ void small_mul_kernel(const Descs<ProductDesc> descs, uint64_t n) {
   for (uint64_t i = w; i < d.nout; ++i) d.out[i] = 0;
 }
 
+// Descriptor arrays come from a pool of the library's own that keeps up to
+// kKeptDescs bytes between calls: from the device's default pool, which gives
+// everything back at each synchronisation, an allocation took about 200 us.
+constexpr uint64_t kKeptDescs = uint64_t(64) << 20;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool = nullptr;
+
+cudaError_t desc_alloc(void **p, size_t bytes, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (!g_pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = lib_device();
+    cudaError_t e = cudaMemPoolCreate(&g_pool, &props);
+    if (e != cudaSuccess) {
+      g_pool = nullptr;
+      return e;
+    }
+    uint64_t keep = kKeptDescs;
+    if ((e = cudaMemPoolSetAttribute(g_pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
+  }
+  return cudaMallocFromPoolAsync(p, bytes, g_pool, st);
+}
+
 template <class Desc, class Launch>
 int run_batch(const Desc *host, size_t n, cudaStream_t st, const char *what, Launch launch) {
   if (n == 0) return HG_OK;
@@ -245,7 +272,7 @@ int run_batch(const Desc *host, size_t n, cudaStream_t st, const char *what, Lau
     return e == cudaSuccess ? HG_OK : lib_cuda_fail(e, what);
   }
   Desc *dev = nullptr;
-  cudaError_t e = cudaMallocAsync(&dev, n * sizeof(Desc), st);
+  cudaError_t e = desc_alloc(reinterpret_cast<void **>(&dev), n * sizeof(Desc), st);
   if (e != cudaSuccess) return lib_cuda_fail(e, what);
   e = cudaMemcpyAsync(dev, host, n * sizeof(Desc), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
@@ -261,6 +288,13 @@ int run_batch(const Desc *host, size_t n, cudaStream_t st, const char *what, Lau
 }
 
 }  // namespace
+
+void lib_release_descs() {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (g_pool) cudaMemPoolDestroy(g_pool);
+  g_pool = nullptr;
+}
+
 #if HG_CHECKED
 HG_CHECKED_READER(checked_fault_sum)
 #endif
@@ -287,7 +321,7 @@ int hg_add_batch_device(const hg_sum *sums, size_t n, int64_t *result, void *str
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   for (size_t k = 0; k < n; ++k) {
     const hg_sum &s = sums[k];
-    if ((s.na > s.nb ? s.na : s.nb) >= kLargeSum) {
+    if ((s.na > s.nb ? s.na : s.nb) >= (n == 1 ? kLargeSumAlone : kLargeSum)) {
       const int rc = large_sum_device(s.a, s.na, s.sa, s.b, s.nb, s.sb, s.out, s.nout, result + 2 * k, st);
       if (rc) return rc;
     } else {
