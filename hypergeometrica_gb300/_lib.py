@@ -64,6 +64,13 @@ class HgProduct(ctypes.Structure):
     _fields_ = [("x", _vp), ("nx", _sz), ("y", _vp), ("ny", _sz), ("out", _vp), ("nout", _sz)]
 
 
+class HgSum(ctypes.Structure):
+    """hg_sum: one signed sum of device magnitudes."""
+
+    _fields_ = [("a", _vp), ("na", _sz), ("b", _vp), ("nb", _sz), ("out", _vp), ("nout", _sz), ("sa", ctypes.c_int64),
+                ("sb", ctypes.c_int64)]
+
+
 HG_BATCH_AUTOTUNE = 1
 HG_BATCH_PER_PASS = 2
 HG_BATCH_PERSISTENT = 4
@@ -115,6 +122,9 @@ SIGNATURES = {
     "hg_batch_schedule": (ctypes.c_int, [_vp, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(_sz)]),
     "hg_mul_batch_device": (ctypes.c_int, [ctypes.POINTER(HgProduct), _sz, _vp]),
     "hg_add_batch_device": (ctypes.c_int, [_vp, _sz, _vp, _vp]),
+    "hg_sums_and_sizes": (ctypes.c_int, [_vp, _vp, _vp, _sz, _vp, _vp, _sz, _vp, _vp]),
+    "hg_mul_sized_device": (ctypes.c_int, [_vp, _sz, _vp, _sz, _vp, _sz, ctypes.c_int, _vp, _vp]),
+    "hg_svc_mul": (ctypes.c_int, [_vp, _vp, _vp, _vp]),
     "hg_trim_batch_device": (ctypes.c_int, [_vp, _sz, _vp, _vp]),
     "hg_mul_small_batch_device": (ctypes.c_int, [_vp, _sz, _vp]),
     "hg_series_leaves_device": (ctypes.c_int, [_vp, ctypes.c_uint64, ctypes.c_uint64, _vp, _vp, _vp]),

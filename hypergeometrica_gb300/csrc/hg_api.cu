@@ -119,6 +119,32 @@ struct DevBuf {
   uint64_t *u64() const { return static_cast<uint64_t *>(p); }
 };
 
+// Page-locked host memory that the device addresses too.
+struct HostBuf {
+  void *p = nullptr, *dev = nullptr;
+  size_t bytes = 0;
+  cudaError_t ensure(size_t b) {
+    if (b <= bytes) return cudaSuccess;
+    release();
+    cudaError_t e = cudaHostAlloc(&p, b, cudaHostAllocMapped);
+    if (e != cudaSuccess) {
+      p = nullptr;
+      return e;
+    }
+    if ((e = cudaHostGetDevicePointer(&dev, p, 0)) != cudaSuccess) {
+      release();
+      return e;
+    }
+    bytes = b;
+    return cudaSuccess;
+  }
+  void release() {
+    if (p) cudaFreeHost(p);
+    p = dev = nullptr;
+    bytes = 0;
+  }
+};
+
 // Column slices of an operand upload from host memory (ntt_product_device).
 constexpr int kUploadSlices = 4;
 
@@ -129,6 +155,7 @@ constexpr int kUploadSlices = 4;
 struct Lane {
   cudaStream_t stream = nullptr;
   DevBuf A, B, X, Y, OUT, flags;
+  HostBuf stage;  // short host products: operands, then the result, then the error word
   DevBuf misc;  // bytes [0, 4) carry-scan finished count, [8, 12) error word (lane 0's is the library's), [16, 40) a long sum's SumWords
   uint32_t epoch = 0;
   cudaEvent_t ws_done = nullptr;
@@ -1182,14 +1209,7 @@ int read_device_error(cudaStream_t st) {
     if (rc) return rc;
   }
 #endif
-  if (err) {
-    HG_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), st), "error word reset");
-    HG_CUDA(cudaStreamSynchronize(st), "stream synchronise");
-    if (err == kDevCarryOverflow) return fail(HG_ERR_INCONSISTENT, "a carry left the top of the result storage");
-    if (err == kDevCopyTimeout) return fail(HG_ERR_CUDA, "a tile copy did not complete within its wait limit");
-    return fail(HG_ERR_CUDA, "device error %d", err);
-  }
-  return HG_OK;
+  return lib_device_error(err, st);
 }
 
 // Device address of a page-locked host buffer (cudaHostAlloc, pinned torch
@@ -1205,8 +1225,63 @@ const void *pinned_view(const void *h) {
   return nullptr;
 }
 
+// Page-locked, device-mapped words that kernels write results into and the
+// host reads after a stream synchronisation: taken for one call at a time,
+// kept until hg_shutdown.
+constexpr size_t kWordsBytes = 64;
+std::mutex g_words_mu;
+std::vector<void *> g_words_pages;
+std::vector<HostWords> g_words_free;
+
 // Host-memory wrapper: stage operands, run, copy back, check.
 enum class Kind { Ntt, Square, Schoolboy, Digit };
+
+// Products of up to this many limbs go through one page-locked buffer of the
+// library's: operands copied in by the host, up in one copy (the quadratic
+// kernels read them in place), the result written in place by the last
+// kernel, the error word beside it, one synchronisation.  The general path's
+// copies from and to pageable memory each wait in the driver and its upload
+// slices launch the first pass eight times.  mpz_mul of 64 x 48 limbs 37.9 us
+// that way, 28.3 this way; 3000 x 2500 142.9 and 77.3; 16000 x 16000 260.8 and
+// 146.6; 65536 x 65536 249 and 227, about where they meet.
+constexpr size_t kStagedLimbs = size_t(1) << 17;
+
+int staged_product(Kind kind, const uint64_t *x, size_t nx, const uint64_t *y, size_t ny, uint64_t d, uint64_t *out,
+                   size_t nout) {
+  Context &c = g_ctx;
+  Lane &L = *c.lane;
+  cudaStream_t st = L.stream;
+  const bool two = kind == Kind::Ntt || kind == Kind::Schoolboy;
+  const size_t size = nx + ny;
+  const size_t oy = (nx + 1) & ~size_t(1), oout = (oy + (two ? ny : 0) + 1) & ~size_t(1), oerr = oout + size;
+  HG_CUDA(L.stage.ensure((3 * kStagedLimbs + 8) * 8), "staging buffer");
+  uint64_t *h = static_cast<uint64_t *>(L.stage.p), *hd = static_cast<uint64_t *>(L.stage.dev);
+  memcpy(h, x, nx * 8);
+  if (two) memcpy(h + oy, y, ny * 8);
+  const uint64_t *dx = hd, *dy = hd + oy;
+  int rc = HG_OK;
+  if (kind == Kind::Ntt || kind == Kind::Square) {
+    HG_CUDA(L.X.ensure((kStagedLimbs + 4) * 8), "operand allocation");
+    HG_CUDA(cudaMemcpyAsync(L.X.p, h, (two ? oy + ny : nx) * 8, cudaMemcpyHostToDevice, st), "operand upload");
+    dx = L.X.u64();
+    dy = dx + oy;
+    rc = ntt_product_device(dx, nx, two ? dy : nullptr, two ? ny : 0, hd + oout, size, st);
+  } else {
+    rc = small_product_device(dx, nx, two ? dy : nullptr, two ? ny : 0, d, hd + oout, size, st);
+  }
+  if (rc) return rc;
+  HG_CUDA(cudaMemcpyAsync(h + oerr, err_word(), sizeof(int), cudaMemcpyDeviceToHost, st), "error word read");
+  HG_CUDA(cudaStreamSynchronize(st), "stream synchronise");
+#if HG_CHECKED
+  if ((rc = read_checked_faults())) return rc;
+#endif
+  int err;
+  memcpy(&err, h + oerr, sizeof err);
+  if ((rc = lib_device_error(err, st))) return rc;
+  memcpy(out, h + oout, size * 8);
+  if (nout > size) memset(out + size, 0, (nout - size) * 8);
+  return HG_OK;
+}
 
 int host_product(Kind kind, const uint64_t *x, size_t nx, const uint64_t *y, size_t ny, uint64_t d, uint64_t *out,
                  size_t nout) {
@@ -1231,6 +1306,7 @@ int host_product(Kind kind, const uint64_t *x, size_t nx, const uint64_t *y, siz
   }
   const size_t nd = size;  // limbs computed on the device; the rest are zero
   cudaStream_t st = c.lane->stream;
+  if (size <= kStagedLimbs) return staged_product(kind, x, nx, y, ny, d, out, nout);
   // Pinned (page-locked) host buffers are addressable from the device over
   // the host link, so the kernels read the operands and write the product
   // in place; pageable buffers go through device staging buffers.
@@ -1464,8 +1540,8 @@ struct hg_batch {
 namespace hg {
 namespace {
 
-// Enqueue group gi with the given schedule.  The group's ticket and flags
-// must be zero.
+// Enqueue group gi with the given schedule.  The group's count must be zero
+// (its carry leaves it so); its flags are written before they are read.
 int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::vector<PassPlan> &plan,
               cudaStream_t st) {
   const int nops = g.square ? 1 : 2;
@@ -1745,12 +1821,6 @@ int persist_run(hg_batch *b, cudaStream_t st) {
   return HG_OK;
 }
 
-int batch_clear_scan(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st) {
-  if (bp.flag_words) HG_CUDA(cudaMemsetAsync(bb.flags, 0, bp.flag_words * 8, st), "scan flags reset");
-  if (!bp.groups.empty()) HG_CUDA(cudaMemsetAsync(bb.tickets, 0, bp.groups.size() * 8, st), "scan tickets reset");
-  return HG_OK;
-}
-
 // Time each candidate schedule of each group (twice; the second run counts)
 // and keep the fastest.
 int batch_autotune(hg_batch *b) {
@@ -1776,7 +1846,6 @@ int batch_autotune(hg_batch *b) {
     for (const auto &plan : cands) {
       float ms = 0;
       for (int rep = 0; rep < 2 && rc == HG_OK; ++rep) {
-        if ((rc = batch_clear_scan(b->bp, bb, st))) break;
         cudaEventRecord(e0, st);
         if ((rc = run_group(g, gi, bb, plan, st))) break;
         cudaEventRecord(e1, st);
@@ -1866,7 +1935,8 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
   }
   if (bp.ws_words) HG_CUDA(b->ws.ensure(bp.ws_words * 8), "batch workspace");
   if (bp.flag_words) HG_CUDA(b->flags.ensure(bp.flag_words * 8), "batch scan flags");
-  HG_CUDA(b->tickets.ensure(std::max<size_t>(1, bp.groups.size()) * 8), "batch tickets");
+  HG_CUDA(b->tickets.ensure(std::max<size_t>(1, bp.groups.size()) * 8), "batch scan counts");
+  HG_CUDA(cudaMemset(b->tickets.p, 0, b->tickets.bytes), "batch scan counts");
   if ((flags & HG_BATCH_PER_PASS) && (flags & HG_BATCH_PERSISTENT))
     return fail(HG_ERR_ARG, "a batch runs either per pass or persistently, not both");
   if (flags & HG_BATCH_AUTOTUNE) {
@@ -1992,22 +2062,59 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
 }
 
 int enqueue_batch(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st) {
-  int rc = batch_clear_scan(bp, bb, st);
-  if (rc) return rc;
+  int rc = HG_OK;
   if (bp.nzero) HG_CUDA(launch_zero_tails(bb.desc + bp.zero_first, bp.nzero, 0, st), "zero products");
   for (size_t gi = 0; gi < bp.groups.size(); ++gi)
     if ((rc = run_group(bp.groups[gi], gi, bb, bp.groups[gi].plan, st))) return rc;
   return HG_OK;
 }
 
+int host_words_take(HostWords *w) {
+  std::lock_guard<std::mutex> lk(g_words_mu);
+  if (g_words_free.empty()) {
+    constexpr size_t kPage = 4096;
+    void *h = nullptr, *d = nullptr;
+    HG_CUDA(cudaHostAlloc(&h, kPage, cudaHostAllocMapped), "result words");
+    const cudaError_t e = cudaHostGetDevicePointer(&d, h, 0);
+    if (e != cudaSuccess) {
+      cudaFreeHost(h);
+      return cuda_fail(e, "result words");
+    }
+    g_words_pages.push_back(h);
+    for (size_t o = 0; o < kPage; o += kWordsBytes)
+      g_words_free.push_back(HostWords{reinterpret_cast<int64_t *>(static_cast<char *>(h) + o),
+                                       reinterpret_cast<int64_t *>(static_cast<char *>(d) + o)});
+  }
+  *w = g_words_free.back();
+  g_words_free.pop_back();
+  return HG_OK;
+}
+
+void host_words_give(const HostWords &w) {
+  std::lock_guard<std::mutex> lk(g_words_mu);
+  if (!g_words_pages.empty()) g_words_free.push_back(w);
+}
+
+int *lib_err_word() { return err_word(); }
+
+// Reset the library's error word after `err` was read from it, and report it.
+int lib_device_error(int err, cudaStream_t st) {
+  if (!err) return HG_OK;
+  HG_CUDA(cudaMemsetAsync(err_word(), 0, sizeof(int), st), "error word reset");
+  HG_CUDA(cudaStreamSynchronize(st), "stream synchronise");
+  if (err == kDevCarryOverflow) return fail(HG_ERR_INCONSISTENT, "a carry left the top of the result storage");
+  if (err == kDevCopyTimeout) return fail(HG_ERR_CUDA, "a tile copy did not complete within its wait limit");
+  return fail(HG_ERR_CUDA, "device error %d", err);
+}
+
 std::recursive_mutex &lib_mutex() { return g_ctx.mu; }
 bool lib_ready() { return g_ctx.ready; }
-int large_sum_device(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t *b, uint64_t nb, int64_t sb,
-                     uint64_t *out, uint64_t nout, int64_t *result, cudaStream_t st) {
+int large_sum_device(const SumOperand &a, int64_t sa, const SumOperand &b, int64_t sb, uint64_t *out, uint64_t nout,
+                     int64_t *result, cudaStream_t st) {
   std::lock_guard<std::recursive_mutex> lock(g_ctx.mu);
   int rc = ensure_init();
   if (rc) return rc;
-  const uint64_t n = na > nb ? na : nb;
+  const uint64_t n = std::max(a.end(), b.end());
   const uint64_t nproc = sa != sb ? n : n + 1;
   HG_CUDA(ws_acquire(st), "workspace ordering");
   if (nout > nproc) HG_CUDA(cudaMemsetAsync(out + nproc, 0, (nout - nproc) * sizeof(uint64_t), st), "zero tail");
@@ -2018,7 +2125,7 @@ int large_sum_device(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t 
   {
     // (top search,) scan (and fix), sign and size
     ProfScope ps(HG_KC_OTHER, st, 24.0 * static_cast<double>(nproc), (sa != sb ? 3 : 2) + (carry_short(nproc) ? 0 : 1));
-    HG_CUDA(launch_large_sum(a, na, sa, b, nb, sb, out, words, result, ss, st), "large sum");
+    HG_CUDA(launch_large_sum(a, sa, b, sb, out, words, result, ss, st), "large sum");
   }
   HG_CUDA(ws_release(st), "workspace ordering");
   return HG_OK;
@@ -2128,6 +2235,7 @@ int hg_shutdown(void) {
     L.Y.release();
     L.OUT.release();
     L.flags.release();
+    L.stage.release();
     L.misc.release();
     for (cudaStream_t *st : {&L.stream, &L.copy_stream, &L.d2h_stream}) {
       if (*st) cudaStreamDestroy(*st);
@@ -2149,6 +2257,12 @@ int hg_shutdown(void) {
   c.tables.release();
   release_pass_twiddles();
   lib_release_descs();
+  {
+    std::lock_guard<std::mutex> lk(g_words_mu);
+    for (void *p : g_words_pages) cudaFreeHost(p);
+    g_words_pages.clear();
+    g_words_free.clear();
+  }
   c.ready = false;
   // The scratch array's device address belongs to the module as loaded in
   // the current context: after a context reset the module loads again, so
@@ -2277,6 +2391,20 @@ int hg_mul_schoolboy_device(const uint64_t *x, size_t nx, const uint64_t *y, siz
   if (rc) return rc;
   if (!y) return fail(HG_ERR_ARG, "null pointer");
   return small_product_device(x, nx, y, ny, 0, out, nout, static_cast<cudaStream_t>(stream));
+}
+
+int hg_mul_sized_device(const uint64_t *x, size_t nx, const uint64_t *y, size_t ny, uint64_t *out, size_t nout,
+                        int schoolboy, void *stream, size_t *size) {
+  if (!size) return fail(HG_ERR_ARG, "null pointer");
+  const int rc = schoolboy ? hg_mul_schoolboy_device(x, nx, y, ny, out, nout, stream)
+                           : (y ? hg_mul_device(x, nx, y, ny, out, nout, stream)
+                                : hg_sqr_device(x, nx, out, nout, stream));
+  if (rc) return rc;
+  const hg_vec v{out, y ? nx + ny : 2 * nx};
+  uint64_t n = 0;
+  const int e = hg_sums_and_sizes(nullptr, nullptr, nullptr, 0, nullptr, &v, 1, &n, stream);
+  *size = n;
+  return e;
 }
 
 int hg_butterfly_peak(double *butterflies_per_s) {

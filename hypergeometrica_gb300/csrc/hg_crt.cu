@@ -145,11 +145,11 @@ struct ConvProducer {
 // %subtract-storages/unsafe, src/mpz-ram.lisp:184-274): position i holds
 // x_i + y_i as (low, carry).  With opposite signs y is the smaller
 // magnitude's complement over n = max(na, nb) limbs plus 1 at position 0,
-// and the carry out of the top is dropped.  `top` is then the highest index
+// and the carry out of the top is dropped (n: the longer operand's end).  `top` is then the highest index
 // where a and b differ (or -1), found before the scan; it picks the larger.
 struct SumProducer {
-  const uint64_t *a, *b;
-  uint64_t na, nb, n;
+  SumOperand a, b;
+  uint64_t n;
   const long long *top;  // subtraction only
 
   __host__ __device__ __forceinline__ bool drop_top() const { return top != nullptr; }
@@ -159,15 +159,14 @@ struct SumProducer {
     const long long t = *top;
     if (t < 0) return true;
     const uint64_t u = static_cast<uint64_t>(t);
-    return (u < na ? a[u] : 0) >= (u < nb ? b[u] : 0);
+    return a.at(u) >= b.at(u);
   }
 
   __device__ __forceinline__ V3 value(uint64_t i, bool ax) const {
     if (i >= n) return V3{0, 0, 0};
-    const uint64_t *X = ax ? a : b, *Y = ax ? b : a;
-    const uint64_t nX = ax ? na : nb, nY = ax ? nb : na;
-    const uint64_t x = i < nX ? X[i] : 0;
-    uint64_t y = i < nY ? Y[i] : 0;
+    const uint64_t va = a.at(i), vb = b.at(i);
+    const uint64_t x = ax ? va : vb;
+    uint64_t y = ax ? vb : va;
     if (top) y = ~y;
     uint64_t lo = x + y;
     uint64_t c = lo < x ? 1 : 0;
@@ -200,13 +199,12 @@ __device__ __forceinline__ void grid_max(long long best, long long *top) {
 }
 
 // *top = max index i < n with a_i != b_i.
-__global__ void top_diff_kernel(const uint64_t *a, uint64_t na, const uint64_t *b, uint64_t nb, uint64_t n,
-                                long long *top) {
+__global__ void top_diff_kernel(const SumOperand a, const SumOperand b, uint64_t n, long long *top) {
   pdl_wait();
   long long best = -1;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
-    if ((i < na ? a[i] : 0) != (i < nb ? b[i] : 0)) best = static_cast<long long>(i);
+    if (a.at(i) != b.at(i)) best = static_cast<long long>(i);
   grid_max(best, top);
 }
 
@@ -483,17 +481,17 @@ cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, int
                       tiles, carry_short(nproc), ss, st);
 }
 
-cudaError_t launch_large_sum(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t *b, uint64_t nb, int64_t sb,
-                             uint64_t *out, SumWords *words, int64_t *result, const ScanState &ss, cudaStream_t st) {
-  const uint64_t n = na > nb ? na : nb;
+cudaError_t launch_large_sum(const SumOperand &a, int64_t sa, const SumOperand &b, int64_t sb, uint64_t *out,
+                             SumWords *words, int64_t *result, const ScanState &ss, cudaStream_t st) {
+  const uint64_t n = a.end() > b.end() ? a.end() : b.end();
   const bool sub = sa != sb;
   const uint64_t nproc = sub ? n : n + 1;
   const uint64_t tiles = carry_tiles(nproc);
   if (tiles == 0 || tiles > 0x7fffffffull) return cudaErrorInvalidValue;
-  const SumProducer prod{a, b, na, nb, n, sub ? &words->top_diff : nullptr};
+  const SumProducer prod{a, b, n, sub ? &words->top_diff : nullptr};
   const auto grid = [](uint64_t m) { return dim3(static_cast<unsigned>(m < 152 * 4 * 1024 ? (m + 1023) / 1024 : 152 * 4)); };
   cudaError_t e = cudaSuccess;
-  if (sub) e = launch_dep(top_diff_kernel, grid(n), 256, 0, st, a, na, b, nb, n, &words->top_diff);
+  if (sub) e = launch_dep(top_diff_kernel, grid(n), 256, 0, st, a, b, n, &words->top_diff);
   if (e == cudaSuccess) e = launch_carry(prod, out, nproc, tiles, carry_short(nproc), ss, st);
   if (e == cudaSuccess) e = launch_dep(sum_finish_kernel, grid(nproc), 256, 0, st, out, nproc, prod, sa, sb, result, words);
   return e;

@@ -42,7 +42,7 @@ struct BatchBufs {
   const ProductDesc *desc;    // device copy of BatchPlan::desc
   uint64_t *ws;               // ws_words words
   unsigned long long *flags;  // flag_words words
-  unsigned long long *tickets;  // one per group
+  unsigned long long *tickets;  // one per group (the carry's finished-tile count), zero between runs
   int *err;                   // device error word
 };
 
@@ -53,16 +53,28 @@ uint64_t product_workspace_bytes(uint64_t nx, uint64_t ny, bool square);
 // so that none needs more than ws_cap_bytes of workspace.
 int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchPlan &bp);
 
-// sa |a| + sb |b| into out[0, nout) over the whole GPU (nout >= max(na,
-// nb) + 1; limbs past the sum are zeroed); (sign, size) into result[0, 2)
+// sa |a| + sb |b| into out[0, nout) over the whole GPU (nout >= the longer
+// operand's end + 1; limbs past the sum are zeroed); (sign, size) into result[0, 2)
 // on the device.  Uses the library's carry-scan state, ordered like the
 // products' workspace.
-int large_sum_device(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t *b, uint64_t nb, int64_t sb,
-                     uint64_t *out, uint64_t nout, int64_t *result, cudaStream_t st);
+int large_sum_device(const SumOperand &a, int64_t sa, const SumOperand &b, int64_t sb, uint64_t *out, uint64_t nout,
+                     int64_t *result, cudaStream_t st);
 
 // Enqueue a planned batch on st: clear its scan state, zero the empty
 // products, run every group.  Takes no lock and allocates nothing.
 int enqueue_batch(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st);
+
+// Words that kernels write and the host reads after a synchronisation.
+struct HostWords {
+  int64_t *host, *dev;
+};
+int host_words_take(HostWords *w);
+void host_words_give(const HostWords &w);
+
+// The library's device error word; lib_device_error resets it when `err`,
+// read from it, is not 0, and returns the error.
+int *lib_err_word();
+int lib_device_error(int err, cudaStream_t st);
 
 // Give back the descriptor memory that hg_sum.cu keeps (hg_shutdown).
 void lib_release_descs();

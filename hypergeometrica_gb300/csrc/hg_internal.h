@@ -214,6 +214,14 @@ cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint
 cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, int logN, uint64_t chunk,
                                     uint64_t nchunks, const CrtConst &cc, uint64_t *out, uint64_t nproc,
                                     const ScanState &ss, cudaStream_t st, uint64_t *tiles_used);
+// An operand of a signed sum: n limbs, `shift` whole limbs up.
+struct SumOperand {
+  const uint64_t *p;
+  uint64_t n, shift;
+  __host__ __device__ __forceinline__ uint64_t end() const { return n ? n + shift : 0; }
+  __device__ __forceinline__ uint64_t at(uint64_t i) const { return i - shift < n ? p[i - shift] : 0; }  // i < shift wraps
+};
+
 // Search words of a long sum, in device memory: -1, -1 and 0 before and after
 // every sum (sums that share them are ordered).
 struct SumWords {
@@ -221,11 +229,11 @@ struct SumWords {
   long long top_out;   // highest nonzero limb of the result
   unsigned done;
 };
-// sa |a| + sb |b| into out[0, n + 1) (n = max(na, nb); out[0, n) when the
-// signs differ) over the whole GPU, with the carry scan of the products;
+// sa |a| + sb |b| into out[0, n + 1) (n = the longer operand's end; out[0, n)
+// when the signs differ) over the whole GPU, with the carry scan of the products;
 // result = (sign, size).
-cudaError_t launch_large_sum(const uint64_t *a, uint64_t na, int64_t sa, const uint64_t *b, uint64_t nb, int64_t sb,
-                             uint64_t *out, SumWords *words, int64_t *result, const ScanState &ss, cudaStream_t st);
+cudaError_t launch_large_sum(const SumOperand &a, int64_t sa, const SumOperand &b, int64_t sb, uint64_t *out,
+                             SumWords *words, int64_t *result, const ScanState &ss, cudaStream_t st);
 // Zero out[N, nout) of every product (out[0, nout) when N == 0), N the
 // residues per prime.
 cudaError_t launch_zero_tails(const ProductDesc *batch, uint64_t nprod, uint64_t N, cudaStream_t st);

@@ -3,9 +3,10 @@
 // Callers (binary splitting, Newton steps) submit products whose operands and
 // results already live in device memory; the service runs them on the GPU
 // with continuous batching:
-//   - a worker thread owns S slots, each a CUDA stream with its own workspace,
+//   - there are S slots, each a CUDA stream with its own workspace,
 //     descriptor buffers, carry-scan state and device error word, all
-//     allocated once when the service opens;
+//     allocated once when the service opens; a worker thread and the clients
+//     that wait fill them and retire their batches;
 //   - pending products are admitted first in, first out into a free slot
 //     while their transform workspace fits in the slot's free memory (and up
 //     to max_batch products); one admitted set runs as one batch: one launch
@@ -41,6 +42,7 @@ struct SvcRequest {
   ProductDesc d;
   uint64_t ticket;
   uint64_t ws_bytes;
+  uint64_t *size;  // device-addressable word for the product's length, or null
   Clock::time_point t_submit;
 };
 
@@ -56,6 +58,7 @@ struct SvcSlot {
   int *h_err = nullptr;  // pinned copy of the error word after the batch
   uint64_t flag_cap = 0;
   bool busy = false;
+  bool launching = false;  // a thread is enqueuing its batch, without the lock
   std::vector<SvcRequest> batch;
   BatchPlan plan;
 };
@@ -78,6 +81,7 @@ struct hg_svc {
   std::vector<float> lat_us;  // since the last stats reset
   bool have_first = false;
   hg::Clock::time_point t_first, t_last;
+  int helpers = 0;  // clients inside wait_helping
   bool closing = false;
   std::thread worker;
 };
@@ -113,7 +117,9 @@ int slot_alloc(SvcSlot &s, uint64_t ws_bytes, size_t max_batch) {
   // most N / 2048 + 1 flag words.
   s.flag_cap = ws_bytes / 8 / 3 / 2048 + max_batch + 64;
   SVC_CUDA(cudaMalloc(&s.flags, s.flag_cap * 8), "service scan flags");
-  SVC_CUDA(cudaMalloc(&s.tickets, kSlotTickets * 8), "service scan tickets");
+  SVC_CUDA(cudaMemset(s.flags, 0, s.flag_cap * 8), "service scan flags");
+  SVC_CUDA(cudaMalloc(&s.tickets, kSlotTickets * 8), "service scan counts");
+  SVC_CUDA(cudaMemset(s.tickets, 0, kSlotTickets * 8), "service scan counts");
   SVC_CUDA(cudaMalloc(&s.d_err, sizeof(int)), "service error word");
   SVC_CUDA(cudaMemset(s.d_err, 0, sizeof(int)), "service error word");
   SVC_CUDA(cudaMallocHost(&s.h_err, sizeof(int)), "service error staging");
@@ -143,8 +149,12 @@ int slot_launch(hg_svc *svc, SvcSlot &s) {
   if (e != cudaSuccess) return lib_cuda_fail(e, "service descriptor upload");
   const BatchBufs bb{s.d_desc, s.ws, s.flags, s.tickets, s.d_err};
   if ((rc = enqueue_batch(s.plan, bb, s.st))) return rc;
+  for (const SvcRequest &r : s.batch) {
+    if (!r.size) continue;
+    const hg_vec v{r.d.out, r.d.nx + r.d.ny};
+    if ((rc = hg_trim_batch_device(&v, 1, r.size, s.st))) return rc;
+  }
   if ((e = cudaMemcpyAsync(s.h_err, s.d_err, sizeof(int), cudaMemcpyDeviceToHost, s.st)) != cudaSuccess ||
-      (e = cudaMemsetAsync(s.d_err, 0, sizeof(int), s.st)) != cudaSuccess ||
       (e = cudaEventRecord(s.done, s.st)) != cudaSuccess)
     return lib_cuda_fail(e, "service batch completion");
   return HG_OK;
@@ -165,62 +175,123 @@ void settle(hg_svc *svc, std::vector<SvcRequest> &batch, int code, Clock::time_p
   batch.clear();
 }
 
+// A slot's batch has ended with `code` (the device error word read by then).
+void retire(hg_svc *svc, SvcSlot &s, cudaError_t q) {
+  int code = HG_OK;
+  if (q != cudaSuccess) code = HG_ERR_CUDA;
+  else if (*s.h_err) code = err_code(*s.h_err);
+  if (*s.h_err) cudaMemsetAsync(s.d_err, 0, sizeof(int), s.st);
+  *s.h_err = 0;
+  s.busy = false;
+  settle(svc, s.batch, code, Clock::now());
+  svc->cv_done.notify_all();
+}
+
+// One step of the service, with the lock held: retire the batches that have
+// ended and admit pending products into a free slot.  The worker and every
+// waiting client run it, so that a client's product starts and ends without
+// waiting for another thread to be scheduled.  True when it did something.
+bool pump(hg_svc *svc, std::unique_lock<std::mutex> &lk) {
+  bool progress = false;
+  for (SvcSlot &s : svc->slots) {
+    if (!s.busy) continue;
+    const cudaError_t q = cudaEventQuery(s.done);
+    if (q == cudaErrorNotReady) continue;
+    retire(svc, s, q);
+    progress = true;
+  }
+  SvcSlot *slot = nullptr;
+  for (SvcSlot &s : svc->slots)
+    if (!s.busy && !s.launching) {
+      slot = &s;
+      break;
+    }
+  if (!slot || svc->pending.empty()) return progress;
+  uint64_t used = 0;
+  while (!svc->pending.empty() && slot->batch.size() < svc->max_batch) {
+    const SvcRequest &r = svc->pending.front();
+    if (!slot->batch.empty() && used + r.ws_bytes > svc->slot_ws_bytes) break;
+    used += r.ws_bytes;
+    slot->batch.push_back(r);
+    svc->pending.pop_front();
+  }
+  svc->peak_batch_bytes = std::max(svc->peak_batch_bytes, used);
+  svc->peak_batch_products = std::max<uint64_t>(svc->peak_batch_products, slot->batch.size());
+  slot->launching = true;
+  lk.unlock();
+  const int rc = slot_launch(svc, *slot);
+  if (rc) cudaStreamSynchronize(slot->st);
+  lk.lock();
+  slot->launching = false;
+  if (rc) {
+    settle(svc, slot->batch, rc, Clock::now());
+    svc->cv_done.notify_all();
+  } else {
+    slot->busy = true;
+    ++svc->batches;
+    svc->cv_work.notify_one();  // the worker watches it from now on
+  }
+  return true;
+}
+
+bool any_busy(const hg_svc *svc) {
+  for (const SvcSlot &s : svc->slots)
+    if (s.busy || s.launching) return true;
+  return false;
+}
+
 void worker_loop(hg_svc *svc) {
   cudaSetDevice(svc->device);
   std::unique_lock<std::mutex> lk(svc->mu);
   for (;;) {
-    bool busy = false;
-    for (SvcSlot &s : svc->slots) {
-      if (!s.busy) continue;
-      const cudaError_t q = cudaEventQuery(s.done);
-      if (q == cudaErrorNotReady) {
-        busy = true;
-        continue;
-      }
-      int code = HG_OK;
-      if (q != cudaSuccess) code = HG_ERR_CUDA;
-      else if (*s.h_err) code = err_code(*s.h_err);
-      *s.h_err = 0;
-      s.busy = false;
-      settle(svc, s.batch, code, Clock::now());
-      svc->cv_done.notify_all();
-    }
-    SvcSlot *slot = nullptr;
-    for (SvcSlot &s : svc->slots)
-      if (!s.busy) {
-        slot = &s;
-        break;
-      }
-    if (slot && !svc->pending.empty()) {
-      uint64_t used = 0;
-      while (!svc->pending.empty() && slot->batch.size() < svc->max_batch) {
-        const SvcRequest &r = svc->pending.front();
-        if (!slot->batch.empty() && used + r.ws_bytes > svc->slot_ws_bytes) break;
-        used += r.ws_bytes;
-        slot->batch.push_back(r);
-        svc->pending.pop_front();
-      }
-      svc->peak_batch_bytes = std::max(svc->peak_batch_bytes, used);
-      svc->peak_batch_products = std::max<uint64_t>(svc->peak_batch_products, slot->batch.size());
-      lk.unlock();
-      const int rc = slot_launch(svc, *slot);
-      lk.lock();
-      if (rc) {
-        cudaStreamSynchronize(slot->st);
-        settle(svc, slot->batch, rc, Clock::now());
-        svc->cv_done.notify_all();
-      } else {
-        slot->busy = true;
-        ++svc->batches;
-      }
-      continue;
-    }
+    if (pump(svc, lk)) continue;
+    const bool busy = any_busy(svc);
     if (svc->closing && svc->pending.empty() && !busy) break;
     if (busy)
-      svc->cv_work.wait_for(lk, std::chrono::microseconds(20));
+      svc->cv_work.wait_for(lk, std::chrono::microseconds(svc->helpers ? 500 : 20));
     else
-      svc->cv_work.wait(lk, [&] { return svc->closing || !svc->pending.empty(); });
+      svc->cv_work.wait(lk, [&] { return svc->closing || !svc->pending.empty() || any_busy(svc); });
   }
+}
+
+// The library's device for the calling thread, while it runs a service's work.
+struct DeviceGuard {
+  int before = -1;
+  explicit DeviceGuard(int device) {
+    if (cudaGetDevice(&before) != cudaSuccess || before == device || cudaSetDevice(device) != cudaSuccess) before = -1;
+  }
+  ~DeviceGuard() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+};
+
+// Wait until pred() or for timeout_s (< 0: no limit), doing the service's
+// work meanwhile; false when the time ran out.  Spins for the first
+// kSpin of a wait (a small batch ends within it), then sleeps between looks.
+template <class Pred>
+bool wait_helping(hg_svc *svc, std::unique_lock<std::mutex> &lk, double timeout_s, Pred pred) {
+  constexpr auto kSpin = std::chrono::microseconds(300);
+  if (pred()) return true;
+  DeviceGuard dev(svc->device);
+  const auto t0 = Clock::now();
+  ++svc->helpers;
+  bool done = false;
+  for (;;) {
+    const bool progress = pump(svc, lk);
+    if ((done = pred())) break;
+    const auto waited = Clock::now() - t0;
+    if (timeout_s >= 0 && waited >= std::chrono::duration<double>(timeout_s)) break;
+    if (progress) continue;
+    if (waited < kSpin) {
+      lk.unlock();
+      std::this_thread::yield();
+      lk.lock();
+    } else {
+      svc->cv_done.wait_for(lk, std::chrono::microseconds(20));
+    }
+  }
+  --svc->helpers;
+  return done;
 }
 
 }  // namespace
@@ -265,7 +336,8 @@ int hg_svc_open(size_t workspace_bytes, int slots, size_t max_batch, hg_svc **ou
   return HG_OK;
 }
 
-int hg_svc_submit(hg_svc *svc, const hg_product *prods, size_t n, uint64_t *first_ticket) {
+namespace {
+int submit(hg_svc *svc, const hg_product *prods, size_t n, uint64_t *first_ticket, uint64_t *size_word) {
   if (!svc || (n && !prods)) return lib_fail(HG_ERR_ARG, "null pointer");
   std::vector<SvcRequest> reqs(n);
   for (size_t i = 0; i < n; ++i) {
@@ -285,6 +357,7 @@ int hg_svc_submit(hg_svc *svc, const hg_product *prods, size_t n, uint64_t *firs
                       (unsigned long long)ws, (unsigned long long)svc->slot_ws_bytes);
     reqs[i].d = ProductDesc{p.x, p.y, p.nx, square ? p.nx : p.ny, p.out, p.nout};
     reqs[i].ws_bytes = ws;
+    reqs[i].size = size_word;
   }
   const Clock::time_point now = Clock::now();
   {
@@ -306,6 +379,11 @@ int hg_svc_submit(hg_svc *svc, const hg_product *prods, size_t n, uint64_t *firs
   svc->cv_work.notify_one();
   return HG_OK;
 }
+}  // namespace
+
+int hg_svc_submit(hg_svc *svc, const hg_product *prods, size_t n, uint64_t *first_ticket) {
+  return submit(svc, prods, n, first_ticket, nullptr);
+}
 
 int hg_svc_status(hg_svc *svc, uint64_t ticket) {
   if (!svc) return lib_fail(HG_ERR_ARG, "null pointer");
@@ -318,10 +396,7 @@ int hg_svc_wait(hg_svc *svc, uint64_t ticket, double timeout_s) {
   if (!svc) return lib_fail(HG_ERR_ARG, "null pointer");
   std::unique_lock<std::mutex> lk(svc->mu);
   if (ticket >= svc->next_ticket) return lib_fail(HG_ERR_ARG, "unknown ticket %llu", (unsigned long long)ticket);
-  const auto pred = [&] { return svc->status[ticket] != 0; };
-  if (timeout_s < 0)
-    svc->cv_done.wait(lk, pred);
-  else if (!svc->cv_done.wait_for(lk, std::chrono::duration<double>(timeout_s), pred))
+  if (!wait_helping(svc, lk, timeout_s, [&] { return svc->status[ticket] != 0; }))
     return lib_fail(HG_ERR_TIMEOUT, "product %llu not finished within %.3f s", (unsigned long long)ticket, timeout_s);
   const int st = svc->status[ticket];
   return st == 1 ? HG_OK : lib_fail(st, "product %llu failed on the device", (unsigned long long)ticket);
@@ -330,13 +405,28 @@ int hg_svc_wait(hg_svc *svc, uint64_t ticket, double timeout_s) {
 int hg_svc_wait_all(hg_svc *svc, double timeout_s) {
   if (!svc) return lib_fail(HG_ERR_ARG, "null pointer");
   std::unique_lock<std::mutex> lk(svc->mu);
-  const auto pred = [&] { return svc->completed + svc->failed == svc->submitted; };
-  if (timeout_s < 0)
-    svc->cv_done.wait(lk, pred);
-  else if (!svc->cv_done.wait_for(lk, std::chrono::duration<double>(timeout_s), pred))
+  if (!wait_helping(svc, lk, timeout_s, [&] { return svc->completed + svc->failed == svc->submitted; }))
     return lib_fail(HG_ERR_TIMEOUT, "%llu products not finished within %.3f s",
                     (unsigned long long)(svc->submitted - svc->completed - svc->failed), timeout_s);
   return svc->failed ? lib_fail(HG_ERR_CUDA, "%llu products failed", (unsigned long long)svc->failed) : HG_OK;
+}
+
+int hg_svc_mul(hg_svc *svc, const hg_product *prod, void *stream, size_t *size) {
+  if (!svc || !prod || !size) return lib_fail(HG_ERR_ARG, "null pointer");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // The service's streams are not ordered after the caller's.
+  cudaError_t e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return lib_cuda_fail(e, "stream synchronise");
+  HostWords w;
+  int rc = host_words_take(&w);
+  if (rc) return rc;
+  w.host[0] = 0;
+  uint64_t ticket = 0;
+  rc = submit(svc, prod, 1, &ticket, reinterpret_cast<uint64_t *>(w.dev));
+  if (rc == HG_OK) rc = hg_svc_wait(svc, ticket, -1.0);
+  *size = static_cast<size_t>(w.host[0]);
+  host_words_give(w);
+  return rc;
 }
 
 int hg_svc_stats(hg_svc *svc, hg_svc_report *out, int reset) {

@@ -14,6 +14,8 @@
 // thread forms its limbs' generate/propagate pair, the CTA scans the pairs
 // (warp shuffles, then the eight warp totals), and the chunk's carry-out
 // feeds the next chunk.
+#include <algorithm>
+
 #include "hg_host.h"
 #include "hypergeometrica_gb300.h"
 
@@ -25,10 +27,7 @@ constexpr int kSumPer = 8;
 constexpr uint64_t kSumChunk = kSumThreads * kSumPer;
 
 struct SumDesc {
-  const uint64_t *a;
-  uint64_t na;
-  const uint64_t *b;
-  uint64_t nb;
+  SumOperand a, b;
   uint64_t *out;
   uint64_t nout;
   int64_t sa, sb;
@@ -57,18 +56,16 @@ struct Descs {
   __device__ __forceinline__ Desc operator[](uint64_t i) const { return p ? p[i] : inl[i]; }
 };
 
-// Highest index < n whose limb is nonzero (or differs between a and b when
-// b != nullptr), -1 if none; scanned from the top one chunk at a time.
-__device__ long long top_index(const uint64_t *a, uint64_t na, const uint64_t *b, uint64_t nb, uint64_t n) {
+// Highest index < n where a and b differ, -1 if none; scanned from the top one
+// chunk at a time.
+__device__ long long top_index(const SumOperand &a, const SumOperand &b, uint64_t n) {
   __shared__ long long s_top;
   if (threadIdx.x == 0) s_top = -1;
   __syncthreads();
   for (uint64_t hi = n; hi > 0;) {
     const uint64_t lo = hi > kSumChunk ? hi - kSumChunk : 0;
     for (uint64_t i = lo + threadIdx.x; i < hi; i += kSumThreads) {
-      const uint64_t x = i < na ? a[i] : 0;
-      const uint64_t y = b ? (i < nb ? b[i] : 0) : 0;
-      if (x != y) atomicMax(&s_top, static_cast<long long>(i));
+      if (a.at(i) != b.at(i)) atomicMax(&s_top, static_cast<long long>(i));
     }
     __syncthreads();
     // Every thread reads the flag before any thread can move on and update
@@ -86,13 +83,12 @@ __device__ long long top_index(const uint64_t *a, uint64_t na, const uint64_t *b
 __global__ void __launch_bounds__(kSumThreads) sum_kernel(const Descs<SumDesc> descs) {
   const SumDesc d = descs[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const uint64_t n = d.na > d.nb ? d.na : d.nb;
+  const uint64_t n = d.a.end() > d.b.end() ? d.a.end() : d.b.end();
   const bool sub = d.sa != d.sb;
-  const uint64_t *X = d.a, *Y = d.b;
-  uint64_t nX = d.na, nY = d.nb;
+  SumOperand X = d.a, Y = d.b;
   int64_t sign = d.sa;
   if (sub) {
-    const long long t = top_index(d.a, d.na, d.b, d.nb, n);
+    const long long t = top_index(d.a, d.b, n);
     if (t < 0) {  // equal magnitudes: zero
       for (uint64_t i = tid; i < d.nout; i += kSumThreads) d.out[i] = 0;
       if (tid == 0) {
@@ -101,13 +97,9 @@ __global__ void __launch_bounds__(kSumThreads) sum_kernel(const Descs<SumDesc> d
       }
       return;
     }
-    const uint64_t at = static_cast<uint64_t>(t) < d.na ? d.a[t] : 0;
-    const uint64_t bt = static_cast<uint64_t>(t) < d.nb ? d.b[t] : 0;
-    if (bt > at) {
+    if (d.b.at(static_cast<uint64_t>(t)) > d.a.at(static_cast<uint64_t>(t))) {
       X = d.b;
-      nX = d.nb;
       Y = d.a;
-      nY = d.na;
       sign = d.sb;
     }
   }
@@ -132,8 +124,8 @@ __global__ void __launch_bounds__(kSumThreads) sum_kernel(const Descs<SumDesc> d
       const uint64_t i = i0 + j;
       uint64_t x = 0, y = 0;
       if (i < span) {
-        x = i < nX ? X[i] : 0;
-        y = i < nY ? Y[i] : 0;
+        x = X.at(i);
+        y = Y.at(i);
         if (sub) y = ~y;
       }
       s[j] = x + y;
@@ -187,7 +179,7 @@ __global__ void __launch_bounds__(kSumThreads) sum_kernel(const Descs<SumDesc> d
 
 __global__ void __launch_bounds__(kSumThreads) trim_kernel(const Descs<VecDesc> descs, uint64_t *sizes) {
   const VecDesc d = descs[blockIdx.x];
-  const long long t = top_index(d.p, d.n, nullptr, 0, d.n);
+  const long long t = top_index(SumOperand{d.p, d.n, 0}, SumOperand{nullptr, 0, 0}, d.n);
   if (threadIdx.x == 0) sizes[blockIdx.x] = static_cast<uint64_t>(t + 1);
 }
 
@@ -287,12 +279,101 @@ int run_batch(const Desc *host, size_t n, cudaStream_t st, const char *what, Lau
   return HG_OK;
 }
 
+// Host-mapped words for one call's results: a block of the library's, or for
+// many results one larger buffer that calls take turns on.
+std::mutex g_many_mu;
+int64_t *g_many = nullptr, *g_many_dev = nullptr;
+size_t g_many_words = 0;
+
+class ResultWords {
+ public:
+  int64_t *host = nullptr, *dev = nullptr;
+  int take(size_t words) {
+    if (words <= 8) {
+      const int rc = host_words_take(&block_);
+      if (rc) return rc;
+      taken_ = true;
+      host = block_.host;
+      dev = block_.dev;
+      return HG_OK;
+    }
+    lock_ = std::unique_lock<std::mutex>(g_many_mu);
+    if (words > g_many_words) {
+      if (g_many) cudaFreeHost(g_many);
+      g_many = nullptr;
+      g_many_words = 0;
+      void *h = nullptr, *d = nullptr;
+      cudaError_t e = cudaHostAlloc(&h, 2 * words * sizeof(int64_t), cudaHostAllocMapped);
+      if (e != cudaSuccess) return lib_cuda_fail(e, "result words");
+      if ((e = cudaHostGetDevicePointer(&d, h, 0)) != cudaSuccess) {
+        cudaFreeHost(h);
+        return lib_cuda_fail(e, "result words");
+      }
+      g_many = static_cast<int64_t *>(h);
+      g_many_dev = static_cast<int64_t *>(d);
+      g_many_words = 2 * words;
+    }
+    host = g_many;
+    dev = g_many_dev;
+    return HG_OK;
+  }
+  ~ResultWords() {
+    if (taken_) host_words_give(block_);
+  }
+
+ private:
+  HostWords block_{};
+  bool taken_ = false;
+  std::unique_lock<std::mutex> lock_;
+};
+
+// Check the sums and enqueue them; sign and size of sum k to result[2 k], result[2 k + 1].
+int sums_enqueue(const hg_sum *sums, const size_t *a_shift, const size_t *b_shift, size_t n, int64_t *result,
+                 cudaStream_t st) {
+  if (n && !sums) return lib_fail(HG_ERR_ARG, "null pointer");
+  if (!lib_ready()) return lib_fail(HG_ERR_NOT_INIT, "hg_add_batch_device: call hg_init first");
+  const auto operands = [&](size_t k, SumOperand &a, SumOperand &b) {
+    a = SumOperand{sums[k].a, sums[k].na, a_shift ? a_shift[k] : 0};
+    b = SumOperand{sums[k].b, sums[k].nb, b_shift ? b_shift[k] : 0};
+  };
+  SumOperand a, b;
+  for (size_t k = 0; k < n; ++k) {
+    const hg_sum &s = sums[k];
+    operands(k, a, b);
+    if ((s.na && !s.a) || (s.nb && !s.b) || (s.nout && !s.out)) return lib_fail(HG_ERR_ARG, "sum %zu: null pointer", k);
+    if ((s.sa != 1 && s.sa != -1) || (s.sb != 1 && s.sb != -1))
+      return lib_fail(HG_ERR_ARG, "sum %zu: signs must be +1 or -1", k);
+    if (a.end() < a.n || b.end() < b.n) return lib_fail(HG_ERR_ARG, "sum %zu: shift out of range", k);
+    const size_t need = std::max(a.end(), b.end()) + 1;
+    if (s.nout < need) return lib_fail(HG_ERR_ARG, "sum %zu: nout = %zu cannot hold %zu limbs", k, s.nout, need);
+  }
+  std::vector<SumDesc> d;
+  d.reserve(n);
+  for (size_t k = 0; k < n; ++k) {
+    const hg_sum &s = sums[k];
+    operands(k, a, b);
+    if (std::max(a.end(), b.end()) >= (n == 1 ? kLargeSumAlone : kLargeSum)) {
+      const int rc = large_sum_device(a, s.sa, b, s.sb, s.out, s.nout, result + 2 * k, st);
+      if (rc) return rc;
+    } else {
+      d.push_back(SumDesc{a, b, s.out, s.nout, s.sa, s.sb, result + 2 * k});
+    }
+  }
+  return run_batch(d.data(), d.size(), st, "signed sums", [&](const Descs<SumDesc> &dev, unsigned grid) {
+    sum_kernel<<<grid, kSumThreads, 0, st>>>(dev);
+  });
+}
+
 }  // namespace
 
 void lib_release_descs() {
   std::lock_guard<std::mutex> lk(g_pool_mu);
   if (g_pool) cudaMemPoolDestroy(g_pool);
   g_pool = nullptr;
+  std::lock_guard<std::mutex> lm(g_many_mu);
+  if (g_many) cudaFreeHost(g_many);
+  g_many = g_many_dev = nullptr;
+  g_many_words = 0;
 }
 
 #if HG_CHECKED
@@ -306,31 +387,32 @@ using namespace hg;
 extern "C" {
 
 int hg_add_batch_device(const hg_sum *sums, size_t n, int64_t *result, void *stream) {
-  if (n && (!sums || !result)) return lib_fail(HG_ERR_ARG, "null pointer");
-  if (!lib_ready()) return lib_fail(HG_ERR_NOT_INIT, "hg_add_batch_device: call hg_init first");
-  std::vector<SumDesc> d;
-  d.reserve(n);
-  for (size_t k = 0; k < n; ++k) {
-    const hg_sum &s = sums[k];
-    if ((s.na && !s.a) || (s.nb && !s.b) || (s.nout && !s.out)) return lib_fail(HG_ERR_ARG, "sum %zu: null pointer", k);
-    if ((s.sa != 1 && s.sa != -1) || (s.sb != 1 && s.sb != -1))
-      return lib_fail(HG_ERR_ARG, "sum %zu: signs must be +1 or -1", k);
-    const size_t need = (s.na > s.nb ? s.na : s.nb) + 1;
-    if (s.nout < need) return lib_fail(HG_ERR_ARG, "sum %zu: nout = %zu cannot hold %zu limbs", k, s.nout, need);
-  }
+  if (n && !result) return lib_fail(HG_ERR_ARG, "null pointer");
+  return sums_enqueue(sums, nullptr, nullptr, n, result, static_cast<cudaStream_t>(stream));
+}
+
+int hg_sums_and_sizes(const hg_sum *sums, const size_t *a_shift, const size_t *b_shift, size_t n, int64_t *results,
+                      const hg_vec *vecs, size_t m, uint64_t *sizes, void *stream) {
+  if ((n && !results) || (m && !sizes)) return lib_fail(HG_ERR_ARG, "null pointer");
+  if (!lib_ready()) return lib_fail(HG_ERR_NOT_INIT, "hg_sums_and_sizes: call hg_init first");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  for (size_t k = 0; k < n; ++k) {
-    const hg_sum &s = sums[k];
-    if ((s.na > s.nb ? s.na : s.nb) >= (n == 1 ? kLargeSumAlone : kLargeSum)) {
-      const int rc = large_sum_device(s.a, s.na, s.sa, s.b, s.nb, s.sb, s.out, s.nout, result + 2 * k, st);
-      if (rc) return rc;
-    } else {
-      d.push_back(SumDesc{s.a, s.na, s.b, s.nb, s.out, s.nout, s.sa, s.sb, result + 2 * k});
-    }
-  }
-  return run_batch(d.data(), d.size(), st, "signed sums", [&](const Descs<SumDesc> &dev, unsigned grid) {
-    sum_kernel<<<grid, kSumThreads, 0, st>>>(dev);
-  });
+  const size_t words = 2 * n + m + 1;  // results, sizes, the error word
+  ResultWords w;
+  int rc = w.take(words);
+  if (rc) return rc;
+  if (n) rc = sums_enqueue(sums, a_shift, b_shift, n, w.dev, st);
+  if (rc == HG_OK && m) rc = hg_trim_batch_device(vecs, m, reinterpret_cast<uint64_t *>(w.dev) + 2 * n, stream);
+  w.host[words - 1] = 0;
+  cudaError_t e = cudaSuccess;
+  if (rc == HG_OK)
+    e = cudaMemcpyAsync(w.host + words - 1, lib_err_word(), sizeof(int), cudaMemcpyDeviceToHost, st);
+  // Nothing enqueued may write the words after they are given back.
+  const cudaError_t f = cudaStreamSynchronize(st);
+  if (rc) return rc;
+  if (e != cudaSuccess || f != cudaSuccess) return lib_cuda_fail(e != cudaSuccess ? e : f, "sums and sizes");
+  for (size_t k = 0; k < 2 * n; ++k) results[k] = w.host[k];
+  for (size_t k = 0; k < m; ++k) sizes[k] = static_cast<uint64_t>(w.host[2 * n + k]);
+  return lib_device_error(static_cast<int>(w.host[words - 1]), st);
 }
 
 int hg_mul_small_batch_device(const hg_product *prods, size_t n, void *stream) {

@@ -176,6 +176,19 @@ class Service:
         check(load().hg_svc_submit(self._h, arr, n, ctypes.byref(first)))
         return range(first.value, first.value + n)
 
+    def mul(self, x: int, nx: int, y: int | None, ny: int, out: int, nout: int, stream=None) -> int:
+        """One product by device addresses (hg_svc_mul; y None squares x): waits
+        for the work on stream and for the product, and returns its length
+        without high zero limbs."""
+        import ctypes
+
+        from ._lib import HgProduct
+
+        size = ctypes.c_size_t()
+        check(load().hg_svc_mul(self._h, ctypes.byref(HgProduct(x, nx, y, ny, out, nout)), _stream(stream),
+                                ctypes.byref(size)))
+        return size.value
+
     def status(self, ticket: int) -> int:
         return load().hg_svc_status(self._h, ticket)
 

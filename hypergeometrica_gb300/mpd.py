@@ -32,12 +32,12 @@ sqrt) are computed on the host exactly as SBCL computes them.
 
 from __future__ import annotations
 
+import ctypes
 import math
 import struct
 
-import numpy as np
-
 from . import series as S
+from ._lib import HgSum, check, load
 from .series import DeviceInt
 
 BASE = 1 << 64
@@ -85,20 +85,22 @@ def _shift(x: DeviceInt, limbs: int) -> DeviceInt:
     return DeviceInt(x.sign, t, x.size + limbs)
 
 
-def mpz_add(x: DeviceInt, y: DeviceInt) -> DeviceInt:
-    """mpz-+ (src/mpz-ram.lisp:292-306)."""
+def mpz_add(x: DeviceInt, y: DeviceInt, x_shift: int = 0, y_shift: int = 0) -> DeviceInt:
+    """mpz-+ (src/mpz-ram.lisp:292-306) of x 2^(64 x_shift) and y 2^(64 y_shift)."""
     import torch
 
     if x.size == 0:
-        return y
+        return _shift(y, y_shift)
     if y.size == 0:
-        return x
-    nout = max(x.size, y.size) + 1
+        return _shift(x, x_shift)
+    nout = max(x.size + x_shift, y.size + y_shift) + 1
     out = torch.empty(nout, dtype=torch.int64, device="cuda")
-    rec = np.array([[x.ptr(), x.size, y.ptr(), y.size, out.data_ptr(), nout,
-                     np.int64(x.sign).view(np.uint64), np.int64(y.sign).view(np.uint64)]], dtype=np.uint64)
-    (sign, size), = S._sum_records(rec)
-    return DeviceInt(int(sign), out, int(size))
+    res = (ctypes.c_int64 * 2)()
+    check(load().hg_sums_and_sizes(
+        ctypes.byref(HgSum(x.ptr(), x.size, y.ptr(), y.size, out.data_ptr(), nout, x.sign, y.sign)),
+        ctypes.byref(ctypes.c_size_t(x_shift)), ctypes.byref(ctypes.c_size_t(y_shift)), 1, res, None, 0, None,
+        torch.cuda.current_stream().cuda_stream))
+    return DeviceInt(res[0], out, res[1])
 
 
 def mpd_mul(a: MPD, b: MPD, service=None) -> MPD:
@@ -107,7 +109,7 @@ def mpd_mul(a: MPD, b: MPD, service=None) -> MPD:
 
 def mpd_add(a: MPD, b: MPD) -> MPD:
     lo = min(a.exponent, b.exponent)
-    return MPD(mpz_add(_shift(a.mantissa, a.exponent - lo), _shift(b.mantissa, b.exponent - lo)), lo)
+    return MPD(mpz_add(a.mantissa, b.mantissa, a.exponent - lo, b.exponent - lo), lo)
 
 
 def mpd_negate(a: MPD) -> MPD:

@@ -48,12 +48,14 @@ def int_from_digits(d) -> int:
 
 
 def _size(d: np.ndarray) -> int:
+    if d.size and d[-1]:  # the usual case: no scan
+        return d.size
     nz = np.flatnonzero(d)
     return int(nz[-1]) + 1 if nz.size else 0
 
 
-def _ptr(a: np.ndarray):
-    return a.ctypes.data_as(ctypes.c_void_p)
+def _ptr(a: np.ndarray) -> int:
+    return a.ctypes.data
 
 
 class MPZ:
@@ -102,6 +104,12 @@ def optimize_mpz(x: MPZ) -> MPZ:
     return x
 
 
+def _fresh(sign: int, storage: np.ndarray) -> MPZ:
+    """optimize-mpz of a result whose storage no one else holds."""
+    n = _size(storage)
+    return MPZ(sign, storage if n == storage.size else storage[:n].copy())
+
+
 def least_power_of_two_ge(n: int) -> int:
     """least-power-of-two->= (src/math-utilities.lisp:18-22)."""
     return n if n > 0 and n & (n - 1) == 0 else 1 << n.bit_length()
@@ -111,20 +119,21 @@ def _mag(x: MPZ) -> np.ndarray:
     return np.ascontiguousarray(x.storage[: mpz_size(x)])
 
 
-def mpz_mul_ntt(x: MPZ, y: MPZ) -> MPZ:
-    """mpz-*/ntt (src/ntt-multiply.lisp:174-254)."""
+def mpz_mul_ntt(x: MPZ, y: MPZ, short: bool = False) -> MPZ:
+    """mpz-*/ntt (src/ntt-multiply.lisp:174-254); short: a storage of size(x) +
+    size(y) digits, which hold the product, instead of the transform length."""
     a, b = _mag(x), _mag(y)
-    length = least_power_of_two_ge(len(a) + len(b))
-    out = np.zeros(length, dtype=np.uint64)
+    length = len(a) + len(b) if short else least_power_of_two_ge(len(a) + len(b))
+    out = np.empty(length, dtype=np.uint64)
     check(load().hg_mul(_ptr(a), len(a), _ptr(b), len(b), _ptr(out), length))
     return MPZ(x.sign * y.sign, out)
 
 
-def mpz_square(x: MPZ) -> MPZ:
-    """mpz-square (src/ntt-multiply.lisp:101-172)."""
+def mpz_square(x: MPZ, short: bool = False) -> MPZ:
+    """mpz-square (src/ntt-multiply.lisp:101-172); short as in mpz_mul_ntt."""
     a = _mag(x)
-    length = least_power_of_two_ge(2 * len(a))
-    out = np.zeros(length, dtype=np.uint64)
+    length = 2 * len(a) if short else least_power_of_two_ge(2 * len(a))
+    out = np.empty(length, dtype=np.uint64)
     check(load().hg_sqr(_ptr(a), len(a), _ptr(out), length))
     return MPZ(1, out)
 
@@ -158,7 +167,7 @@ def multiply_storage_schoolboy(a: np.ndarray, a_size: int, b: np.ndarray, b_size
     1 + a_size + b_size digits."""
     a = np.ascontiguousarray(a[:a_size], dtype=np.uint64)
     b = np.ascontiguousarray(b[:b_size], dtype=np.uint64)
-    out = np.zeros(1 + a_size + b_size, dtype=np.uint64)
+    out = np.empty(1 + a_size + b_size, dtype=np.uint64)
     check(load().hg_mul_schoolboy(_ptr(a), a_size, _ptr(b), b_size, _ptr(out), len(out)))
     return out
 
@@ -167,7 +176,7 @@ def mpz_multiply_by_digit(d: int, x: MPZ) -> MPZ:
     """The by-digit branch of mpz-* (src/multiply.lisp:33-38): a fresh MPZ with
     a storage of size(x) + 2 holding x * d."""
     a = _mag(x)
-    out = np.zeros(len(a) + 2, dtype=np.uint64)
+    out = np.empty(len(a) + 2, dtype=np.uint64)
     check(load().hg_mul_digit(_ptr(a), len(a), ctypes.c_uint64(d), _ptr(out), len(out)))
     return MPZ(x.sign, out)
 
@@ -189,14 +198,11 @@ def mpz_mul(x: MPZ, y: MPZ, threshold: int | None = None) -> MPZ:
         d = int(y.storage[0])
         if d == 1:
             return x if y.sign == 1 else MPZ(-x.sign, x.storage.copy())
-        r = mpz_multiply_by_digit(d, x)
-        r.sign = x.sign * y.sign
-        return optimize_mpz(r)
+        return _fresh(x.sign * y.sign, mpz_multiply_by_digit(d, x).storage)
     if ny <= thr:
-        return optimize_mpz(MPZ(x.sign * y.sign, multiply_storage_schoolboy(x.storage, nx, y.storage, ny)))
-    if same:
-        return optimize_mpz(mpz_square(x))
-    return optimize_mpz(mpz_mul_ntt(x, y))
+        return _fresh(x.sign * y.sign, multiply_storage_schoolboy(x.storage, nx, y.storage, ny))
+    r = mpz_square(x, True) if same else mpz_mul_ntt(x, y, True)
+    return _fresh(r.sign, r.storage)
 
 
 def f_expt(a, n: int, one, multiply):

@@ -146,34 +146,26 @@ def multiply(x: DeviceInt, y: DeviceInt, service=None) -> DeviceInt:
     given).  x is y squares (mpz-square's single forward transform)."""
     import torch
 
-    from . import device as D
-
     square = x is y
     n = max(1, x.size + y.size)
     out = torch.empty(n, dtype=torch.int64, device="cuda")
     if x.size == 0 or y.size == 0:
         out.zero_()
         return DeviceInt(1, out, 0)
-    xs, ys = x.t[: x.size], (None if square else y.t[: y.size])
-    if not square and min(x.size, y.size) <= NTT_MULTIPLY_THRESHOLD:
-        # mpz-*'s dispatch: a smaller operand of at most 100 limbs goes to the
-        # quadratic method (src/multiply.lisp:37-42), here on the device
-        big, small = (xs, ys) if x.size >= y.size else (ys, xs)
-        D.mul_schoolboy(big, small, out)
-        sizes = trim_sizes([(out, n)])
-        return DeviceInt(x.sign * y.sign, out, int(sizes[0]))
-    if service is not None:
-        torch.cuda.current_stream().synchronize()
-        (t,) = service.submit([(xs, ys, out)])
-        service.wait(t)
-    elif square:
-        D.sqr(xs, out)
-        D.sync()
+    st = torch.cuda.current_stream().cuda_stream
+    # mpz-*'s dispatch: a smaller operand of at most 100 limbs goes to the
+    # quadratic method (src/multiply.lisp:37-42), here on the device
+    schoolboy = not square and min(x.size, y.size) <= NTT_MULTIPLY_THRESHOLD
+    if schoolboy and x.size < y.size:
+        x, y = y, x
+    if service is not None and not schoolboy:
+        size = service.mul(x.ptr(), x.size, None if square else y.ptr(), 0 if square else y.size, out.data_ptr(), n, st)
     else:
-        D.mul(xs, ys, out)
-        D.sync()
-    sizes = trim_sizes([(out, n)])
-    return DeviceInt(x.sign * y.sign, out, int(sizes[0]))
+        size = ctypes.c_size_t()
+        check(load().hg_mul_sized_device(x.ptr(), x.size, None if square else y.ptr(), 0 if square else y.size,
+                                         out.data_ptr(), n, 1 if schoolboy else 0, st, ctypes.byref(size)))
+        size = size.value
+    return DeviceInt(x.sign * y.sign, out, size)
 
 
 def mpz_expt_device(a, n: int, service=None) -> DeviceInt:
@@ -235,6 +227,24 @@ def _trim_records(rec: np.ndarray) -> np.ndarray:
     st = torch.cuda.current_stream()
     check(load().hg_trim_batch_device(rec.ctypes.data_as(ctypes.c_void_p), n, sizes.data_ptr(), st.cuda_stream))
     return sizes.cpu().numpy()
+
+
+def _sums_and_sizes(sums: np.ndarray, vecs: np.ndarray | None = None, shifts: np.ndarray | None = None):
+    """hg_sums_and_sizes on (n, 8) hg_sum and (m, 2) hg_vec records: ((n, 2)
+    signs and sizes of the sums, m sizes of the vectors); shifts (2, n) moves
+    the sums' operands up by whole limbs.  Waits."""
+    import torch
+
+    n, m = sums.shape[0], 0 if vecs is None else vecs.shape[0]
+    res, sizes = np.empty((n, 2), dtype=np.int64), np.empty(m, dtype=np.int64)
+    sums = np.ascontiguousarray(sums, dtype=np.uint64)
+    vecs = None if vecs is None else np.ascontiguousarray(vecs, dtype=np.uint64)
+    sh = None if shifts is None else np.ascontiguousarray(shifts, dtype=np.uint64)
+    check(load().hg_sums_and_sizes(sums.ctypes.data, None if sh is None else sh[0].ctypes.data,
+                                   None if sh is None else sh[1].ctypes.data, n, res.ctypes.data,
+                                   vecs.ctypes.data if m else None, m, sizes.ctypes.data,
+                                   torch.cuda.current_stream().cuda_stream))
+    return res, sizes
 
 
 def _sum_records(rec: np.ndarray) -> np.ndarray:
@@ -436,10 +446,9 @@ def binary_split(series: Series, lower: int, upper: int, service=None, timings: 
             sgT3, sgT4 = gR[2] * sgT1, gL[2] * sgT2
             sums = np.stack([t3, szT3.astype(np.uint64), t4, szT4.astype(np.uint64), aR, szR.astype(np.uint64),
                              sgT3.astype(np.int64).view(np.uint64), sgT4.astype(np.int64).view(np.uint64)], axis=1)
-            res = _sum_records(sums)
             trims = np.stack([np.concatenate([aP, aQ, aB]),
                               np.concatenate([szP, szQ, szB]).astype(np.uint64)], axis=1)
-            tsz = _trim_records(trims)
+            res, tsz = _sums_and_sizes(sums, trims)
             if timings is not None:
                 timings.append((h, int(k), t1 - t0, time.perf_counter() - t1))
             ptr[0, idx], ptr[1, idx], ptr[2, idx], ptr[3, idx] = aP, aQ, aB, aR

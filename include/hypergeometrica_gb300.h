@@ -165,6 +165,12 @@ int hg_sqr_device(const uint64_t *x, size_t nx, uint64_t *out, size_t nout, void
 int hg_mul_schoolboy_device(const uint64_t *x, size_t nx, const uint64_t *y, size_t ny, uint64_t *out,
                             size_t nout, void *stream);
 
+/* hg_mul_device (hg_sqr_device when y is NULL, hg_mul_schoolboy_device when
+ * schoolboy is nonzero) that waits for the product and returns its length
+ * without high zero limbs in *size. */
+int hg_mul_sized_device(const uint64_t *x, size_t nx, const uint64_t *y, size_t ny, uint64_t *out, size_t nout,
+                        int schoolboy, void *stream, size_t *size);
+
 /* ---- products without allocation -------------------------------------- */
 
 /* Largest product (nx + ny limbs, transform length 2^16) that
@@ -279,6 +285,20 @@ typedef struct hg_sum {
  * (a carry-lookahead scan ordered with the library's products). */
 int hg_add_batch_device(const hg_sum *sums, size_t n, int64_t *result, void *stream);
 
+typedef struct hg_vec {
+    const uint64_t *p; /* device limbs */
+    size_t n;
+} hg_vec;
+
+/* n sums as hg_add_batch_device, operands a and b of sum k moved up by
+ * a_shift[k] and b_shift[k] whole limbs (null: none; mpz-left-shift by whole
+ * digits, src/mpz-ram.lisp:310-332, without a shifted copy; nout >= the longer
+ * operand's end + 1), and m lengths as hg_trim_batch_device, in one call that
+ * waits: results (2n) and sizes (m) are host arrays.  Reports any device error
+ * latched before, as hg_sync does. */
+int hg_sums_and_sizes(const hg_sum *sums, const size_t *a_shift, const size_t *b_shift, size_t n, int64_t *results,
+                      const hg_vec *vecs, size_t m, uint64_t *sizes, void *stream);
+
 /* Largest operand of hg_mul_small_batch_device. */
 #define HG_SMALL_MAX_LIMBS 64
 
@@ -289,11 +309,6 @@ int hg_add_batch_device(const hg_sum *sums, size_t n, int64_t *result, void *str
  * most 100 limbs this way (src/multiply.lisp:37-42); binary splitting's
  * lowest tree levels consist of them. */
 int hg_mul_small_batch_device(const hg_product *prods, size_t n, void *stream);
-
-typedef struct hg_vec {
-    const uint64_t *p; /* device limbs */
-    size_t n;
-} hg_vec;
 
 /* mpz-size (vec-digit-length*, src/vec.lisp:218-229) of n device integers:
  * sizes[k] = length of vecs[k] without high zero limbs (device array). */
@@ -376,6 +391,10 @@ int hg_svc_status(hg_svc *svc, uint64_t ticket);
 int hg_svc_wait(hg_svc *svc, uint64_t ticket, double timeout_s);
 /* Wait for every product submitted so far. */
 int hg_svc_wait_all(hg_svc *svc, double timeout_s);
+/* One product through the service, from submission to completion: waits for
+ * the work on stream (which wrote the operands), submits, waits, and returns
+ * the product's length without high zero limbs in *size. */
+int hg_svc_mul(hg_svc *svc, const hg_product *prod, void *stream, size_t *size);
 /* Counters and latency percentiles; reset != 0 starts a new latency window. */
 int hg_svc_stats(hg_svc *svc, hg_svc_report *out, int reset);
 /* Finish the queued products, stop the worker, free the service. */

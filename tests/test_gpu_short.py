@@ -84,3 +84,84 @@ def test_spectrum_scaling(hg, L, offset):
         D.ntt_reverse(t, mod)
         D.sync()
         assert np.array_equal(t.cpu().numpy().view(np.uint64), a), (L, mod)
+
+
+@pytest.mark.parametrize("na,sa,nb,sb", [(3, 0, 5, 2), (5, 7, 3, 0), (1, 100, 100, 0), (2048, 1, 2047, 2), (4000, 4200, 8190, 0),
+                                         (9000, 0, 1, 9000), (70000, 3, 70001, 2), (1, 1 << 17, 1 << 17, 0)])
+def test_shifted_sums_and_sizes(hg, na, sa, nb, sb):
+    """hg_sums_and_sizes: operands moved up by whole limbs, with the sizes of
+    other integers in the same call."""
+    import torch
+
+    from hypergeometrica_gb300 import series as S
+
+    u, v = W.limbs(na, na), W.limbs(nb + 1, nb)
+    w = np.concatenate([W.limbs(3, 11), np.zeros(5000, dtype=np.uint64)])
+    ta, tb, tw = _dev(u), _dev(v), _dev(w)
+    n = max(na + sa, nb + sb)
+    for ga, gb in ((1, 1), (1, -1), (-1, 1), (-1, -1)):
+        want = ga * (hg.int_from_digits(u) << (64 * sa)) + gb * (hg.int_from_digits(v) << (64 * sb))
+        out = torch.full((n + 4,), -1, dtype=torch.int64, device="cuda")
+        rec = np.array([[ta.data_ptr(), na, tb.data_ptr(), nb, out.data_ptr(), n + 4, np.int64(ga).view(np.uint64),
+                         np.int64(gb).view(np.uint64)]], dtype=np.uint64)
+        vecs = np.array([[tw.data_ptr(), w.size], [tw.data_ptr() + 8 * 11, 5000]] * 20, dtype=np.uint64)
+        res, sizes = S._sums_and_sizes(rec, vecs, np.array([[sa], [sb]]))
+        assert hg.int_from_digits(out.cpu().numpy().view(np.uint64)) == abs(want)
+        assert tuple(res[0]) == (-1 if want < 0 else 1, (abs(want).bit_length() + 63) // 64)
+        assert sizes.tolist() == [11, 0] * 20
+
+
+@pytest.mark.parametrize("size", [2, 3, 1024, 1025, (1 << 17) - 1, 1 << 17, (1 << 17) + 1])
+def test_staged_host_products(hg, size):
+    """Host products on both sides of the staging buffer's limit, results longer
+    than the product, operands with high zeros."""
+    import ctypes
+
+    from hypergeometrica_gb300._lib import check, load
+
+    nx = size - size * 2 // 5
+    x, y = W.limbs(size, nx, "ones"), W.limbs(size + 1, size - nx)
+    xz = np.concatenate([x, np.zeros(7, dtype=np.uint64)])
+    vx, vy = hg.int_from_digits(x), hg.int_from_digits(y)
+    out = np.full(size + 9, np.uint64(7))
+    check(load().hg_mul(xz.ctypes.data, xz.size, y.ctypes.data, y.size, out.ctypes.data, out.size))
+    assert hg.int_from_digits(out) == vx * vy
+    out = np.full(2 * nx + 1, np.uint64(7))
+    check(load().hg_sqr(x.ctypes.data, nx, out.ctypes.data, out.size))
+    assert hg.int_from_digits(out) == vx * vx
+    out = np.full(nx + 3, np.uint64(7))
+    check(load().hg_mul_digit(x.ctypes.data, nx, ctypes.c_uint64(0xFFFFFFFFFFFFFFF1), out.ctypes.data, out.size))
+    assert hg.int_from_digits(out) == vx * 0xFFFFFFFFFFFFFFF1
+
+
+def test_service_sized_products(hg):
+    """hg_svc_mul from several threads, among submitted products, against the direct product."""
+    import threading
+
+    import torch
+
+    from hypergeometrica_gb300 import device as D
+
+    wrong = []
+    with D.Service(workspace_bytes=256 << 20, slots=2) as svc:
+        def client(k):
+            st = torch.cuda.Stream()
+            with torch.cuda.stream(st):
+                for j in range(12):
+                    nx, ny = 150 + 997 * j * (k + 1), 101 + 311 * j
+                    x, y = _dev(W.limbs(100 * k + j, nx)), _dev(W.limbs(5000 + 100 * k + j, ny))
+                    square = j % 3 == 2
+                    n = 2 * nx if square else nx + ny
+                    out, want = torch.empty(n, dtype=torch.int64, device="cuda"), torch.empty(n, dtype=torch.int64, device="cuda")
+                    size = svc.mul(x.data_ptr(), nx, None if square else y.data_ptr(), 0 if square else ny, out.data_ptr(), n)
+                    D.sqr(x, want) if square else D.mul(x, y, want)
+                    torch.cuda.current_stream().synchronize()
+                    w = want.cpu().numpy()
+                    if not torch.equal(out, want) or size != int(np.flatnonzero(w)[-1]) + 1:
+                        wrong.append((k, j))
+        ts = [threading.Thread(target=client, args=(k,)) for k in range(3)]
+        [t.start() for t in ts]
+        [t.join() for t in ts]
+        assert not wrong
+        st = svc.stats()
+        assert st["completed"] == st["submitted"] == 36 and st["failed"] == 0
