@@ -986,7 +986,20 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
       HG_CUDA(cudaMemcpyAsync(const_cast<uint64_t *>(y), host->hy, ny * 8, cudaMemcpyHostToDevice, st),
               "operand upload");
   }
-  if (host && plan.size() > 1) {
+  // Slices of a short product would be many rows of a few hundred bytes each:
+  // its operands go up whole.
+  constexpr int kSliceMinL = 19;
+  if (host && plan.size() > 1 && L < kSliceMinL) {
+    HG_CUDA(cudaMemcpyAsync(const_cast<uint64_t *>(x), host->hx, nx * 8, cudaMemcpyHostToDevice, c.lane->copy_stream),
+            "operand upload");
+    if (!square)
+      HG_CUDA(cudaMemcpyAsync(const_cast<uint64_t *>(y), host->hy, ny * 8, cudaMemcpyHostToDevice,
+                              c.lane->copy_stream),
+              "operand upload");
+    HG_CUDA(cudaEventRecord(c.lane->copy_done, c.lane->copy_stream), "operand upload");
+    HG_CUDA(cudaStreamWaitEvent(st, c.lane->copy_done, 0), "operand upload ordering");
+  }
+  if (host && plan.size() > 1 && L >= kSliceMinL) {
     // The first strided pass covers one block of 2^L = R S residues; its tile
     // t reads columns [t C, (t + 1) C) (C = 4096 / R) of every row.
     const PassPlan &p0 = plan[0];
@@ -1529,6 +1542,7 @@ std::map<std::tuple<int, int, bool, uint64_t>, std::vector<PassPlan>> g_tuned;
 struct hg_batch {
   hg::BatchPlan bp;
   hg::DevBuf d_desc, ws, flags, tickets;
+  hg::SideStreams side;
   // The persistent schedule: its work list and its counters.
   std::vector<hg::PersistPhase> phases;
   uint64_t items = 0;
@@ -1548,7 +1562,7 @@ int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::ve
   const uint64_t N = kept_points(g.L, g.kh);
   const uint64_t slab = static_cast<uint64_t>(kPrimes) * N;
   const ProductDesc *d = bb.desc + g.first;
-  uint64_t *ws = bb.ws;
+  uint64_t *ws = bb.ws + g.ws_off;
   if (g.tails) HG_CUDA(launch_zero_tails(d, g.nprod, N, st), "zero tails");
   PassArgs a = base_args(g.L, nops, N);
   a.err = bb.err;
@@ -1587,7 +1601,7 @@ int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::ve
 BatchBufs batch_bufs(hg_batch *b) {
   return BatchBufs{static_cast<const ProductDesc *>(b->d_desc.p), b->ws.u64(),
                    static_cast<unsigned long long *>(b->flags.p), static_cast<unsigned long long *>(b->tickets.p),
-                   err_word()};
+                   err_word(), b->side.n ? &b->side : nullptr};
 }
 
 // ---- the persistent schedule (hg_persist.cu) -------------------------------
@@ -1937,6 +1951,7 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
   if (bp.flag_words) HG_CUDA(b->flags.ensure(bp.flag_words * 8), "batch scan flags");
   HG_CUDA(b->tickets.ensure(std::max<size_t>(1, bp.groups.size()) * 8), "batch scan counts");
   HG_CUDA(cudaMemset(b->tickets.p, 0, b->tickets.bytes), "batch scan counts");
+  if (bp.parallel && bp.groups.size() > 1) HG_CUDA(b->side.create(), "batch streams");
   if ((flags & HG_BATCH_PER_PASS) && (flags & HG_BATCH_PERSISTENT))
     return fail(HG_ERR_ARG, "a batch runs either per pass or persistently, not both");
   if (flags & HG_BATCH_AUTOTUNE) {
@@ -1977,9 +1992,14 @@ uint64_t product_workspace_bytes(uint64_t nx, uint64_t ny, bool square) {
 }
 
 // Points a batch's cut must save per prime and operand to be a group of its
-// own: about 40 us of a full GPU's work, what a group's chain of launches
-// takes at least.
-constexpr uint64_t kCutPoints = uint64_t(1) << 19;
+// own.  The 4096-pair batch takes 3316, 3281 and 3231 us at 2^19, 2^18 and
+// 2^17, 1024 pairs 974, 959 and 929; 300 pairs of 2^12 to 2^14 limbs 753, 772
+// and 786.
+constexpr uint64_t kCutPoints = uint64_t(1) << 17;
+
+// What a chain of launches costs beside its residues, in the same units as
+// their stages (points x (L + 4)): about 30 us.
+constexpr double kChainWork = 4e7;
 
 int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchPlan &bp) {
   bp = BatchPlan();
@@ -1991,6 +2011,7 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
   };
   std::vector<Item> live;
   std::vector<size_t> zeros;
+  uint64_t ws_all = 0;  // words of all groups together
   live.reserve(n);
   for (size_t i = 0; i < n; ++i) {
     const ProductDesc &p = items[i];
@@ -2050,23 +2071,86 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
         if (bp.desc.back().nout > N) g.tails = true;
       }
       bp.flag_words += carry_tiles(N, g.nprod) * g.nprod;
+      g.ws_off = ws_all;
+      ws_all += per / 8 * g.nprod;
       bp.ws_words = std::max<uint64_t>(bp.ws_words, per / 8 * g.nprod);
       bp.groups.push_back(std::move(g));
     }
     s = e;
   }
+  bp.parallel = ws_all * 8 <= ws_cap_bytes;
+  if (bp.parallel)
+    bp.ws_words = ws_all;
+  else
+    for (BatchGroup &g : bp.groups) g.ws_off = 0;
   bp.zero_first = bp.desc.size();
   bp.nzero = zeros.size();
   for (size_t z : zeros) bp.desc.push_back(items[z]);
   return HG_OK;
 }
 
+cudaError_t SideStreams::create() {
+  cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+  for (; e == cudaSuccess && n < kMax; ++n) {
+    if ((e = cudaStreamCreateWithFlags(&st[n], cudaStreamNonBlocking)) != cudaSuccess) break;
+    if ((e = cudaEventCreateWithFlags(&join[n], cudaEventDisableTiming)) != cudaSuccess) {
+      cudaStreamDestroy(st[n]);
+      break;
+    }
+  }
+  if (e != cudaSuccess) destroy();
+  return e;
+}
+
+void SideStreams::destroy() {
+  for (int i = 0; i < n; ++i) {
+    cudaStreamDestroy(st[i]);
+    cudaEventDestroy(join[i]);
+  }
+  if (fork) cudaEventDestroy(fork);
+  *this = SideStreams();
+}
+
+// A group is a chain of four to six dependent launches, each of which ends
+// with SMs running dry; chains of different groups fill them for each other.
+// The groups go, largest first, to the stream with the least work so far.
+// Four streams against one after another: 256 pairs of 2^6 to 2^14 limbs 372
+// -> 265 us, 1024 pairs 1166 -> 974, 4096 pairs 3420 -> 3316, 4096 of 2^6 to
+// 2^9 314 -> 256; two streams 287, 973, 3278 and 261, six 255, 981, 3331, 259.
 int enqueue_batch(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st) {
   int rc = HG_OK;
   if (bp.nzero) HG_CUDA(launch_zero_tails(bb.desc + bp.zero_first, bp.nzero, 0, st), "zero products");
-  for (size_t gi = 0; gi < bp.groups.size(); ++gi)
-    if ((rc = run_group(bp.groups[gi], gi, bb, bp.groups[gi].plan, st))) return rc;
-  return HG_OK;
+  const size_t ng = bp.groups.size();
+  if (!bb.side || !bp.parallel || ng < 2) {
+    for (size_t gi = 0; gi < ng; ++gi)
+      if ((rc = run_group(bp.groups[gi], gi, bb, bp.groups[gi].plan, st))) return rc;
+    return HG_OK;
+  }
+  const SideStreams &side = *bb.side;
+  const int ns = std::min<int>(side.n + 1, static_cast<int>(ng));  // st and ns - 1 side streams
+  const auto work = [&](size_t gi) {
+    const BatchGroup &g = bp.groups[gi];
+    return static_cast<double>(kept_points(g.L, g.kh)) * static_cast<double>(g.nprod) * (g.L + 4) * (g.square ? 2 : 3) +
+           kChainWork;
+  };
+  std::vector<size_t> order(ng);
+  for (size_t gi = 0; gi < ng; ++gi) order[gi] = gi;
+  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return work(a) > work(b); });
+  double load[SideStreams::kMax + 1] = {};
+  HG_CUDA(cudaEventRecord(side.fork, st), "batch fork");
+  for (int i = 0; i + 1 < ns; ++i) HG_CUDA(cudaStreamWaitEvent(side.st[i], side.fork, 0), "batch fork");
+  for (size_t gi : order) {
+    const int k = static_cast<int>(std::min_element(load, load + ns) - load);
+    load[k] += work(gi);
+    if ((rc = run_group(bp.groups[gi], gi, bb, bp.groups[gi].plan, k ? side.st[k - 1] : st))) break;
+  }
+  // Joined also after a failed launch: st must not run ahead of what was enqueued.
+  for (int i = 0; i + 1 < ns; ++i) {
+    cudaError_t e = cudaEventRecord(side.join[i], side.st[i]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, side.join[i], 0);
+    if (e != cudaSuccess && rc == HG_OK) rc = cuda_fail(e, "batch join");
+  }
+  return rc;
 }
 
 int host_words_take(HostWords *w) {
@@ -2195,6 +2279,7 @@ int hg_batch_destroy(hg_batch *batch) {
   batch->ws.release();
   batch->flags.release();
   batch->tickets.release();
+  batch->side.destroy();
   delete batch;
   return HG_OK;
 }

@@ -25,13 +25,27 @@ struct BatchGroup {
   std::vector<PassPlan> plan;
   uint64_t first = 0, nprod = 0;   // descriptors [first, first + nprod)
   uint64_t flags_off = 0;          // first carry-scan flag word
+  uint64_t ws_off = 0;             // first workspace word
+};
+
+// Streams beside a batch's own, for groups that run at the same time.  Each
+// batch (and service slot) has its own: a captured batch captures them too.
+struct SideStreams {
+  static constexpr int kMax = 3;
+  int n = 0;
+  cudaStream_t st[kMax] = {};
+  cudaEvent_t fork = nullptr, join[kMax] = {};
+  cudaError_t create();
+  void destroy();
 };
 
 // A planned batch: groups contiguous in desc, then the products with an empty
-// operand (zeroed, no transform).  Groups run one after another and share
-// one workspace of ws_words words.
+// operand (zeroed, no transform).  Where the workspace of all groups fits the
+// cap (parallel), each has its own part of it and groups may run at the same
+// time; else they run one after another and share it.
 struct BatchPlan {
   std::vector<BatchGroup> groups;
+  bool parallel = false;
   std::vector<ProductDesc> desc;
   uint64_t zero_first = 0, nzero = 0;
   uint64_t ws_words = 0, flag_words = 0;
@@ -44,6 +58,7 @@ struct BatchBufs {
   unsigned long long *flags;  // flag_words words
   unsigned long long *tickets;  // one per group (the carry's finished-tile count), zero between runs
   int *err;                   // device error word
+  const SideStreams *side;    // or null: groups one after another
 };
 
 // Workspace bytes one product occupies while its group runs.

@@ -48,6 +48,7 @@ struct SvcRequest {
 
 struct SvcSlot {
   cudaStream_t st = nullptr;
+  SideStreams side;
   cudaEvent_t done = nullptr;
   uint64_t *ws = nullptr;
   ProductDesc *d_desc = nullptr;
@@ -92,6 +93,7 @@ namespace {
 void slot_free(SvcSlot &s) {
   if (s.done) cudaEventDestroy(s.done);
   if (s.st) cudaStreamDestroy(s.st);
+  s.side.destroy();
   if (s.ws) cudaFree(s.ws);
   if (s.d_desc) cudaFree(s.d_desc);
   if (s.h_desc) cudaFreeHost(s.h_desc);
@@ -109,6 +111,7 @@ int slot_alloc(SvcSlot &s, uint64_t ws_bytes, size_t max_batch) {
     if (e_ != cudaSuccess) return lib_cuda_fail(e_, what);   \
   } while (0)
   SVC_CUDA(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking), "service stream");
+  SVC_CUDA(s.side.create(), "service streams");
   SVC_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming), "service event");
   SVC_CUDA(cudaMalloc(&s.ws, ws_bytes), "service workspace");
   SVC_CUDA(cudaMalloc(&s.d_desc, max_batch * sizeof(ProductDesc)), "service descriptors");
@@ -147,7 +150,7 @@ int slot_launch(hg_svc *svc, SvcSlot &s) {
   cudaError_t e = cudaMemcpyAsync(s.d_desc, s.h_desc, s.plan.desc.size() * sizeof(ProductDesc),
                                   cudaMemcpyHostToDevice, s.st);
   if (e != cudaSuccess) return lib_cuda_fail(e, "service descriptor upload");
-  const BatchBufs bb{s.d_desc, s.ws, s.flags, s.tickets, s.d_err};
+  const BatchBufs bb{s.d_desc, s.ws, s.flags, s.tickets, s.d_err, &s.side};
   if ((rc = enqueue_batch(s.plan, bb, s.st))) return rc;
   for (const SvcRequest &r : s.batch) {
     if (!r.size) continue;
