@@ -319,7 +319,8 @@ int init_locked(const uint64_t *moduli, int k, const uint64_t *roots, int maxlg,
   for (int i = 0; i < kPrimes; ++i) {
     const uint64_t p = dm[i];
     c.moduli[i] = p;
-    c.pc[i] = PrimeConst{p, static_cast<uint32_t>(p >> kShift), 0};
+    const uint64_t cp = p >> kShift;
+    c.pc[i] = PrimeConst{p, static_cast<uint32_t>(cp), static_cast<uint32_t>(((uint64_t(1) << 39) + cp - 1) / cp)};
     c.gens[i] = generator_h(p);
     const uint64_t w30 = powmod_h(c.gens[i], (p - 1) >> kLogNmax, p);
     const uint64_t w30i = invmod_h(w30, p);
@@ -441,61 +442,73 @@ std::vector<PassPlan> plan_passes(int L) {
   return v;
 }
 
-// ---- truncated transforms -------------------------------------------------
+// ---- transform plans ----------------------------------------------------
 //
-// A product of n limbs needs n points.  Where n is at most 7/8 of the power
-// of two above it, the transform keeps 5, 6 or 7 eighths of the 2^L points
-// (hg_ntt_strided.cu): the passes inside the outer one, the middle and the
-// workspace shrink by that factor.  The outer pass cuts by its top row bits,
-// so it needs 16, 128 or 256 rows (64 for 6/8).  Products, us, beside the
-// whole transform of the same size (one product, warm):
-//   points   5/8            6/8            7/8            8/8
-//   2^18     59.8 (74.2)    61.8 (74.2)    72.8 (74.1)    74.4
-//   2^21     272 (363)      302 (365)      329 (367)      369
-//   2^25     3947 (5521)    4543 (5561)    5132 (5600)    5638
-// Below 2^17 points a product is bound by the latency of its launches and the
-// cut gives 1-6%; it is nowhere slower.
-uint64_t kept_points(int L, int kh) { return kh == 8 ? uint64_t(1) << L : (uint64_t(1) << (L - 3)) * kh; }
+// A product of n coefficients needs n points, not the power of two above: the
+// transform keeps 9 to 15 sixteenths of the 2^L points where that is enough
+// (hg_ntt_strided.cu), and the passes inside the outer one, the middle and
+// the workspace shrink by that factor.  The outer pass cuts by its top row
+// bits, so it needs 16 or 256 rows (128 for even numbers of sixteenths, 64
+// for 12).
+//
+// And the coefficients need not be limbs.  Three primes hold coefficients
+// below p0 p1 p2 = 2^187; limbs give 2^128 times the shorter operand's
+// length, digits of 80 bits 2^160 times: up to 2^27 digits fit, and a product
+// has 4/5 as many of them.
+// Products, us, beside the whole transform on limbs (one product, warm):
+//   limbs     5/8            6/8            7/8            8/8
+//   2^18      37.8 (60.2)    49.4 (60.2)    52.9 (60.6)    59.4 (60.1)
+//   2^21      186 (341)      265 (343)      294 (343)      319 (345)
+//   2^25      2750 (5387)    3974 (5425)    4554 (5464)    4933 (5503)
+// (cut to eighths on limbs, 5/8 and 7/8 of 2^25 limbs took 3866 and 5100).
+// Below 2^17 points a product is bound by the latency of its launches.
+uint64_t kept_points(int L, int k16) { return k16 == 16 ? uint64_t(1) << L : (uint64_t(1) << (L - 4)) * k16; }
 
 struct TransformPlan {
   int L = 0;
-  int kh = 8;  // eighths kept
+  int k16 = 16;        // sixteenths kept
+  bool dig80 = false;  // coefficients are 80-bit digits
   std::vector<PassPlan> passes;
-  uint64_t points() const { return kept_points(L, kh); }
+  uint64_t points() const { return kept_points(L, k16); }
 };
 
 // Tiles of 4096 residues (three primes) up to which a launch leaves SMs idle:
 // plans for it spread the work instead of saving passes over memory.
 constexpr uint64_t kIdleTiles = 192;
 
-// Passes of a 2^L-point transform that keeps kh eighths: the outer pass has
-// 16 rows where the other bits still fit the same number of passes (the
-// smaller the outer pass, the more of the work is cut), else the plan of the
-// whole transform, else 128 rows (2^17 and 2^18 points).
+// Passes of a 2^L-point transform that keeps k16 sixteenths: the outer pass
+// has 16 rows where the other bits still fit the same number of passes (the
+// smaller the outer pass, the more of the work is cut), else it is the whole
+// transform's where that can cut, else it has 256 rows.
 //
 // nprod products at a time that leave SMs idle (kIdleTiles) take contiguous
 // blocks of 2^9 residues (2^10 from 2^17 points on): more CTAs, and more of
 // the stages where both operands run side by side.  A product of 2^16 points:
 // 43.1 us with 2^12-residue blocks, 37.0 with 2^9; of 2^17: 49.2 and 45.6; of
 // 2^18: 73.0 and 68.8 (one product, warm).
-std::vector<PassPlan> plan_kept(int L, int kh, uint64_t nprod = 1) {
+std::vector<PassPlan> plan_kept(int L, int k16, uint64_t nprod = 1) {
   std::vector<PassPlan> v = plan_passes(L);
   if (L > kTileBits && L <= 18 && (3 * nprod << L) >> kTileBits <= kIdleTiles) {
     const int T = L < 17 ? 9 : 10;
-    if (truncation_ok(L - T, kh)) return {{L - T, T, kTileBits}, {T, 0, T}};
+    if (truncation_ok(L - T, k16)) return {{L - T, T, kTileBits}, {T, 0, T}};
   }
-  if (kh == 8) return v;
-  const int rem = L - v.back().logT;
+  if (k16 == 16) return v;
+  const int T = v.back().logT, rem = L - T;
   const int k = static_cast<int>(v.size()) - 1;
   std::vector<int> parts;
-  if (k >= 2 && rem - 4 >= 4 * (k - 1) && rem - 4 <= 8 * (k - 1)) {
-    parts.push_back(4);
-    for (int i = 0; i < k - 1; ++i) parts.push_back((rem - 4) / (k - 1) + (i < (rem - 4) % (k - 1) ? 1 : 0));
-  } else if (!truncation_ok(v[0].logR, kh)) {
-    parts.push_back(7);
-  } else {
+  const auto rest = [&](int first) {  // the outer pass, then the other bits in k - 1 passes
+    parts.push_back(first);
+    for (int i = 0; i < k - 1; ++i)
+      parts.push_back((rem - first) / (k - 1) + (i < (rem - first) % (k - 1) ? 1 : 0));
+  };
+  if (k >= 2 && rem - 4 >= 4 * (k - 1) && rem - 4 <= 8 * (k - 1))
+    rest(4);
+  else if (truncation_ok(v[0].logR, k16))
     return v;
-  }
+  else if (k >= 2)
+    rest(8);
+  else
+    parts.push_back(8);
   v.clear();
   int logS = L;
   for (int part : parts) {
@@ -506,22 +519,55 @@ std::vector<PassPlan> plan_kept(int L, int kh, uint64_t nprod = 1) {
   return v;
 }
 
-// Eighths of 2^L points that a product of `size` limbs keeps (2^(L-1) < size
-// <= 2^L): transforms of one contiguous pass (L <= 12) are whole, and so is
-// every one with chunking off (hg_set_chunking).
-std::atomic<int> g_chunking{1};  // hg_set_chunking
-int plan_eighths(int L, uint64_t size, bool whole = false) {
-  if (whole || L <= kTileBits || !g_chunking.load()) return 8;
-  const uint64_t eighth = uint64_t(1) << (L - 3);
-  const uint64_t kh = (size + eighth - 1) / eighth;
-  return kh < 5 ? 5 : static_cast<int>(kh);
+// Sixteenths of 2^L points that n coefficients keep (2^(L-1) < n <= 2^L):
+// transforms of one contiguous pass (L <= 12) are whole; 2^16, 2^17 and 2^19
+// points keep an even number (a 7-bit outer pass; an odd number's 4- or 8-bit
+// one made 2^16 points 36.9 us instead of 28.5).
+int plan_sixteenths(int L, uint64_t n) {
+  if (L <= kTileBits) return 16;
+  const uint64_t part = uint64_t(1) << (L - 4);
+  int k = static_cast<int>((n + part - 1) / part);
+  if (k < 9) k = 9;
+  return L == 16 || L == 17 || L == 19 ? (k + 1) & ~1 : k;
 }
 
-TransformPlan plan_transform(int L, uint64_t size, bool whole = false) {
+// Cost of a transform of `points` of 2^L points in units of one radix-2 stage over one
+// point: L stages plus about kPassCost stages' worth of memory passes.  On
+// GB300 the measured time of chunked products is 0.93-0.97 of this model's
+// ratio to one transform (2^16..2^25 long operands, ratios 0.17-0.80).
+constexpr double kPassCost = 4.0;
+double transform_cost(int L, int k16) { return static_cast<double>(kept_points(L, k16)) * (L + kPassCost); }
+
+// Digits of 80 bits: the largest shorter operand whose coefficients stay below
+// p0 p1 p2 (2^187.09 > 2^160 2^27), and how much cheaper the transform has to
+// be.  Below 2^17 limbs a product is bound by latency and forming digits only
+// adds to it (2^16 limbs: 36.3 us, 28.5 without); up to 2^19 whole waves of
+// CTAs count, not points (2^19 limbs, 14/16 of the points: 97.4 us, 93.5
+// without; 5/8 of that, 4/5 of the points: 61.8 and 75.5).  Products that fill
+// the GPU together (busy) gain by their points at every length.
+constexpr uint64_t kMaxDigits = uint64_t(1) << 27;
+constexpr int kMinDigitL = 17;
+double digit_gain(int L, bool busy) { return L <= 19 && !busy ? 0.85 : 0.97; }
+
+std::atomic<int> g_chunking{1};  // hg_set_chunking
+
+// The transform of an nx x ny-limb product.  whole (or with chunking off): the
+// reference's, of the power of two above nx + ny points on limbs.
+TransformPlan plan_product(uint64_t nx, uint64_t ny, bool whole = false, bool busy = false) {
   TransformPlan t;
-  t.L = L;
-  t.kh = plan_eighths(L, size, whole);
-  t.passes = plan_kept(L, t.kh);
+  t.L = ilog2_ceil(nx + ny);
+  if (whole || t.L <= kTileBits || !g_chunking.load()) return t;
+  t.k16 = plan_sixteenths(t.L, nx + ny);
+  const uint64_t dx = coefs_of(nx, true), dy = coefs_of(ny, true);
+  const int L = ilog2_ceil(dx + dy);
+  if (L > kTileBits && (busy || t.L >= kMinDigitL) && std::min(dx, dy) <= kMaxDigits) {
+    const int k = plan_sixteenths(L, dx + dy);
+    if (transform_cost(L, k) < digit_gain(t.L, busy) * transform_cost(t.L, t.k16)) {
+      t.L = L;
+      t.k16 = k;
+      t.dig80 = true;
+    }
+  }
   return t;
 }
 
@@ -782,42 +828,53 @@ int check_len(int L) {
 // product is the same integer: sum_k chunk_k * short * 2^(64 C k)).
 struct ChunkPlan {
   int L = 0;
-  uint64_t chunk = 0, nchunks = 0;
+  uint64_t chunk = 0, nchunks = 0;  // chunk in limbs
+  int k16 = 16;        // a chunk's transform, as in TransformPlan
+  bool dig80 = false;
 };
 
-// Cost of a transform of 2^L points in units of one radix-2 stage over one
-// point: L stages plus about kPassCost stages' worth of memory passes.  On
-// GB300 the measured time of chunked products is 0.93-0.97 of this model's
-// ratio to one transform (2^16..2^25 long operands, ratios 0.17-0.80).
-constexpr double kPassCost = 4.0;
-// Chunk only when the estimate is below this fraction of one transform.
+// Chunk when the estimate is below this fraction of one transform, or when a
+// pair is so unbalanced that this holds for whole transforms and chunks are
+// within kChunkLoss of one cut transform: the model's error there, and the
+// chunks' workspace is smaller (hg_chunk_plan's pairs stay chunked).
 constexpr double kChunkGain = 0.95;
+constexpr double kChunkLoss = 1.10;
 
 // The cheapest chunking of a long operand of nl limbs and a short one of ns
 // <= nl limbs, or false when one transform of the whole product is cheaper.
 // C = (2^L - ns) rounded down to a multiple of 8 (>= 2^(L-1) because
 // 2^L >= 2 pow2(ns) >= 16), so that at most two chunk products meet at any
-// position of the result.
+// position of the result.  Where it can be a multiple of 40 limbs (whole
+// 80-bit digits, a multiple of 8 of them) and still 2^(L-1), the chunks'
+// transforms run on digits and keep 13 of 16 parts (14 at 2^19 points).
 bool plan_chunks(uint64_t nl, uint64_t ns, ChunkPlan &cp) {
   if (ns == 0 || nl < ns || !g_chunking.load()) return false;
   const int Lf = ilog2_ceil(nl + ns);
-  const auto cost = [](double transforms, int L) { return transforms * std::ldexp(L + kPassCost, L); };
-  double best = kChunkGain * cost(3.0, Lf) / 8 * plan_eighths(Lf, nl + ns);
+  const TransformPlan one = plan_product(nl, ns);
+  const double single = 3.0 * transform_cost(one.L, one.k16), whole = 3.0 * transform_cost(Lf, 16);
+  double best = kChunkLoss * single;
+  bool unbalanced = false;
   bool found = false;
   const int Lmin = std::max(4, ilog2_ceil(ns) + 1);
   for (int L = Lmin; L < Lf && L <= Lmin + 4; ++L) {
     const uint64_t T = uint64_t(1) << L;
-    const uint64_t c = (T - ns) & ~uint64_t(7);
+    uint64_t c = (T - ns) & ~uint64_t(7);
+    const uint64_t c40 = (T - ns) / 40 * 40;
+    const bool dig80 = L > kTileBits && 2 * c40 >= T && coefs_of(ns, true) <= kMaxDigits / 2;
+    if (dig80) c = c40;
+    const int k16 = dig80 ? plan_sixteenths(L, coefs_of(c, true) + coefs_of(ns, true)) : 16;
     const uint64_t k = (nl + c - 1) / c;
     if (k < 2) continue;
-    const double e = cost(2.0 * static_cast<double>(k) + 1.0, L);
+    const double transforms = 2.0 * static_cast<double>(k) + 1.0;
+    const double e = transforms * transform_cost(L, k16);
+    unbalanced = unbalanced || transforms * transform_cost(L, 16) < kChunkGain * whole;
     if (e < best) {
       best = e;
-      cp = ChunkPlan{L, c, k};
+      cp = ChunkPlan{L, c, k, k16, dig80};
       found = true;
     }
   }
-  return found;
+  return found && (unbalanced || best < kChunkGain * single);
 }
 
 // The chunked schedule of ntt_product_device.  Chunk k's residues occupy
@@ -831,17 +888,18 @@ int chunk_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint
   const uint64_t *lng = x_long ? x : y, *sht = x_long ? y : x;
   const uint64_t nl = x_long ? nx : ny, ns = x_long ? ny : nx;
   const int L = cp.L;
-  const uint64_t T = uint64_t(1) << L;
-  const uint64_t slab = static_cast<uint64_t>(kPrimes) * T;
+  const uint64_t N = kept_points(L, cp.k16);
+  const uint64_t slab = static_cast<uint64_t>(kPrimes) * N;
   HG_CUDA(ws_acquire(st), "workspace ordering");
   if (c.lane->A.bytes < cp.nchunks * slab * 8 || c.lane->B.bytes < slab * 8) {
     HG_CUDA(cudaDeviceSynchronize(), "sync before workspace growth");
     HG_CUDA(c.lane->A.ensure(cp.nchunks * slab * 8), "workspace allocation");
     HG_CUDA(c.lane->B.ensure(slab * 8), "workspace allocation");
   }
-  const std::vector<PassPlan> plan = plan_passes(L);
+  const std::vector<PassPlan> plan = plan_kept(L, cp.k16, cp.nchunks);
   const bool one_pass = plan.size() == 1;
-  PassArgs a = base_args(L, 1);  // the chunks
+  PassArgs a = base_args(L, 1, N);  // the chunks
+  a.dig80 = cp.dig80;
   a.data[0] = c.lane->A.u64();
   a.data[1] = c.lane->B.u64();
   a.limbs[0] = lng;
@@ -849,7 +907,8 @@ int chunk_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint
   a.chunk = cp.chunk;
   a.nprod = cp.nchunks;
   a.ws_stride = slab;
-  PassArgs sp = base_args(L, 1);  // the short operand's spectrum
+  PassArgs sp = base_args(L, 1, N);  // the short operand's spectrum
+  sp.dig80 = cp.dig80;
   sp.data[0] = c.lane->B.u64();
   sp.limbs[0] = sht;
   sp.nlimbs[0] = ns;
@@ -874,7 +933,7 @@ int chunk_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint
     if (!one_pass) m.limbs[0] = nullptr;
     HG_CUDA(run_contig(m, plan.back(), kContigMulSpec, st), "middle pass");
   }
-  PassArgs inv = base_args(L, 1);
+  PassArgs inv = base_args(L, 1, N);
   inv.data[0] = c.lane->A.u64();
   inv.nprod = cp.nchunks;
   inv.ws_stride = slab;
@@ -884,13 +943,15 @@ int chunk_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint
   const uint64_t size = nx + ny;
   if (nout > size) HG_CUDA(cudaMemsetAsync(out + size, 0, (nout - size) * sizeof(uint64_t), st), "zero tail");
   ScanState ss;
-  rc = scan_state(carry_tiles(size), &ss);
+  const uint64_t ncoef = coefs_of(size, cp.dig80);
+  rc = scan_state(carry_tiles(ncoef), &ss);
   if (rc) return rc;
   uint64_t tiles = 0;
   {
-    ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(size), carry_short(size) ? 1 : 2);
-    HG_CUDA(launch_crt_carry_chunks(c.lane->A.u64(), slab, L, cp.chunk, cp.nchunks, crt_const(L, scaled), out, size,
-                                    ss, st, &tiles),
+    ProfScope ps(HG_KC_CARRY, st, 24.0 * static_cast<double>(ncoef) + 8.0 * static_cast<double>(size),
+                 carry_short(ncoef) ? 1 : 2);
+    HG_CUDA(launch_crt_carry_chunks(c.lane->A.u64(), slab, N, cp.dig80, coefs_of(cp.chunk, cp.dig80), cp.nchunks,
+                                    crt_const(L, scaled), out, size, ss, st, &tiles),
             "reconstruction");
   }
   HG_CUDA(ws_release(st), "workspace ordering");
@@ -957,10 +1018,11 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
     }
     return chunk_product_device(x, nx, y, ny, out, nout, cp, st, y_ready);
   }
-  const int L = ilog2_ceil(size);
-  int rc = check_len(L);
+  int rc = check_len(ilog2_ceil(size));
   if (rc) return rc;
-  const TransformPlan tp = plan_transform(L, size);
+  TransformPlan tp = plan_product(nx, ny);
+  tp.passes = plan_kept(tp.L, tp.k16);
+  const int L = tp.L;
   const uint64_t N = tp.points();
   const size_t words = static_cast<size_t>(kPrimes) * N;
   HG_CUDA(ws_acquire(st), "workspace ordering");
@@ -973,6 +1035,7 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
   // operands + pointwise product + first inverse pass), strided inverse passes.
   const std::vector<PassPlan> &plan = tp.passes;
   PassArgs a = base_args(L, square ? 1 : 2, N);
+  a.dig80 = tp.dig80;
   a.data[0] = c.lane->A.u64();
   a.data[1] = c.lane->B.u64();
   a.limbs[0] = x;
@@ -1001,10 +1064,10 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
   }
   if (host && plan.size() > 1 && L >= kSliceMinL) {
     // The first strided pass covers one block of 2^L = R S residues; its tile
-    // t reads columns [t C, (t + 1) C) (C = 4096 / R) of every row.
+    // t reads columns [t C, (t + 1) C) (C = 4096 / R) of every row, here in limbs.
     const PassPlan &p0 = plan[0];
-    const uint64_t S = uint64_t(1) << p0.logS;
-    const uint64_t C = uint64_t(1) << (kTileBits - p0.logR);
+    const uint64_t S = limbs_of(uint64_t(1) << p0.logS, tp.dig80);
+    const uint64_t C = limbs_of(uint64_t(1) << (kTileBits - p0.logR), tp.dig80);
     const uint64_t ntiles = (uint64_t(1) << L) >> kTileBits;
     const int K = static_cast<int>(std::min<uint64_t>(kUploadSlices, ntiles));
     const int nops = square ? 1 : 2;
@@ -1056,15 +1119,17 @@ int ntt_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64
   uint64_t sc[kPrimes];
   bool scaled = false;
   HG_CUDA(run_strided(inv, plan, true, st, prescale_factors(L, sc) ? sc : nullptr, &scaled), "inverse transform");
-  if (nout > N) HG_CUDA(cudaMemsetAsync(out + N, 0, (nout - N) * sizeof(uint64_t), st), "zero tail");
+  const uint64_t nl = limbs_of(N, tp.dig80);  // limbs the coefficients fill
+  if (nout > nl) HG_CUDA(cudaMemsetAsync(out + nl, 0, (nout - nl) * sizeof(uint64_t), st), "zero tail");
   ScanState ss;
-  const uint64_t nproc = nout < N ? nout : N;
-  rc = scan_state(carry_tiles(nproc), &ss);
+  const uint64_t nproc = nout < nl ? nout : nl, ncoef = coefs_of(nproc, tp.dig80);
+  rc = scan_state(carry_tiles(ncoef), &ss);
   if (rc) return rc;
   uint64_t tiles = 0;
   {
-    ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(nproc), carry_short(nproc) ? 1 : 2);
-    HG_CUDA(launch_crt_carry(c.lane->A.u64(), N, crt_const(L, scaled), out, nout, ss, st, &tiles),
+    ProfScope ps(HG_KC_CARRY, st, 24.0 * static_cast<double>(ncoef) + 8.0 * static_cast<double>(nproc),
+                 carry_short(ncoef) ? 1 : 2);
+    HG_CUDA(launch_crt_carry(c.lane->A.u64(), N, tp.dig80, crt_const(L, scaled), out, nout, ss, st, &tiles),
             "reconstruction");
   }
   HG_CUDA(ws_release(st), "workspace ordering");
@@ -1159,7 +1224,7 @@ int noalloc_product_device(const uint64_t *x, uint64_t nx, const uint64_t *y, ui
   ss.epoch = 1;
   ss.err = err_word();
   uint64_t used = 0;
-  HG_CUDA(launch_crt_carry(scratch, N, crt_const(L), out, nout, ss, st, &used), "reconstruction");
+  HG_CUDA(launch_crt_carry(scratch, N, false, crt_const(L), out, nout, ss, st, &used), "reconstruction");
   return HG_OK;
 }
 
@@ -1503,9 +1568,9 @@ int spectrum(uint64_t *a, size_t n, int mod_num, bool inverse, cudaStream_t st) 
 // Candidate pass splits of a 2^L transform: the default plan and, for
 // L >= 12, every contiguous block size T with the remaining L - T bits in
 // as few strided passes of 4..8 bits as possible (where the outer one can
-// keep kh eighths of its rows).
-std::vector<std::vector<PassPlan>> plan_candidates(int L, int kh, uint64_t nprod) {
-  std::vector<std::vector<PassPlan>> out{plan_kept(L, kh, nprod)};
+// keep k16 sixteenths of its rows).
+std::vector<std::vector<PassPlan>> plan_candidates(int L, int k16, uint64_t nprod) {
+  std::vector<std::vector<PassPlan>> out{plan_kept(L, k16, nprod)};
   if (L < kTileBits) return out;
   for (int T = 4; T <= kTileBits; ++T) {
     const int rem = L - T;
@@ -1522,7 +1587,7 @@ std::vector<std::vector<PassPlan>> plan_candidates(int L, int kh, uint64_t nprod
     // A strided pass over R rows needs columns of at least 2^(12 - logR)
     // words so that its 4096-word tile spans whole rows.
     if (logS + v.back().logR < kTileBits) continue;
-    if (!truncation_ok(v[0].logR, kh)) continue;
+    if (!truncation_ok(v[0].logR, k16)) continue;
     v.push_back({logS, 0, logS});
     bool same = v.size() == out[0].size();
     for (size_t i = 0; same && i < v.size(); ++i)
@@ -1532,15 +1597,18 @@ std::vector<std::vector<PassPlan>> plan_candidates(int L, int kh, uint64_t nprod
   return out;
 }
 
-// Schedules chosen by timing, keyed by (L, eighths kept, square, products in the group).
+// Schedules chosen by timing, keyed by (L, sixteenths kept, digits, square, products in the group).
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, bool, uint64_t>, std::vector<PassPlan>> g_tuned;
+std::map<std::tuple<int, int, bool, bool, uint64_t>, std::vector<PassPlan>> g_tuned;
+auto tune_key(const BatchGroup &g) { return std::make_tuple(g.L, g.k16, g.dig80, g.square, g.nprod); }
 
 }  // namespace
 }  // namespace hg
 
 struct hg_batch {
-  hg::BatchPlan bp;
+  hg::BatchPlan bp;     // one launch per pass
+  hg::BatchPlan whole;  // the persistent schedule's groups: whole transforms on limbs
+  hg::DevBuf d_whole;   // device copy of whole.desc
   hg::DevBuf d_desc, ws, flags, tickets;
   hg::SideStreams side;
   // The persistent schedule: its work list and its counters.
@@ -1559,12 +1627,13 @@ namespace {
 int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::vector<PassPlan> &plan,
               cudaStream_t st) {
   const int nops = g.square ? 1 : 2;
-  const uint64_t N = kept_points(g.L, g.kh);
+  const uint64_t N = kept_points(g.L, g.k16);
   const uint64_t slab = static_cast<uint64_t>(kPrimes) * N;
   const ProductDesc *d = bb.desc + g.first;
   uint64_t *ws = bb.ws + g.ws_off;
-  if (g.tails) HG_CUDA(launch_zero_tails(d, g.nprod, N, st), "zero tails");
+  if (g.tails) HG_CUDA(launch_zero_tails(d, g.nprod, limbs_of(N, g.dig80), st), "zero tails");
   PassArgs a = base_args(g.L, nops, N);
+  a.dig80 = g.dig80;
   a.err = bb.err;
   a.batch = d;
   a.read_limbs = 1;
@@ -1593,7 +1662,7 @@ int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::ve
   {
     ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(N) * static_cast<double>(g.nprod),
                  carry_short(N, g.nprod) ? 1 : 2);
-    HG_CUDA(launch_crt_carry_batch(ws, slab, N, crt_const(g.L, scaled), d, g.nprod, ss, st), "reconstruction");
+    HG_CUDA(launch_crt_carry_batch(ws, slab, N, g.dig80, crt_const(g.L, scaled), d, g.nprod, ss, st), "reconstruction");
   }
   return HG_OK;
 }
@@ -1611,33 +1680,23 @@ BatchBufs batch_bufs(hg_batch *b) {
 // one, with the same arguments.
 constexpr uint64_t kPersistWorkspaceCap = uint64_t(16) << 30;  // bytes
 
-// The persistent schedule's groups: whole transforms, all products of one
-// length and kind together (they are contiguous in the descriptors).  Its
+// The persistent schedule's groups: all products of one length and kind
+// together (they are contiguous in the descriptors of the whole plan).  Its
 // phases run the per-thread-load bodies, whose outer inverse pass is not
 // truncated.
-std::vector<BatchGroup> persist_groups(const BatchPlan &bp) {
+std::vector<BatchGroup> persist_groups(const BatchPlan &whole) {
   std::vector<BatchGroup> v;
-  uint64_t tuned = 0;  // products of the part whose tuned plan the group takes
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  for (const BatchGroup &g : bp.groups) {
+  for (const BatchGroup &g : whole.groups) {
     if (v.empty() || v.back().L != g.L || v.back().square != g.square) {
       v.push_back(g);
-      v.back().kh = 8;
-      v.back().tails = false;
-      v.back().nprod = 0;
-      v.back().plan = plan_passes(g.L);
-      tuned = 0;
-    }
-    v.back().nprod += g.nprod;
-    const auto it = g_tuned.find(std::make_tuple(g.L, g.kh, g.square, g.nprod));
-    if (it != g_tuned.end() && g.nprod > tuned) {
-      v.back().plan = it->second;
-      tuned = g.nprod;
+      const auto it = g_tuned.find(tune_key(g));
+      if (it != g_tuned.end()) v.back().plan = it->second;
+    } else {
+      v.back().nprod += g.nprod;
+      v.back().tails = v.back().tails || g.tails;
     }
   }
-  for (BatchGroup &g : v)
-    for (uint64_t k = g.first; k < g.first + g.nprod; ++k)
-      if (bp.desc[k].nout > (uint64_t(1) << g.L)) g.tails = true;
   return v;
 }
 
@@ -1757,7 +1816,7 @@ std::vector<PersistPhase> group_phases(const BatchGroup &g, const BatchBufs &bb,
 int persist_build(hg_batch *b) {
   b->phases.clear();
   b->items = 0;
-  const BatchPlan &bp = b->bp;
+  const BatchPlan &bp = b->whole;
   if (bp.groups.empty() || !persist_grid()) return HG_OK;
   const std::vector<BatchGroup> groups = persist_groups(bp);
   const PersistLayout l = persist_layout(groups);
@@ -1765,7 +1824,8 @@ int persist_build(hg_batch *b) {
   if (b->ws.bytes < l.ws_words * 8) HG_CUDA(b->ws.ensure(l.ws_words * 8), "batch workspace");
   if (b->flags.bytes < l.flag_words * 8) HG_CUDA(b->flags.ensure(l.flag_words * 8), "batch scan flags");
   b->persist_flag_words = l.flag_words;
-  const BatchBufs bb = batch_bufs(b);
+  BatchBufs bb = batch_bufs(b);
+  bb.desc = static_cast<const ProductDesc *>(b->d_whole.p);
   std::vector<std::vector<PersistPhase>> per;
   std::vector<PersistPhase> indep;  // zeroing: waits for nothing
   for (size_t gi = 0; gi < groups.size(); ++gi) {
@@ -1846,7 +1906,7 @@ int batch_autotune(hg_batch *b) {
   const BatchBufs bb = batch_bufs(b);
   for (size_t gi = 0; gi < b->bp.groups.size() && rc == HG_OK; ++gi) {
     BatchGroup &g = b->bp.groups[gi];
-    const auto key = std::make_tuple(g.L, g.kh, g.square, g.nprod);
+    const auto key = tune_key(g);
     {
       std::lock_guard<std::mutex> lk(g_tune_mu);
       auto it = g_tuned.find(key);
@@ -1855,7 +1915,7 @@ int batch_autotune(hg_batch *b) {
         continue;
       }
     }
-    const auto cands = plan_candidates(g.L, g.kh, g.nprod);
+    const auto cands = plan_candidates(g.L, g.k16, g.nprod);
     float best = 1e30f;
     for (const auto &plan : cands) {
       float ms = 0;
@@ -1959,11 +2019,17 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
   } else {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     for (BatchGroup &g : b->bp.groups) {
-      auto it = g_tuned.find(std::make_tuple(g.L, g.kh, g.square, g.nprod));
+      auto it = g_tuned.find(tune_key(g));
       if (it != g_tuned.end()) g.plan = it->second;
     }
   }
   if (!(flags & HG_BATCH_PER_PASS)) {
+    if ((rc = plan_batch(items.data(), items.size(), kBatchWorkspaceCap, b->whole, true))) return rc;
+    if (!b->whole.desc.empty()) {
+      const size_t bytes = b->whole.desc.size() * sizeof(ProductDesc);
+      HG_CUDA(b->d_whole.ensure(bytes), "batch descriptors");
+      HG_CUDA(cudaMemcpy(b->d_whole.p, b->whole.desc.data(), bytes, cudaMemcpyHostToDevice), "batch descriptors upload");
+    }
     if ((rc = persist_build(b.get()))) return rc;
     b->persistent = b->items > 0;
     if ((flags & HG_BATCH_PERSISTENT) && !b->persistent && !b->bp.groups.empty())
@@ -1992,26 +2058,32 @@ uint64_t product_workspace_bytes(uint64_t nx, uint64_t ny, bool square) {
 }
 
 // Points a batch's cut must save per prime and operand to be a group of its
-// own.  The 4096-pair batch takes 3316, 3281 and 3231 us at 2^19, 2^18 and
-// 2^17, 1024 pairs 974, 959 and 929; 300 pairs of 2^12 to 2^14 limbs 753, 772
-// and 786.
+// own.  The 4096-pair batch takes 3081, 2908, 2914 and 2877 us at 2^20 down to
+// 2^17, 1024 pairs 855, 877, 878 and 828; 300 pairs of 2^12 to 2^14 limbs 646,
+// 646, 646 and 671.
 constexpr uint64_t kCutPoints = uint64_t(1) << 17;
+
+// Tiles of 4096 residues (three primes, one operand) that fill the GPU several times.
+constexpr uint64_t kBusyTiles = 4 * kIdleTiles;
 
 // What a chain of launches costs beside its residues, in the same units as
 // their stages (points x (L + 4)): about 30 us.
 constexpr double kChainWork = 4e7;
 
-int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchPlan &bp) {
+int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchPlan &bp, bool whole) {
   bp = BatchPlan();
   struct Item {
     int L;
-    bool square;
-    int kh;
+    bool square, dig80;
+    int k16;
     size_t i;
+    // Whether the two share transforms, whatever they keep of them.
+    bool like(const Item &o) const { return L == o.L && square == o.square && dig80 == o.dig80; }
   };
   std::vector<Item> live;
   std::vector<size_t> zeros;
   uint64_t ws_all = 0;  // words of all groups together
+  uint64_t per_length[kLogNmax + 1] = {};  // products by the bits of their length in limbs
   live.reserve(n);
   for (size_t i = 0; i < n; ++i) {
     const ProductDesc &p = items[i];
@@ -2021,10 +2093,18 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
       continue;
     }
     const int L = ilog2_ceil(p.nx + p.ny);
-    live.push_back({L, square, plan_eighths(L, p.nx + p.ny), i});
+    if (L <= kLogNmax) per_length[L] += 1;
+    live.push_back({L, square, false, 16, i});
+  }
+  for (Item &it : live) {
+    const bool busy = (3 * per_length[std::min(it.L, kLogNmax)] << it.L) >> kTileBits > kBusyTiles;
+    const TransformPlan t = plan_product(items[it.i].nx, items[it.i].ny, whole, busy);
+    it.L = t.L;
+    it.dig80 = t.dig80;
+    it.k16 = t.k16;
   }
   std::stable_sort(live.begin(), live.end(), [](const Item &a, const Item &c) {
-    return a.L != c.L ? a.L < c.L : a.square != c.square ? a.square < c.square : a.kh < c.kh;
+    return std::make_tuple(a.L, a.square, a.dig80, a.k16) < std::make_tuple(c.L, c.square, c.dig80, c.k16);
   });
   // Every group is a chain of launches that depend on each other, so a cut
   // that few products would use is not worth a group of its own: they join
@@ -2032,12 +2112,12 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
   // kCutPoints points more.
   for (size_t s = 0; s < live.size();) {
     size_t e = s;
-    while (e < live.size() && live[e].L == live[s].L && live[e].square == live[s].square) ++e;
+    while (e < live.size() && live[e].like(live[s])) ++e;
     for (size_t c = s; c < e;) {
       size_t d = c;
-      while (d < e && live[d].kh == live[c].kh) ++d;
-      if (d < e && (static_cast<uint64_t>(d - c) * (live[d].kh - live[c].kh) << live[c].L) / 8 < kCutPoints)
-        for (size_t k = c; k < d; ++k) live[k].kh = live[d].kh;
+      while (d < e && live[d].k16 == live[c].k16) ++d;
+      if (d < e && (static_cast<uint64_t>(d - c) * (live[d].k16 - live[c].k16) << live[c].L) / 16 < kCutPoints)
+        for (size_t k = c; k < d; ++k) live[k].k16 = live[d].k16;
       else
         c = d;
     }
@@ -2046,29 +2126,32 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
   bp.desc.reserve(n);
   for (size_t s = 0; s < live.size();) {
     size_t e = s;
-    while (e < live.size() && live[e].L == live[s].L && live[e].square == live[s].square && live[e].kh == live[s].kh)
-      ++e;
+    while (e < live.size() && live[e].like(live[s]) && live[e].k16 == live[s].k16) ++e;
     const int L = live[s].L;
     const bool square = live[s].square;
-    const uint64_t N = kept_points(L, live[s].kh);
+    const uint64_t N = kept_points(L, live[s].k16);
     const uint64_t per = static_cast<uint64_t>(square ? 1 : 2) * kPrimes * N * 8;
-    const uint64_t whole = (static_cast<uint64_t>(square ? 1 : 2) * kPrimes * 8) << L;
-    if (whole > ws_cap_bytes)
-      return fail(HG_ERR_ARG, "a 2^%d-point product needs %llu workspace bytes, more than the %llu available", L,
-                  (unsigned long long)whole, (unsigned long long)ws_cap_bytes);
+    for (size_t k = s; k < e; ++k) {  // refused by the workspace of the whole transform, whatever runs
+      const ProductDesc &p = items[live[k].i];
+      const uint64_t full = product_workspace_bytes(p.nx, p.ny, square);
+      if (full > ws_cap_bytes)
+        return fail(HG_ERR_ARG, "a 2^%d-point product needs %llu workspace bytes, more than the %llu available",
+                    ilog2_ceil(p.nx + p.ny), (unsigned long long)full, (unsigned long long)ws_cap_bytes);
+    }
     const uint64_t chunk = std::max<uint64_t>(1, ws_cap_bytes / per);
     for (size_t c = s; c < e; c += chunk) {
       BatchGroup g;
       g.L = L;
       g.square = square;
-      g.kh = live[s].kh;
-      g.plan = plan_kept(L, g.kh, g.nprod);
+      g.k16 = live[s].k16;
+      g.dig80 = live[s].dig80;
       g.first = bp.desc.size();
       g.nprod = std::min<uint64_t>(chunk, e - c);
+      g.plan = whole ? plan_passes(L) : plan_kept(L, g.k16, g.nprod);
       g.flags_off = bp.flag_words;
       for (size_t k = c; k < c + g.nprod; ++k) {
         bp.desc.push_back(items[live[k].i]);
-        if (bp.desc.back().nout > N) g.tails = true;
+        if (bp.desc.back().nout > limbs_of(N, g.dig80)) g.tails = true;
       }
       bp.flag_words += carry_tiles(N, g.nprod) * g.nprod;
       g.ws_off = ws_all;
@@ -2130,7 +2213,7 @@ int enqueue_batch(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st) {
   const int ns = std::min<int>(side.n + 1, static_cast<int>(ng));  // st and ns - 1 side streams
   const auto work = [&](size_t gi) {
     const BatchGroup &g = bp.groups[gi];
-    return static_cast<double>(kept_points(g.L, g.kh)) * static_cast<double>(g.nprod) * (g.L + 4) * (g.square ? 2 : 3) +
+    return static_cast<double>(kept_points(g.L, g.k16)) * static_cast<double>(g.nprod) * (g.L + 4) * (g.square ? 2 : 3) +
            kChainWork;
   };
   std::vector<size_t> order(ng);
@@ -2265,7 +2348,7 @@ int hg_batch_schedule(const hg_batch *batch, int *persistent, size_t *launches) 
   size_t n = batch->bp.nzero ? 1 : 0;
   for (const hg::BatchGroup &g : batch->bp.groups)
     n += (g.tails ? 1 : 0) + 2 * (g.plan.size() - 1) + 1  // zero tails, passes, middle, carry (+ fix)
-         + (hg::carry_short(hg::kept_points(g.L, g.kh), g.nprod) ? 1 : 2);
+         + (hg::carry_short(hg::kept_points(g.L, g.k16), g.nprod) ? 1 : 2);
   *launches = n;
   return HG_OK;
 }
@@ -2276,6 +2359,7 @@ int hg_batch_destroy(hg_batch *batch) {
   batch->d_phases.release();
   batch->d_state.release();
   batch->d_desc.release();
+  batch->d_whole.release();
   batch->ws.release();
   batch->flags.release();
   batch->tickets.release();

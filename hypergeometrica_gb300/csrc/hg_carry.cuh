@@ -262,6 +262,144 @@ __device__ __forceinline__ void carry_body(const Producer &prod, uint64_t *__res
   }
 }
 
+// carry_body for coefficients that are 80-bit digits: position i of the sum is
+// worth 2^(80 i), and four positions fill five limbs.  Each coefficient splits
+// into three pieces of 80 bits (the third below 2^28), the pieces that meet at
+// a position add up to less than 2^82, and position i's digit before carries
+// is that sum's low 80 bits plus the bits past 80 of position i - 1: at most
+// one carry, as with limbs.  A tile of NT * PER positions is NT * PER * 5/4
+// limbs; a thread passes its neighbour the pieces of its last positions.
+// nproc is in limbs; limbs the digits fill past it must be zero.
+template <class Producer, int NT, int PER>
+__device__ __forceinline__ void carry80_body(const Producer &prod, uint64_t *__restrict__ out, uint64_t nproc,
+                                             const ScanState &ss, const ProductDesc *batch, uint64_t tpp,
+                                             uint64_t ws_stride, uint64_t n, uint64_t gt, uint64_t *s_buf, GP *s_warp) {
+  constexpr int kTile = NT * PER, kOut = PER / 4 * 5;  // digits per tile, limbs per thread
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  uint64_t tile = gt, off = 0;
+  if (batch) {
+    const uint64_t k = gt / tpp;
+    tile = gt - k * tpp;
+    off = k * ws_stride;
+    out = batch[k].out;
+    nproc = batch[k].nout < limbs_of(n, true) ? batch[k].nout : limbs_of(n, true);
+  }
+  const uint64_t ndig = coefs_of(nproc, true);
+  const uint64_t i0 = tile * kTile + static_cast<uint64_t>(tid) * PER;
+  V3 v[PER];
+  prod.template many<PER>(off, i0, ndig, v);
+  // Pieces of a coefficient: bits 0..79 (w0 and the low 16 bits of w1), 80..159, 160...
+  const auto lo1 = [](const V3 &x) { return (x.w1 >> 16) | (x.w2 << 48); };
+  const auto hi1 = [](const V3 &x) { return static_cast<uint32_t>(x.w2 >> 16) & 0xffffu; };
+  const auto lo2 = [](const V3 &x) { return static_cast<uint32_t>(x.w2 >> 32); };
+  // The sum at a position: c0's first piece, c1's second, c2's third.
+  const auto sum = [&](const V3 &c0, uint64_t b1, uint32_t b1h, uint32_t b2, uint32_t &hi) {
+    uint64_t lo = c0.w0 + b1;
+    hi = (static_cast<uint32_t>(c0.w1) & 0xffffu) + b1h + (lo < b1 ? 1u : 0u);
+    lo += b2;
+    hi += lo < b2 ? 1u : 0u;
+    return lo;
+  };
+  // To the next thread: the last position's second piece, the third pieces of
+  // the last two, and the bits past 80 of the last position's sum.
+  uint64_t *s_prev = s_buf;  // [NT][3]
+  {
+    uint32_t h;
+    (void)sum(v[PER - 1], lo1(v[PER - 2]), hi1(v[PER - 2]), lo2(v[PER - 3]), h);
+    s_prev[3 * tid] = lo1(v[PER - 1]);
+    s_prev[3 * tid + 1] = hi1(v[PER - 1]) | (static_cast<uint64_t>(h >> 16) << 32);
+    s_prev[3 * tid + 2] = lo2(v[PER - 1]) | (static_cast<uint64_t>(lo2(v[PER - 2])) << 32);
+  }
+  uint64_t b1 = 0;                    // second piece of the position below
+  uint32_t b1h = 0, b2 = 0, b3 = 0;   // its high bits; third pieces of the two below
+  uint32_t hp = 0;                    // bits past 80 of the sum below
+  if (tid == 0 && i0 >= 3) {
+    const V3 q3 = prod.at(off, i0 - 3), q2 = prod.at(off, i0 - 2), q1 = prod.at(off, i0 - 1);
+    uint32_t h;
+    (void)sum(q1, lo1(q2), hi1(q2), lo2(q3), h);
+    b1 = lo1(q1);
+    b1h = hi1(q1);
+    b2 = lo2(q2);
+    b3 = lo2(q1);
+    hp = h >> 16;
+  }
+  __syncthreads();
+  if (tid > 0) {
+    b1 = s_prev[3 * tid - 3];
+    const uint64_t a = s_prev[3 * tid - 2], c = s_prev[3 * tid - 1];
+    b1h = static_cast<uint32_t>(a);
+    hp = static_cast<uint32_t>(a >> 32);
+    b3 = static_cast<uint32_t>(c);
+    b2 = static_cast<uint32_t>(c >> 32);
+  }
+  uint64_t al[PER];
+  uint32_t ah[PER];  // the digit's bits 64..79
+  uint32_t gbits = 0, pbits = 0;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    uint32_t h;
+    const uint64_t lo = sum(v[k], k ? lo1(v[k - 1]) : b1, k ? hi1(v[k - 1]) : b1h, k >= 2 ? lo2(v[k - 2]) : (k ? b3 : b2), h);
+    const uint64_t a = lo + hp;
+    hp = h >> 16;
+    h = (h & 0xffffu) + (a < lo ? 1u : 0u);
+    al[k] = a;
+    ah[k] = h & 0xffffu;
+    gbits |= (h >> 16) << k;
+    pbits |= (a == ~0ull && h == 0xffffu ? 1u : 0u) << k;
+  }
+  GP t{0, 1};
+#pragma unroll
+  for (int k = 0; k < PER; ++k) t = gp_compose(t, GP{(gbits >> k) & 1u, (pbits >> k) & 1u});
+  GP inc = t;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t og = __shfl_up_sync(0xffffffffu, inc.g, d);
+    const uint32_t op = __shfl_up_sync(0xffffffffu, inc.p, d);
+    if (lane >= d) inc = gp_compose(GP{og, op}, inc);
+  }
+  if (lane == 31) s_warp[wid] = inc;
+  __syncthreads();  // also: every thread has read s_prev
+  GP wpre{0, 1};
+  for (int w = 0; w < wid; ++w) wpre = gp_compose(wpre, s_warp[w]);
+  const uint32_t og = __shfl_up_sync(0xffffffffu, inc.g, 1);
+  const uint32_t op = __shfl_up_sync(0xffffffffu, inc.p, 1);
+  const GP excl = gp_compose(wpre, lane == 0 ? GP{0, 1} : GP{og, op});
+  if (tid == 0) {
+    GP agg{0, 1};
+    for (int w = 0; w < NT / 32; ++w) agg = gp_compose(agg, s_warp[w]);
+    ss.flags[gt] = flag_word(ss.epoch, agg.g, agg.p);
+  }
+  uint32_t cin = excl.g;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {  // the digits with their carries (mod 2^80)
+    const uint64_t z = al[k] + cin;
+    ah[k] = (ah[k] + (z < al[k] ? 1u : 0u)) & 0xffffu;
+    al[k] = z;
+    cin = ((gbits >> k) & 1u) | (((pbits >> k) & 1u) & cin);
+  }
+  uint64_t *s_out = s_buf;
+#pragma unroll
+  for (int q = 0; q < PER; q += 4) {
+    uint64_t *o = s_out + tid * kOut + q / 4 * 5;
+    o[0] = al[q];
+    o[1] = ah[q] | (al[q + 1] << 16);
+    o[2] = (al[q + 1] >> 48) | (static_cast<uint64_t>(ah[q + 1]) << 16) | (al[q + 2] << 32);
+    o[3] = (al[q + 2] >> 32) | (static_cast<uint64_t>(ah[q + 2]) << 32) | (al[q + 3] << 48);
+    o[4] = (al[q + 3] >> 16) | (static_cast<uint64_t>(ah[q + 3]) << 48);
+  }
+  __syncthreads();
+  const uint64_t tbase = tile * (kTile / 4 * 5);
+#pragma unroll
+  for (int k = 0; k < kOut; ++k) {
+    const uint32_t w = static_cast<uint32_t>(tid + k * NT);
+    const uint64_t z = s_out[w];
+    if (tbase + w < nproc)
+      out[tbase + w] = z;
+    else if (z)
+      latch_error(ss.err, kDevCarryOverflow);
+  }
+}
+
 // The second launch of a carry, one warp per tile.  Tile t's carry-in is
 // the composition of the aggregates of tiles t - 1, t - 2, ... up to the
 // nearest one that does not propagate (p = 0), or 0 before the product's
@@ -278,7 +416,11 @@ __device__ __forceinline__ void carry_body(const Producer &prod, uint64_t *__res
 // become 0 and the first limb after them gains 1; a tile that is one run
 // becomes 0 and passes the carry on, as its p = 1 aggregate already says.
 //
-// fix_body is one warp on tile gt of TILE positions.
+// With 80-bit digits a tile is TILE limbs too, all ones exactly when every
+// digit is, so the same holds.
+//
+// fix_body is one warp on tile gt of TILE limbs; a batch's product has at most
+// n limbs.
 constexpr int kFixWarps = 8;
 
 template <int TILE>

@@ -28,7 +28,7 @@ constexpr int kPerThread = 16;  // residues held in registers per thread
 struct PrimeConst {
   uint64_t p;
   uint32_t c;  // p = c * 2^55 + 1
-  uint32_t pad;
+  uint32_t m;  // ceil(2^39 / c): floor(t / c) = (t * m) >> 39 for t < 2^25
 };
 
 // Device error word codes (latched with atomicCAS; first error wins).
@@ -276,6 +276,17 @@ __device__ __forceinline__ uint64_t shoup_mul(uint64_t a, uint64_t w, uint64_t w
 // 2^63, so the first correction compares).
 __device__ __forceinline__ uint64_t reduce64(uint64_t x, uint64_t p) {
   return fold_p(fold_any(x, p << 1), p);
+}
+
+// (hi 2^64 + lo) mod p for hi < 2^16.  With t = floor(v / 2^55) < 2^25, q =
+// floor(t / c) = floor(v / (c 2^55)) is floor(v / p) or one more (p = c 2^55 +
+// 1), so v - q p lies in [-p, p): its sign says whether to add p.  q p mod
+// 2^64 = q + ((q c) mod 2^9) 2^55.
+__device__ __forceinline__ uint64_t reduce80(uint64_t lo, uint32_t hi, const PrimeConst &pc) {
+  const uint32_t t = (hi << 9) | static_cast<uint32_t>(lo >> 55);
+  const uint32_t q = __umulhi(t, pc.m) >> 7;
+  const uint64_t r = lo - q - (static_cast<uint64_t>(q * (pc.c << 23)) << 32);
+  return static_cast<int64_t>(r) < 0 ? r + pc.p : r;
 }
 
 // Carry-lookahead pair for the final carry scan: with carry-in c, a

@@ -236,15 +236,27 @@ __global__ void sum_finish_kernel(const uint64_t *out, uint64_t nproc, SumProduc
   w->top_diff = -1;
 }
 
-// One tile per CTA.
-template <class Producer>
+// One tile per CTA, of PER coefficients per thread (limbs, or 80-bit digits).
+template <class Producer, bool D80, int PER>
+__device__ __forceinline__ void carry_tile(const Producer &prod0, uint64_t *out, uint64_t nproc, const ScanState &ss,
+                                           const ProductDesc *batch, uint64_t tpp, uint64_t ws_stride, uint64_t n,
+                                           uint64_t *s_buf, GP *s_warp) {
+  if constexpr (D80)
+    carry80_body<Producer, kCarryThreads, PER>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, blockIdx.x, s_buf,
+                                               s_warp);
+  else
+    carry_body<Producer, kCarryThreads, PER>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, blockIdx.x,
+                                             reinterpret_cast<uint64_t(*)[9]>(s_buf), s_warp);
+}
+
+template <class Producer, bool D80>
 __global__ void __launch_bounds__(kCarryThreads, kCarryMinBlocks)
     carry_kernel(const Producer prod0, uint64_t *__restrict__ out, uint64_t nproc, ScanState ss,
                  const ProductDesc *batch, uint64_t tpp, uint64_t ws_stride, uint64_t n) {
-  __shared__ uint64_t s_prev[kCarryThreads][9];
+  __shared__ uint64_t s_buf[kCarryThreads * (D80 ? 10 : 9)];
   __shared__ GP s_warp[kCarryThreads / 32];
   pdl_wait();
-  carry_body<Producer, kCarryThreads>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, blockIdx.x, s_prev, s_warp);
+  carry_tile<Producer, D80, kCarryPer>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, s_buf, s_warp);
 }
 
 // The carries of a whole short launch, by the CTA that finished last: thread
@@ -252,6 +264,7 @@ __global__ void __launch_bounds__(kCarryThreads, kCarryMinBlocks)
 // below (fix_body says why only the tile's leading limbs equal to 2^64 - 1
 // and the first limb after them change).  Most tiles are done by their
 // thread's first limb; the others go to whole warps.
+template <int TILE>
 __device__ __forceinline__ void fix_all(uint64_t *out, uint64_t nproc, uint64_t tiles, const ScanState &ss,
                                         bool drop_top, const ProductDesc *batch, uint64_t tpp, uint64_t n,
                                         GP *s_warp, uint32_t *s_long) {
@@ -264,7 +277,7 @@ __device__ __forceinline__ void fix_all(uint64_t *out, uint64_t nproc, uint64_t 
     out = batch[k].out;
     nproc = batch[k].nout < n ? batch[k].nout : n;
   }
-  const uint64_t ntiles = carry_tiles_dev<kShortTile>(nproc);
+  const uint64_t ntiles = carry_tiles_dev<TILE>(nproc);
   const bool live = gt < tiles && t < ntiles;
   GP own{0, 0};
   if (live) {
@@ -290,9 +303,9 @@ __device__ __forceinline__ void fix_all(uint64_t *out, uint64_t nproc, uint64_t 
   const uint32_t cin = live && t > 0 ? below.g : 0;
   if (live && t == ntiles - 1 && !drop_top && (own.g | (own.p & cin))) atomicCAS(ss.err, kDevOk, kDevCarryOverflow);
   if (cin) {
-    const uint64_t w = __ldcg(out + t * kShortTile);
+    const uint64_t w = __ldcg(out + t * TILE);
     if (w != ~0ull)
-      out[t * kShortTile] = w + 1;
+      out[t * TILE] = w + 1;
     else
       s_long[tid] = 1;
   }
@@ -307,8 +320,8 @@ __device__ __forceinline__ void fix_all(uint64_t *out, uint64_t nproc, uint64_t 
       o = batch[pr].out;
       np = batch[pr].nout < n ? batch[pr].nout : n;
     }
-    const uint64_t end = (tile + 1) * kShortTile < np ? (tile + 1) * kShortTile : np;
-    for (uint64_t i = tile * kShortTile; i < end; i += 32) {
+    const uint64_t end = (tile + 1) * TILE < np ? (tile + 1) * TILE : np;
+    for (uint64_t i = tile * TILE; i < end; i += 32) {
       const uint64_t at = i + lane;
       const uint64_t w = at < end ? __ldcg(o + at) : 0;
       const unsigned stop = __ballot_sync(0xffffffffu, at < end && w != ~0ull);
@@ -322,16 +335,15 @@ __device__ __forceinline__ void fix_all(uint64_t *out, uint64_t nproc, uint64_t 
 
 // A short launch: tiles, then the carries by the CTA that finishes last.
 // ss.done counts the launch's finished CTAs and wraps back to 0 with the last.
-template <class Producer>
+template <class Producer, bool D80>
 __global__ void __launch_bounds__(kCarryThreads, kCarryMinBlocks)
     carry_short_kernel(const Producer prod0, uint64_t *out, uint64_t nproc, ScanState ss, const ProductDesc *batch,
                        uint64_t tpp, uint64_t ws_stride, uint64_t n, bool drop_top) {
-  __shared__ uint64_t s_prev[kCarryThreads][9];
+  __shared__ uint64_t s_buf[kCarryThreads * 9];
   __shared__ GP s_warp[kCarryThreads / 32];
   __shared__ unsigned s_done;
   pdl_wait();
-  carry_body<Producer, kCarryThreads, kShortPer>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, blockIdx.x, s_prev,
-                                                 s_warp);
+  carry_tile<Producer, D80, kShortPer>(prod0, out, nproc, ss, batch, tpp, ws_stride, n, s_buf, s_warp);
   __threadfence();  // this thread's limbs (thread 0: also the aggregate) before the count
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -340,20 +352,22 @@ __global__ void __launch_bounds__(kCarryThreads, kCarryMinBlocks)
   }
   __syncthreads();
   if (s_done != gridDim.x - 1) return;
-  fix_all(out, nproc, gridDim.x, ss, drop_top, batch, tpp, n, s_warp, reinterpret_cast<uint32_t *>(&s_prev[0][0]));
+  fix_all<D80 ? kShortTile / 4 * 5 : kShortTile>(out, nproc, gridDim.x, ss, drop_top, batch, tpp, limbs_of(n, D80),
+                                                 s_warp, reinterpret_cast<uint32_t *>(s_buf));
 }
 
+template <bool D80>
 __global__ void __launch_bounds__(kFixWarps * 32)
     carry_fix_kernel(uint64_t *out, uint64_t nproc, uint64_t tiles, ScanState ss, bool drop_top,
                      const ProductDesc *batch, uint64_t tpp, uint64_t n) {
   pdl_wait();
-  fix_body<kCarryTile>(out, nproc, tiles, ss, drop_top, batch, tpp, n,
-                       static_cast<uint64_t>(blockIdx.x) * kFixWarps + (threadIdx.x >> 5));
+  fix_body<D80 ? kCarryTile / 4 * 5 : kCarryTile>(
+      out, nproc, tiles, ss, drop_top, batch, tpp, limbs_of(n, D80), static_cast<uint64_t>(blockIdx.x) * kFixWarps + (threadIdx.x >> 5));
 }
 
 // A carry over `tiles` tiles (a batch: tpp per product): one launch where it
 // is short, else the tiles and the fix.
-template <class Producer>
+template <bool D80 = false, class Producer>
 cudaError_t launch_carry(const Producer &prod, uint64_t *out, uint64_t nproc, uint64_t tiles, bool is_short,
                          const ScanState &ss, cudaStream_t st, const ProductDesc *batch = nullptr, uint64_t tpp = 0,
                          uint64_t ws_stride = 0, uint64_t n = 0) {
@@ -361,13 +375,13 @@ cudaError_t launch_carry(const Producer &prod, uint64_t *out, uint64_t nproc, ui
   if (tiles > 0x7fffffffull || (is_short && tiles > kCarryThreads)) return cudaErrorInvalidValue;
   const dim3 grid(static_cast<unsigned>(tiles));
   if (is_short)
-    return launch_dep(carry_short_kernel<Producer>, grid, kCarryThreads, 0, st, prod, out, nproc, ss, batch, tpp,
+    return launch_dep(carry_short_kernel<Producer, D80>, grid, kCarryThreads, 0, st, prod, out, nproc, ss, batch, tpp,
                       ws_stride, n, prod.drop_top());
-  cudaError_t e = launch_dep(carry_kernel<Producer>, grid, kCarryThreads, 0, st, prod, out, nproc, ss, batch, tpp,
+  cudaError_t e = launch_dep(carry_kernel<Producer, D80>, grid, kCarryThreads, 0, st, prod, out, nproc, ss, batch, tpp,
                              ws_stride, n);
   if (e != cudaSuccess) return e;
   const uint64_t blocks = (tiles + kFixWarps - 1) / kFixWarps;
-  return launch_dep(carry_fix_kernel, dim3(static_cast<unsigned>(blocks)), kFixWarps * 32, 0, st, out, nproc, tiles,
+  return launch_dep(carry_fix_kernel<D80>, dim3(static_cast<unsigned>(blocks)), kFixWarps * 32, 0, st, out, nproc, tiles,
                     ss, prod.drop_top(), batch, tpp, n);
 }
 
@@ -441,18 +455,30 @@ uint64_t carry_tiles(uint64_t n, uint64_t nprod) {
   return (n + tile - 1) / tile;
 }
 
-cudaError_t launch_crt_carry(const uint64_t *res, uint64_t n, const CrtConst &cc, uint64_t *out, uint64_t nout,
-                             const ScanState &ss, cudaStream_t st, uint64_t *tiles_used) {
-  const uint64_t nproc = nout < n ? nout : n;
-  const uint64_t tiles = carry_tiles(nproc);
+namespace {
+// The carry of coefficients that `prod` reconstructs, limbs or digits.
+template <class Producer>
+cudaError_t launch_coefs(const Producer &prod, bool dig80, uint64_t *out, uint64_t nproc, uint64_t tiles, bool sh,
+                         const ScanState &ss, cudaStream_t st, const ProductDesc *batch = nullptr, uint64_t tpp = 0,
+                         uint64_t ws_stride = 0, uint64_t n = 0) {
+  return dig80 ? launch_carry<true>(prod, out, nproc, tiles, sh, ss, st, batch, tpp, ws_stride, n)
+               : launch_carry<false>(prod, out, nproc, tiles, sh, ss, st, batch, tpp, ws_stride, n);
+}
+using Prescaled = carry::CrtProducerT<false, true>;
+}  // namespace
+
+cudaError_t launch_crt_carry(const uint64_t *res, uint64_t n, bool dig80, const CrtConst &cc, uint64_t *out,
+                             uint64_t nout, const ScanState &ss, cudaStream_t st, uint64_t *tiles_used) {
+  const uint64_t nproc = nout < limbs_of(n, dig80) ? nout : limbs_of(n, dig80);
+  const uint64_t ncoef = coefs_of(nproc, dig80), tiles = carry_tiles(ncoef);
   *tiles_used = tiles;
   if (tiles == 0) return cudaSuccess;
-  const bool sh = carry_short(nproc);
-  if (cc.prescaled) return launch_carry(carry::CrtProducerT<false, true>{res, n, cc}, out, nproc, tiles, sh, ss, st);
-  return launch_carry(CrtProducer{res, n, cc}, out, nproc, tiles, sh, ss, st);
+  const bool sh = carry_short(ncoef);
+  if (cc.prescaled) return launch_coefs(Prescaled{res, n, cc}, dig80, out, nproc, tiles, sh, ss, st);
+  return launch_coefs(CrtProducer{res, n, cc}, dig80, out, nproc, tiles, sh, ss, st);
 }
 
-cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint64_t n, const CrtConst &cc,
+cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint64_t n, bool dig80, const CrtConst &cc,
                                    const ProductDesc *batch, uint64_t nprod, const ScanState &ss, cudaStream_t st) {
   const uint64_t tpp = carry_tiles(n, nprod);
   const uint64_t tiles = tpp * nprod;
@@ -460,25 +486,24 @@ cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint
   if (tiles == 0) return cudaSuccess;
   if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
   if (cc.prescaled)
-    return launch_carry(carry::CrtProducerT<false, true>{res, n, cc}, nullptr, 0, tiles, sh, ss, st, batch, tpp,
-                        ws_stride, n);
-  return launch_carry(CrtProducer{res, n, cc}, nullptr, 0, tiles, sh, ss, st, batch, tpp, ws_stride, n);
+    return launch_coefs(Prescaled{res, n, cc}, dig80, nullptr, 0, tiles, sh, ss, st, batch, tpp, ws_stride, n);
+  return launch_coefs(CrtProducer{res, n, cc}, dig80, nullptr, 0, tiles, sh, ss, st, batch, tpp, ws_stride, n);
 }
 
-cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, int logN, uint64_t chunk,
+cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, uint64_t n, bool dig80, uint64_t chunk,
                                     uint64_t nchunks, const CrtConst &cc, uint64_t *out, uint64_t nproc,
                                     const ScanState &ss, cudaStream_t st, uint64_t *tiles_used) {
-  const uint64_t n = 1ull << logN;
-  if (chunk % 8 || 2 * chunk < n || chunk > n || ws_stride % 2) return cudaErrorInvalidValue;
-  const uint64_t tiles = carry_tiles(nproc);
+  if (chunk % 8 || chunk > n || ws_stride % 2) return cudaErrorInvalidValue;
+  const uint64_t ncoef = coefs_of(nproc, dig80), tiles = carry_tiles(ncoef);
   *tiles_used = tiles;
   if (tiles == 0) return cudaSuccess;
   if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
+  const bool sh = carry_short(ncoef);
   if (cc.prescaled)
-    return launch_carry(ChunkProducerT<carry::CrtProducerT<false, true>>{{res, n, cc}, ws_stride, chunk, nchunks}, out,
-                        nproc, tiles, carry_short(nproc), ss, st);
-  return launch_carry(ChunkProducerT<CrtProducer>{CrtProducer{res, n, cc}, ws_stride, chunk, nchunks}, out, nproc,
-                      tiles, carry_short(nproc), ss, st);
+    return launch_coefs(ChunkProducerT<Prescaled>{{res, n, cc}, ws_stride, chunk, nchunks}, dig80, out, nproc, tiles,
+                        sh, ss, st);
+  return launch_coefs(ChunkProducerT<CrtProducer>{CrtProducer{res, n, cc}, ws_stride, chunk, nchunks}, dig80, out,
+                      nproc, tiles, sh, ss, st);
 }
 
 cudaError_t launch_large_sum(const SumOperand &a, int64_t sa, const SumOperand &b, int64_t sb, uint64_t *out,

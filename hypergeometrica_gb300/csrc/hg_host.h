@@ -19,7 +19,8 @@ struct PassPlan {
 // Products of one transform length and kind, run as one launch per pass.
 struct BatchGroup {
   int L = 0;
-  int kh = 8;                      // eighths of the 2^L points that are kept (8: a whole transform)
+  int k16 = 16;                    // sixteenths of the 2^L points that are kept (16: a whole transform)
+  bool dig80 = false;              // coefficients are 80-bit digits
   bool square = false;
   bool tails = false;              // some product has nout > N
   std::vector<PassPlan> plan;
@@ -65,8 +66,9 @@ struct BatchBufs {
 uint64_t product_workspace_bytes(uint64_t nx, uint64_t ny, bool square);
 
 // Group validated descriptors by (transform length, square) and split groups
-// so that none needs more than ws_cap_bytes of workspace.
-int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchPlan &bp);
+// so that none needs more than ws_cap_bytes of workspace.  whole: every product
+// by the whole transform of its limbs.
+int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchPlan &bp, bool whole = false);
 
 // sa |a| + sb |b| into out[0, nout) over the whole GPU (nout >= the longer
 // operand's end + 1; limbs past the sum are zeroed); (sign, size) into result[0, 2)

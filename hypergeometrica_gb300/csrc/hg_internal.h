@@ -81,6 +81,9 @@ struct PassArgs {
   uint64_t chunk;              // single product cut into chunks: product k reads
                                // operand 0's limbs [k * chunk, (k + 1) * chunk)
   int read_limbs;              // batch: this pass reads and reduces limbs
+  // The operands' coefficients are digits of 80 bits (5 limbs hold 4) instead
+  // of limbs; a pass that reads limbs then forms them.
+  int dig80;
   int nops;                    // operands handled by this launch
   int logN;
   int logR;                    // log2 rows (transform points) of this pass
@@ -151,10 +154,31 @@ struct ScanState {
   int *err;                    // device error word
 };
 
-// Whether a truncated transform's outer pass of 2^logR rows can keep kh
-// eighths of them (8: all).
-__host__ __device__ __forceinline__ constexpr bool truncation_ok(int logR, int kh) {
-  return kh == 8 || (kh == 6 && logR == 6) || (kh >= 5 && kh <= 7 && (logR == 4 || logR >= 7));
+// Whether a truncated transform's outer pass of 2^logR rows can keep k
+// sixteenths of them (16: all): its last round holds the top four row bits of
+// a 4- or 8-bit pass in registers, three of a 7-bit one, two of a 6-bit one.
+__host__ __device__ __forceinline__ constexpr bool truncation_ok(int logR, int k) {
+  return k == 16 || (k >= 9 && k < 16 &&
+                     (logR == 4 || logR == 8 || (logR == 7 && k % 2 == 0) || (logR == 6 && k == 12)));
+}
+
+// The 80-bit digit at bit 80 j of a vector whose limb 5 (j / 4) + i the two
+// words are: word (80 j) / 64 and the next.
+__device__ __forceinline__ uint64_t digit80(uint64_t a, uint64_t b, uint32_t j, const PrimeConst &pc) {
+  const uint32_t s = (j & 3u) << 4;  // bits of `a` below the digit
+  return reduce80((a >> s) | ((b << 1) << (63 - s)), static_cast<uint32_t>(b >> s) & 0xffffu, pc);
+}
+
+// Coefficient j of an operand of nl limbs modulo p: limb j, or 80-bit digit j.
+template <bool D80>
+__device__ __forceinline__ uint64_t coefficient(const uint64_t *limbs, uint64_t nl, uint64_t j, const PrimeConst &pc) {
+  if constexpr (D80) {
+    const uint64_t w = (5 * j) >> 2;
+    if (w >= nl) return 0;
+    return digit80(__ldg(limbs + w), w + 1 < nl ? __ldg(limbs + w + 1) : 0, static_cast<uint32_t>(j), pc);
+  } else {
+    return j < nl ? reduce64(__ldg(limbs + j), pc.p) : 0;
+  }
 }
 
 // ---- dependent launches ----------------------------------------------------
@@ -199,19 +223,20 @@ cudaError_t launch_ntt_strided(const PassArgs &a, bool inverse, cudaStream_t st)
 // logR == logT <= 12.
 constexpr int kContigFwd = 0, kContigInv = 1, kContigMul = 2, kContigSqr = 3, kContigMulSpec = 4;
 cudaError_t launch_ntt_contig(const PassArgs &a, int mode, cudaStream_t st);
-cudaError_t launch_crt_carry(const uint64_t *res, uint64_t n, const CrtConst &cc, uint64_t *out, uint64_t nout,
+cudaError_t launch_crt_carry(const uint64_t *res, uint64_t n, bool dig80, const CrtConst &cc, uint64_t *out, uint64_t nout,
                              const ScanState &ss, cudaStream_t st, uint64_t *tiles_used);
 // Reconstruction + carry for nprod products of n residues per prime that
 // start ws_stride words apart at res.
-cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint64_t n, const CrtConst &cc,
+cudaError_t launch_crt_carry_batch(const uint64_t *res, uint64_t ws_stride, uint64_t n, bool dig80, const CrtConst &cc,
                                    const ProductDesc *batch, uint64_t nprod, const ScanState &ss, cudaStream_t st);
 // Reconstruction + carry of a product computed in chunks: chunk k's
 // residues ([3][2^logN], unscaled inverse) start k * ws_stride words past
 // res and hold the product of limbs [k * chunk, (k + 1) * chunk) of the long
 // operand with the short one; position i of the result sums chunk i / chunk
 // at i % chunk and the chunk before it at i % chunk + chunk.  Writes
-// out[0, nproc).  Needs 2^(logN-1) <= chunk, chunk a multiple of 8.
-cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, int logN, uint64_t chunk,
+// out[0, nproc).  n residues per prime hold a chunk's product of at most
+// 2 chunk coefficients; chunk (in coefficients) is a multiple of 8.
+cudaError_t launch_crt_carry_chunks(const uint64_t *res, uint64_t ws_stride, uint64_t n, bool dig80, uint64_t chunk,
                                     uint64_t nchunks, const CrtConst &cc, uint64_t *out, uint64_t nproc,
                                     const ScanState &ss, cudaStream_t st, uint64_t *tiles_used);
 // An operand of a signed sum: n limbs, `shift` whole limbs up.
@@ -246,10 +271,17 @@ cudaError_t launch_digit_carry(const uint64_t *x, uint64_t nx, uint64_t d, uint6
 cudaError_t launch_pass_twiddles(uint64_t *out, int logM, int logR, bool inverse, const NttTables *tb,
                                  const PrimeConst *pc, int nprimes, cudaStream_t st, const uint64_t *scale = nullptr);
 
-// Tiles per product that a carry over nprod products of n positions uses, and
-// whether it is one launch (short) or two.
+// Tiles per product that a carry over nprod products of n coefficients uses,
+// and whether it is one launch (short) or two.
 uint64_t carry_tiles(uint64_t n, uint64_t nprod = 1);
 bool carry_short(uint64_t n, uint64_t nprod = 1);
+// Coefficients that n limbs hold, and limbs that n coefficients (a multiple of 4) fill.
+__host__ __device__ __forceinline__ constexpr uint64_t coefs_of(uint64_t n, bool dig80) {
+  return dig80 ? n - n / 5 : n;  // ceil(4 n / 5)
+}
+__host__ __device__ __forceinline__ constexpr uint64_t limbs_of(uint64_t n, bool dig80) {
+  return dig80 ? n + n / 4 : n;
+}
 
 #if HG_CHECKED
 // The fault word of each translation unit with kernels (checked builds),

@@ -24,7 +24,8 @@ constexpr int kFwd = 0, kInv = 1, kMul = 2, kSqr = 3, kMulSpec = 4;
 // and reduces limbs from batch descriptors or chunks runs here.
 // CUT: forward, the outer pass of a truncated transform, which keeps P.krows
 // rows; inverse, a transform's last pass that scales by P.scale.
-template <int LOGR, bool INV, bool CUT = false>
+// D80: the operands' coefficients are 80-bit digits.
+template <int LOGR, bool INV, bool CUT = false, bool D80 = false>
 __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid, ulonglong2 *tw, uint64_t *sm) {
   constexpr int T = kTileBits;
   constexpr int LOGTC = T - LOGR;  // log2 columns per tile
@@ -73,7 +74,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
                           (static_cast<uint64_t>(rhi) << (4 + logS)) + s;
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        if (CUT && LOGR == 4 && i >= 10 && i >= P.krows) break;  // rows a truncated transform drops
+        if (CUT && LOGR == 4 && i >= 9 && i >= P.krows) break;  // rows a truncated transform drops
         v[i] = mont_mul(v[i], __ldg(t + (static_cast<uint64_t>(i) << logS)), p, c);
       }
       return;
@@ -96,8 +97,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     if (limbs) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const uint64_t o = off + i * step;
-        v[i] = o < nl ? reduce64(__ldg(limbs + o), p) : 0;
+        v[i] = coefficient<D80>(limbs, nl, off + i * step, P.pc[prime]);
       }
     } else {
 #pragma unroll
@@ -116,7 +116,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
       from_smem<A0>(v, sm, xt);
     }
     // The thread's 16 rows, of which a truncated transform keeps the first
-    // `keep` (the rows of a 16-row group together; 10, 12 or 14 of 16 when R = 16).
+    // `keep` (the rows of a 16-row group together; 9 to 15 of 16 when R = 16).
     const int keep = CUT ? P.krows - static_cast<int>((xt >> (ROWOFF + 4)) << 4) : 16;
     if (CUT && LOGR > 4 && keep <= 0) return;
     stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true>(v, tw, xt, p, c);  // then the inter-pass twiddle
@@ -124,7 +124,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     offsets(xt, A0, off, step);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      if (CUT && LOGR == 4 && i >= 10 && i >= keep) break;
+      if (CUT && LOGR == 4 && i >= 9 && i >= keep) break;
       const uint64_t o = off + i * step;
       check_below(v[i], p);
       if (check_index(o, P.points)) data[o] = v[i];

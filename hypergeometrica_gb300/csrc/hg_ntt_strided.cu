@@ -31,9 +31,13 @@
 // rows of outputs (krows S >= n): the passes inside then run on krows of the
 // R blocks, and the outer inverse pass solves each column's krows values
 // from krows outputs and the R - krows results known to be zero
-// (TruncatedInverse).  krows is 5/8, 6/8 or 7/8 of R, cut by the top three row
-// bits (by the top two for R = 64: 6/8 only), which sit in one thread's
-// registers in the round that ends the pass.
+// (TruncatedInverse).  krows is 9 to 15 sixteenths of R, cut by the top four
+// row bits (the top three for R = 128, the top two for R = 64), which sit in
+// one thread's registers in the round that ends the pass.
+//
+// A product's coefficients are limbs or, where that needs fewer points, digits
+// of 80 bits (5 limbs hold 4 digits): the first forward pass then forms the
+// digits from its limbs.
 #include <algorithm>
 #include <cudaTypedefs.h>
 #include <mutex>
@@ -50,15 +54,15 @@ using namespace bodies;
 // Four CTAs of 256 threads per SM (64 registers, a few spilled words): on
 // the 2^25-point passes faster than three (80 registers), two (128) or five
 // (48).
-template <int LOGR, bool INV, bool CUT = false>
+template <int LOGR, bool INV, bool CUT = false, bool D80 = false>
 __global__ void __launch_bounds__(kTileThreads, 4) ntt_strided_kernel(const PassArgs P) {
   __shared__ ulonglong2 tw[1 << (LOGR - 1)];
   __shared__ uint64_t sm[LOGR > 4 ? (1 << kTileBits) : 1];
   pdl_wait();
-  strided_ldg_body<LOGR, INV, CUT>(P, blockIdx.x, tw, sm);
+  strided_ldg_body<LOGR, INV, CUT, D80>(P, blockIdx.x, tw, sm);
 }
 
-constexpr int kCut = 0;  // KH of a truncated transform's outer forward pass
+constexpr int kCut = 0;  // KQ of a truncated transform's outer forward pass
 
 // Tensor maps of one TMA-staged pass: the box each CTA loads (residues, or
 // the limbs of a first forward pass) and stores, per operand, and the box of
@@ -93,8 +97,12 @@ struct TmaLimbs {
 // the upper half of the block lies past the limbs (P.ztop bit op), the first
 // stage skips its zero inputs.
 //
-// KH < 8: the outer pass of a truncated transform.  Inverse: KH/8 of the rows
-// are known.  Forward (KH = kCut, whatever the number): the kept rows are
+// D80 (with LIMBS): the coefficients are 80-bit digits.  The limbs' rows have
+// 5 S / 4 limbs and the tile's box 5 C / 4 of them (two boxes for R = 16, whose
+// 320 limbs pass the 256 of a box); a digit lies in two words of its row.
+//
+// KQ < 16: the outer pass of a truncated transform.  Inverse: KQ/16 of the rows
+// are known.  Forward (KQ = kCut, whatever the number): the kept rows are
 // P.krows, and threads whose 16 rows are all dropped stop after the exchange
 // (R > 16).  A whole transform's passes are instances of their own: taking the
 // rows from P.krows there made the 2^25-point product 2% slower.
@@ -102,7 +110,7 @@ struct TmaLimbs {
 // SCALE (inverse only): the last pass of the spectrum entry point, which
 // multiplies every residue by P.scale as it leaves (a launch and a pass over
 // memory less: 2^20 points there and back 67.4 -> 61.0 us).
-template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KH, bool SCALE>
+template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KQ, bool SCALE, bool D80>
 __global__ void __launch_bounds__(kTileThreads, 4)
     ntt_strided_tma_kernel(const __grid_constant__ TmaMaps maps, const PassArgs P, const TmaLimbs L) {
   constexpr int T = kTileBits;
@@ -115,15 +123,18 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   constexpr uint32_t kTileBytes = (1u << T) * sizeof(uint64_t);
   static_assert(LOGR >= 4 && LOGR <= 8, "strided passes have 4..8 row bits");
   static_assert(!LIMBS || !INV, "only a forward pass reads limbs");
-  static_assert(KH == 8 || (!INV && KH == kCut && LIMBS) || (INV && KH >= 5 && (LOGR == 4 || LOGR >= 7 || (LOGR == 6 && KH == 6))),
+  static_assert(KQ == 16 || (!INV && KQ == kCut && LIMBS) || (INV && truncation_ok(LOGR, KQ)),
                 "rows a truncated inverse can cut");
-  constexpr int KI = INV ? KH : 8;
-  constexpr int kRows = (1 << LOGR) * KI / 8;  // inverse: known rows
-  constexpr bool kCutFwd = !INV && KH < 8;
+  static_assert(!D80 || LIMBS, "digits are formed from limbs");
+  constexpr int KI = INV ? KQ : 16;
+  constexpr int kRows = (1 << LOGR) * KI / 16;  // inverse: known rows
+  constexpr bool kCutFwd = !INV && KQ < 16;
+  constexpr uint32_t kInWords = (D80 ? 5u : 4u) << (T - 2);  // words of the input box
+  constexpr uint32_t kRowWords = D80 ? 5u << (LOGTC - 2) : 1u << LOGTC;  // words of an input row of the tile
   const int krows = kCutFwd ? P.krows : kRows;
   extern __shared__ __align__(128) uint64_t tile[];  // [1 << T] residues, then [1 << T] twiddles
   __shared__ ulonglong2 tw[1 << (LOGR - 1)];
-  __shared__ ulonglong2 twf[INV && KH < 8 ? 1 << (LOGR - 1) : 1];
+  __shared__ ulonglong2 twf[INV && KQ < 16 ? 1 << (LOGR - 1) : 1];
   __shared__ __align__(8) uint64_t bar;
 
   const uint32_t tid = threadIdx.x;
@@ -141,7 +152,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   const uint64_t ncg = 1ull << (logS - LOGTC);
   const int blk = static_cast<int>(t / ncg);
   const int s0 = static_cast<int>((t % ncg) << LOGTC);
-  uint64_t *twt = tile + (1u << T);
+  uint64_t *twt = tile + kInWords;
 
   if (tid == 0) {
     tma::mbar_init(&bar, 1);
@@ -150,17 +161,20 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   __syncthreads();
   if (tid == 0) {
     const uint32_t row_bytes = kTileBytes >> LOGR;
-    tma::mbar_arrive_expect_tx(&bar, (INV ? kRows * row_bytes : kTileBytes) +
+    tma::mbar_arrive_expect_tx(&bar, (INV ? kRows * row_bytes : kInWords * 8u) +
                                          (TABLE ? static_cast<uint32_t>(krows) * row_bytes : 0u));
     if (TABLE) tma::load_3d(twt, &maps.tw, &bar, s0, 0, prime);  // no kernel of the stream writes the tables
     pdl_wait();
-    if constexpr (LIMBS)
-      tma::load_2d(tile, &maps.in[op], &bar, s0, blk << LOGR);
+    if constexpr (D80 && LOGR == 4) {
+      tma::load_2d(tile, &maps.in[op], &bar, s0 / 4 * 5, blk << LOGR);
+      tma::load_2d(tile + kInWords / 2, &maps.in[op], &bar, s0 / 4 * 5 + static_cast<int>(kRowWords) / 2, blk << LOGR);
+    } else if constexpr (LIMBS)
+      tma::load_2d(tile, &maps.in[op], &bar, D80 ? s0 / 4 * 5 : s0, blk << LOGR);
     else
       tma::load_5d(tile, &maps.in[op], &bar, s0, 0, blk, prime - P.prime_lo, static_cast<int>(prod));
   }
   load_sub_twiddles(tw, INV ? tb.sub_inv : tb.sub_fwd, LOGR, tid, kTileThreads);
-  if constexpr (INV && KH < 8) load_sub_twiddles(twf, tb.sub_fwd, LOGR, tid, kTileThreads);
+  if constexpr (INV && KQ < 16) load_sub_twiddles(twf, tb.sub_fwd, LOGR, tid, kTileThreads);
   if constexpr (LIMBS) pdl_wait();  // a partial row's limbs are read by every thread
   const bool landed = tma::mbar_wait_bounded(&bar, 0);
   if (!__syncthreads_and(landed)) {  // also orders the sub-twiddle table
@@ -174,7 +188,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     if constexpr (TABLE) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        if (LOGR == 4 && KH < 8 && i >= 10 && i >= krows) break;  // rows that are not kept
+        if (LOGR == 4 && KQ < 16 && i >= 9 && i >= krows) break;  // rows that are not kept
         v[i] = mont_mul(v[i], twt[xt | (static_cast<uint32_t>(i) << A0)], p, c);
       }
     } else {
@@ -204,10 +218,21 @@ __global__ void __launch_bounds__(kTileThreads, 4)
       const bool has_tail = tail != 0 && tr >= row0 && tr < row0 + (1u << LOGR);
       auto limb = [&](int i) {
         const uint32_t x = xt | (static_cast<uint32_t>(i) << AL);
-        uint64_t w = tile[x];
-        if (has_tail && row0 + (x >> ROWOFF) == tr && s0 + (x & ((1u << LOGTC) - 1u)) < tail)
-          w = __ldg(lp + tr * (uint64_t(1) << logS) + s0 + (x & ((1u << LOGTC) - 1u)));
-        return reduce64(w, p);
+        const uint32_t row = x >> ROWOFF, col = x & ((1u << LOGTC) - 1u);
+        if constexpr (D80) {
+          if (has_tail && row0 + row == tr)
+            return coefficient<true>(lp, tr * (uint64_t(5) << (logS - 2)) + tail,
+                                     (tr << logS) + static_cast<uint64_t>(s0) + col, P.pc[prime]);
+          // R = 16: columns 0 .. C/2 - 1 in the first box, the others in the second.
+          const uint32_t half = LOGR == 4 ? col >> (LOGTC - 1) : 0u;
+          const uint32_t lc = LOGR == 4 ? col & ((1u << (LOGTC - 1)) - 1u) : col;
+          const uint32_t at = half * (kInWords / 2) + row * (LOGR == 4 ? kRowWords / 2 : kRowWords) + ((5u * lc) >> 2);
+          return digit80(tile[at], tile[at + 1], lc, P.pc[prime]);
+        } else {
+          uint64_t w = tile[x];
+          if (has_tail && row0 + row == tr && s0 + col < tail) w = __ldg(lp + (tr << logS) + s0 + col);
+          return reduce64(w, p);
+        }
       };
       if (G == 2 && ((L.ztop >> op) & 1)) {
         // Registers 8..15 hold the top row bit's upper half, past the limbs:
@@ -254,9 +279,9 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   } else {
     // Registers of the rows [0, kRows) hold the known outputs, the others nothing.
     constexpr int NK0 = LOGR == 4 ? kRows : 16;  // layout A0: registers of a thread with known rows
-    constexpr int NK1 = 2 * KI;                  // the pass's last layout: register i is row bits LOGR-4 .. LOGR-1
+    constexpr int NK1 = KI;                      // the pass's last layout: register i is row bits LOGR-4 .. LOGR-1
     xt = thread_base<A0>(tid);
-    const bool known = KI == 8 || LOGR == 4 || static_cast<int>((xt >> (ROWOFF + 4)) << 4) < kRows;
+    const bool known = KI == 16 || LOGR == 4 || static_cast<int>((xt >> (ROWOFF + 4)) << 4) < kRows;
     if (known) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -268,16 +293,18 @@ __global__ void __launch_bounds__(kTileThreads, 4)
         check_below(v[i], 2 * p);  // inverse residues live in [0, 2p)
       }
       inter_pass(v, xt, tb.hi_inv, tb.lo_inv);
-      if constexpr (KI == 8 || LOGR > 4) {
+      if constexpr (KI == 16 || LOGR > 4) {
         stages<4, 0, A0, ROWOFF, 0, LOGR, true, true, true>(v, tw, xt, p, c);
-      } else {  // the stage on row bit 0 of the known rows, then the top three bits
+      } else if constexpr (KI % 2 == 0) {  // the stage on row bit 0 of the known rows, then the top three bits
 #pragma unroll
         for (int i = 0; i < kRows; i += 2) {
           const uint64_t u = v[i], w = v[i + 1];
           v[i] = u + w;
           v[i + 1] = u - w + p;
         }
-        TruncatedInverse<LOGR, A0, ROWOFF, true>{tw, twf, xt, p, c}.template run<3, 1, KI, 0, true>(v);
+        TruncatedInverse<LOGR, A0, ROWOFF, true>{tw, twf, xt, p, c}.template run<3, 1, KI / 2, 0, true>(v);
+      } else {
+        TruncatedInverse<LOGR, A0, ROWOFF, true>{tw, twf, xt, p, c}.template run<3, 0, KI, 0, true>(v);
       }
     }
     constexpr int AS = (G == 2) ? A1 : A0;
@@ -288,18 +315,11 @@ __global__ void __launch_bounds__(kTileThreads, 4)
       xt = thread_base<A1>(tid);
 #pragma unroll
       for (int i = 0; i < NK1; ++i) v[i] = tile[xt | (static_cast<uint32_t>(i) << A1)];
-      if constexpr (KI == 8) {
+      if constexpr (KI == 16) {
         stages<NB1, 4 - NB1, A1, ROWOFF, 4, LOGR, true, false>(v, tw, xt, p, c);
       } else {
-        const TruncatedInverse<LOGR, A1, ROWOFF, false> top{tw, twf, xt, p, c};
-        if constexpr (LOGR == 8) {
-#pragma unroll
-          for (int i = 0; i < NK1; i += 2) top.template butterfly<0>(v, i);  // row bit 4 of the known rows
-        }
-        if constexpr (LOGR == 6)
-          top.template run<3, 2, KI / 2, 0, true>(v);
-        else
-          top.template run<3, 1, KI, 0, true>(v);
+        constexpr int JL = 8 - LOGR;  // register bit of the lowest row bit that this round still owes
+        TruncatedInverse<LOGR, A1, ROWOFF, false>{tw, twf, xt, p, c}.template run<3, JL, (KI >> JL), 0, true>(v);
       }
     }
     if constexpr (SCALE) {
@@ -343,12 +363,23 @@ __global__ void pass_twiddles_kernel(uint64_t *out, int logM, int logR, bool inv
   }
 }
 
+bool reads_limbs(const PassArgs &a) {
+  if (a.batch) return a.read_limbs != 0;
+  return a.limbs[0] != nullptr || (a.nops > 1 && a.limbs[1] != nullptr);
+}
+
 template <int LOGR>
 cudaError_t launch_r(const PassArgs &a, bool inverse, unsigned grid, cudaStream_t st) {
   if (inverse && a.scale) return launch_dep(ntt_strided_kernel<LOGR, true, true>, grid, kTileThreads, 0, st, a);
   if (inverse)
     return launch_dep(ntt_strided_kernel<LOGR, true>, grid, kTileThreads, 0, st, a);
-  if (a.krows < (1 << LOGR)) return launch_dep(ntt_strided_kernel<LOGR, false, true>, grid, kTileThreads, 0, st, a);
+  const bool digits = a.dig80 && reads_limbs(a);
+  if constexpr (LOGR != 5) {
+    if (a.krows < (1 << LOGR))
+      return digits ? launch_dep(ntt_strided_kernel<LOGR, false, true, true>, grid, kTileThreads, 0, st, a)
+                    : launch_dep(ntt_strided_kernel<LOGR, false, true>, grid, kTileThreads, 0, st, a);
+  }
+  if (digits) return launch_dep(ntt_strided_kernel<LOGR, false, false, true>, grid, kTileThreads, 0, st, a);
   return launch_dep(ntt_strided_kernel<LOGR, false>, grid, kTileThreads, 0, st, a);
 }
 
@@ -408,20 +439,40 @@ cudaError_t twiddle_map(CUtensorMap *m, const uint64_t *ptw, const PassArgs &a) 
   return encode(m, ptw, 3, dims, strides, box);
 }
 
-template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KH = 8, bool SCALE = false>
+template <int LOGR, bool INV, bool TABLE, bool LIMBS, int KQ = 16, bool SCALE = false, bool D80 = false>
 cudaError_t launch_tma_v(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l, unsigned grid, cudaStream_t st) {
-  constexpr size_t bytes = (TABLE ? 2 : 1) * (size_t(1) << kTileBits) * sizeof(uint64_t);
+  constexpr size_t bytes = ((D80 ? 5 : 4) + (TABLE ? 4 : 0)) * (size_t(1) << (kTileBits - 2)) * sizeof(uint64_t);
   // Raise the dynamic shared-memory limit once per instantiation (not on
   // every launch, so that launches can be captured in a CUDA graph).
   static bool raised = false;
   if (bytes > 48 * 1024 && !raised) {
-    cudaError_t e = cudaFuncSetAttribute(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH, SCALE>,
+    cudaError_t e = cudaFuncSetAttribute(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KQ, SCALE, D80>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e != cudaSuccess) return e;
     raised = true;
   }
-  return launch_dep(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KH, SCALE>, grid, kTileThreads, bytes, st, m, a,
+  return launch_dep(ntt_strided_tma_kernel<LOGR, INV, TABLE, LIMBS, KQ, SCALE, D80>, grid, kTileThreads, bytes, st, m, a,
                     l);
+}
+
+// The outer inverse pass of a truncated transform that keeps KQ sixteenths.
+template <int LOGR, int KQ>
+cudaError_t launch_cut(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l, unsigned grid, cudaStream_t st) {
+  if constexpr (truncation_ok(LOGR, KQ))
+    return a.ptw ? launch_tma_v<LOGR, true, true, false, KQ>(m, a, l, grid, st)
+                 : launch_tma_v<LOGR, true, false, false, KQ>(m, a, l, grid, st);
+  return cudaErrorInvalidValue;
+}
+
+template <int LOGR, bool D80>
+cudaError_t launch_limbs(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l, unsigned grid, cudaStream_t st) {
+  if constexpr (LOGR != 5) {
+    if (a.krows < (1 << LOGR))
+      return a.ptw ? launch_tma_v<LOGR, false, true, true, kCut, false, D80>(m, a, l, grid, st)
+                   : launch_tma_v<LOGR, false, false, true, kCut, false, D80>(m, a, l, grid, st);
+  }
+  return a.ptw ? launch_tma_v<LOGR, false, true, true, 16, false, D80>(m, a, l, grid, st)
+               : launch_tma_v<LOGR, false, false, true, 16, false, D80>(m, a, l, grid, st);
 }
 
 template <int LOGR>
@@ -429,51 +480,42 @@ cudaError_t launch_tma_r(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l,
                          unsigned grid, cudaStream_t st) {
   const bool table = a.ptw != nullptr;
   if (inverse && a.krows < (1 << LOGR)) {
-    const int kh = 8 * a.krows >> LOGR;
-    if constexpr (LOGR != 5) {
-      if (kh == 6)
-        return table ? launch_tma_v<LOGR, true, true, false, 6>(m, a, l, grid, st)
-                     : launch_tma_v<LOGR, true, false, false, 6>(m, a, l, grid, st);
+    switch (16 * a.krows >> LOGR) {
+      case 9: return launch_cut<LOGR, 9>(m, a, l, grid, st);
+      case 10: return launch_cut<LOGR, 10>(m, a, l, grid, st);
+      case 11: return launch_cut<LOGR, 11>(m, a, l, grid, st);
+      case 12: return launch_cut<LOGR, 12>(m, a, l, grid, st);
+      case 13: return launch_cut<LOGR, 13>(m, a, l, grid, st);
+      case 14: return launch_cut<LOGR, 14>(m, a, l, grid, st);
+      case 15: return launch_cut<LOGR, 15>(m, a, l, grid, st);
+      default: return cudaErrorInvalidValue;
     }
-    if constexpr (LOGR != 5 && LOGR != 6) {
-      if (kh == 5)
-        return table ? launch_tma_v<LOGR, true, true, false, 5>(m, a, l, grid, st)
-                     : launch_tma_v<LOGR, true, false, false, 5>(m, a, l, grid, st);
-      if (kh == 7)
-        return table ? launch_tma_v<LOGR, true, true, false, 7>(m, a, l, grid, st)
-                     : launch_tma_v<LOGR, true, false, false, 7>(m, a, l, grid, st);
-    }
-    return cudaErrorInvalidValue;
   }
   if (inverse && a.scale)
-    return table ? launch_tma_v<LOGR, true, true, false, 8, true>(m, a, l, grid, st)
-                 : launch_tma_v<LOGR, true, false, false, 8, true>(m, a, l, grid, st);
+    return table ? launch_tma_v<LOGR, true, true, false, 16, true>(m, a, l, grid, st)
+                 : launch_tma_v<LOGR, true, false, false, 16, true>(m, a, l, grid, st);
   if (inverse)
     return table ? launch_tma_v<LOGR, true, true, false>(m, a, l, grid, st)
                  : launch_tma_v<LOGR, true, false, false>(m, a, l, grid, st);
-  if (limbs && a.krows < (1 << LOGR))
-    return table ? launch_tma_v<LOGR, false, true, true, kCut>(m, a, l, grid, st)
-                 : launch_tma_v<LOGR, false, false, true, kCut>(m, a, l, grid, st);
   if (limbs)
-    return table ? launch_tma_v<LOGR, false, true, true>(m, a, l, grid, st)
-                 : launch_tma_v<LOGR, false, false, true>(m, a, l, grid, st);
+    return a.dig80 ? launch_limbs<LOGR, true>(m, a, l, grid, st) : launch_limbs<LOGR, false>(m, a, l, grid, st);
   return table ? launch_tma_v<LOGR, false, true, false>(m, a, l, grid, st)
                : launch_tma_v<LOGR, false, false, false>(m, a, l, grid, st);
 }
 
-// The limbs of a single product's operand as rows of S limbs: a 2-D map
-// over the complete rows (none when the operand is shorter than a row).
-cudaError_t limb_map(CUtensorMap *m, const uint64_t *limbs, uint64_t nl, const PassArgs &a) {
-  const uint64_t S = uint64_t(1) << a.logS, R = uint64_t(1) << a.logR;
-  const cuuint64_t dims[2] = {S, nl / S};
-  const cuuint64_t strides[1] = {S * 8};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>((uint64_t(1) << kTileBits) / R), static_cast<cuuint32_t>(R)};
-  return encode(m, limbs, 2, dims, strides, box);
-}
+// The limbs of a single product's operand as rows of S limbs (5 S / 4 for
+// 80-bit digits): a 2-D map over the complete rows (none when the operand is
+// shorter than a row).
+uint64_t limb_row(const PassArgs &a) { return limbs_of(uint64_t(1) << a.logS, a.dig80 != 0); }
 
-bool reads_limbs(const PassArgs &a) {
-  if (a.batch) return a.read_limbs != 0;
-  return a.limbs[0] != nullptr || (a.nops > 1 && a.limbs[1] != nullptr);
+cudaError_t limb_map(CUtensorMap *m, const uint64_t *limbs, uint64_t nl, const PassArgs &a) {
+  const uint64_t W = limb_row(a), R = uint64_t(1) << a.logR;
+  const cuuint64_t dims[2] = {W, nl / W};
+  const cuuint64_t strides[1] = {W * 8};
+  uint64_t cols = limbs_of((uint64_t(1) << kTileBits) / R, a.dig80 != 0);
+  if (cols > 256) cols /= 2;  // R = 16: two boxes
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(cols), static_cast<cuuint32_t>(R)};
+  return encode(m, limbs, 2, dims, strides, box);
 }
 
 // A first forward pass of one product (not a batch, not chunks) whose block
@@ -484,7 +526,7 @@ bool tma_limbs_ok(const PassArgs &a) {
   if (a.batch || a.chunk || a.nprod != 1 || a.logS + a.logR != a.logN) return false;
   for (int op = 0; op < a.nops; ++op) {
     if (!a.limbs[op] || (reinterpret_cast<uintptr_t>(a.limbs[op]) & 15u)) return false;
-    if ((a.nlimbs[op] >> a.logS) == 0 || a.nlimbs[op] > (uint64_t(1) << a.logN)) return false;
+    if (a.nlimbs[op] < limb_row(a) || coefs_of(a.nlimbs[op], a.dig80 != 0) > (uint64_t(1) << a.logN)) return false;
   }
   return true;
 }
@@ -524,7 +566,7 @@ cudaError_t launch_ntt_strided(const PassArgs &a, bool inverse, cudaStream_t st)
   const bool limbs = reads_limbs(a);
   const int R = 1 << a.logR;
   if (a.krows < R) {  // truncated: the outer pass, its forward side from limbs, by rows the kernels can cut
-    if (a.logR + a.logS != a.logN || !truncation_ok(a.logR, 8 * a.krows >> a.logR) || (8 * a.krows) % R ||
+    if (a.logR + a.logS != a.logN || !truncation_ok(a.logR, 16 * a.krows >> a.logR) || (16 * a.krows) % R ||
         a.points != static_cast<uint64_t>(a.krows) << a.logS || (inverse ? !tma_aligned(a) : !limbs))
       return cudaErrorInvalidValue;
   } else if (a.krows != R || (a.points >> (a.logR + a.logS)) == 0) {
@@ -544,11 +586,11 @@ cudaError_t launch_ntt_strided(const PassArgs &a, bool inverse, cudaStream_t st)
       }
       const int lo = op < a.nops ? op : 0;
       l.limbs[op] = a.limbs[lo];
-      l.full_rows[op] = a.nlimbs[lo] >> a.logS;
-      l.tail[op] = a.nlimbs[lo] & ((uint64_t(1) << a.logS) - 1);
+      l.full_rows[op] = a.nlimbs[lo] / limb_row(a);
+      l.tail[op] = a.nlimbs[lo] % limb_row(a);
       // Every limb lies in the lower half of the block: the first stage's
       // upper inputs are zero.
-      if (a.nlimbs[lo] <= (uint64_t(1) << (a.logS + a.logR - 1))) l.ztop |= 1u << op;
+      if (coefs_of(a.nlimbs[lo], a.dig80 != 0) <= (uint64_t(1) << (a.logS + a.logR - 1))) l.ztop |= 1u << op;
       e = limb_map(&m.in[op], a.limbs[lo], a.nlimbs[lo], a);
     }
     if (e == cudaSuccess) e = a.ptw ? twiddle_map(&m.tw, a.ptw, a) : residue_map(&m.tw, a.data[0], a);

@@ -1,9 +1,9 @@
-"""Truncated transforms: a product whose size is at most 7/8 of the power of
-two above it keeps 5, 6 or 7 eighths of the points.  Every length class that
-has its own plan (13 .. 22 bits: one or two strided passes, outer passes of
-16, 64, 128 and 256 rows) at the edges of each cut, against the oracle where
-that is quick and against the whole transform (set_chunking(False)) limb for
-limb.
+"""Truncated transforms and 80-bit digits: a product keeps 9 to 15 sixteenths
+of the points where its size allows, and its coefficients may be digits of 80
+bits.  Every length class that has its own plan (13 .. 22 bits: one or two
+strided passes, outer passes of 16, 64, 128 and 256 rows) at the edges of each
+cut, of limbs and of digits, against the oracle where that is quick and
+against the whole transform on limbs (set_chunking(False)) limb for limb.
 """
 
 import numpy as np
@@ -25,12 +25,18 @@ def _np(t):
 
 
 def _sizes(L):
-    """Product sizes around every cut of 2^L points, and odd ones between."""
+    """Product sizes (limbs) around the cuts of 2^L points on limbs and of
+    2^(L-1) and 2^L points on 80-bit digits, and odd ones between."""
     n, e = 1 << L, 1 << (L - 3)
-    out = [n // 2 + 1]
+    out = [n // 2 + 1, n - 1, n, n // 2 + e // 3, 6 * e + e // 5]
     for k in (5, 6, 7):
         out += [k * e - 1, k * e, k * e + 1]
-    return out + [n - 1, n, n // 2 + e // 3, 6 * e + e // 5]
+    for k in range(9, 17):  # 5 limbs hold 4 digits
+        for m in (L - 1, L):
+            d = (k << (m - 4)) * 5 // 4
+            if n // 2 < d <= n:
+                out += [d - 5, d - 1, d]
+    return out
 
 
 @pytest.mark.parametrize("L", range(13, 23))

@@ -109,7 +109,7 @@ class Column:
 
 
 @pytest.mark.parametrize("p", PS)
-@pytest.mark.parametrize("n,K", [(8, 5), (8, 6), (8, 7), (8, 8), (4, 3), (4, 4)])
+@pytest.mark.parametrize("n,K", [(16, k) for k in range(9, 17)] + [(8, 5), (8, 6), (8, 7), (8, 8), (4, 3), (4, 4)])
 def test_truncated_inverse_returns_the_column(p, n, K):
     rng = random.Random(n * 100 + K)
     for low, m in ((0, 2), (1, 2), (5, 16), (15, 16)):
