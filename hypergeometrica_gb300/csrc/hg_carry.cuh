@@ -36,6 +36,13 @@ __device__ __forceinline__ void add128_to(V3 &acc, uint64_t lo, uint64_t hi) {
   acc.w2 += c1 + c2;
 }
 
+// acc += x y.  As one 128-bit product: a pair of 64-bit low and high products
+// costs a third more (mont_mul).
+__device__ __forceinline__ void add_product_to(V3 &acc, uint64_t x, uint64_t y) {
+  const unsigned __int128 v = static_cast<unsigned __int128>(x) * y;
+  add128_to(acc, static_cast<uint64_t>(v), static_cast<uint64_t>(v >> 64));
+}
+
 // COHERENT: the residues were written earlier in the same launch (the
 // persistent batch kernel), so they are read through L2 (ld.global.cg)
 // rather than the read-only data path, which is coherent only for data no
@@ -112,9 +119,11 @@ struct CrtProducerT {
     }
     // V = y0 + p0 t1 + (p0 p1) t2 < p0 p1 p2 < 2^188
     V3 v{y0, 0, 0};
-    add128_to(v, p0 * t1, __umul64hi(p0, t1));
-    const uint64_t a0 = k.p01_lo * t2, a1 = __umul64hi(k.p01_lo, t2);
-    const uint64_t b0 = k.p01_hi * t2, b1 = __umul64hi(k.p01_hi, t2);
+    add_product_to(v, p0, t1);
+    const unsigned __int128 a = static_cast<unsigned __int128>(k.p01_lo) * t2;
+    const unsigned __int128 b = static_cast<unsigned __int128>(k.p01_hi) * t2;
+    const uint64_t a0 = static_cast<uint64_t>(a), a1 = static_cast<uint64_t>(a >> 64);
+    const uint64_t b0 = static_cast<uint64_t>(b), b1 = static_cast<uint64_t>(b >> 64);
     // (p0p1) t2 = a0 + (a1 + b0) 2^64 + b1 2^128
     const uint64_t m1 = a1 + b0;
     const uint64_t mc = m1 < a1;

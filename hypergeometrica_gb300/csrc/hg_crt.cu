@@ -135,7 +135,7 @@ struct ConvProducer {
     const uint64_t jhi = i < ny - 1 ? i : ny - 1;
     for (uint64_t j = jlo; j <= jhi; ++j) {
       const uint64_t a = x[i - j], b = y[j];
-      add128_to(v, a * b, __umul64hi(a, b));
+      add_product_to(v, a, b);
     }
     return v;
   }
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kSchoolMax)
 #pragma unroll 4
     for (uint32_t j = jlo; j < jhi; ++j) {
       const uint64_t a = s_x[i - j], b = s_y[j];
-      add128_to(v, a * b, __umul64hi(a, b));
+      add_product_to(v, a, b);
     }
   }
   __syncthreads();

@@ -189,7 +189,8 @@ __device__ int mul_by(uint64_t *out, const uint64_t *x, int n, const U256 &m, in
     for (int t = 0; t < 4; ++t) {
       if (t >= ms) break;
       const uint64_t xt = t ? below(xi, xprev, t) : xi;
-      const uint64_t lo = xt * m.w[t], hi = __umul64hi(xt, m.w[t]);
+      const unsigned __int128 xm = static_cast<unsigned __int128>(xt) * m.w[t];
+      const uint64_t lo = static_cast<uint64_t>(xm), hi = static_cast<uint64_t>(xm >> 64);
       v0 += lo;
       const uint64_t c0 = v0 < lo ? 1 : 0;
       const uint64_t s = v1 + hi;
