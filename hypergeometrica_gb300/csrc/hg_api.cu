@@ -1943,8 +1943,10 @@ int batch_autotune(hg_batch *b) {
   return rc;
 }
 
-// Time the whole batch on both schedules (twice each; the second run
-// counts) and keep the faster.
+// Time the whole batch on both schedules and keep the faster: one run after
+// one that warms up and, below half a millisecond, four in a row instead, so
+// that a schedule whose launches take the host longer than the GPU is charged
+// for it.
 int schedule_autotune(hg_batch *b) {
   cudaStream_t st = g_ctx.lane->stream;
   cudaEvent_t e0, e1;
@@ -1954,13 +1956,19 @@ int schedule_autotune(hg_batch *b) {
   float ms[2] = {0, 0};
   for (int sched = 0; sched < 2 && rc == HG_OK; ++sched) {
     b->persistent = sched == 1;
-    for (int rep = 0; rep < 2 && rc == HG_OK; ++rep) {
+    bool warm = false;
+    for (int runs : {1, 1, 4}) {
       cudaEventRecord(e0, st);
-      rc = b->persistent ? persist_run(b, st) : enqueue_batch(b->bp, batch_bufs(b), st);
+      for (int k = 0; k < runs && rc == HG_OK; ++k)
+        rc = b->persistent ? persist_run(b, st) : enqueue_batch(b->bp, batch_bufs(b), st);
       if (rc) break;
       cudaEventRecord(e1, st);
       if (cudaEventSynchronize(e1) != cudaSuccess) rc = fail(HG_ERR_CUDA, "schedule timing failed");
       else cudaEventElapsedTime(&ms[sched], e0, e1);
+      if (rc) break;
+      ms[sched] /= runs;
+      if (warm && ms[sched] > 0.5f) break;
+      warm = true;
     }
   }
   cudaEventDestroy(e0);
@@ -1999,7 +2007,10 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
   std::vector<ProductDesc> items;
   int rc = product_descs(prods, n, items);
   if (rc) return rc;
-  std::unique_ptr<hg_batch> b(new hg_batch());
+  struct Destroy {
+    void operator()(hg_batch *p) const { hg_batch_destroy(p); }
+  };
+  std::unique_ptr<hg_batch, Destroy> b(new hg_batch());
   if ((rc = plan_batch(items.data(), items.size(), kBatchWorkspaceCap, b->bp))) return rc;
   const BatchPlan &bp = b->bp;
   if (!bp.desc.empty()) {

@@ -29,7 +29,7 @@ using namespace rounds;
 using namespace bodies;
 
 template <int T, int MODE>
-__global__ void __launch_bounds__(kTileThreads, contig_min_blocks(T)) ntt_contig_kernel(const PassArgs P) {
+__global__ void __launch_bounds__(kTileThreads, kContigMinBlocks) ntt_contig_kernel(const PassArgs P) {
   extern __shared__ uint64_t smem[];
   const uint64_t bx = blockIdx.x;
   const int by = static_cast<int>(blockIdx.y);
