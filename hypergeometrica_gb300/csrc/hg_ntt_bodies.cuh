@@ -94,9 +94,13 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     offsets(xt, AL, off, step);
     uint64_t nl = 0;
     const uint64_t *limbs = pass_limbs(P, prod, op, nl);
+    // Limbs in the lower half of the block only: registers 8..15 are zeros that
+    // the first stage (ZTOP) never reads.
+    const bool ztop = limbs && blk == 0 && coefs_of(nl, D80) <= (uint64_t(1) << (logM - 1));
     if (limbs) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
+        if (i == 8 && ztop) break;
         v[i] = coefficient<D80>(limbs, nl, off + i * step, P.pc[prime]);
       }
     } else {
@@ -109,7 +113,10 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     }
     __syncthreads();  // twiddle table ready
     if constexpr (G == 2) {
-      stages<NB1, 4 - NB1, A1, ROWOFF, 4, LOGR, false, false>(v, tw, xt, p, c);
+      if (ztop)
+        stages<NB1, 4 - NB1, A1, ROWOFF, 4, LOGR, false, false, false, true>(v, tw, xt, p, c);
+      else
+        stages<NB1, 4 - NB1, A1, ROWOFF, 4, LOGR, false, false>(v, tw, xt, p, c);
       to_smem<A1>(sm, v, xt);
       __syncthreads();
       xt = thread_base<A0>(tid);
@@ -119,7 +126,10 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     // `keep` (the rows of a 16-row group together; 9 to 15 of 16 when R = 16).
     const int keep = CUT ? P.krows - static_cast<int>((xt >> (ROWOFF + 4)) << 4) : 16;
     if (CUT && LOGR > 4 && keep <= 0) return;
-    stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true>(v, tw, xt, p, c);  // then the inter-pass twiddle
+    if (G == 1 && ztop)
+      stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true, G == 1>(v, tw, xt, p, c);
+    else
+      stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true>(v, tw, xt, p, c);  // then the inter-pass twiddle
     inter_pass(v, xt, tb.hi_fwd, tb.lo_fwd);
     offsets(xt, A0, off, step);
 #pragma unroll

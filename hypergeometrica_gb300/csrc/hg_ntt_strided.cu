@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   if (!INV) {
     constexpr int AL = (G == 2) ? A1 : A0;
     xt = thread_base<AL>(tid);
+    const bool ztop = LIMBS && ((L.ztop >> op) & 1);
     if constexpr (LIMBS) {
       // Row tr (in the limbs' rows of S) is the partial one: limbs
       // [tr S, tr S + tail) exist past the complete rows the map covers.
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
           return reduce64(w, p);
         }
       };
-      if (G == 2 && ((L.ztop >> op) & 1)) {
+      if (ztop) {
         // Registers 8..15 hold the top row bit's upper half, past the limbs:
         // zeros that the first stage (ZTOP) never reads, so neither read nor
         // reduced here.
@@ -265,7 +266,10 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     // (the thread's, warp by warp), or the last rows of the one group (R = 16).
     const bool kept = !kCutFwd || LOGR == 4 || static_cast<int>((xt >> (ROWOFF + 4)) << 4) < krows;
     if (kept) {
-      stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true>(v, tw, xt, p, c);
+      if (G == 1 && ztop)
+        stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true, G == 1>(v, tw, xt, p, c);
+      else
+        stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true>(v, tw, xt, p, c);
       inter_pass(v, xt, tb.hi_fwd, tb.lo_fwd);
     }
     __syncthreads();

@@ -121,3 +121,40 @@ def test_batches(hg, autotune):
         for k, (it, w) in enumerate(zip(items, want)):
             assert torch.equal(it[2], w), (schedule, sizes[k])
         b.close()
+
+
+@pytest.mark.parametrize("L", [13, 14, 16, 17])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_half_full_operands(hg, oracle, L, offset):
+    """Operands that just fill, or just miss filling, the lower half of a
+    transform's points (the first forward pass then skips its upper rows), as
+    limbs and as digits, on and off a 16-byte boundary, alone and in batches."""
+    import torch
+
+    from hypergeometrica_gb300 import device as D
+
+    items, want = [], []
+    for half in (1 << (L - 1), (1 << (L - 1)) * 5 // 4):
+        for nx in (half - 1, half, half + 1):
+            ny = half // 2 + nx % 7
+            x, y = W.limbs(L + nx, nx), W.limbs(2 * L + nx, ny, "ones")
+            tx, ty = torch.zeros(nx + offset, dtype=torch.int64, device="cuda"), _dev(y)
+            tx[offset:] = _dev(x)
+            out = torch.full((nx + ny,), -1, dtype=torch.int64, device="cuda")
+            D.mul(tx[offset:], ty, out)
+            D.sync()
+            w = oracle.mpz_mul_ntt(x, y)[: nx + ny]
+            assert np.array_equal(_np(out), w), (L, nx, offset)
+            items.append((tx[offset:], ty, out))
+            want.append(torch.from_numpy(w.view(np.int64).copy()).cuda())
+    for copies in (1, 40 if L < 16 else 4):  # a batch that fills the GPU runs on digits
+        many = [(x, y, torch.empty_like(o)) for _ in range(copies) for x, y, o in items]
+        for schedule in ("per_pass", "persistent"):
+            b = D.Batch(many, autotune=False, schedule=schedule)
+            for _, _, o in many:
+                o.fill_(-1)
+            b.run()
+            D.sync()
+            for k, (_, _, o) in enumerate(many):
+                assert torch.equal(o, want[k % len(want)]), (L, k, copies, schedule)
+            b.close()
