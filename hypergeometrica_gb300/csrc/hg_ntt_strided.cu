@@ -73,9 +73,11 @@ struct TmaMaps {
   CUtensorMap tw;
 };
 
-// A first forward pass's limbs per operand: the complete rows of S limbs the
-// load map covers, the limbs of the partial row after them, and (bit op of
-// ztop) whether every limb lies in the lower half of the block.
+// A first forward pass's limbs per load map: the complete rows of S limbs it
+// covers, the limbs of the partial row after them, and (bit k of ztop) whether
+// every limb of map k lies in the lower half of the block.  Map op is operand
+// op's; a long operand cut into chunks has its last chunk in map 1 and the
+// others, one after another in its third dimension, in map 0.
 struct TmaLimbs {
   const uint64_t *limbs[2];
   uint64_t full_rows[2];
@@ -91,8 +93,8 @@ struct TmaLimbs {
 // faster than with 80).
 //
 // LIMBS (forward only): the pass reads the operand's limbs, viewed as rows
-// of S limbs (a 2-D map over the rows that are complete; the copy fills the
-// rows past them with zeros) and patches the partial row past the last
+// of S limbs (a map over the rows that are complete, and over the chunks of a
+// long operand; the copy fills the rows past them with zeros) and patches the partial row past the last
 // complete one with plain loads before reducing every limb modulo p.  When
 // the upper half of the block lies past the limbs (P.ztop bit op), the first
 // stage skips its zero inputs.
@@ -153,6 +155,8 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   const int blk = static_cast<int>(t / ncg);
   const int s0 = static_cast<int>((t % ncg) << LOGTC);
   uint64_t *twt = tile + kInWords;
+  // The load map: an operand's, or the last chunk's.
+  const int sel = LIMBS && P.chunk ? (prod == P.nprod - 1 ? 1 : 0) : op;
 
   if (tid == 0) {
     tma::mbar_init(&bar, 1);
@@ -165,11 +169,12 @@ __global__ void __launch_bounds__(kTileThreads, 4)
                                          (TABLE ? static_cast<uint32_t>(krows) * row_bytes : 0u));
     if (TABLE) tma::load_3d(twt, &maps.tw, &bar, s0, 0, prime);  // no kernel of the stream writes the tables
     pdl_wait();
+    const int z = sel == op ? static_cast<int>(prod) : 0;  // chunk
     if constexpr (D80 && LOGR == 4) {
-      tma::load_2d(tile, &maps.in[op], &bar, s0 / 4 * 5, blk << LOGR);
-      tma::load_2d(tile + kInWords / 2, &maps.in[op], &bar, s0 / 4 * 5 + static_cast<int>(kRowWords) / 2, blk << LOGR);
+      tma::load_3d(tile, &maps.in[sel], &bar, s0 / 4 * 5, blk << LOGR, z);
+      tma::load_3d(tile + kInWords / 2, &maps.in[sel], &bar, s0 / 4 * 5 + static_cast<int>(kRowWords) / 2, blk << LOGR, z);
     } else if constexpr (LIMBS)
-      tma::load_2d(tile, &maps.in[op], &bar, D80 ? s0 / 4 * 5 : s0, blk << LOGR);
+      tma::load_3d(tile, &maps.in[sel], &bar, D80 ? s0 / 4 * 5 : s0, blk << LOGR, z);
     else
       tma::load_5d(tile, &maps.in[op], &bar, s0, 0, blk, prime - P.prime_lo, static_cast<int>(prod));
   }
@@ -208,13 +213,13 @@ __global__ void __launch_bounds__(kTileThreads, 4)
   if (!INV) {
     constexpr int AL = (G == 2) ? A1 : A0;
     xt = thread_base<AL>(tid);
-    const bool ztop = LIMBS && ((L.ztop >> op) & 1);
+    const bool ztop = LIMBS && ((L.ztop >> sel) & 1);
     if constexpr (LIMBS) {
       // Row tr (in the limbs' rows of S) is the partial one: limbs
       // [tr S, tr S + tail) exist past the complete rows the map covers.
-      const uint64_t tr = op ? L.full_rows[1] : L.full_rows[0];
-      const uint64_t tail = op ? L.tail[1] : L.tail[0];
-      const uint64_t *lp = op ? L.limbs[1] : L.limbs[0];
+      const uint64_t tr = sel ? L.full_rows[1] : L.full_rows[0];
+      const uint64_t tail = sel ? L.tail[1] : L.tail[0];
+      const uint64_t *lp = (op ? L.limbs[1] : L.limbs[0]) + prod * P.chunk;
       const uint64_t row0 = static_cast<uint64_t>(blk) << LOGR;
       const bool has_tail = tail != 0 && tr >= row0 && tr < row0 + (1u << LOGR);
       auto limb = [&](int i) {
@@ -507,27 +512,36 @@ cudaError_t launch_tma_r(const TmaMaps &m, const PassArgs &a, const TmaLimbs &l,
                : launch_tma_v<LOGR, false, false, false>(m, a, l, grid, st);
 }
 
-// The limbs of a single product's operand as rows of S limbs (5 S / 4 for
-// 80-bit digits): a 2-D map over the complete rows (none when the operand is
-// shorter than a row).
+// `count` operands of nl limbs, `stride` limbs apart, as rows of S limbs (5 S / 4
+// for 80-bit digits): a 3-D map over their complete rows.
 uint64_t limb_row(const PassArgs &a) { return limbs_of(uint64_t(1) << a.logS, a.dig80 != 0); }
 
-cudaError_t limb_map(CUtensorMap *m, const uint64_t *limbs, uint64_t nl, const PassArgs &a) {
+cudaError_t limb_map(CUtensorMap *m, const uint64_t *limbs, uint64_t nl, uint64_t count, uint64_t stride,
+                     const PassArgs &a) {
   const uint64_t W = limb_row(a), R = uint64_t(1) << a.logR;
-  const cuuint64_t dims[2] = {W, nl / W};
-  const cuuint64_t strides[1] = {W * 8};
+  const cuuint64_t dims[3] = {W, nl / W, count};
+  const cuuint64_t strides[2] = {W * 8, stride * 8};
   uint64_t cols = limbs_of((uint64_t(1) << kTileBits) / R, a.dig80 != 0);
   if (cols > 256) cols /= 2;  // R = 16: two boxes
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(cols), static_cast<cuuint32_t>(R)};
-  return encode(m, limbs, 2, dims, strides, box);
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(cols), static_cast<cuuint32_t>(R), 1};
+  return encode(m, limbs, 3, dims, strides, box);
 }
 
-// A first forward pass of one product (not a batch, not chunks) whose block
-// is the whole transform reads its limbs through TMA: each operand's limbs
+// The limbs of a cut operand's last chunk.
+uint64_t last_chunk(const PassArgs &a) { return a.nlimbs[0] - (a.nprod - 1) * a.chunk; }
+
+// A first forward pass of one product (not a batch) whose block is the whole
+// transform reads its limbs through TMA: each operand's limbs (each chunk's)
 // fill at least one row of S, start on a 16-byte boundary and lie in the
-// pass's single block.
+// pass's single block.  Chunks against per-thread loads: 2^24 x 2^16 limbs
+// 1709 -> 1692 us, 20000 x 500 35.8 -> 34.5, 2^22 x 2^14 439.7 -> 434.9.
 bool tma_limbs_ok(const PassArgs &a) {
-  if (a.batch || a.chunk || a.nprod != 1 || a.logS + a.logR != a.logN) return false;
+  if (a.batch || a.logS + a.logR != a.logN) return false;
+  if (a.chunk)
+    return a.nops == 1 && a.nprod > 1 && a.limbs[0] && (reinterpret_cast<uintptr_t>(a.limbs[0]) & 15u) == 0 &&
+           a.chunk % 2 == 0 && a.chunk >= limb_row(a) && coefs_of(a.chunk, a.dig80 != 0) <= (uint64_t(1) << a.logN) &&
+           a.nlimbs[0] > (a.nprod - 1) * a.chunk && last_chunk(a) <= a.chunk && last_chunk(a) >= limb_row(a);
+  if (a.nprod != 1) return false;
   for (int op = 0; op < a.nops; ++op) {
     if (!a.limbs[op] || (reinterpret_cast<uintptr_t>(a.limbs[op]) & 15u)) return false;
     if (a.nlimbs[op] < limb_row(a) || coefs_of(a.nlimbs[op], a.dig80 != 0) > (uint64_t(1) << a.logN)) return false;
@@ -577,27 +591,36 @@ cudaError_t launch_ntt_strided(const PassArgs &a, bool inverse, cudaStream_t st)
     return cudaErrorInvalidValue;
   }
   if (tma_aligned(a) && (!limbs || tma_limbs_ok(a))) {
-    TmaMaps m;
+    TmaMaps m{};
     TmaLimbs l{};
     cudaError_t e = cudaSuccess;
     for (int op = 0; op < 2 && e == cudaSuccess; ++op) {
-      const uint64_t *d = (op < a.nops) ? a.data[op] : a.data[0];
-      e = residue_map(&m.out[op], d, a);
+      if (op >= a.nops && !(limbs && a.chunk)) break;  // no CTA uses map 1; an encode is 0.5 to 1 us of host time
+      if (op < a.nops) e = residue_map(&m.out[op], a.data[op], a);
       if (e != cudaSuccess) break;
       if (!limbs) {
         m.in[op] = m.out[op];
         continue;
       }
       const int lo = op < a.nops ? op : 0;
-      l.limbs[op] = a.limbs[lo];
-      l.full_rows[op] = a.nlimbs[lo] / limb_row(a);
-      l.tail[op] = a.nlimbs[lo] % limb_row(a);
+      const uint64_t *p = a.limbs[lo];
+      uint64_t nl = a.nlimbs[lo], count = 1, stride = limb_row(a);
+      l.limbs[op] = p;
+      if (a.chunk && op == 0) {
+        nl = stride = a.chunk;
+        count = a.nprod - 1;
+      } else if (a.chunk) {
+        nl = last_chunk(a);
+        p += (a.nprod - 1) * a.chunk;
+      }
+      l.full_rows[op] = nl / limb_row(a);
+      l.tail[op] = nl % limb_row(a);
       // Every limb lies in the lower half of the block: the first stage's
       // upper inputs are zero.
-      if (coefs_of(a.nlimbs[lo], a.dig80 != 0) <= (uint64_t(1) << (a.logS + a.logR - 1))) l.ztop |= 1u << op;
-      e = limb_map(&m.in[op], a.limbs[lo], a.nlimbs[lo], a);
+      if (coefs_of(nl, a.dig80 != 0) <= (uint64_t(1) << (a.logS + a.logR - 1))) l.ztop |= 1u << op;
+      e = limb_map(&m.in[op], p, nl, count, stride, a);
     }
-    if (e == cudaSuccess) e = a.ptw ? twiddle_map(&m.tw, a.ptw, a) : residue_map(&m.tw, a.data[0], a);
+    if (e == cudaSuccess && a.ptw) e = twiddle_map(&m.tw, a.ptw, a);
     if (e != cudaSuccess) return e;
     switch (a.logR) {
       case 4: return launch_tma_r<4>(m, a, l, inverse, limbs, g, st);

@@ -158,3 +158,36 @@ def test_half_full_operands(hg, oracle, L, offset):
             for k, (_, _, o) in enumerate(many):
                 assert torch.equal(o, want[k % len(want)]), (L, k, copies, schedule)
             b.close()
+
+
+@pytest.mark.parametrize("ny", [1 << 9, 5000, 1 << 15])
+def test_chunk_edges(hg, ny):
+    """A long operand in chunks whose last one has a limb, a row less one, a
+    row, half a chunk and a whole chunk, on and off a 16-byte boundary (bulk
+    copies, or per-thread loads), against one transform."""
+    import torch
+
+    from hypergeometrica_gb300 import device as D
+    from hypergeometrica_gb300._lib import chunk_plan, set_chunking
+
+    L, C, _ = chunk_plan(64 * ny, ny)
+    y = _dev(W.limbs(ny, ny, "ones"))
+    for K in (2, 3, 9):
+        for rest in (1, 15, 16, 319, 320, 1023, 1024, 1281, C // 2 - 1, C // 2, C // 2 + 1, C - 1, C):
+            nx = (K - 1) * C + rest
+            x = torch.zeros(nx + 1, dtype=torch.int64, device="cuda")
+            x[:nx] = _dev(W.limbs(nx, nx, ("uniform", "ones")[rest % 2]))
+            got = torch.full((nx + ny + 3,), -1, dtype=torch.int64, device="cuda")
+            off, want = torch.empty_like(got), torch.empty_like(got)
+            D.mul(x[:nx], y, got)
+            shifted = torch.zeros(nx + 1, dtype=torch.int64, device="cuda")
+            shifted[1:] = x[:nx]
+            D.mul(y, shifted[1:], off)
+            assert set_chunking(False)
+            try:
+                D.mul(x[:nx], y, want)
+                D.sync()
+            finally:
+                set_chunking(True)
+            assert torch.equal(got, want), (ny, K, rest)
+            assert torch.equal(off, want), (ny, K, rest)
