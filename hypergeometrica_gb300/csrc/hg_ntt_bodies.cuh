@@ -25,7 +25,10 @@ constexpr int kFwd = 0, kInv = 1, kMul = 2, kSqr = 3, kMulSpec = 4;
 // CUT: forward, the outer pass of a truncated transform, which keeps P.krows
 // rows; inverse, a transform's last pass that scales by P.scale.
 // D80: the operands' coefficients are 80-bit digits.
-template <int LOGR, bool INV, bool CUT = false, bool D80 = false>
+// SKIP: limbs that lie in the lower half of the block leave registers 8..15 to
+// the first stage's ZTOP form.  Not in the persistent kernel: the second copy
+// of the rounds took its 4096-pair batch from 3.90 to 4.44 ms.
+template <int LOGR, bool INV, bool CUT = false, bool D80 = false, bool SKIP = false>
 __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid, ulonglong2 *tw, uint64_t *sm) {
   constexpr int T = kTileBits;
   constexpr int LOGTC = T - LOGR;  // log2 columns per tile
@@ -94,9 +97,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     offsets(xt, AL, off, step);
     uint64_t nl = 0;
     const uint64_t *limbs = pass_limbs(P, prod, op, nl);
-    // Limbs in the lower half of the block only: registers 8..15 are zeros that
-    // the first stage (ZTOP) never reads.
-    const bool ztop = limbs && blk == 0 && coefs_of(nl, D80) <= (uint64_t(1) << (logM - 1));
+    const bool ztop = SKIP && limbs && blk == 0 && coefs_of(nl, D80) <= (uint64_t(1) << (logM - 1));
     if (limbs) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -114,7 +115,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     __syncthreads();  // twiddle table ready
     if constexpr (G == 2) {
       if (ztop)
-        stages<NB1, 4 - NB1, A1, ROWOFF, 4, LOGR, false, false, false, true>(v, tw, xt, p, c);
+        stages<NB1, 4 - NB1, A1, ROWOFF, 4, LOGR, false, false, false, SKIP>(v, tw, xt, p, c);
       else
         stages<NB1, 4 - NB1, A1, ROWOFF, 4, LOGR, false, false>(v, tw, xt, p, c);
       to_smem<A1>(sm, v, xt);
@@ -127,7 +128,7 @@ __device__ __forceinline__ void strided_ldg_body(const PassArgs &P, uint64_t bid
     const int keep = CUT ? P.krows - static_cast<int>((xt >> (ROWOFF + 4)) << 4) : 16;
     if (CUT && LOGR > 4 && keep <= 0) return;
     if (G == 1 && ztop)
-      stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true, G == 1>(v, tw, xt, p, c);
+      stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true, SKIP && G == 1>(v, tw, xt, p, c);
     else
       stages<4, 0, A0, ROWOFF, 0, LOGR, false, true, true>(v, tw, xt, p, c);  // then the inter-pass twiddle
     inter_pass(v, xt, tb.hi_fwd, tb.lo_fwd);

@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) ntt_strided_kernel(const Pass
   __shared__ ulonglong2 tw[1 << (LOGR - 1)];
   __shared__ uint64_t sm[LOGR > 4 ? (1 << kTileBits) : 1];
   pdl_wait();
-  strided_ldg_body<LOGR, INV, CUT, D80>(P, blockIdx.x, tw, sm);
+  strided_ldg_body<LOGR, INV, CUT, D80, true>(P, blockIdx.x, tw, sm);
 }
 
 constexpr int kCut = 0;  // KQ of a truncated transform's outer forward pass
