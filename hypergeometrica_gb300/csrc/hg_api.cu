@@ -1944,7 +1944,7 @@ int batch_autotune(hg_batch *b) {
 }
 
 // Time the whole batch on both schedules and keep the faster: one run after
-// one that warms up and, below half a millisecond, four in a row instead, so
+// one that warms up and, below half a millisecond, three in a row instead, so
 // that a schedule whose launches take the host longer than the GPU is charged
 // for it.
 int schedule_autotune(hg_batch *b) {
@@ -1956,8 +1956,8 @@ int schedule_autotune(hg_batch *b) {
   float ms[2] = {0, 0};
   for (int sched = 0; sched < 2 && rc == HG_OK; ++sched) {
     b->persistent = sched == 1;
-    bool warm = false;
-    for (int runs : {1, 1, 4}) {
+    for (int timed = 0; timed < 2 && rc == HG_OK; ++timed) {
+      const int runs = timed && ms[sched] < 0.5f ? 3 : 1;
       cudaEventRecord(e0, st);
       for (int k = 0; k < runs && rc == HG_OK; ++k)
         rc = b->persistent ? persist_run(b, st) : enqueue_batch(b->bp, batch_bufs(b), st);
@@ -1967,8 +1967,6 @@ int schedule_autotune(hg_batch *b) {
       else cudaEventElapsedTime(&ms[sched], e0, e1);
       if (rc) break;
       ms[sched] /= runs;
-      if (warm && ms[sched] > 0.5f) break;
-      warm = true;
     }
   }
   cudaEventDestroy(e0);
