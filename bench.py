@@ -464,7 +464,7 @@ def run_sweep(stream, peak_gbs: float) -> dict:
     """The balanced single-product sweep: a x b and a^2 with |a| = |b| = 2^18 ..
     2^26 limbs (uniform limbs, seeds 11, 12), device-resident, CUDA events.
     Each line: ms per product, output limbs/s, and the minimum-pass HBM
-    bytes (16 (na + nb) + 192 N for a product, 24 n + 96 N for a square) over
+    bytes (16 (na + nb) + 192 P for a product, 24 n + 96 P for a square, P the points kept) over
     the time as a fraction of the measured copy bandwidth."""
     import numpy as np
     import torch
@@ -486,7 +486,6 @@ def run_sweep(stream, peak_gbs: float) -> dict:
         a = torch.from_numpy(W.limbs(11, n).view(np.int64)).cuda()
         b = torch.from_numpy(W.limbs(12, n).view(np.int64)).cuda()
         o = torch.empty(2 * n, dtype=torch.int64, device="cuda")
-        N = 1 << (k + 1)
         reps = max(2, min(20, (1 << 26) // n))
         for kind in ("mul", "sqr"):
             f = (lambda: D.mul(a, b, o, stream=stream)) if kind == "mul" else (lambda: D.sqr(a, o, stream=stream))
@@ -504,7 +503,8 @@ def run_sweep(stream, peak_gbs: float) -> dict:
             x = W.limbs(11, n)
             ok, how = exact.check((kind, k), o.cpu().numpy().view(np.uint64), x,
                                   x if kind == "sqr" else W.limbs(12, n))
-            algo = (16 * 2 * n + 192 * N) if kind == "mul" else (24 * n + 96 * N)
+            pts = _kept_points(n)[0]
+            algo = (16 * 2 * n + 192 * pts) if kind == "mul" else (24 * n + 96 * pts)
             out["lines"].append({"log_size": k, "kind": kind, "ms": ms, "limbs_per_s": 2 * n / (ms / 1000.0),
                                  "hbm_frac": algo / (ms / 1000.0) / 1e9 / peak_gbs, "correct": ok, "check": how})
         del a, b, o
@@ -649,16 +649,28 @@ def run_expt() -> dict:
 
 # Thread instructions per radix-2 butterfly of the middle kernel (ncu,
 # profiles/ntt_contig_mul_2e22.md): the fewest any pass of the product spends.
-INSTR_PER_BUTTERFLY = 29.2
+INSTR_PER_BUTTERFLY = 27.9
 
 
-def _int_roofline(N: int, ms_per_product: float, sm_mhz) -> dict:
-    """The product's radix-2 butterflies (3 primes x 3 transforms x N/2 log2 N)
-    per second against two ceilings: hg_butterfly_peak, a memory-free network
-    of the same modular butterflies over every SM measured now, and the
-    issue-rate floor, every SM sub-partition issuing one warp instruction
-    per clock at the clock sampled under load, with the middle kernel's
-    29.2 thread instructions per butterfly."""
+def _kept_points(n: int) -> tuple[int, int]:
+    """(points, log2 of the transform) that a balanced product of n limbs per
+    operand keeps: sixteenths of the power of two above its 80-bit digits
+    (products above 2^19 limbs; the whole transform up to there)."""
+    if 2 * n <= 1 << 19:
+        return 1 << (2 * n - 1).bit_length(), (2 * n - 1).bit_length()
+    d = 2 * ((4 * n + 4) // 5)
+    L = (d - 1).bit_length()
+    k = max(9, -(-d // (1 << (L - 4))))
+    return k << (L - 4), L
+
+
+def _int_roofline(n: int, ms_per_product: float, sm_mhz) -> dict:
+    """The radix-2 butterflies of an n x n-limb product (3 primes x 3 transforms
+    x points/2 log2 N, the points kept of N) per second against two ceilings:
+    hg_butterfly_peak, a memory-free network of the same modular butterflies
+    over every SM measured now, and the issue-rate floor, every SM
+    sub-partition issuing one warp instruction per clock at the clock sampled
+    under load, with the middle kernel's 27.9 thread instructions per butterfly."""
     import ctypes
 
     import torch
@@ -667,7 +679,8 @@ def _int_roofline(N: int, ms_per_product: float, sm_mhz) -> dict:
 
     pk = ctypes.c_double()
     _lib.check(_lib.load().hg_butterfly_peak(ctypes.byref(pk)))
-    bf = 3 * 3 * (N // 2) * (N.bit_length() - 1)
+    points, log_n = _kept_points(n)
+    bf = 3 * 3 * (points // 2) * log_n
     achieved = bf / (ms_per_product / 1000.0)
     sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
     mhz = sm_mhz or 2070.0
@@ -832,8 +845,7 @@ def run_ours(args) -> None:
     peak, peak_kind = _peaks()
     d = prof[dom]
     achieved = (d["bytes"] / d["launches"]) / (d["ms"] / d["launches"] / 1000.0) / 1e9 if d["ms"] > 0 else 0.0
-    N = 1 << (args.log_size + 1)
-    b_mul = 16 * n_out + 192 * N  # minimum-pass algorithmic bytes of one product
+    b_mul = 16 * n_out + 192 * _kept_points(na)[0]  # minimum-pass algorithmic bytes of one product
     prod_gbs = b_mul / (ms / args.steps / 1000.0) / 1e9
     traffic = _traffic(dom)
 
@@ -862,8 +874,8 @@ def run_ours(args) -> None:
                      "launches": d["launches"], "ms_per_launch": d["ms"] / max(1, d["launches"]),
                      "pipes": _pipes(dom)},
         "roofline_product": {"algorithmic_bytes": b_mul, "achieved": prod_gbs, "frac": prod_gbs / peak,
-                             "unit": "GB/s", "formula": "16(na+nb) + 192 N"},
-        "roofline_int": _int_roofline(N, ms / args.steps, clocks["sm_mhz"]),
+                             "unit": "GB/s", "formula": "16(na+nb) + 192 x points kept"},
+        "roofline_int": _int_roofline(na, ms / args.steps, clocks["sm_mhz"]),
         "kernels": {k: {"launches": v["launches"], "ms": v["ms"]} for k, v in prof.items() if v["launches"]},
         "clocks": {"sm_mhz": clocks["sm_mhz"], "sm_max_mhz": clocks["sm_max_mhz"], "reasons": clocks["reasons"],
                    "samples": clocks["samples"]},

@@ -35,7 +35,7 @@ struct PrimeConst {
 enum DevErr : int {
   kDevOk = 0,
   kDevCarryOverflow = 2,  // a carry left the top of the result
-  kDevTicket = 3,         // a carry tile ticket fell outside its launch, or a tile aggregate of another launch
+  kDevTicket = 3,         // a carry met a tile aggregate of another launch
   kDevCopyTimeout = 4,    // a tile copy (TMA) did not land within its wait limit
   kDevQueueTimeout = 5,   // a persistent batch's item waited past its limit for the phase before it
   // Checked builds (HG_CHECKED) only:

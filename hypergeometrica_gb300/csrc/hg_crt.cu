@@ -11,7 +11,8 @@
 // within a CTA by warp shuffles.  Across CTAs each tile is written with
 // carry-in 0 and publishes its (generate, propagate) aggregate; a second
 // launch composes every tile's carry-in from the aggregates below it and
-// applies it.  No kernel here waits on another CTA.
+// applies it (in a short launch, the CTA that finishes last does).  No kernel
+// here waits on another CTA.  80-bit digits add up at 2^(80 i) the same way.
 //
 // The same overlap-add + scan finishes the schoolboy and by-digit products
 // (src/mpz-ram.lisp:367-431), with V_i = sum_j x_(i-j) y_j.
@@ -38,12 +39,12 @@ constexpr int kShortPer = 4;
 constexpr int kShortTile = kCarryThreads * kShortPer;
 constexpr uint64_t kShortCarry = static_cast<uint64_t>(kShortTile) * kCarryThreads;
 
-// The product of a long operand cut into chunks of `chunk` limbs with a
-// short one: chunk k's cyclic product (2^logN > chunk + short - 1 points, no
-// wrap) covers result positions [k chunk, k chunk + 2^logN), and chunk >=
-// 2^(logN-1) makes at most two chunks meet at a position.  Their residues
-// are added before the reconstruction: the sum of the two coefficients is
-// below 2 * short * 2^128, far below p0 p1 p2, so Garner's value of the
+// The product of a long operand cut into chunks of `chunk` coefficients (limbs
+// or 80-bit digits) with a short one: chunk k's cyclic product (n > chunk +
+// short - 1 points, no wrap) covers result positions k chunk .. k chunk + chunk
+// + short - 2, and chunk >= short makes at most two chunks meet at a position.
+// Their residues are added before the reconstruction: the sum is the product's
+// own coefficient, below short * 2^160 < p0 p1 p2 (2^128 on limbs), so Garner's value of the
 // summed residues is the exact sum.  The inverse leaves residues in
 // [0, 2p); each is folded to [0, p) before the sum, and Garner's Shoup
 // products take the sum in [0, 2p) as it is.

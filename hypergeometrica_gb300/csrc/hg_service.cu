@@ -36,7 +36,7 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 constexpr int kMaxSlots = 8;
-constexpr size_t kSlotTickets = 512;  // carry-scan tickets per slot (one per group)
+constexpr size_t kSlotTickets = 512;  // finished-tile counts of the carries per slot (one per group)
 
 struct SvcRequest {
   ProductDesc d;

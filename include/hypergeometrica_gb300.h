@@ -98,14 +98,16 @@ size_t hg_ntt_length(size_t nx, size_t ny);
 // counterpart in the reference, whose mpz-*/ntt always runs one transform of
 // hg_ntt_length(nx, ny) points).  Returns 1 when the longer operand is cut
 // into *nchunks chunks of *chunk limbs, each multiplied by the shorter one
-// with transforms of 2^*log_len points (the result is the same integer);
+// with transforms of at most 2^*log_len points (the result is the same integer);
 // 0 when the product runs as one transform, or on a null pointer.  Host
 // arithmetic only: needs no device and no hg_init.
 int hg_chunk_plan(size_t nx, size_t ny, int *log_len, size_t *chunk, size_t *nchunks);
 
-// Whether unbalanced products may run in chunks (hg_chunk_plan); on by
-// default.  With 0 every product runs as the reference's one transform of
-// hg_ntt_length(nx, ny) points.  Returns the previous setting.  Process-wide;
+// Whether products may leave the reference's one transform of
+// hg_ntt_length(nx, ny) points on limbs: unbalanced ones for chunks
+// (hg_chunk_plan), others for 9 to 15 sixteenths of the points and for 80-bit
+// digits.  On by default; the result is the same integer.  Returns the previous
+// setting.  Process-wide;
 // takes effect for products enqueued after it returns.  No counterpart in
 // the reference.
 int hg_set_chunking(int enable);
@@ -194,7 +196,7 @@ int hg_mul_sized_device(const uint64_t *x, size_t nx, const uint64_t *y, size_t 
  *    capture begins.  A call with another device current is HG_ERR_ARG.
  *  - nx + ny > HG_NOALLOC_MAX_LIMBS is rejected with HG_ERR_ARG before
  *    anything is enqueued.
- *  - The carry scan's ticket and flag words in the scratch must be zero
+ *  - The carry scan's count and flag words in the scratch must be zero
  *    when its kernel starts; the call clears them on stream itself
  *    (cudaMemsetAsync), so the caller zeroes nothing.
  *  - There is one scratch array per device, shared by every call: calls
