@@ -172,7 +172,8 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     const int z = sel == op ? static_cast<int>(prod) : 0;  // chunk
     if constexpr (D80 && LOGR == 4) {
       tma::load_3d(tile, &maps.in[sel], &bar, s0 / 4 * 5, blk << LOGR, z);
-      tma::load_3d(tile + kInWords / 2, &maps.in[sel], &bar, s0 / 4 * 5 + static_cast<int>(kRowWords) / 2, blk << LOGR, z);
+      tma::load_3d(tile + kInWords / 2, &maps.in[sel], &bar, s0 / 4 * 5 + static_cast<int>(kRowWords) / 2, blk << LOGR,
+                   z);
     } else if constexpr (LIMBS)
       tma::load_3d(tile, &maps.in[sel], &bar, D80 ? s0 / 4 * 5 : s0, blk << LOGR, z);
     else
@@ -232,8 +233,9 @@ __global__ void __launch_bounds__(kTileThreads, 4)
           // R = 16: columns 0 .. C/2 - 1 in the first box, the others in the second.
           const uint32_t half = LOGR == 4 ? col >> (LOGTC - 1) : 0u;
           const uint32_t lc = LOGR == 4 ? col & ((1u << (LOGTC - 1)) - 1u) : col;
-          const uint32_t at = half * (kInWords / 2) + row * (LOGR == 4 ? kRowWords / 2 : kRowWords) + ((5u * lc) >> 2);
-          return digit80(tile[at], tile[at + 1], lc, P.pc[prime]);
+          const uint32_t at = half * (kInWords / 2) + row * (LOGR == 4 ? kRowWords / 2 : kRowWords);
+          const uint32_t *w = reinterpret_cast<const uint32_t *>(tile + at) + ((5u * lc) >> 1);
+          return digit80_words(w[0], w[1], w[2], lc & 1u, P.pc[prime]);
         } else {
           uint64_t w = tile[x];
           if (has_tail && row0 + row == tr && s0 + col < tail) w = __ldg(lp + (tr << logS) + s0 + col);
