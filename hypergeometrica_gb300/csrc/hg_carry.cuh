@@ -43,23 +43,16 @@ __device__ __forceinline__ void add_product_to(V3 &acc, uint64_t x, uint64_t y) 
   add128_to(acc, static_cast<uint64_t>(v), static_cast<uint64_t>(v >> 64));
 }
 
-// COHERENT: the residues were written earlier in the same launch (the
-// persistent batch kernel), so they are read through L2 (ld.global.cg)
-// rather than the read-only data path, which is coherent only for data no
-// CTA of the launch writes.  PRESCALED: the residues are the coefficients
-// mod p_j (CrtConst::prescaled).
-template <bool COHERENT = false, bool PRESCALED = false>
+// The residues are read through L2 (ld.global.cg), not by the read-only data
+// path: the launch before wrote them (or, in the persistent batch kernel, an
+// earlier phase of the same launch), and a dependent launch is resident before
+// those writes are visible.  PRESCALED: the residues are the coefficients mod
+// p_j (CrtConst::prescaled).
+template <bool PRESCALED = false>
 struct CrtProducerT {
   const uint64_t *res;  // [3][N] natural-order residues from the unscaled inverse
   uint64_t n;           // N
   CrtConst k;
-
-  __device__ __forceinline__ static ulonglong2 load2(const ulonglong2 *p) {
-    if constexpr (COHERENT)
-      return __ldcg(p);
-    else
-      return __ldg(p);
-  }
 
   // Coefficient i of the product whose residues start `off` words past res.
   __device__ __forceinline__ V3 at(uint64_t off, uint64_t i) const {
@@ -77,7 +70,7 @@ struct CrtProducerT {
         const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(res + off + j * n + i0);
 #pragma unroll
         for (int q = 0; q < PER / 2; ++q) {
-          const ulonglong2 w = load2(src + q);
+          const ulonglong2 w = __ldcg(src + q);
           r[j][2 * q] = w.x;
           r[j][2 * q + 1] = w.y;
         }
@@ -133,7 +126,7 @@ struct CrtProducerT {
   }
 };
 
-using CrtProducer = CrtProducerT<false>;
+using CrtProducer = CrtProducerT<>;
 
 // A tile's published aggregate: the launch's epoch in the high word, then
 // p, g and the state bit 1 ("published").

@@ -96,8 +96,8 @@ struct ChunkProducerT {
 #pragma unroll
       for (int q = 0; q < PER / 2; ++q) {
         ulonglong2 a = make_ulonglong2(0, 0), b = make_ulonglong2(0, 0);
-        if (r0) a = __ldg(reinterpret_cast<const ulonglong2 *>(r0 + j * crt.n) + q);
-        if (r1) b = __ldg(reinterpret_cast<const ulonglong2 *>(r1 + j * crt.n) + q);
+        if (r0) a = __ldcg(reinterpret_cast<const ulonglong2 *>(r0 + j * crt.n) + q);
+        if (r1) b = __ldcg(reinterpret_cast<const ulonglong2 *>(r1 + j * crt.n) + q);
         r[j][2 * q] = sum2(a.x, b.x, p);
         r[j][2 * q + 1] = sum2(a.y, b.y, p);
       }
@@ -465,7 +465,7 @@ cudaError_t launch_coefs(const Producer &prod, bool dig80, uint64_t *out, uint64
   return dig80 ? launch_carry<true>(prod, out, nproc, tiles, sh, ss, st, batch, tpp, ws_stride, n)
                : launch_carry<false>(prod, out, nproc, tiles, sh, ss, st, batch, tpp, ws_stride, n);
 }
-using Prescaled = carry::CrtProducerT<false, true>;
+using Prescaled = carry::CrtProducerT<true>;
 }  // namespace
 
 cudaError_t launch_crt_carry(const uint64_t *res, uint64_t n, bool dig80, const CrtConst &cc, uint64_t *out,

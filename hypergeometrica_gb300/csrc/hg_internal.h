@@ -186,9 +186,9 @@ __device__ __forceinline__ uint64_t coefficient(const uint64_t *limbs, uint64_t 
   if constexpr (D80) {
     const uint64_t w = (5 * j) >> 2;
     if (w >= nl) return 0;
-    return digit80(__ldg(limbs + w), w + 1 < nl ? __ldg(limbs + w + 1) : 0, static_cast<uint32_t>(j), pc);
+    return digit80(limbs[w], w + 1 < nl ? limbs[w + 1] : 0, static_cast<uint32_t>(j), pc);
   } else {
-    return j < nl ? reduce64(__ldg(limbs + j), pc.p) : 0;
+    return j < nl ? reduce64(limbs[j], pc.p) : 0;
   }
 }
 
@@ -200,7 +200,10 @@ __device__ __forceinline__ uint64_t coefficient(const uint64_t *limbs, uint64_t 
 // and waits in pdl_wait, which returns once the kernels before have completed
 // and their writes are visible.  Every kernel launched by launch_dep calls
 // pdl_wait before its first access to memory that another kernel writes or
-// reads.  A product of 2^13 points 31.8 -> 23.2 us, of 2^16 points 37.0 ->
+// reads, and reads such memory (residues, spectra, operands) by plain, .cg or
+// volatile loads: the read-only path (__ldg) is for memory that nothing writes
+// while the kernel is resident, which here leaves the twiddle tables, and a
+// load in asm that is not volatile may be moved above the wait.  A product of 2^13 points 31.8 -> 23.2 us, of 2^16 points 37.0 ->
 // 28.0, a 2^20-limb square 261 -> 244, 2^24 x 2^24 limbs 5528 -> 5508, the
 // 4096-pair batch 3545 -> 3438.  No kernel triggers its successor early
 // (griddepcontrol.launch_dependents): CTAs that become resident beside a

@@ -280,7 +280,7 @@ __device__ __forceinline__ void load_block(uint64_t (&v)[16], const uint64_t *da
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const uint64_t o = base + (xt | (static_cast<uint32_t>(i) << A));
-      v[i] = o < nl ? reduce64(__ldg(limbs + o), p) : 0;
+      v[i] = o < nl ? reduce64(limbs[o], p) : 0;
     }
   } else {
 #pragma unroll

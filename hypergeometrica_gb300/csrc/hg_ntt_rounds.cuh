@@ -23,7 +23,7 @@ namespace rounds {
 // ms; marking the tables' loads evict-last as well measured 2.334 ms).
 __device__ __forceinline__ uint64_t ld_once(const uint64_t *p) {
   uint64_t v;
-  asm("ld.global.L1::no_allocate.u64 %0, [%1];" : "=l"(v) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.u64 %0, [%1];" : "=l"(v) : "l"(p));
   return v;
 }
 

@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
         if constexpr (D80)
           w = coefficient<true>(lp, tr * (uint64_t(5) << (logS - 2)) + tail, at, P.pc[prime]);
         else if (s0 + col < tail)
-          w = reduce64(__ldg(lp + at), p);
+          w = reduce64(lp[at], p);
 #pragma unroll
         for (int i = 0; i < 16; ++i)
           v[i] = i < nreg && (d >> (AL - ROWOFF)) == static_cast<uint32_t>(i) ? w : v[i];
