@@ -370,7 +370,7 @@ int init_locked(const uint64_t *moduli, int k, const uint64_t *roots, int maxlg,
     }
   }
   HG_CUDA(c.tables.ensure(host.size() * sizeof(uint64_t)), "table allocation");
-  HG_CUDA(cudaMemcpy(c.tables.p, host.data(), host.size() * sizeof(uint64_t), cudaMemcpyHostToDevice), "table upload");
+  HG_CUDA(upload_now(c.tables.p, host.data(), host.size() * sizeof(uint64_t)), "table upload");
   for (int i = 0; i < kPrimes; ++i) {
     const uint64_t *t = c.tables.u64() + i * kPrimeTableWords;
     c.tb[i].sub_fwd = reinterpret_cast<const ulonglong2 *>(t);
@@ -392,8 +392,8 @@ int init_locked(const uint64_t *moduli, int k, const uint64_t *roots, int maxlg,
     HG_CUDA(cudaEventCreateWithFlags(&L.carry_done, cudaEventDisableTiming), "event creation");
     HG_CUDA(cudaEventCreateWithFlags(&L.d2h_done, cudaEventDisableTiming), "event creation");
     HG_CUDA(L.misc.ensure(64), "scan state allocation");
-    HG_CUDA(cudaMemset(L.misc.p, 0, 64), "scan state init");
-    HG_CUDA(cudaMemset(static_cast<char *>(L.misc.p) + 16, 0xff, 2 * sizeof(long long)), "scan state init");
+    HG_CUDA(fill_now(L.misc.p, 0, 64), "scan state init");
+    HG_CUDA(fill_now(static_cast<char *>(L.misc.p) + 16, 0xff, 2 * sizeof(long long)), "scan state init");
   }
   c.lane = &c.lanes[0];
   c.ready = true;
@@ -801,7 +801,7 @@ int scan_state(uint64_t tiles, ScanState *ss) {
   if (need > c.lane->flags.bytes) {
     HG_CUDA(cudaDeviceSynchronize(), "sync before flag growth");
     HG_CUDA(c.lane->flags.ensure(need * 2), "flag allocation");
-    HG_CUDA(cudaMemset(c.lane->flags.p, 0, c.lane->flags.bytes), "flag init");
+    HG_CUDA(fill_now(c.lane->flags.p, 0, c.lane->flags.bytes), "flag init");
   }
   if (++c.lane->epoch == 0) c.lane->epoch = 1;
   ss->done = static_cast<unsigned *>(c.lane->misc.p);
@@ -1876,8 +1876,7 @@ int persist_build(hg_batch *b) {
     first += p.count;
   }
   HG_CUDA(b->d_phases.ensure(out.size() * sizeof(PersistPhase)), "batch work list");
-  HG_CUDA(cudaMemcpy(b->d_phases.p, out.data(), out.size() * sizeof(PersistPhase), cudaMemcpyHostToDevice),
-          "batch work list upload");
+  HG_CUDA(upload_now(b->d_phases.p, out.data(), out.size() * sizeof(PersistPhase)), "batch work list upload");
   HG_CUDA(b->d_state.ensure(persist_state_bytes(static_cast<int>(out.size()))), "batch work counters");
   b->phases.swap(out);
   b->items = first;
@@ -2013,13 +2012,12 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
   const BatchPlan &bp = b->bp;
   if (!bp.desc.empty()) {
     HG_CUDA(b->d_desc.ensure(bp.desc.size() * sizeof(ProductDesc)), "batch descriptors");
-    HG_CUDA(cudaMemcpy(b->d_desc.p, bp.desc.data(), bp.desc.size() * sizeof(ProductDesc), cudaMemcpyHostToDevice),
-            "batch descriptors upload");
+    HG_CUDA(upload_now(b->d_desc.p, bp.desc.data(), bp.desc.size() * sizeof(ProductDesc)), "batch descriptors upload");
   }
   if (bp.ws_words) HG_CUDA(b->ws.ensure(bp.ws_words * 8), "batch workspace");
   if (bp.flag_words) HG_CUDA(b->flags.ensure(bp.flag_words * 8), "batch scan flags");
   HG_CUDA(b->tickets.ensure(std::max<size_t>(1, bp.groups.size()) * 8), "batch scan counts");
-  HG_CUDA(cudaMemset(b->tickets.p, 0, b->tickets.bytes), "batch scan counts");
+  HG_CUDA(fill_now(b->tickets.p, 0, b->tickets.bytes), "batch scan counts");
   if (bp.parallel && bp.groups.size() > 1) HG_CUDA(b->side.create(), "batch streams");
   if ((flags & HG_BATCH_PER_PASS) && (flags & HG_BATCH_PERSISTENT))
     return fail(HG_ERR_ARG, "a batch runs either per pass or persistently, not both");
@@ -2037,7 +2035,7 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
     if (!b->whole.desc.empty()) {
       const size_t bytes = b->whole.desc.size() * sizeof(ProductDesc);
       HG_CUDA(b->d_whole.ensure(bytes), "batch descriptors");
-      HG_CUDA(cudaMemcpy(b->d_whole.p, b->whole.desc.data(), bytes, cudaMemcpyHostToDevice), "batch descriptors upload");
+      HG_CUDA(upload_now(b->d_whole.p, b->whole.desc.data(), bytes), "batch descriptors upload");
     }
     if ((rc = persist_build(b.get()))) return rc;
     b->persistent = b->items > 0;

@@ -81,6 +81,18 @@ int large_sum_device(const SumOperand &a, int64_t sa, const SumOperand &b, int64
 // products, run every group.  Takes no lock and allocates nothing.
 int enqueue_batch(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st);
 
+// Fill or upload device memory, done on return.  cudaMemset and cudaMemcpy from
+// pageable memory may return before the device is done, and neither the
+// library's streams nor a caller's are ordered after the null stream.
+inline cudaError_t fill_now(void *p, int byte, size_t bytes) {
+  const cudaError_t e = cudaMemset(p, byte, bytes);
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
+inline cudaError_t upload_now(void *dst, const void *src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
+
 // Words that kernels write and the host reads after a synchronisation.
 struct HostWords {
   int64_t *host, *dev;

@@ -120,11 +120,11 @@ int slot_alloc(SvcSlot &s, uint64_t ws_bytes, size_t max_batch) {
   // most N / 2048 + 1 flag words.
   s.flag_cap = ws_bytes / 8 / 3 / 2048 + max_batch + 64;
   SVC_CUDA(cudaMalloc(&s.flags, s.flag_cap * 8), "service scan flags");
-  SVC_CUDA(cudaMemset(s.flags, 0, s.flag_cap * 8), "service scan flags");
+  SVC_CUDA(fill_now(s.flags, 0, s.flag_cap * 8), "service scan flags");
   SVC_CUDA(cudaMalloc(&s.tickets, kSlotTickets * 8), "service scan counts");
-  SVC_CUDA(cudaMemset(s.tickets, 0, kSlotTickets * 8), "service scan counts");
+  SVC_CUDA(fill_now(s.tickets, 0, kSlotTickets * 8), "service scan counts");
   SVC_CUDA(cudaMalloc(&s.d_err, sizeof(int)), "service error word");
-  SVC_CUDA(cudaMemset(s.d_err, 0, sizeof(int)), "service error word");
+  SVC_CUDA(fill_now(s.d_err, 0, sizeof(int)), "service error word");
   SVC_CUDA(cudaMallocHost(&s.h_err, sizeof(int)), "service error staging");
   *s.h_err = 0;
   return HG_OK;
