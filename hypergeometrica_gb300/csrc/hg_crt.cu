@@ -37,6 +37,7 @@ constexpr int kCarryTile = kCarryThreads * kCarryPer;
 // 35.9 -> 31.8 us, of 2^16 points 47.2 -> 43.1.
 constexpr int kShortPer = 4;
 constexpr int kShortTile = kCarryThreads * kShortPer;
+static_assert(kShortTile == kCarryMinTile && kCarryTile > kShortTile, "flag words are reserved for this tile");
 constexpr uint64_t kShortCarry = static_cast<uint64_t>(kShortTile) * kCarryThreads;
 
 // The product of a long operand cut into chunks of `chunk` coefficients (limbs

@@ -285,6 +285,8 @@ cudaError_t launch_digit_carry(const uint64_t *x, uint64_t nx, uint64_t d, uint6
 cudaError_t launch_pass_twiddles(uint64_t *out, int logM, int logR, bool inverse, const NttTables *tb,
                                  const PrimeConst *pc, int nprimes, cudaStream_t st, const uint64_t *scale = nullptr);
 
+// Coefficients of the smallest tile of a carry (short launches).
+constexpr uint64_t kCarryMinTile = 1024;
 // Tiles per product that a carry over nprod products of n coefficients uses,
 // and whether it is one launch (short) or two.
 uint64_t carry_tiles(uint64_t n, uint64_t nprod = 1);

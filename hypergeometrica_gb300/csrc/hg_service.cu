@@ -116,9 +116,9 @@ int slot_alloc(SvcSlot &s, uint64_t ws_bytes, size_t max_batch) {
   SVC_CUDA(cudaMalloc(&s.ws, ws_bytes), "service workspace");
   SVC_CUDA(cudaMalloc(&s.d_desc, max_batch * sizeof(ProductDesc)), "service descriptors");
   SVC_CUDA(cudaMallocHost(&s.h_desc, max_batch * sizeof(ProductDesc)), "service descriptor staging");
-  // Every admitted product holds at least 3N workspace words and needs at
-  // most N / 2048 + 1 flag words.
-  s.flag_cap = ws_bytes / 8 / 3 / 2048 + max_batch + 64;
+  // A product is admitted with at least 3N workspace words (a square of 2^k =
+  // N points) and keeps at most N of them, in tiles of kCarryMinTile or more.
+  s.flag_cap = ws_bytes / 8 / 3 / kCarryMinTile + max_batch + 64;
   SVC_CUDA(cudaMalloc(&s.flags, s.flag_cap * 8), "service scan flags");
   SVC_CUDA(fill_now(s.flags, 0, s.flag_cap * 8), "service scan flags");
   SVC_CUDA(cudaMalloc(&s.tickets, kSlotTickets * 8), "service scan counts");
