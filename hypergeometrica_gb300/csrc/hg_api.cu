@@ -1611,6 +1611,7 @@ struct hg_batch {
   hg::DevBuf d_whole;   // device copy of whole.desc
   hg::DevBuf d_desc, ws, flags, tickets;
   hg::SideStreams side;
+  hg::ScanEpoch epoch;
   // The persistent schedule: its work list and its counters.
   std::vector<hg::PersistPhase> phases;
   uint64_t items = 0;
@@ -1623,7 +1624,7 @@ namespace hg {
 namespace {
 
 // Enqueue group gi with the given schedule.  The group's count must be zero
-// (its carry leaves it so); its flags are written before they are read.
+// (its carry leaves it so); flags of another run than bb.epoch's are an error.
 int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::vector<PassPlan> &plan,
               cudaStream_t st) {
   const int nops = g.square ? 1 : 2;
@@ -1657,7 +1658,7 @@ int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::ve
   ScanState ss;
   ss.done = reinterpret_cast<unsigned *>(bb.tickets + gi);
   ss.flags = bb.flags + g.flags_off;
-  ss.epoch = 1;
+  ss.epoch = bb.epoch;
   ss.err = bb.err;
   {
     ProfScope ps(HG_KC_CARRY, st, 32.0 * static_cast<double>(N) * static_cast<double>(g.nprod),
@@ -1667,10 +1668,19 @@ int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::ve
   return HG_OK;
 }
 
+// Flag words for a schedule, zeroed when they are allocated.
+int batch_flags(hg_batch *b, uint64_t words) {
+  if (b->flags.bytes >= words * 8) return HG_OK;
+  HG_CUDA(b->flags.ensure(words * 8), "batch scan flags");
+  HG_CUDA(fill_now(b->flags.p, 0, b->flags.bytes), "batch scan flags");
+  return HG_OK;
+}
+
+// The batch's buffers for one run (its epoch is the run's).
 BatchBufs batch_bufs(hg_batch *b) {
   return BatchBufs{static_cast<const ProductDesc *>(b->d_desc.p), b->ws.u64(),
                    static_cast<unsigned long long *>(b->flags.p), static_cast<unsigned long long *>(b->tickets.p),
-                   err_word(), b->side.n ? &b->side : nullptr};
+                   err_word(), b->side.n ? &b->side : nullptr, b->epoch.next()};
 }
 
 // ---- the persistent schedule (hg_persist.cu) -------------------------------
@@ -1800,7 +1810,7 @@ std::vector<PersistPhase> group_phases(const BatchGroup &g, const BatchBufs &bb,
   c.tiles = c.tpp * g.nprod;
   c.ss.done = nullptr;
   c.ss.flags = flags;
-  c.ss.epoch = 1;
+  c.ss.epoch = kPersistEpoch;
   c.ss.err = bb.err;
   v.push_back(c);
   PersistPhase f = c;
@@ -1822,7 +1832,7 @@ int persist_build(hg_batch *b) {
   const PersistLayout l = persist_layout(groups);
   if (l.ws_words * 8 > kPersistWorkspaceCap) return HG_OK;
   if (b->ws.bytes < l.ws_words * 8) HG_CUDA(b->ws.ensure(l.ws_words * 8), "batch workspace");
-  if (b->flags.bytes < l.flag_words * 8) HG_CUDA(b->flags.ensure(l.flag_words * 8), "batch scan flags");
+  if (const int rc = batch_flags(b, l.flag_words)) return rc;
   b->persist_flag_words = l.flag_words;
   BatchBufs bb = batch_bufs(b);
   bb.desc = static_cast<const ProductDesc *>(b->d_whole.p);
@@ -1902,7 +1912,6 @@ int batch_autotune(hg_batch *b) {
   HG_CUDA(cudaEventCreate(&e0), "event creation");
   HG_CUDA(cudaEventCreate(&e1), "event creation");
   int rc = HG_OK;
-  const BatchBufs bb = batch_bufs(b);
   for (size_t gi = 0; gi < b->bp.groups.size() && rc == HG_OK; ++gi) {
     BatchGroup &g = b->bp.groups[gi];
     const auto key = tune_key(g);
@@ -1920,7 +1929,7 @@ int batch_autotune(hg_batch *b) {
       float ms = 0;
       for (int rep = 0; rep < 2 && rc == HG_OK; ++rep) {
         cudaEventRecord(e0, st);
-        if ((rc = run_group(g, gi, bb, plan, st))) break;
+        if ((rc = run_group(g, gi, batch_bufs(b), plan, st))) break;
         cudaEventRecord(e1, st);
         if (cudaEventSynchronize(e1) != cudaSuccess) rc = fail(HG_ERR_CUDA, "autotune timing failed");
         else cudaEventElapsedTime(&ms, e0, e1);
@@ -2015,7 +2024,7 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
     HG_CUDA(upload_now(b->d_desc.p, bp.desc.data(), bp.desc.size() * sizeof(ProductDesc)), "batch descriptors upload");
   }
   if (bp.ws_words) HG_CUDA(b->ws.ensure(bp.ws_words * 8), "batch workspace");
-  if (bp.flag_words) HG_CUDA(b->flags.ensure(bp.flag_words * 8), "batch scan flags");
+  if ((rc = batch_flags(b.get(), bp.flag_words))) return rc;
   HG_CUDA(b->tickets.ensure(std::max<size_t>(1, bp.groups.size()) * 8), "batch scan counts");
   HG_CUDA(fill_now(b->tickets.p, 0, b->tickets.bytes), "batch scan counts");
   if (bp.parallel && bp.groups.size() > 1) HG_CUDA(b->side.create(), "batch streams");
@@ -2209,6 +2218,10 @@ void SideStreams::destroy() {
 // 2^9 314 -> 256; two streams 287, 973, 3278 and 261, six 255, 981, 3331, 259.
 int enqueue_batch(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st) {
   int rc = HG_OK;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cudaGetLastError();
+  if (cs != cudaStreamCaptureStatusNone && bp.flag_words)
+    HG_CUDA(cudaMemsetAsync(bb.flags, 0, bp.flag_words * 8, st), "scan flags reset");
   if (bp.nzero) HG_CUDA(launch_zero_tails(bb.desc + bp.zero_first, bp.nzero, 0, st), "zero products");
   const size_t ng = bp.groups.size();
   if (!bb.side || !bp.parallel || ng < 2) {

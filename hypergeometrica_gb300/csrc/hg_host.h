@@ -7,6 +7,7 @@
 #include <mutex>
 #include <vector>
 
+#include "hg_epoch.h"
 #include "hg_internal.h"
 
 namespace hg {
@@ -60,6 +61,7 @@ struct BatchBufs {
   unsigned long long *tickets;  // one per group (the carry's finished-tile count), zero between runs
   int *err;                   // device error word
   const SideStreams *side;    // or null: groups one after another
+  uint32_t epoch;             // this run's (ScanEpoch)
 };
 
 // Workspace bytes one product occupies while its group runs.
@@ -77,8 +79,8 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
 int large_sum_device(const SumOperand &a, int64_t sa, const SumOperand &b, int64_t sb, uint64_t *out, uint64_t nout,
                      int64_t *result, cudaStream_t st);
 
-// Enqueue a planned batch on st: clear its scan state, zero the empty
-// products, run every group.  Takes no lock and allocates nothing.
+// Enqueue a planned batch on st: zero the empty products, run every group.  A
+// captured run, whose epoch is the same on every replay, clears its flags.  Takes no lock and allocates nothing.
 int enqueue_batch(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st);
 
 // Fill or upload device memory, done on return.  cudaMemset and cudaMemcpy from

@@ -58,6 +58,7 @@ struct SvcSlot {
   int *d_err = nullptr;
   int *h_err = nullptr;  // pinned copy of the error word after the batch
   uint64_t flag_cap = 0;
+  ScanEpoch epoch;
   bool busy = false;
   bool launching = false;  // a thread is enqueuing its batch, without the lock
   std::vector<SvcRequest> batch;
@@ -150,7 +151,7 @@ int slot_launch(hg_svc *svc, SvcSlot &s) {
   cudaError_t e = cudaMemcpyAsync(s.d_desc, s.h_desc, s.plan.desc.size() * sizeof(ProductDesc),
                                   cudaMemcpyHostToDevice, s.st);
   if (e != cudaSuccess) return lib_cuda_fail(e, "service descriptor upload");
-  const BatchBufs bb{s.d_desc, s.ws, s.flags, s.tickets, s.d_err, &s.side};
+  const BatchBufs bb{s.d_desc, s.ws, s.flags, s.tickets, s.d_err, &s.side, s.epoch.next()};
   if ((rc = enqueue_batch(s.plan, bb, s.st))) return rc;
   for (const SvcRequest &r : s.batch) {
     if (!r.size) continue;
