@@ -2018,12 +2018,20 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
   };
   std::unique_ptr<hg_batch, Destroy> b(new hg_batch());
   if ((rc = plan_batch(items.data(), items.size(), kBatchWorkspaceCap, b->bp))) return rc;
-  const BatchPlan &bp = b->bp;
+  BatchPlan &bp = b->bp;
   if (!bp.desc.empty()) {
     HG_CUDA(b->d_desc.ensure(bp.desc.size() * sizeof(ProductDesc)), "batch descriptors");
     HG_CUDA(upload_now(b->d_desc.p, bp.desc.data(), bp.desc.size() * sizeof(ProductDesc)), "batch descriptors upload");
   }
-  if (bp.ws_words) HG_CUDA(b->ws.ensure(bp.ws_words * 8), "batch workspace");
+  if (bp.ws_words) {
+    cudaError_t e = b->ws.ensure(bp.ws_words * 8);
+    if (e == cudaErrorMemoryAllocation && bp.ws_words > bp.in_turn_words) {  // no room for all groups at once
+      cudaGetLastError();
+      bp.run_in_turn();
+      e = b->ws.ensure(bp.ws_words * 8);
+    }
+    HG_CUDA(e, "batch workspace");
+  }
   if ((rc = batch_flags(b.get(), bp.flag_words))) return rc;
   HG_CUDA(b->tickets.ensure(std::max<size_t>(1, bp.groups.size()) * 8), "batch scan counts");
   HG_CUDA(fill_now(b->tickets.p, 0, b->tickets.bytes), "batch scan counts");
@@ -2172,16 +2180,14 @@ int plan_batch(const ProductDesc *items, size_t n, uint64_t ws_cap_bytes, BatchP
       bp.flag_words += carry_tiles(N, g.nprod) * g.nprod;
       g.ws_off = ws_all;
       ws_all += per / 8 * g.nprod;
-      bp.ws_words = std::max<uint64_t>(bp.ws_words, per / 8 * g.nprod);
+      bp.in_turn_words = std::max<uint64_t>(bp.in_turn_words, per / 8 * g.nprod);
       bp.groups.push_back(std::move(g));
     }
     s = e;
   }
-  bp.parallel = ws_all * 8 <= ws_cap_bytes;
-  if (bp.parallel)
-    bp.ws_words = ws_all;
-  else
-    for (BatchGroup &g : bp.groups) g.ws_off = 0;
+  bp.parallel = true;
+  bp.ws_words = ws_all;
+  if (ws_all * 8 > ws_cap_bytes) bp.run_in_turn();
   bp.zero_first = bp.desc.size();
   bp.nzero = zeros.size();
   for (size_t z : zeros) bp.desc.push_back(items[z]);

@@ -51,6 +51,12 @@ struct BatchPlan {
   std::vector<ProductDesc> desc;
   uint64_t zero_first = 0, nzero = 0;
   uint64_t ws_words = 0, flag_words = 0;
+  uint64_t in_turn_words = 0;  // ws_words of groups that run one after another
+  void run_in_turn() {
+    parallel = false;
+    ws_words = in_turn_words;
+    for (BatchGroup &g : groups) g.ws_off = 0;
+  }
 };
 
 // Device buffers a planned batch runs in.
