@@ -1303,13 +1303,11 @@ const void *pinned_view(const void *h) {
   return nullptr;
 }
 
-// Page-locked, device-mapped words that kernels write results into and the
-// host reads after a stream synchronisation: taken for one call at a time,
-// kept until hg_shutdown.
-constexpr size_t kWordsBytes = 64;
+// Blocks of HostWords that no call holds (whole pages, kKeptWords at most).
+constexpr size_t kMinWords = 512, kKeptWords = size_t(1) << 23;
 std::mutex g_words_mu;
-std::vector<void *> g_words_pages;
 std::vector<HostWords> g_words_free;
+size_t g_words_kept = 0;
 
 // Host-memory wrapper: stage operands, run, copy back, check.
 enum class Kind { Ntt, Square, Schoolboy, Digit };
@@ -2262,30 +2260,52 @@ int enqueue_batch(const BatchPlan &bp, const BatchBufs &bb, cudaStream_t st) {
   return rc;
 }
 
-int host_words_take(HostWords *w) {
-  std::lock_guard<std::mutex> lk(g_words_mu);
-  if (g_words_free.empty()) {
-    constexpr size_t kPage = 4096;
-    void *h = nullptr, *d = nullptr;
-    HG_CUDA(cudaHostAlloc(&h, kPage, cudaHostAllocMapped), "result words");
-    const cudaError_t e = cudaHostGetDevicePointer(&d, h, 0);
-    if (e != cudaSuccess) {
-      cudaFreeHost(h);
-      return cuda_fail(e, "result words");
+int host_words_take(size_t words, HostWords *w) {
+  {
+    std::lock_guard<std::mutex> lk(g_words_mu);
+    size_t best = g_words_free.size();
+    for (size_t i = 0; i < g_words_free.size(); ++i)
+      if (g_words_free[i].words >= words && (best == g_words_free.size() || g_words_free[i].words < g_words_free[best].words))
+        best = i;
+    if (best < g_words_free.size()) {
+      *w = g_words_free[best];
+      g_words_free[best] = g_words_free.back();
+      g_words_free.pop_back();
+      g_words_kept -= w->words;
+      return HG_OK;
     }
-    g_words_pages.push_back(h);
-    for (size_t o = 0; o < kPage; o += kWordsBytes)
-      g_words_free.push_back(HostWords{reinterpret_cast<int64_t *>(static_cast<char *>(h) + o),
-                                       reinterpret_cast<int64_t *>(static_cast<char *>(d) + o)});
   }
-  *w = g_words_free.back();
-  g_words_free.pop_back();
+  size_t n = kMinWords;
+  while (n < words) n *= 2;
+  void *h = nullptr, *d = nullptr;
+  HG_CUDA(cudaHostAlloc(&h, n * sizeof(int64_t), cudaHostAllocMapped), "result words");
+  const cudaError_t e = cudaHostGetDevicePointer(&d, h, 0);
+  if (e != cudaSuccess) {
+    cudaFreeHost(h);
+    return cuda_fail(e, "result words");
+  }
+  *w = HostWords{static_cast<int64_t *>(h), static_cast<int64_t *>(d), n};
   return HG_OK;
 }
 
 void host_words_give(const HostWords &w) {
+  {
+    std::lock_guard<std::mutex> lk(g_words_mu);
+    if (g_words_kept + w.words <= kKeptWords) {
+      g_words_free.push_back(w);
+      g_words_kept += w.words;
+      return;
+    }
+  }
+  cudaFreeHost(w.host);
+}
+
+// The blocks that calls hold are theirs still: they come back to the list.
+void release_words() {
   std::lock_guard<std::mutex> lk(g_words_mu);
-  if (!g_words_pages.empty()) g_words_free.push_back(w);
+  for (const HostWords &w : g_words_free) cudaFreeHost(w.host);
+  g_words_free.clear();
+  g_words_kept = 0;
 }
 
 int *lib_err_word() { return err_word(); }
@@ -2293,8 +2313,10 @@ int *lib_err_word() { return err_word(); }
 // Reset the library's error word after `err` was read from it, and report it.
 int lib_device_error(int err, cudaStream_t st) {
   if (!err) return HG_OK;
-  HG_CUDA(cudaMemsetAsync(err_word(), 0, sizeof(int), st), "error word reset");
-  HG_CUDA(cudaStreamSynchronize(st), "stream synchronise");
+  if (g_ctx.ready) {
+    HG_CUDA(cudaMemsetAsync(err_word(), 0, sizeof(int), st), "error word reset");
+    HG_CUDA(cudaStreamSynchronize(st), "stream synchronise");
+  }
   if (err == kDevCarryOverflow) return fail(HG_ERR_INCONSISTENT, "a carry left the top of the result storage");
   if (err == kDevCopyTimeout) return fail(HG_ERR_CUDA, "a tile copy did not complete within its wait limit");
   return fail(HG_ERR_CUDA, "device error %d", err);
@@ -2452,12 +2474,7 @@ int hg_shutdown(void) {
   c.tables.release();
   release_pass_twiddles();
   lib_release_descs();
-  {
-    std::lock_guard<std::mutex> lk(g_words_mu);
-    for (void *p : g_words_pages) cudaFreeHost(p);
-    g_words_pages.clear();
-    g_words_free.clear();
-  }
+  release_words();
   c.ready = false;
   // The scratch array's device address belongs to the module as loaded in
   // the current context: after a context reset the module loads again, so

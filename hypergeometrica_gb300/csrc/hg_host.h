@@ -101,11 +101,15 @@ inline cudaError_t upload_now(void *dst, const void *src, size_t bytes) {
   return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
 }
 
-// Words that kernels write and the host reads after a synchronisation.
+// Page-locked words that kernels write and the host reads after a
+// synchronisation: one call's from take to give, then kept for the next (64 MB
+// of them) until hg_shutdown.  Taking and giving hold no lock that
+// any other is taken under.
 struct HostWords {
-  int64_t *host, *dev;
+  int64_t *host = nullptr, *dev = nullptr;
+  size_t words = 0;
 };
-int host_words_take(HostWords *w);
+int host_words_take(size_t words, HostWords *w);
 void host_words_give(const HostWords &w);
 
 // The library's device error word; lib_device_error resets it when `err`,

@@ -422,7 +422,7 @@ int hg_svc_mul(hg_svc *svc, const hg_product *prod, void *stream, size_t *size) 
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return lib_cuda_fail(e, "stream synchronise");
   HostWords w;
-  int rc = host_words_take(&w);
+  int rc = host_words_take(1, &w);
   if (rc) return rc;
   w.host[0] = 0;
   uint64_t ticket = 0;

@@ -279,54 +279,6 @@ int run_batch(const Desc *host, size_t n, cudaStream_t st, const char *what, Lau
   return HG_OK;
 }
 
-// Host-mapped words for one call's results: a block of the library's, or for
-// many results one larger buffer that calls take turns on.
-std::mutex g_many_mu;
-int64_t *g_many = nullptr, *g_many_dev = nullptr;
-size_t g_many_words = 0;
-
-class ResultWords {
- public:
-  int64_t *host = nullptr, *dev = nullptr;
-  int take(size_t words) {
-    if (words <= 8) {
-      const int rc = host_words_take(&block_);
-      if (rc) return rc;
-      taken_ = true;
-      host = block_.host;
-      dev = block_.dev;
-      return HG_OK;
-    }
-    lock_ = std::unique_lock<std::mutex>(g_many_mu);
-    if (words > g_many_words) {
-      if (g_many) cudaFreeHost(g_many);
-      g_many = nullptr;
-      g_many_words = 0;
-      void *h = nullptr, *d = nullptr;
-      cudaError_t e = cudaHostAlloc(&h, 2 * words * sizeof(int64_t), cudaHostAllocMapped);
-      if (e != cudaSuccess) return lib_cuda_fail(e, "result words");
-      if ((e = cudaHostGetDevicePointer(&d, h, 0)) != cudaSuccess) {
-        cudaFreeHost(h);
-        return lib_cuda_fail(e, "result words");
-      }
-      g_many = static_cast<int64_t *>(h);
-      g_many_dev = static_cast<int64_t *>(d);
-      g_many_words = 2 * words;
-    }
-    host = g_many;
-    dev = g_many_dev;
-    return HG_OK;
-  }
-  ~ResultWords() {
-    if (taken_) host_words_give(block_);
-  }
-
- private:
-  HostWords block_{};
-  bool taken_ = false;
-  std::unique_lock<std::mutex> lock_;
-};
-
 // Check the sums and enqueue them; sign and size of sum k to result[2 k], result[2 k + 1].
 int sums_enqueue(const hg_sum *sums, const size_t *a_shift, const size_t *b_shift, size_t n, int64_t *result,
                  cudaStream_t st) {
@@ -370,10 +322,6 @@ void lib_release_descs() {
   std::lock_guard<std::mutex> lk(g_pool_mu);
   if (g_pool) cudaMemPoolDestroy(g_pool);
   g_pool = nullptr;
-  std::lock_guard<std::mutex> lm(g_many_mu);
-  if (g_many) cudaFreeHost(g_many);
-  g_many = g_many_dev = nullptr;
-  g_many_words = 0;
 }
 
 #if HG_CHECKED
@@ -394,25 +342,39 @@ int hg_add_batch_device(const hg_sum *sums, size_t n, int64_t *result, void *str
 int hg_sums_and_sizes(const hg_sum *sums, const size_t *a_shift, const size_t *b_shift, size_t n, int64_t *results,
                       const hg_vec *vecs, size_t m, uint64_t *sizes, void *stream) {
   if ((n && !results) || (m && !sizes)) return lib_fail(HG_ERR_ARG, "null pointer");
-  if (!lib_ready()) return lib_fail(HG_ERR_NOT_INIT, "hg_sums_and_sizes: call hg_init first");
+  const auto not_init = [] { return lib_fail(HG_ERR_NOT_INIT, "hg_sums_and_sizes: call hg_init first"); };
+  if (!lib_ready()) return not_init();
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t words = 2 * n + m + 1;  // results, sizes, the error word
-  ResultWords w;
-  int rc = w.take(words);
+  struct Held : HostWords {
+    ~Held() {
+      if (host) host_words_give(*this);
+    }
+  } w;
+  int rc = host_words_take(words, &w);
   if (rc) return rc;
-  if (n) rc = sums_enqueue(sums, a_shift, b_shift, n, w.dev, st);
-  if (rc == HG_OK && m) rc = hg_trim_batch_device(vecs, m, reinterpret_cast<uint64_t *>(w.dev) + 2 * n, stream);
   w.host[words - 1] = 0;
   cudaError_t e = cudaSuccess;
-  if (rc == HG_OK)
-    e = cudaMemcpyAsync(w.host + words - 1, lib_err_word(), sizeof(int), cudaMemcpyDeviceToHost, st);
+  {
+    // Enqueued whole before or after an hg_shutdown in another thread, which
+    // waits for what is enqueued; the wait below holds no lock.
+    std::lock_guard<std::recursive_mutex> lock(lib_mutex());
+    if (!lib_ready()) return not_init();
+    if (n) rc = sums_enqueue(sums, a_shift, b_shift, n, w.dev, st);
+    if (rc == HG_OK && m) rc = hg_trim_batch_device(vecs, m, reinterpret_cast<uint64_t *>(w.dev) + 2 * n, stream);
+    if (rc == HG_OK)
+      e = cudaMemcpyAsync(w.host + words - 1, lib_err_word(), sizeof(int), cudaMemcpyDeviceToHost, st);
+  }
   // Nothing enqueued may write the words after they are given back.
   const cudaError_t f = cudaStreamSynchronize(st);
   if (rc) return rc;
   if (e != cudaSuccess || f != cudaSuccess) return lib_cuda_fail(e != cudaSuccess ? e : f, "sums and sizes");
   for (size_t k = 0; k < 2 * n; ++k) results[k] = w.host[k];
   for (size_t k = 0; k < m; ++k) sizes[k] = static_cast<uint64_t>(w.host[2 * n + k]);
-  return lib_device_error(static_cast<int>(w.host[words - 1]), st);
+  const int err = static_cast<int>(w.host[words - 1]);
+  if (!err) return HG_OK;
+  std::lock_guard<std::recursive_mutex> lock(lib_mutex());
+  return lib_device_error(err, st);
 }
 
 int hg_mul_small_batch_device(const hg_product *prods, size_t n, void *stream) {
