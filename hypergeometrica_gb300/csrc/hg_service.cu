@@ -83,7 +83,7 @@ struct hg_svc {
   std::vector<float> lat_us;  // since the last stats reset
   bool have_first = false;
   hg::Clock::time_point t_first, t_last;
-  int helpers = 0;  // clients inside wait_helping
+  int helpers = 0;  // clients inside wait_helping that are looking at the slots
   bool closing = false;
   std::thread worker;
 };
@@ -191,11 +191,18 @@ void retire(hg_svc *svc, SvcSlot &s, cudaError_t q) {
   svc->cv_done.notify_all();
 }
 
+// A client that stops looking at the slots (it leaves, or enqueues a batch):
+// with no other looking, the worker has to, at its own short interval.
+void looks_away(hg_svc *svc) {
+  if (--svc->helpers == 0) svc->cv_work.notify_one();
+}
+
 // One step of the service, with the lock held: retire the batches that have
 // ended and admit pending products into a free slot.  The worker and every
 // waiting client run it, so that a client's product starts and ends without
 // waiting for another thread to be scheduled.  True when it did something.
-bool pump(hg_svc *svc, std::unique_lock<std::mutex> &lk) {
+// helper: the caller is a waiting client.
+bool pump(hg_svc *svc, std::unique_lock<std::mutex> &lk, bool helper) {
   bool progress = false;
   for (SvcSlot &s : svc->slots) {
     if (!s.busy) continue;
@@ -222,10 +229,12 @@ bool pump(hg_svc *svc, std::unique_lock<std::mutex> &lk) {
   svc->peak_batch_bytes = std::max(svc->peak_batch_bytes, used);
   svc->peak_batch_products = std::max<uint64_t>(svc->peak_batch_products, slot->batch.size());
   slot->launching = true;
+  if (helper) looks_away(svc);
   lk.unlock();
   const int rc = slot_launch(svc, *slot);
   if (rc) cudaStreamSynchronize(slot->st);
   lk.lock();
+  if (helper) ++svc->helpers;
   slot->launching = false;
   if (rc) {
     settle(svc, slot->batch, rc, Clock::now());
@@ -248,7 +257,7 @@ void worker_loop(hg_svc *svc) {
   cudaSetDevice(svc->device);
   std::unique_lock<std::mutex> lk(svc->mu);
   for (;;) {
-    if (pump(svc, lk)) continue;
+    if (pump(svc, lk, false)) continue;
     const bool busy = any_busy(svc);
     if (svc->closing && svc->pending.empty() && !busy) break;
     if (busy)
@@ -281,7 +290,7 @@ bool wait_helping(hg_svc *svc, std::unique_lock<std::mutex> &lk, double timeout_
   ++svc->helpers;
   bool done = false;
   for (;;) {
-    const bool progress = pump(svc, lk);
+    const bool progress = pump(svc, lk, true);
     if ((done = pred())) break;
     const auto waited = Clock::now() - t0;
     if (timeout_s >= 0 && waited >= std::chrono::duration<double>(timeout_s)) break;
@@ -294,7 +303,7 @@ bool wait_helping(hg_svc *svc, std::unique_lock<std::mutex> &lk, double timeout_
       svc->cv_done.wait_for(lk, std::chrono::microseconds(20));
     }
   }
-  --svc->helpers;
+  looks_away(svc);
   return done;
 }
 
