@@ -392,7 +392,7 @@ cudaError_t launch_carry(const Producer &prod, uint64_t *out, uint64_t nproc, ui
 // above gives such a product a handful of threads with four positions each
 // and reads the operands from global memory: 64 x 48 limbs took 25 us (eight
 // positions a thread; four: the whole host call 57.5 us, with this kernel 46.9).
-constexpr uint32_t kSchoolMax = 1024;
+static_assert(kSchoolMax == 1024, "a thread per position");
 
 __global__ void __launch_bounds__(kSchoolMax)
     school_kernel(const uint64_t *x, uint32_t nx, const uint64_t *y, uint32_t ny, uint64_t *out, uint32_t n, int *err) {

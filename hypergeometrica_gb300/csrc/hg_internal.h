@@ -276,6 +276,8 @@ cudaError_t launch_large_sum(const SumOperand &a, int64_t sa, const SumOperand &
 // Zero out[N, nout) of every product (out[0, nout) when N == 0), N the
 // residues per prime.
 cudaError_t launch_zero_tails(const ProductDesc *batch, uint64_t nprod, uint64_t N, cudaStream_t st);
+// Schoolboy products of up to kSchoolMax limbs read every operand limb once.
+constexpr uint32_t kSchoolMax = 1024;
 cudaError_t launch_schoolboy_carry(const uint64_t *x, uint64_t nx, const uint64_t *y, uint64_t ny, uint64_t *out,
                                    uint64_t nout, const ScanState &ss, cudaStream_t st, uint64_t *tiles_used);
 cudaError_t launch_digit_carry(const uint64_t *x, uint64_t nx, uint64_t d, uint64_t *out, uint64_t nout,
