@@ -1317,10 +1317,17 @@ enum class Kind { Ntt, Square, Schoolboy, Digit };
 // that reads them once does so in place), the result written in place by the last
 // kernel, the error word beside it, one synchronisation.  The general path's
 // copies from and to pageable memory each wait in the driver and its upload
-// slices launch the first pass eight times.  mpz_mul of 64 x 48 limbs 37.9 us
-// that way, 28.3 this way; 3000 x 2500 142.9 and 77.3; 16000 x 16000 260.8 and
-// 146.6; 65536 x 65536 249 and 227, about where they meet.
-constexpr size_t kStagedLimbs = size_t(1) << 17;
+// slices launch the first pass eight times, but it does not copy on the host.
+// From and to pageable memory, us this way and the general one, products of
+//   limbs          256          2^12         2^14         2^15         49152        2^17
+//   half x half    33.5 (45.5)  43.9 (53.9)  55.6 (61.2)  67.0 (76.4)  80.2 (77.4)  172.5 (97.1)
+//   by a digit     25.5 (36.1)  26.5 (37.8)  33.8 (46.1)  44.3 (47.6)  57.0 (49.6)  147.6 (56.4)
+// Page-locked operands and results need no copy by the host and are read and
+// written in place by the general path: half x half 40.0 (40.8), 44.0 (42.9),
+// 55.2 (48.3), 67.4 (48.9), 80.8 (48.8), 173.1 (65.2); they take it above
+// kStagedPinned limbs (quadratic products, which would be read in place, do not).
+constexpr size_t kStagedLimbs = size_t(1) << 15;
+constexpr size_t kStagedPinned = size_t(1) << 12;
 
 int staged_product(Kind kind, const uint64_t *x, size_t nx, const uint64_t *y, size_t ny, uint64_t d, uint64_t *out,
                    size_t nout) {
@@ -1388,11 +1395,13 @@ int host_product(Kind kind, const uint64_t *x, size_t nx, const uint64_t *y, siz
   }
   const size_t nd = size;  // limbs computed on the device; the rest are zero
   cudaStream_t st = c.lane->stream;
-  if (size <= kStagedLimbs) return staged_product(kind, x, nx, y, ny, d, out, nout);
+  const bool two = (kind == Kind::Ntt || kind == Kind::Schoolboy);
+  const auto pinned = [&] { return pinned_view(out) && pinned_view(x) && (!two || pinned_view(y)); };
+  if (size <= kStagedPinned || (size <= kStagedLimbs && (kind == Kind::Schoolboy || !pinned())))
+    return staged_product(kind, x, nx, y, ny, d, out, nout);
   // Pinned (page-locked) host buffers are addressable from the device over
   // the host link, so the kernels read the operands and write the product
   // in place; pageable buffers go through device staging buffers.
-  const bool two = (kind == Kind::Ntt || kind == Kind::Schoolboy);
   const uint64_t *dx = static_cast<const uint64_t *>(pinned_view(x));
   const uint64_t *dy = two ? static_cast<const uint64_t *>(pinned_view(y)) : nullptr;
   uint64_t *dout = static_cast<uint64_t *>(const_cast<void *>(pinned_view(out)));

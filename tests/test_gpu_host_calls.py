@@ -49,3 +49,33 @@ def test_quadratic_product_reads_device_memory(hg, oracle):
     assert np.array_equal(out, dout.cpu().numpy().view(np.uint64))
     assert np.array_equal(out, oracle.mpz_mul_ntt(x, y)[:2 * n])
     assert th < 1.25 * td + 100, (th, td)
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("n", [4095, 4096, 32767, 32768, 131000])
+def test_by_digit_at_the_ends_of_the_staged_sizes(hg, pinned, n):
+    """A product by a digit moves 16 n bytes over a link of about 200 GB/s beside
+    what the shortest one costs (25 us): twice that, and the driver's copies of
+    pageable memory, hold it below 2 x + 40 us.  Copied on the host both ways,
+    131000 limbs take 150 us."""
+    import torch
+
+    from hypergeometrica_gb300._lib import check, load
+
+    d = 12345678901234567
+
+    def buffers(k):
+        x, out = W.limbs(3, k), np.full(k + 1, 7, dtype=np.uint64)
+        if pinned:
+            x, out = (torch.from_numpy(a.view(np.int64)).pin_memory().numpy().view(np.uint64) for a in (x, out))
+        return x, out
+
+    def call(x, out):
+        return lambda: check(load().hg_mul_digit(x.ctypes.data, len(x), ctypes.c_uint64(d), out.ctypes.data, len(out)))
+
+    x0, out0 = buffers(256)
+    x, out = buffers(n)
+    t0, t = _median_us(call(x0, out0), 31), _median_us(call(x, out), 31)
+    want = int.from_bytes(x.tobytes(), "little") * d
+    assert int.from_bytes(out.tobytes(), "little") == want
+    assert t < 2 * t0 + 40, (t, t0)
