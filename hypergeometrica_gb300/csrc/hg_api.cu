@@ -1681,14 +1681,6 @@ int run_group(const BatchGroup &g, size_t gi, const BatchBufs &bb, const std::ve
   return HG_OK;
 }
 
-// Flag words for a schedule, zeroed when they are allocated.
-int batch_flags(hg_batch *b, uint64_t words) {
-  if (b->flags.bytes >= words * 8) return HG_OK;
-  HG_CUDA(b->flags.ensure(words * 8), "batch scan flags");
-  HG_CUDA(fill_now(b->flags.p, 0, b->flags.bytes), "batch scan flags");
-  return HG_OK;
-}
-
 // The batch's buffers for one run (its epoch is the run's).
 BatchBufs batch_bufs(hg_batch *b) {
   return BatchBufs{static_cast<const ProductDesc *>(b->d_desc.p), b->ws.u64(),
@@ -1845,7 +1837,11 @@ int persist_build(hg_batch *b) {
   const PersistLayout l = persist_layout(groups);
   if (l.ws_words * 8 > kPersistWorkspaceCap) return HG_OK;
   if (b->ws.bytes < l.ws_words * 8) HG_CUDA(b->ws.ensure(l.ws_words * 8), "batch workspace");
-  if (const int rc = batch_flags(b, l.flag_words)) return rc;
+  if (b->flags.bytes < l.flag_words * 8) {
+    HG_CUDA(b->flags.ensure(l.flag_words * 8), "batch scan flags");
+    // For the per-pass schedule beside this one, which clears its own.
+    if (!b->bp.groups.empty()) HG_CUDA(fill_now(b->flags.p, 0, b->flags.bytes), "batch scan flags");
+  }
   b->persist_flag_words = l.flag_words;
   BatchBufs bb = batch_bufs(b);
   bb.desc = static_cast<const ProductDesc *>(b->d_whole.p);
@@ -2020,22 +2016,11 @@ int product_descs(const hg_product *prods, size_t n, std::vector<ProductDesc> &o
   return HG_OK;
 }
 
-int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
-  if (!out) return fail(HG_ERR_ARG, "null pointer");
-  *out = nullptr;
-  std::vector<ProductDesc> items;
-  int rc = product_descs(prods, n, items);
-  if (rc) return rc;
-  struct Destroy {
-    void operator()(hg_batch *p) const { hg_batch_destroy(p); }
-  };
-  std::unique_ptr<hg_batch, Destroy> b(new hg_batch());
-  if ((rc = plan_batch(items.data(), items.size(), kBatchWorkspaceCap, b->bp))) return rc;
+// Plan the schedule of one launch per pass, with what its runs need.
+int per_pass_build(hg_batch *b, const std::vector<ProductDesc> &items) {
   BatchPlan &bp = b->bp;
-  if (!bp.desc.empty()) {
-    HG_CUDA(b->d_desc.ensure(bp.desc.size() * sizeof(ProductDesc)), "batch descriptors");
-    HG_CUDA(upload_now(b->d_desc.p, bp.desc.data(), bp.desc.size() * sizeof(ProductDesc)), "batch descriptors upload");
-  }
+  int rc = plan_batch(items.data(), items.size(), kBatchWorkspaceCap, bp);
+  if (rc) return rc;
   if (bp.ws_words) {
     cudaError_t e = b->ws.ensure(bp.ws_words * 8);
     if (e == cudaErrorMemoryAllocation && bp.ws_words > bp.in_turn_words) {  // no room for all groups at once
@@ -2045,21 +2030,43 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
     }
     HG_CUDA(e, "batch workspace");
   }
-  if ((rc = batch_flags(b.get(), bp.flag_words))) return rc;
-  HG_CUDA(b->tickets.ensure(std::max<size_t>(1, bp.groups.size()) * 8), "batch scan counts");
-  HG_CUDA(fill_now(b->tickets.p, 0, b->tickets.bytes), "batch scan counts");
+  if (!bp.groups.empty()) {
+    // Counts and flags start at zero: done when the upload behind them is.
+    HG_CUDA(b->flags.ensure(bp.flag_words * 8), "batch scan flags");
+    HG_CUDA(cudaMemsetAsync(b->flags.p, 0, b->flags.bytes, nullptr), "batch scan flags");
+    HG_CUDA(b->tickets.ensure(bp.groups.size() * 8), "batch scan counts");
+    HG_CUDA(cudaMemsetAsync(b->tickets.p, 0, b->tickets.bytes, nullptr), "batch scan counts");
+  }
+  if (!bp.desc.empty()) {
+    HG_CUDA(b->d_desc.ensure(bp.desc.size() * sizeof(ProductDesc)), "batch descriptors");
+    HG_CUDA(upload_now(b->d_desc.p, bp.desc.data(), bp.desc.size() * sizeof(ProductDesc)), "batch descriptors upload");
+  }
   if (bp.parallel && bp.groups.size() > 1) HG_CUDA(b->side.create(), "batch streams");
+  std::lock_guard<std::mutex> lk(g_tune_mu);
+  for (BatchGroup &g : bp.groups) {
+    const auto it = g_tuned.find(tune_key(g));
+    if (it != g_tuned.end()) g.plan = it->second;
+  }
+  return HG_OK;
+}
+
+// Without HG_BATCH_AUTOTUNE the persistent schedule runs where it can, and the
+// other one is not planned beside it (its descriptors, counts and streams took
+// 25 to 45 us of a small batch's 130 to 180).
+int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
+  if (!out) return fail(HG_ERR_ARG, "null pointer");
+  *out = nullptr;
+  std::vector<ProductDesc> items;
+  int rc = product_descs(prods, n, items);
+  if (rc) return rc;
   if ((flags & HG_BATCH_PER_PASS) && (flags & HG_BATCH_PERSISTENT))
     return fail(HG_ERR_ARG, "a batch runs either per pass or persistently, not both");
-  if (flags & HG_BATCH_AUTOTUNE) {
-    if ((rc = batch_autotune(b.get()))) return rc;
-  } else {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    for (BatchGroup &g : b->bp.groups) {
-      auto it = g_tuned.find(tune_key(g));
-      if (it != g_tuned.end()) g.plan = it->second;
-    }
-  }
+  struct Destroy {
+    void operator()(hg_batch *p) const { hg_batch_destroy(p); }
+  };
+  std::unique_ptr<hg_batch, Destroy> b(new hg_batch());
+  const bool tune = (flags & HG_BATCH_AUTOTUNE) != 0;
+  if (tune && ((rc = per_pass_build(b.get(), items)) || (rc = batch_autotune(b.get())))) return rc;
   if (!(flags & HG_BATCH_PER_PASS)) {
     if ((rc = plan_batch(items.data(), items.size(), kBatchWorkspaceCap, b->whole, true))) return rc;
     if (!b->whole.desc.empty()) {
@@ -2069,13 +2076,12 @@ int batch_create(const hg_product *prods, size_t n, int flags, hg_batch **out) {
     }
     if ((rc = persist_build(b.get()))) return rc;
     b->persistent = b->items > 0;
-    if ((flags & HG_BATCH_PERSISTENT) && !b->persistent && !b->bp.groups.empty())
+    if ((flags & HG_BATCH_PERSISTENT) && !b->persistent && !b->whole.groups.empty())
       return fail(HG_ERR_ARG, "this batch cannot run as one persistent launch (more than %d phases, or group "
                               "workspaces above %llu bytes)", kPersistMaxPhases, (unsigned long long)kPersistWorkspaceCap);
-    if ((flags & HG_BATCH_AUTOTUNE) && !(flags & HG_BATCH_PERSISTENT) && b->persistent &&
-        (rc = schedule_autotune(b.get())))
-      return rc;
+    if (tune && !(flags & HG_BATCH_PERSISTENT) && b->persistent && (rc = schedule_autotune(b.get()))) return rc;
   }
+  if (!tune && !b->persistent && (rc = per_pass_build(b.get(), items))) return rc;
   *out = b.release();
   return HG_OK;
 }
