@@ -1281,12 +1281,6 @@ int read_device_error(cudaStream_t st) {
   int *d_err = err_word();
   HG_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st), "error word read");
   HG_CUDA(cudaStreamSynchronize(st), "stream synchronise");
-#if HG_CHECKED
-  {
-    const int rc = read_checked_faults();
-    if (rc) return rc;
-  }
-#endif
   return lib_device_error(err, st);
 }
 
@@ -1361,9 +1355,6 @@ int staged_product(Kind kind, const uint64_t *x, size_t nx, const uint64_t *y, s
   if (rc) return rc;
   HG_CUDA(cudaMemcpyAsync(h + oerr, err_word(), sizeof(int), cudaMemcpyDeviceToHost, st), "error word read");
   HG_CUDA(cudaStreamSynchronize(st), "stream synchronise");
-#if HG_CHECKED
-  if ((rc = read_checked_faults())) return rc;
-#endif
   int err;
   memcpy(&err, h + oerr, sizeof err);
   if ((rc = lib_device_error(err, st))) return rc;
@@ -2331,9 +2322,14 @@ void release_words() {
 
 int *lib_err_word() { return err_word(); }
 
-// Reset the library's error word after `err` was read from it, and report it.
+// Report `err`, which was read from the library's error word after the work was
+// done, and reset the word; in checked builds, a fault that a check latched.
 int lib_device_error(int err, cudaStream_t st) {
+#if HG_CHECKED
+  if (const int rc = read_checked_faults()) return rc;
+#endif
   if (!err) return HG_OK;
+  std::lock_guard<std::recursive_mutex> lock(g_ctx.mu);
   if (g_ctx.ready) {
     HG_CUDA(cudaMemsetAsync(err_word(), 0, sizeof(int), st), "error word reset");
     HG_CUDA(cudaStreamSynchronize(st), "stream synchronise");

@@ -113,7 +113,8 @@ int host_words_take(size_t words, HostWords *w);
 void host_words_give(const HostWords &w);
 
 // The library's device error word; lib_device_error resets it when `err`,
-// read from it, is not 0, and returns the error.
+// read from it, is not 0, and returns the error (in checked builds also a
+// fault that a check latched).
 int *lib_err_word();
 int lib_device_error(int err, cudaStream_t st);
 

@@ -371,10 +371,7 @@ int hg_sums_and_sizes(const hg_sum *sums, const size_t *a_shift, const size_t *b
   if (e != cudaSuccess || f != cudaSuccess) return lib_cuda_fail(e != cudaSuccess ? e : f, "sums and sizes");
   for (size_t k = 0; k < 2 * n; ++k) results[k] = w.host[k];
   for (size_t k = 0; k < m; ++k) sizes[k] = static_cast<uint64_t>(w.host[2 * n + k]);
-  const int err = static_cast<int>(w.host[words - 1]);
-  if (!err) return HG_OK;
-  std::lock_guard<std::recursive_mutex> lock(lib_mutex());
-  return lib_device_error(err, st);
+  return lib_device_error(static_cast<int>(w.host[words - 1]), st);
 }
 
 int hg_mul_small_batch_device(const hg_product *prods, size_t n, void *stream) {
