@@ -141,6 +141,15 @@ def partial_denominator(x: Partial, service=None) -> DeviceInt:
     return multiply(x.b, x.q, service)
 
 
+def _limbs(x: DeviceInt) -> tuple[int, int]:
+    """Address and length of x's limbs: a contiguous CUDA tensor's first x.size
+    words, or all of a shorter one."""
+    t = x.t if x.t.is_contiguous() else x.t[: x.size]
+    if not t.is_cuda or not t.is_contiguous():
+        raise ValueError("expected a contiguous CUDA tensor")
+    return t.data_ptr(), min(x.size, t.numel())
+
+
 def multiply(x: DeviceInt, y: DeviceInt, service=None) -> DeviceInt:
     """mpz-* of two device integers (one product; through the service when
     given).  x is y squares (mpz-square's single forward transform)."""
@@ -158,12 +167,14 @@ def multiply(x: DeviceInt, y: DeviceInt, service=None) -> DeviceInt:
     schoolboy = not square and min(x.size, y.size) <= NTT_MULTIPLY_THRESHOLD
     if schoolboy and x.size < y.size:
         x, y = y, x
+    xp, nx = _limbs(x)
+    yp, ny = (None, 0) if square else _limbs(y)
     if service is not None and not schoolboy:
-        size = service.mul(x.ptr(), x.size, None if square else y.ptr(), 0 if square else y.size, out.data_ptr(), n, st)
+        size = service.mul(xp, nx, yp, ny, out.data_ptr(), n, st)
     else:
         size = ctypes.c_size_t()
-        check(load().hg_mul_sized_device(x.ptr(), x.size, None if square else y.ptr(), 0 if square else y.size,
-                                         out.data_ptr(), n, 1 if schoolboy else 0, st, ctypes.byref(size)))
+        check(load().hg_mul_sized_device(xp, nx, yp, ny, out.data_ptr(), n, 1 if schoolboy else 0, st,
+                                         ctypes.byref(size)))
         size = size.value
     return DeviceInt(x.sign * y.sign, out, size)
 
