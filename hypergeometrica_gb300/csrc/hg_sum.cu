@@ -296,8 +296,8 @@ int sums_enqueue(const hg_sum *sums, const size_t *a_shift, const size_t *b_shif
     if ((s.sa != 1 && s.sa != -1) || (s.sb != 1 && s.sb != -1))
       return lib_fail(HG_ERR_ARG, "sum %zu: signs must be +1 or -1", k);
     if (a.end() < a.n || b.end() < b.n) return lib_fail(HG_ERR_ARG, "sum %zu: shift out of range", k);
-    const size_t need = std::max(a.end(), b.end()) + 1;
-    if (s.nout < need) return lib_fail(HG_ERR_ARG, "sum %zu: nout = %zu cannot hold %zu limbs", k, s.nout, need);
+    const size_t end = std::max(a.end(), b.end());  // and a limb for the carry
+    if (s.nout <= end) return lib_fail(HG_ERR_ARG, "sum %zu: nout = %zu cannot hold %zu limbs and a carry", k, s.nout, end);
   }
   std::vector<SumDesc> d;
   d.reserve(n);
