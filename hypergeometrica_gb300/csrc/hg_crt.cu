@@ -521,6 +521,10 @@ cudaError_t launch_large_sum(const SumOperand &a, int64_t sa, const SumOperand &
   if (sub) e = launch_dep(top_diff_kernel, grid(n), 256, 0, st, a, b, n, &words->top_diff);
   if (e == cudaSuccess) e = launch_carry(prod, out, nproc, tiles, carry_short(nproc), ss, st);
   if (e == cudaSuccess) e = launch_dep(sum_finish_kernel, grid(nproc), 256, 0, st, out, nproc, prod, sa, sb, result, words);
+  if (e != cudaSuccess) {  // what was launched may have set the search words, which the next sum expects clear
+    cudaMemsetAsync(words, 0xff, 2 * sizeof(long long), st);
+    cudaMemsetAsync(&words->done, 0, sizeof words->done, st);
+  }
   return e;
 }
 
