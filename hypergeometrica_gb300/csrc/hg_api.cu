@@ -2354,12 +2354,15 @@ int large_sum_device(const SumOperand &a, int64_t sa, const SumOperand &b, int64
   rc = scan_state(carry_tiles(nproc), &ss);
   if (rc) return rc;
   SumWords *words = reinterpret_cast<SumWords *>(static_cast<char *>(g_ctx.lane->misc.p) + 16);
+  cudaError_t e;
   {
     // (top search,) scan (and fix), sign and size
     ProfScope ps(HG_KC_OTHER, st, 24.0 * static_cast<double>(nproc), (sa != sb ? 3 : 2) + (carry_short(nproc) ? 0 : 1));
-    HG_CUDA(launch_large_sum(a, sa, b, sb, out, words, result, ss, st), "large sum");
+    e = launch_large_sum(a, sa, b, sb, out, words, result, ss, st);
   }
-  HG_CUDA(ws_release(st), "workspace ordering");
+  const cudaError_t f = ws_release(st);  // the next sum's launches come after a failed one's too
+  HG_CUDA(e, "large sum");
+  HG_CUDA(f, "workspace ordering");
   return HG_OK;
 }
 
