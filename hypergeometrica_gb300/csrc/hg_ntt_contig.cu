@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(MODE == kMul ? 2 << (T - 4) : 1 << (T - 4)) nt
     } else {
       const uint64_t *spec = P.data[1] + static_cast<uint64_t>(prime - P.prime_lo) * P.prime_stride + base;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = mont_mul(v[i], __ldcg(spec + (xt | (static_cast<uint32_t>(i) << A0))), p, c);
+      for (int i = 0; i < 16; ++i) v[i] = mont_mul(v[i], spec[xt | (static_cast<uint32_t>(i) << A0)], p, c);
     }
     inverse_rounds<T, true, TWO ? NT : 0>(v, through(sm), swz_table(tb, T, true), xt, lt, p, c);
     store_block<ATOP>(v, P.data[0] + poff, base, xt, 2 * p);
