@@ -43,12 +43,14 @@ __device__ __forceinline__ void add_product_to(V3 &acc, uint64_t x, uint64_t y) 
   add128_to(acc, static_cast<uint64_t>(v), static_cast<uint64_t>(v >> 64));
 }
 
-// The residues are read through L2 (ld.global.cg), not by the read-only data
-// path: the launch before wrote them (or, in the persistent batch kernel, an
-// earlier phase of the same launch), and a dependent launch is resident before
-// those writes are visible.  PRESCALED: the residues are the coefficients mod
-// p_j (CrtConst::prescaled).
-template <bool PRESCALED = false>
+// PRESCALED: the residues are the coefficients mod p_j (CrtConst::prescaled).
+// SAME_LAUNCH: an earlier phase of the same launch (the persistent batch kernel)
+// wrote them, so they are read through L2 (ld.global.cg).  Else the launch
+// before did: plain loads, whose L1 serves the other half of the sectors that a
+// thread's 16-byte loads touch (the 4096-pair batch 2650 us through L2, 2621
+// this way), and not the read-only path, since a dependent launch is resident
+// before those writes are visible.
+template <bool PRESCALED = false, bool SAME_LAUNCH = false>
 struct CrtProducerT {
   const uint64_t *res;  // [3][N] natural-order residues from the unscaled inverse
   uint64_t n;           // N
@@ -70,7 +72,7 @@ struct CrtProducerT {
         const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(res + off + j * n + i0);
 #pragma unroll
         for (int q = 0; q < PER / 2; ++q) {
-          const ulonglong2 w = __ldcg(src + q);
+          const ulonglong2 w = SAME_LAUNCH ? __ldcg(src + q) : src[q];
           r[j][2 * q] = w.x;
           r[j][2 * q + 1] = w.y;
         }

@@ -97,8 +97,8 @@ struct ChunkProducerT {
 #pragma unroll
       for (int q = 0; q < PER / 2; ++q) {
         ulonglong2 a = make_ulonglong2(0, 0), b = make_ulonglong2(0, 0);
-        if (r0) a = __ldcg(reinterpret_cast<const ulonglong2 *>(r0 + j * crt.n) + q);
-        if (r1) b = __ldcg(reinterpret_cast<const ulonglong2 *>(r1 + j * crt.n) + q);
+        if (r0) a = reinterpret_cast<const ulonglong2 *>(r0 + j * crt.n)[q];
+        if (r1) b = reinterpret_cast<const ulonglong2 *>(r1 + j * crt.n)[q];
         r[j][2 * q] = sum2(a.x, b.x, p);
         r[j][2 * q + 1] = sum2(a.y, b.y, p);
       }

@@ -87,7 +87,7 @@ __device__ __noinline__ void run_tiny(const PersistPhase &ph, uint64_t item) {
 // or not: each reconstruction has its own body.
 template <bool PRESCALED>
 __device__ __noinline__ void run_carry_t(const PersistPhase &ph, uint64_t item, uint64_t *dyn, GP *s_warp) {
-  using Producer = carry::CrtProducerT<PRESCALED>;
+  using Producer = carry::CrtProducerT<PRESCALED, true>;
   carry::carry_body<Producer, kPersistThreads>(Producer{ph.res, ph.n, ph.cc}, nullptr, 0, ph.ss, ph.batch, ph.tpp,
                                                ph.ws_stride, ph.n, item, reinterpret_cast<uint64_t(*)[9]>(dyn),
                                                s_warp);
