@@ -1318,10 +1318,12 @@ enum class Kind { Ntt, Square, Schoolboy, Digit };
 //   by a digit     25.5 (36.1)  26.5 (37.8)  33.8 (46.1)  44.3 (47.6)  57.0 (49.6)  147.6 (56.4)
 // Page-locked operands and results need no copy by the host and are read and
 // written in place by the general path: half x half 40.0 (40.8), 44.0 (42.9),
-// 55.2 (48.3), 67.4 (48.9), 80.8 (48.8), 173.1 (65.2); they take it above
-// kStagedPinned limbs (quadratic products, which would be read in place, do not).
+// 55.2 (48.3), 67.4 (48.9), 80.8 (48.8), 173.1 (65.2), at 2^13 limbs 49.3
+// (48.3); they take it above kStagedPinned limbs (quadratic products, which
+// would be read in place, do not).  Below, asking the driver what a buffer is
+// would cost what it saves, about a microsecond.
 constexpr size_t kStagedLimbs = size_t(1) << 15;
-constexpr size_t kStagedPinned = size_t(1) << 12;
+constexpr size_t kStagedPinned = size_t(1) << 13;
 
 int staged_product(Kind kind, const uint64_t *x, size_t nx, const uint64_t *y, size_t ny, uint64_t d, uint64_t *out,
                    size_t nout) {
